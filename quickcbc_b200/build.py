@@ -6,7 +6,8 @@ Steps:
    reference) read from the reference tree given by QCBC_REFERENCE (default: a
    `reference` directory beside this repository).  The generated file is a
    build output and is not committed.
-   When the reference tree is absent the existing generated file is reused.
+   When the reference tree is absent the existing generated file is reused, or
+   the table is computed (qnm.py).
 2. nvcc -gencode arch=compute_100a,code=sm_100a for the kernels and the C ABI.
 
 Usage:  python -m quickcbc_b200.build [--force]
@@ -37,26 +38,27 @@ def gen_qnm(force: bool = False) -> str:
     src = os.path.join(reference_dir(), "IMRPhenomD_internals.h")
     if os.path.exists(out) and not force:
         return out
-    if not os.path.exists(src):
-        if os.path.exists(out):
-            return out
-        raise FileNotFoundError(
-            f"{src} not found: the QNM table is read from the QuickCBC reference at build time "
-            "(set QCBC_REFERENCE to the reference checkout)")
-    text = open(src).read()
     arrays = {}
-    for name in ("QNMData_a", "QNMData_fring", "QNMData_fdamp"):
-        m = re.search(r"static const double " + name + r"\[\]\s*=\s*\{(.*?)\};", text, re.S)
-        if not m:
-            raise RuntimeError(f"{name} not found in {src}")
-        body = m.group(1).replace("\\", " ")
-        arrays[name] = [float(x) for x in re.findall(r"[-+]?[0-9]*\.?[0-9]+(?:[eE][-+]?[0-9]+)?", body)]
+    names = ("QNMData_a", "QNMData_fring", "QNMData_fdamp")
+    if os.path.exists(src):
+        text = open(src).read()
+        for name in names:
+            m = re.search(r"static const double " + name + r"\[\]\s*=\s*\{(.*?)\};", text, re.S)
+            if not m:
+                raise RuntimeError(f"{name} not found in {src}")
+            body = m.group(1).replace("\\", " ")
+            arrays[name] = [float(x) for x in re.findall(r"[-+]?[0-9]*\.?[0-9]+(?:[eE][-+]?[0-9]+)?", body)]
+        origin = "read from the reference's IMRPhenomD_internals.h"
+    else:
+        from quickcbc_b200 import qnm
+        arrays = dict(zip(names, qnm.table()))
+        origin = "computed by quickcbc_b200/qnm.py"
     n = len(arrays["QNMData_a"])
     if any(len(v) != n for v in arrays.values()):
         raise RuntimeError("QNM tables differ in length")
     os.makedirs(GEN, exist_ok=True)
     with open(out, "w") as f:
-        f.write("// generated by quickcbc_b200/build.py from the reference's IMRPhenomD_internals.h\n")
+        f.write(f"// generated by quickcbc_b200/build.py: {origin}\n")
         f.write("#pragma once\n")
         f.write(f"#define QCBC_QNM_N {n}\n")
         for cname, key in (("QCBC_QNM_A", "QNMData_a"), ("QCBC_QNM_FRING", "QNMData_fring"),
