@@ -696,56 +696,85 @@ extern "C" int qcbc_het_export(const qcbc_event* ev, int* fgrid, double* freq, d
   HetData d = het_data(ev);
   const HetDev& h = ev->het;
   int nI = ev->g.nifo, M = h.M, NR = h.NR, J1 = h.J + 1;
+  // the tables are one device buffer: one copy, then the parts
+  std::vector<double> all(het_doubles(nI, M, h.J));
+  CU(cudaMemcpy(all.data(), h.buf, all.size() * sizeof(double), cudaMemcpyDeviceToHost));
   struct { double* dst; const double* src; size_t n; } parts[] = {
     {freq, d.freq, (size_t)M}, {amp, d.amp, (size_t)nI * M}, {phase, d.phase, (size_t)nI * M},
     {IP, d.IP, (size_t)NR * J1 * J1}, {SL, d.SL, (size_t)NR * nI * J1}, {lc, d.lc, (size_t)NR * nI * J1},
     {ls, d.ls, (size_t)NR * nI * J1}, {aa, d.aa, (size_t)nI * NR}, {rc, d.rc, (size_t)nI * NR},
     {rs, d.rs, (size_t)nI * NR}};
   for (auto& p : parts)
-    if (p.dst) CU(cudaMemcpy(p.dst, p.src, p.n * sizeof(double), cudaMemcpyDeviceToHost));
+    if (p.dst) memcpy(p.dst, all.data() + (p.src - h.buf), p.n * sizeof(double));
   if (fgrid) memcpy(fgrid, h.fgrid.data(), sizeof(int) * M);
   if (logLb) *logLb = h.logLb;
   return QCBC_OK;
 }
 
-// Transpose of the inverse of the sampled Legendre basis, per region (QuickCBC.c:5232-5253).
-static void invert_small(const double* A, double* Ainv, int n) {
-  double W[4][8];
-  for (int i = 0; i < n; i++)
-    for (int j = 0; j < 2 * n; j++) W[i][j] = j < n ? A[i * n + j] : (j - n == i ? 1.0 : 0.0);
-  for (int col = 0; col < n; col++) {
-    int piv = col;
-    for (int i = col + 1; i < n; i++)
-      if (fabs(W[i][col]) > fabs(W[piv][col])) piv = i;
-    if (piv != col)
-      for (int j = 0; j < 2 * n; j++) std::swap(W[col][j], W[piv][j]);
-    double dd = W[col][col];
-    for (int j = 0; j < 2 * n; j++) W[col][j] /= dd;
-    for (int i = 0; i < n; i++) {
-      if (i == col) continue;
-      double f = W[i][col];
-      for (int j = 0; j < 2 * n; j++) W[i][j] -= f * W[col][j];
-    }
-  }
-  for (int i = 0; i < n; i++)
-    for (int j = 0; j < n; j++) Ainv[i * n + j] = W[i][n + j];
+// Queues the kernels that build the event's heterodyne tables on w->stream; logLb lands in the pinned
+// w->h_lnl[0] (het_setup_finish, after a synchronisation).
+static int het_setup_queue(qcbc_event* ev, Workspace* w, const double* pref, const int* fgrid, int M, int MN, int MM,
+                           int J) {
+  const int nI = ev->g.nifo, nh = ev->g.N / 2;
+  int rc;
+  if ((rc = het_alloc(ev, M, J, MN, MM))) return rc;
+  cudaStream_t s = w->stream;
+  DeviceState& ds = g_dev[current_device()];
+  const int NR = ev->het.NR;
+  int max_region = 0;
+  for (int r = 0; r < NR; r++) max_region = std::max(max_region, fgrid[(r + 1) * J] - fgrid[r * J]);
+  HetBuild q{};
+  q.j0 = std::min(fgrid[0], MN);
+  q.j1 = std::max(fgrid[M - 1] + 1, MM);
+  const size_t n = (size_t)(q.j1 - q.j0);
+  q.npairs = (int)((n + 255) / 256);
+  const size_t npair = (size_t)q.npairs * 2 * kMaxIfo, npart = (size_t)NR * nI * het_chunks(max_region) * 12;
+  if ((rc = grow(w->d_a, w->c_a, 3 * (size_t)nI * n + npair + npart))) return rc;
+  if ((rc = grow(w->d_recs, w->c_recs, 1))) return rc;
+  if ((rc = grow(w->d_status, w->c_status, 1))) return rc;
+  // pinned staging: the setup reads the reference point and the tables kernel writes logLb through
+  // the mapped addresses
+  if ((rc = grow_host(w->h_params, w->ch_params, 11))) return rc;
+  if ((rc = grow_host(w->h_lnl, w->ch_lnl, 1 + kMaxIfo))) return rc;
+  if ((rc = grow_host(w->h_b, w->ch_b, ((size_t)M + 1) / 2))) return rc;
+  if ((rc = mapped_ptr(w->h_params, w->ch_params, w->m_params, w->m_params_of))) return rc;
+  if ((rc = mapped_ptr(w->h_lnl, w->ch_lnl, w->m_lnl, w->m_lnl_of))) return rc;
+  memcpy(w->h_params, pref, 11 * sizeof(double));
+  memcpy(w->h_b, fgrid, (size_t)M * sizeof(int));
+  CU(cudaMemcpyAsync(ev->het.d_fgrid, w->h_b, (size_t)M * sizeof(int), cudaMemcpyHostToDevice, s));
+  const HetData hd = het_data(ev);
+  q.freq = ev->d_freq; q.D = ev->d_D; q.S = ev->d_S; q.sn_stride = nh + 1;
+  q.fgrid = ev->het.d_fgrid;
+  q.MN = MN; q.MM = MM; q.M = M; q.J = J; q.NR = NR;
+  // fulltemplates uses Tobs = 1/freq[1]; the canonical grid has freq[1] = 1/Tobs
+  const double Tt = 1.0 / (1.0 / ev->g.Tobs);
+  q.ts_t = Tt - pref[5];
+  q.sqT_t = sqrt(Tt);
+  q.RC = w->d_a; q.RS = q.RC + nI * n; q.AA = q.RS + nI * n;
+  q.pairs = q.AA + nI * n; q.parts = q.pairs + npair;
+  q.gfreq = (double*)hd.freq; q.amp = (double*)hd.amp; q.phase = (double*)hd.phase; q.IP = (double*)hd.IP;
+  q.SL = (double*)hd.SL; q.lc = (double*)hd.lc; q.ls = (double*)hd.ls;
+  q.aa = (double*)hd.aa; q.rc = (double*)hd.rc; q.rs = (double*)hd.rs;
+  q.logLb = w->m_lnl;
+  launch_setup(w->m_params, 1, ev->g, ds.qnm, w->d_recs, w->d_status, s);
+  launch_het_tables(w->d_recs, ev->g, q, max_region, s);
+  tls_launches += 4;
+  CU(cudaGetLastError());
+  return QCBC_OK;
 }
 
-static void gram_values(int J, int U, int n, double* P) {
-  double c0 = 0.0, c1 = (double)(U - 2 * n), c2 = (double)U;
-  double d0 = c2, d1 = c1 + c1, d2 = d0;
-  P[0] = 1.0;
-  if (J >= 1) P[1] = c1 / (double)U;
-  for (int i = 1; i < J; i++) {
-    d0 += 2.0; d2 -= 2.0; c0 += d0; c1 += d1; c2 += d2;
-    P[i + 1] = (c1 * P[i] - c0 * P[i - 1]) / c2;
-  }
+static void het_setup_finish(qcbc_event* ev, Workspace* w, const double* pref, const int* fgrid, int M) {
+  HetDev& h = ev->het;
+  h.logLb = w->h_lnl[0];
+  h.fgrid.assign(fgrid, fgrid + M);
+  memcpy(h.pref, pref, sizeof(h.pref));
+  h.has_pref = true;
 }
 
 extern "C" int qcbc_het_setup(qcbc_event* ev, const double* pref, const int* fgrid, int M, int MN, int MM, int J) {
   if (!ev || !pref || !fgrid) return fail(QCBC_EINVAL, "NULL argument");
   if (!ev->has_data) return fail(QCBC_EINVAL, "event has no data");
-  const int nI = ev->g.nifo, N = ev->g.N, nh = N / 2;
+  const int nh = ev->g.N / 2;
   for (int i = 0; i < M; i++)
     if (fgrid[i] < 1 || fgrid[i] >= nh || (i && fgrid[i] <= fgrid[i - 1]))
       return fail(QCBC_EINVAL, "fgrid must increase strictly inside [1, N/2)");
@@ -753,88 +782,9 @@ extern "C" int qcbc_het_setup(qcbc_event* ev, const double* pref, const int* fgr
   Workspace* w;
   int rc = workspace(w);
   if (rc) return rc;
-  if ((rc = het_alloc(ev, M, J, MN, MM))) return rc;
-  cudaStream_t s = w->stream;
-  DeviceState& ds = g_dev[current_device()];
-  // scratch: h [nifo][N], amp/phase [nifo][nh], RC/RS/AA [nifo][nh]
-  size_t nA = (size_t)nI * N + 5 * (size_t)nI * nh;
-  if ((rc = grow(w->d_a, w->c_a, nA))) return rc;
-  if ((rc = grow(w->d_params, w->c_params, 11))) return rc;
-  if ((rc = grow(w->d_recs, w->c_recs, 1))) return rc;
-  if ((rc = grow(w->d_status, w->c_status, 1))) return rc;
-  if ((rc = grow(w->d_b, w->c_b, (size_t)2 * kMaxIfo))) return rc;
-  double* d_h = w->d_a;
-  double* d_amp = d_h + (size_t)nI * N;
-  double* d_ph = d_amp + (size_t)nI * nh;
-  double* d_RC = d_ph + (size_t)nI * nh;
-  double* d_RS = d_RC + (size_t)nI * nh;
-  double* d_AA = d_RS + (size_t)nI * nh;
-  CU(cudaMemcpyAsync(w->d_params, pref, 11 * sizeof(double), cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(ev->het.d_fgrid, fgrid, (size_t)M * sizeof(int), cudaMemcpyHostToDevice, s));
-  // fulltemplates uses Tobs = 1/freq[1]; the canonical grid has freq[1] = 1/Tobs
-  NetGeom gt = ev->g;
-  gt.Tobs = 1.0 / (1.0 / ev->g.Tobs);
-  launch_fulltemplates(w->d_params, gt, ds.qnm, ev->d_freq, w->d_recs, w->d_status, d_h, s);
-  launch_fullphaseamp(w->d_params, ev->g, ds.qnm, ev->d_freq, nh, w->d_recs, w->d_status, d_amp, d_ph, s);
-  launch_het_bins(d_h, d_amp, d_ph, ev->d_D, ev->d_S, nh + 1, N, nI, d_RC, d_RS, d_AA, s);
-  HetData hd = het_data(ev);
-  launch_het_region_sums(d_RC, d_RS, d_AA, ev->het.d_fgrid, M, J, nI, nh, (double*)hd.SL, (double*)hd.lc,
-                         (double*)hd.ls, s);
-  launch_nwip_pairs(d_h, ev->d_D, ev->d_S, nh + 1, N, nI, MN, MM, w->d_b, s);
-  tls_launches += 8;
-  CU(cudaGetLastError());
-  // grid gathers and per-region small tables on the host (FP64)
-  std::vector<double> ampb((size_t)nI * nh), phb((size_t)nI * nh), RC((size_t)nI * nh), RS((size_t)nI * nh),
-      AA((size_t)nI * nh);
-  double pairs[2 * kMaxIfo];
-  CU(cudaMemcpyAsync(ampb.data(), d_amp, ampb.size() * 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(phb.data(), d_ph, phb.size() * 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(RC.data(), d_RC, RC.size() * 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(RS.data(), d_RS, RS.size() * 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(AA.data(), d_AA, AA.size() * 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(pairs, w->d_b, sizeof(double) * 2 * nI, cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
-  HetDev& h = ev->het;
-  int NR = h.NR, J1 = J + 1;
-  std::vector<double> freq(M), amp((size_t)nI * M), ph((size_t)nI * M), IP((size_t)NR * J1 * J1), aa((size_t)nI * NR),
-      rcv((size_t)nI * NR), rsv((size_t)nI * NR);
-  for (int j = 0; j < M; j++) freq[j] = (double)fgrid[j] / ev->g.Tobs;
-  for (int id = 0; id < nI; id++)
-    for (int j = 0; j < M; j++) {
-      amp[(size_t)id * M + j] = ampb[(size_t)id * nh + fgrid[j]];
-      ph[(size_t)id * M + j] = phb[(size_t)id * nh + fgrid[j]];
-    }
-  for (int id = 0; id < nI; id++)
-    for (int r = 0; r < NR; r++) {
-      int k = fgrid[r * J];
-      rcv[(size_t)id * NR + r] = RC[(size_t)id * nh + k];
-      rsv[(size_t)id * NR + r] = RS[(size_t)id * nh + k];
-      aa[(size_t)id * NR + r] = AA[(size_t)id * nh + k];
-    }
-  for (int r = 0; r < NR; r++) {
-    int U = fgrid[(r + 1) * J] - fgrid[r * J];
-    double PP[16], inv[16], P[4];
-    for (int k = 0; k <= J; k++) {
-      gram_values(J, U, fgrid[r * J + k] - fgrid[r * J], P);
-      for (int a = 0; a <= J; a++) PP[a * J1 + k] = P[a];
-    }
-    invert_small(PP, inv, J1);
-    for (int a = 0; a <= J; a++)
-      for (int b = 0; b <= J; b++) IP[((size_t)r * J1 + a) * J1 + b] = inv[b * J1 + a];
-  }
-  double L = 0.0;
-  for (int id = 0; id < nI; id++) L += pairs[2 * id + 1] + 0.5 * pairs[2 * id];
-  h.logLb = L;
-  h.fgrid.assign(fgrid, fgrid + M);
-  memcpy(h.pref, pref, sizeof(h.pref));
-  h.has_pref = true;
-  CU(cudaMemcpy((void*)hd.freq, freq.data(), M * 8, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy((void*)hd.amp, amp.data(), amp.size() * 8, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy((void*)hd.phase, ph.data(), ph.size() * 8, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy((void*)hd.IP, IP.data(), IP.size() * 8, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy((void*)hd.aa, aa.data(), aa.size() * 8, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy((void*)hd.rc, rcv.data(), rcv.size() * 8, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy((void*)hd.rs, rsv.data(), rsv.size() * 8, cudaMemcpyHostToDevice));
+  if ((rc = het_setup_queue(ev, w, pref, fgrid, M, MN, MM, J))) return rc;
+  CU(cudaStreamSynchronize(w->stream));
+  het_setup_finish(ev, w, pref, fgrid, M);
   return QCBC_OK;
 }
 
@@ -2488,37 +2438,38 @@ extern "C" int qcbc_lnl_full_noalloc(qcbc_event* ev, const double* d_params, int
 }
 
 // ================================================================== PSD changes (noise marginalisation)
-// After the event's device PSD rows changed: the in-band minimum of each detector (device reduction),
-// sigma = sqrt(min) as at upload, the weighted data rebuilt on the device with the same arithmetic
-// as event_upload, and heterodyne tables built by qcbc_het_setup rebuilt about the same reference
-// point and grid (QuickCBC.c:1994-2010).  Tables given by qcbc_het_set are dropped.
+// After the event's device PSD rows changed: the weighted data rebuilt on the device with the same
+// arithmetic as event_upload (sigma from the in-band minimum, found on the device), and heterodyne
+// tables built by qcbc_het_setup rebuilt about the same reference point and grid
+// (QuickCBC.c:1994-2010).  Tables given by qcbc_het_set are dropped.  Everything is queued on the
+// thread's stream and waited for once: at 128 s, 4096 Hz, three detectors a redraw with its tables
+// takes about 0.14 ms (11.8 ms with two host round trips and the host-side table gathers).
 static int event_psd_changed(qcbc_event* ev, Workspace* w) {
   const int nI = ev->g.nifo, nh = ev->nh;
   const int lo = std::max(ev->g.imin, 1), hi = std::min(ev->g.imax, nh);
   int rc;
-  if ((rc = grow(w->d_b, w->c_b, (size_t)2 * kMaxIfo))) return rc;
+  if ((rc = grow(w->d_b, w->c_b, (size_t)qcbc::kMinBlocks * kMaxIfo))) return rc;
+  if ((rc = grow_host(w->h_lnl, w->ch_lnl, 1 + kMaxIfo))) return rc;
+  if ((rc = mapped_ptr(w->h_lnl, w->ch_lnl, w->m_lnl, w->m_lnl_of))) return rc;
   cudaStream_t s = w->stream;
-  qcbc::launch_band_min(ev->d_S, nh + 1, nI, lo, hi, w->d_b, s);
-  double smin[kMaxIfo];
-  CU(cudaMemcpyAsync(smin, w->d_b, sizeof(double) * nI, cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
-  qcbc::Sigmas sg{{1.0, 1.0, 1.0}};
-  for (int id = 0; id < nI; id++) {
-    double m = smin[id];
-    if (!(m < HUGE_VAL)) m = 1.0;
-    sg.v[id] = sqrt(m);
-    ev->inv_sigma[id] = 1.0 / sg.v[id];
-  }
-  qcbc::launch_event_weights(ev->d_D, ev->g.N, ev->d_S, nh + 1, nI, lo, hi, sg, ev->d_w64, ev->d_wm, s);
+  qcbc::launch_event_weights_min(ev->d_D, ev->g.N, ev->d_S, nh + 1, nI, lo, hi, w->d_b, w->m_lnl + 1, ev->d_w64,
+                                 ev->d_wm, s);
   tls_launches += 2;
   CU(cudaGetLastError());
-  CU(cudaStreamSynchronize(s));
   HetDev& h = ev->het;
-  if (h.buf && h.has_pref) {
-    double pref[11];
+  const bool rebuild = h.buf && h.has_pref;
+  double pref[11];
+  std::vector<int> grid;
+  if (rebuild) {
     memcpy(pref, h.pref, sizeof(pref));
-    std::vector<int> grid = h.fgrid;
-    return qcbc_het_setup(ev, pref, grid.data(), h.M, h.MN, h.MM, h.J);
+    grid = h.fgrid;
+    rc = het_setup_queue(ev, w, pref, grid.data(), h.M, h.MN, h.MM, h.J);
+  }
+  CU(cudaStreamSynchronize(s));
+  for (int id = 0; id < nI; id++) ev->inv_sigma[id] = 1.0 / sqrt(w->h_lnl[1 + id]);
+  if (rebuild) {
+    if (!rc) het_setup_finish(ev, w, pref, grid.data(), h.M);
+    return rc;
   }
   if (h.buf) {
     cudaFree(h.buf);

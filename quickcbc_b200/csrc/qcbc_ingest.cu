@@ -218,11 +218,14 @@ __global__ void k_makespec(ModelDev m, int k, int nh, double Tobs, double* __res
 }
 
 // ---------------------------------------------------------------- event weights
+// Smallest positive PSD of a detector's in-band bins: block x of detector y takes bins lo + x B + t,
+// x B + t + gridDim.x B, ..., and writes its minimum (HUGE_VAL when none) to out[y][x]; the weights
+// kernel takes the minimum over the blocks.
 __global__ void k_band_min(const double* __restrict__ S, int stride, int lo, int hi, double* __restrict__ out) {
   __shared__ double red[32];
-  const double* s = S + (size_t)blockIdx.x * stride;
+  const double* s = S + (size_t)blockIdx.y * stride;
   double m = HUGE_VAL;
-  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+  for (int i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x) {
     const double v = s[i];
     if (v > 0.0 && v < m) m = v;
   }
@@ -232,17 +235,30 @@ __global__ void k_band_min(const double* __restrict__ S, int stride, int lo, int
   if (threadIdx.x < 32) {
     m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : HUGE_VAL;
     for (int o = 16; o; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) out[blockIdx.x] = m;
+    if (threadIdx.x == 0) out[blockIdx.y * gridDim.x + blockIdx.x] = m;
   }
 }
 
 __global__ void k_event_weights(const double* __restrict__ D, int N, const double* __restrict__ S, int stride, int lo,
-                                int hi, int nifo, Sigmas sg, double* __restrict__ w64, float* __restrict__ wm) {
+                                int hi, int nifo, Sigmas sg, const double* __restrict__ mins,
+                                double* __restrict__ out_min, double* __restrict__ w64, float* __restrict__ wm) {
+  __shared__ double s_sigma;
   const int id = blockIdx.y;
+  if (mins && threadIdx.x < 32) {       // sigma = sqrt of the band's minimum, as at upload
+    double m = HUGE_VAL;
+    for (int k = threadIdx.x; k < kMinBlocks; k += 32) m = fmin(m, mins[id * kMinBlocks + k]);
+    for (int o = 16; o; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (!(m < HUGE_VAL)) m = 1.0;
+    if (threadIdx.x == 0) {
+      s_sigma = sqrt(m);
+      if (blockIdx.x == 0) out_min[id] = m;
+    }
+  }
+  __syncthreads();
   const int i = lo + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= hi) return;
   const int nh = N / 2;
-  const double sigma = sg.v[id];
+  const double sigma = mins ? s_sigma : sg.v[id];
   const double s = S[(size_t)id * stride + i];
   const double* Dr = D + (size_t)id * N;
   const double wr = 4.0 * sigma * Dr[i] / s;
@@ -279,15 +295,19 @@ __global__ void k_event_weights(const double* __restrict__ D, int N, const doubl
 
 }  // namespace
 
-void launch_band_min(const double* d_S, int stride, int nifo, int lo, int hi, double* d_out, cudaStream_t s) {
-  k_band_min<<<nifo, 1024, 0, s>>>(d_S, stride, lo, hi, d_out);
-}
-
 void launch_event_weights(const double* d_D, int N, const double* d_S, int stride, int nifo, int lo, int hi,
                           Sigmas sigma, double* d_w64, float* d_wm, cudaStream_t s) {
   if (hi <= lo) return;
   dim3 grid((hi - lo + 255) / 256, nifo);
-  k_event_weights<<<grid, 256, 0, s>>>(d_D, N, d_S, stride, lo, hi, nifo, sigma, d_w64, d_wm);
+  k_event_weights<<<grid, 256, 0, s>>>(d_D, N, d_S, stride, lo, hi, nifo, sigma, nullptr, nullptr, d_w64, d_wm);
+}
+
+void launch_event_weights_min(const double* d_D, int N, const double* d_S, int stride, int nifo, int lo, int hi,
+                              double* d_mins, double* out_min, double* d_w64, float* d_wm, cudaStream_t s) {
+  k_band_min<<<dim3(kMinBlocks, nifo), 256, 0, s>>>(d_S, stride, lo, hi, d_mins);
+  // at least one block per detector, which reports the minimum even when the band is empty
+  dim3 grid(hi > lo ? (hi - lo + 255) / 256 : 1, nifo);
+  k_event_weights<<<grid, 256, 0, s>>>(d_D, N, d_S, stride, lo, hi, nifo, Sigmas{}, d_mins, out_min, d_w64, d_wm);
 }
 
 }  // namespace qcbc

@@ -11,9 +11,6 @@ int psd_model_nifo(const qcbc_psd_model* m);
 // makespec of sample k for every detector into d_S rows (stride doubles apart), queued on s.
 int psd_model_draw_dev(qcbc_psd_model* m, int k, double Tobs, int N, double* d_S, int stride, cudaStream_t s);
 
-// Smallest positive PSD of each detector over bins [lo, hi) (HUGE_VAL when none), into d_out[nifo].
-void launch_band_min(const double* d_S, int stride, int nifo, int lo, int hi, double* d_out, cudaStream_t s);
-
 struct Sigmas {
   double v[3];
 };
@@ -22,5 +19,11 @@ struct Sigmas {
 // in the mixed kernel's FP32 planes (EventData::wm).  Bins outside [lo, hi) are left as they are.
 void launch_event_weights(const double* d_D, int N, const double* d_S, int stride, int nifo, int lo, int hi,
                           Sigmas sigma, double* d_w64, float* d_wm, cudaStream_t s);
+// The same with sigma found on the device: the square root of each detector's smallest positive PSD
+// over [lo, hi) (1 when none), two launches and no host round trip.  d_mins: scratch for
+// kMinBlocks x nifo minima; out_min [nifo] (may be mapped host memory) receives the minima.
+constexpr int kMinBlocks = 64;
+void launch_event_weights_min(const double* d_D, int N, const double* d_S, int stride, int nifo, int lo, int hi,
+                              double* d_mins, double* out_min, double* d_w64, float* d_wm, cudaStream_t s);
 
 }  // namespace qcbc

@@ -2604,110 +2604,210 @@ void launch_fullphaseamp(const double* d_params, const NetGeom& g, const QnmTabl
 }
 
 // ---------------------------------------------------------------- heterodyne setup (FP64)
-// Per bin j in [1, N/2): residual r = D - h, RC = 2 (r_re cos p + r_im sin p) A / S,
-// RS = 2 (-r_re sin p + r_im cos p) A / S, AA = A^2 / S  (QuickCBC.c:5190-5203).
-__global__ void k_het_bins(const double* __restrict__ h, const double* __restrict__ amp,
-                           const double* __restrict__ phase, const double* __restrict__ D,
-                           const double* __restrict__ S, int sn_stride, int N, int nifo, double* __restrict__ RC,
-                           double* __restrict__ RS, double* __restrict__ AA) {
-  const int half = N / 2;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < nifo * half; idx += gridDim.x * blockDim.x) {
-    int id = idx / half, j = idx - id * half;
-    size_t o = (size_t)id * half + j;
-    if (j == 0) { RC[o] = 0.0; RS[o] = 0.0; AA[o] = 0.0; continue; }
-    const double* hr = h + (size_t)id * N;
-    const double* dr = D + (size_t)id * N;
-    double rre = dr[j] - hr[j], rim = dr[N - j] - hr[N - j];
-    double a = amp[o], s = S[(size_t)id * sn_stride + j];
-    double sp, cp;
-    sincos(phase[o], &sp, &cp);
-    double x = a / s;
-    RC[o] = 2.0 * (rre * cp + rim * sp) * x;
-    RS[o] = 2.0 * (-rre * sp + rim * cp) * x;
-    AA[o] = a * a / s;
+// The tables of heterodyne() (QuickCBC.c:5112-5299) in three launches after the reference point's
+// record, with nothing but logLb coming back to the host.  What bounds them is launch latency: the
+// band's raw data and PSD (9.4 MB at 3 x 131 k bins) are read once and the per-bin terms stay in L2.
+// The earlier form wrote the template, amplitude and phase of all N/2 bins to memory in two waveform
+// passes and copied five [nifo][N/2] arrays (31 MB at 128 s, 4096 Hz) to the host to pick out the
+// grid's entries: 11.9 ms per call there against 116 us.
+
+// Discrete Legendre (Gram) polynomials P_0 .. P_J at point n of U + 1 (recurrence of QuickCBC.c:5055-5094).
+__device__ __forceinline__ void gram_values(int J, int U, int n, double (&P)[4]) {
+  double c0 = 0.0, c1 = (double)(U - 2 * n), c2 = (double)U;
+  double d0 = c2, d1 = c1 + c1, d2 = d0;
+  P[0] = 1.0;
+  P[1] = c1 / (double)U;
+  P[2] = P[3] = 0.0;
+#pragma unroll
+  for (int i = 1; i < 3; i++) {
+    if (i >= J) break;
+    d0 += 2.0; d2 -= 2.0; c0 += d0; c1 += d1; c2 += d2;
+    P[i + 1] = (c1 * P[i] - c0 * P[i - 1]) / c2;
   }
 }
 
-void launch_het_bins(const double* d_h, const double* d_amp, const double* d_phase, const double* d_D,
-                     const double* d_S, int sn_stride, int N, int nifo, double* d_RC, double* d_RS, double* d_AA,
-                     cudaStream_t s) {
-  int total = nifo * (N / 2);
-  int blocks = (total + 255) / 256;
-  if (blocks > 4736) blocks = 4736;
-  k_het_bins<<<blocks, 256, 0, s>>>(d_h, d_amp, d_phase, d_D, d_S, sn_stride, N, nifo, d_RC, d_RS, d_AA);
+// One thread per bin j of [j0, j1) (the bins of the regions and of the band [MN, MM)): the reference
+// waveform once, then per detector the template h (hard start at fbegin, ts and sqrt(T) of
+// fulltemplates) and the tapered amplitude A and phase p of fullphaseamp; residual r = D - h,
+//   RC = 2 (r_re cos p + r_im sin p) A / S, RS = 2 (-r_re sin p + r_im cos p) A / S, AA = A^2 / S
+// (QuickCBC.c:5190-5203) to rows of n = j1 - j0; the grid's amplitude, phase and region-edge terms
+// straight into the tables; and the block's partial sums of <h|h>, <r|h> over [MN, MM) per detector.
+__global__ void __launch_bounds__(256) k_het_bins(const PhdRec* __restrict__ recp, NetGeom g, HetBuild q) {
+  __shared__ PhdRec c;
+  __shared__ double red[32 * 2 * kMaxIfo];
+  for (int k = threadIdx.x; k < kRecDoubles; k += blockDim.x)
+    reinterpret_cast<double*>(&c)[k] = reinterpret_cast<const double*>(recp)[k];
+  __syncthreads();
+  const int j = q.j0 + blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = q.j1 - q.j0, N = g.N;
+  double pair[2 * kMaxIfo];
+#pragma unroll
+  for (int k = 0; k < 2 * kMaxIfo; k++) pair[k] = 0.0;
+  if (j < q.j1) {
+    const double f = __ldg(q.freq + j);
+    double amp = 0.0, ph = 0.0, y = 1.0;
+    if (!(f > c.fCut)) { phd_eval64(c, c.Msec * f, amp, ph); amp *= c.amp_scale; }
+    if (f < c.fs) y = exp(10.0 * (f - c.fs) / c.fs);
+    const bool sig = f > c.fs, same = q.ts_t == c.ts && q.sqT_t == c.sqT;
+    const bool in = j >= q.MN && j < q.MM;
+    int lo = 0, hi = q.M;                        // is j a grid bin?
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(q.fgrid + mid) < j) lo = mid + 1; else hi = mid;
+    }
+    const int m = lo < q.M && __ldg(q.fgrid + lo) == j ? lo : -1;
+#pragma unroll
+    for (int id = 0; id < kMaxIfo; id++) {
+      if (id >= g.nifo) break;
+      const double w = c.Fs[id] * kH22fac * amp, A = w / c.sqT * y;
+      const double x = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(kTwoPi, f), c.ts - c.td[id]), c.lam[id]), -ph);
+      double sp, cp;
+      sincos(reduce_2pi(x), &sp, &cp);
+      double hr = 0.0, hi_ = 0.0;
+      if (sig) {
+        double st = sp, ct = cp;
+        if (!same) {
+          const double xt = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(kTwoPi, f), q.ts_t - c.td[id]), c.lam[id]), -ph);
+          sincos(reduce_2pi(xt), &st, &ct);
+        }
+        hr = w / q.sqT_t * ct;
+        hi_ = w / q.sqT_t * st;
+      }
+      const double* d = q.D + (size_t)id * N;
+      const double rr = __ldg(d + j) - hr, ri = __ldg(d + N - j) - hi_;
+      const double s = __ldg(q.S + (size_t)id * q.sn_stride + j), z = A / s;
+      const double rc = 2.0 * (rr * cp + ri * sp) * z, rs = 2.0 * (-rr * sp + ri * cp) * z, aa = A * A / s;
+      const size_t o = (size_t)id * n + (j - q.j0);
+      q.RC[o] = rc;
+      q.RS[o] = rs;
+      q.AA[o] = aa;
+      if (in) {
+        pair[2 * id] = (hr * hr + hi_ * hi_) / s;
+        pair[2 * id + 1] = (rr * hr + ri * hi_) / s;
+      }
+      if (m >= 0) {
+        q.amp[(size_t)id * q.M + m] = A;
+        q.phase[(size_t)id * q.M + m] = x;
+        if (m % q.J == 0 && m / q.J < q.NR) {
+          const size_t e = (size_t)id * q.NR + m / q.J;
+          q.aa[e] = aa;
+          q.rc[e] = rc;
+          q.rs[e] = rs;
+        }
+      }
+    }
+  }
+  block_sum<2 * kMaxIfo>(pair, red);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 2 * kMaxIfo; k++) q.pairs[(size_t)blockIdx.x * 2 * kMaxIfo + k] = pair[k];
 }
 
-// One block per (region, detector): sums over the region's U+1 bins of AA, RC, RS times the
-// discrete Legendre polynomials P_a(n) (QuickCBC.c:5265-5281, recurrence of 5055-5094).
-__global__ void k_het_region_sums(const double* __restrict__ RC, const double* __restrict__ RS,
-                                  const double* __restrict__ AA, const int* __restrict__ fgrid, int M, int J,
-                                  int nifo, int nh, double* __restrict__ SL, double* __restrict__ lc,
-                                  double* __restrict__ ls) {
+// One block per (region, detector, chunk): the chunk's part of the sums over the region's U + 1 bins
+// of AA, RC, RS times P_a(n) (QuickCBC.c:5265-5281).  Regions grow with frequency (from tens to ten
+// thousand bins at 128 s); a chunk is kHetChunk bins, so the largest regions are spread over blocks.
+__global__ void __launch_bounds__(256) k_het_region_sums(HetBuild q, int nifo) {
   __shared__ double red[32 * 12];
-  int r = blockIdx.x / nifo, id = blockIdx.x - r * nifo;
-  int J1 = J + 1;
-  int k0 = fgrid[r * J], U = fgrid[(r + 1) * J] - k0;
+  const int r = blockIdx.x / nifo, id = blockIdx.x - r * nifo, J = q.J, J1 = J + 1;
+  const int k0 = __ldg(q.fgrid + r * J), U = __ldg(q.fgrid + (r + 1) * J) - k0;
+  const int n0 = blockIdx.y * kHetChunk, n1 = min(n0 + kHetChunk - 1, U);
+  if (n0 > U) return;
   double acc[12];
 #pragma unroll
   for (int a = 0; a < 12; a++) acc[a] = 0.0;
-  for (int n = threadIdx.x; n <= U; n += blockDim.x) {
+  const size_t row = (size_t)id * (q.j1 - q.j0) + (k0 - q.j0);
+  for (int n = n0 + threadIdx.x; n <= n1; n += blockDim.x) {
     double P[4];
-    double c0 = 0.0, c1 = (double)(U - 2 * n), c2 = (double)U;
-    double d0 = c2, d1 = c1 + c1, d2 = d0;
-    P[0] = 1.0;
-    if (J >= 1) P[1] = c1 / (double)U;
-    for (int i = 1; i < J && i < 3; i++) {
-      d0 += 2.0; d2 -= 2.0; c0 += d0; c1 += d1; c2 += d2;
-      P[i + 1] = (c1 * P[i] - c0 * P[i - 1]) / c2;
-    }
-    size_t k = (size_t)id * nh + k0 + n;
-    double aa = AA[k], rc = RC[k], rs = RS[k];
-    for (int a = 0; a < J1 && a < 4; a++) {
+    gram_values(J, U, n, P);
+    const double aa = __ldg(q.AA + row + n), rc = __ldg(q.RC + row + n), rs = __ldg(q.RS + row + n);
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
       acc[3 * a] += aa * P[a];
       acc[3 * a + 1] += rc * P[a];
       acc[3 * a + 2] += rs * P[a];
     }
   }
   block_sum<12>(acc, red);
-  if (threadIdx.x == 0) {
-    for (int a = 0; a < J1 && a < 4; a++) {
-      size_t o = ((size_t)r * nifo + id) * J1 + a;
-      SL[o] = acc[3 * a];
-      lc[o] = acc[3 * a + 1];
-      ls[o] = acc[3 * a + 2];
+  if (threadIdx.x == 0)
+    for (int a = 0; a < J1; a++)
+      for (int k = 0; k < 3; k++)
+        q.parts[(((size_t)r * nifo + id) * gridDim.y + blockIdx.y) * 12 + 3 * a + k] = acc[3 * a + k];
+}
+
+// Inverse of an n x n matrix (n <= 4) by Gauss-Jordan elimination with partial pivoting.
+__device__ __forceinline__ void invert_small(const double (&A)[4][4], double (&Ainv)[4][4], int n) {
+  double W[4][8];
+  for (int i = 0; i < n; i++)
+    for (int j = 0; j < 2 * n; j++) W[i][j] = j < n ? A[i][j] : (j - n == i ? 1.0 : 0.0);
+  for (int col = 0; col < n; col++) {
+    int piv = col;
+    for (int i = col + 1; i < n; i++)
+      if (fabs(W[i][col]) > fabs(W[piv][col])) piv = i;
+    if (piv != col)
+      for (int j = 0; j < 2 * n; j++) { const double t = W[col][j]; W[col][j] = W[piv][j]; W[piv][j] = t; }
+    const double d = W[col][col];
+    for (int j = 0; j < 2 * n; j++) W[col][j] /= d;
+    for (int i = 0; i < n; i++) {
+      if (i == col) continue;
+      const double f = W[i][col];
+      for (int j = 0; j < 2 * n; j++) W[i][j] -= f * W[col][j];
     }
   }
+  for (int i = 0; i < n; i++)
+    for (int j = 0; j < n; j++) Ainv[i][j] = W[i][n + j];
 }
 
-void launch_het_region_sums(const double* d_RC, const double* d_RS, const double* d_AA, const int* d_fgrid, int M,
-                            int J, int nifo, int nh, double* d_SL, double* d_lc, double* d_ls, cudaStream_t s) {
-  int NR = (M - 1) / J;
-  if (NR <= 0) return;
-  k_het_region_sums<<<NR * nifo, 256, 0, s>>>(d_RC, d_RS, d_AA, d_fgrid, M, J, nifo, nh, d_SL, d_lc, d_ls);
-}
-
-// <h|h> and <D-h|h> over [imin, imax) per detector, one block per detector (Utilities.c:716-736)
-__global__ void k_nwip_pairs(const double* __restrict__ h, const double* __restrict__ D, const double* __restrict__ S,
-                             int sn_stride, int N, int imin, int imax, double* __restrict__ out) {
-  __shared__ double red[32 * 2];
-  int id = blockIdx.x;
-  const double* hr = h + (size_t)id * N;
-  const double* dr = D + (size_t)id * N;
-  const double* sr = S + (size_t)id * sn_stride;
-  double acc[2] = {0.0, 0.0};
-  for (int i = imin + threadIdx.x; i < imax; i += blockDim.x) {
-    int k = N - i;
-    double s = sr[i];
-    acc[0] += (hr[i] * hr[i] + hr[k] * hr[k]) / s;
-    acc[1] += ((dr[i] - hr[i]) * hr[i] + (dr[k] - hr[k]) * hr[k]) / s;
+// The rest of the tables.  Blocks 0 .. gridDim.x - 2: a thread per (region, detector, P_a, term) adds
+// the chunks in order, a thread per region stores the transpose of the inverse of its sampled basis
+// (QuickCBC.c:5232-5253), a thread per grid point its frequency.  The last block adds the bins
+// kernel's partial sums in a fixed order: logLb = sum (<r|h> + <h|h>/2) to *q.logLb.
+__global__ void __launch_bounds__(128) k_het_tables(HetBuild q, int nifo, int chunks, double Tobs) {
+  const int J = q.J, J1 = J + 1;
+  if (blockIdx.x == gridDim.x - 1) {
+    __shared__ double red[32 * 2 * kMaxIfo];
+    double v[2 * kMaxIfo];
+#pragma unroll
+    for (int k = 0; k < 2 * kMaxIfo; k++) v[k] = 0.0;
+    for (int b = threadIdx.x; b < q.npairs; b += blockDim.x)
+#pragma unroll
+      for (int k = 0; k < 2 * kMaxIfo; k++) v[k] += q.pairs[(size_t)b * 2 * kMaxIfo + k];
+    block_sum<2 * kMaxIfo>(v, red);
+    if (threadIdx.x == 0) {
+      double L = 0.0;
+      for (int id = 0; id < nifo; id++) L += 4.0 * v[2 * id + 1] + 0.5 * (4.0 * v[2 * id]);
+      *q.logLb = L;
+    }
+    return;
   }
-  block_sum<2>(acc, red);
-  if (threadIdx.x == 0) { out[2 * id] = 4.0 * acc[0]; out[2 * id + 1] = 4.0 * acc[1]; }
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nsum = q.NR * nifo * J1 * 3;
+  if (t < nsum) {
+    const int k = t % 3, a = (t / 3) % J1, e = t / (3 * J1), r = e / nifo;     // e = r nifo + id
+    const int U = __ldg(q.fgrid + (r + 1) * J) - __ldg(q.fgrid + r * J);
+    double s = 0.0;
+    for (int c = 0; c <= U / kHetChunk; c++) s += q.parts[((size_t)e * chunks + c) * 12 + 3 * a + k];
+    (k == 0 ? q.SL : k == 1 ? q.lc : q.ls)[(size_t)e * J1 + a] = s;
+  } else if (t < nsum + q.NR) {
+    const int r = t - nsum, k0 = __ldg(q.fgrid + r * J), U = __ldg(q.fgrid + (r + 1) * J) - k0;
+    double PP[4][4], inv[4][4], P[4];
+    for (int k = 0; k <= J; k++) {
+      gram_values(J, U, __ldg(q.fgrid + r * J + k) - k0, P);
+      for (int a = 0; a <= J; a++) PP[a][k] = P[a];
+    }
+    invert_small(PP, inv, J1);
+    for (int a = 0; a <= J; a++)
+      for (int b = 0; b <= J; b++) q.IP[((size_t)r * J1 + a) * J1 + b] = inv[b][a];
+  } else if (t < nsum + q.NR + q.M) {
+    const int m = t - nsum - q.NR;
+    q.gfreq[m] = (double)__ldg(q.fgrid + m) / Tobs;
+  }
 }
 
-void launch_nwip_pairs(const double* d_h, const double* d_D, const double* d_S, int sn_stride, int N, int nifo,
-                       int imin, int imax, double* d_out, cudaStream_t s) {
-  k_nwip_pairs<<<nifo, 1024, 0, s>>>(d_h, d_D, d_S, sn_stride, N, imin, imax, d_out);
+void launch_het_tables(const PhdRec* d_rec, const NetGeom& g, const HetBuild& q, int max_region, cudaStream_t s) {
+  k_het_bins<<<q.npairs, 256, 0, s>>>(d_rec, g, q);
+  const int chunks = het_chunks(max_region);
+  k_het_region_sums<<<dim3(q.NR * g.nifo, chunks), 256, 0, s>>>(q, g.nifo);
+  const int total = q.NR * g.nifo * (q.J + 1) * 3 + q.NR + q.M;
+  k_het_tables<<<(total + 127) / 128 + 1, 128, 0, s>>>(q, g.nifo, chunks, g.Tobs);
 }
 
 __global__ void k_nwip(const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ S,

@@ -184,14 +184,23 @@ void launch_ampphase_out(const double* d_freq, const double* d_amp, const double
 void launch_fullphaseamp(const double* d_params, const NetGeom& g, const QnmTable& q, const double* d_freq, int n,
                          PhdRec* d_rec, int* d_status, double* d_amp, double* d_phase, cudaStream_t s);
 
-// heterodyne setup pieces (FP64)
-void launch_het_bins(const double* d_h, const double* d_amp, const double* d_phase, const double* d_D,
-                     const double* d_S, int sn_stride, int N, int nifo, double* d_RC, double* d_RS, double* d_AA,
-                     cudaStream_t s);
-void launch_het_region_sums(const double* d_RC, const double* d_RS, const double* d_AA, const int* d_fgrid, int M,
-                            int J, int nifo, int nh, double* d_SL, double* d_lc, double* d_ls, cudaStream_t s);
-void launch_nwip_pairs(const double* d_h, const double* d_D, const double* d_S, int sn_stride, int N, int nifo,
-                       int imin, int imax, double* d_out /* nifo x 2: HH, HR */, cudaStream_t s);
+// Heterodyne tables (FP64) of grid fgrid[M] about one record: D, S rows of the event, the bins
+// [j0, j1) that the regions and [MN, MM) cover, scratch rows RC/RS/AA [nifo][j1 - j0], partial sums
+// pairs [npairs][2 kMaxIfo] (one per block of 256 bins) and parts [NR][nifo][chunks][12], and the
+// tables (layouts of HetData).  ts_t, sqT_t: Tobs - tc and sqrt(Tobs) with the Tobs = 1/freq[1] of
+// fulltemplates.  logLb may be mapped host memory.
+constexpr int kHetChunk = 1024;
+inline int het_chunks(int max_region) { return max_region / kHetChunk + 1; }   // of U + 1 bins
+struct HetBuild {
+  const double *freq, *D, *S;
+  const int* fgrid;
+  int sn_stride, j0, j1, MN, MM, M, J, NR, npairs;
+  double ts_t, sqT_t;
+  double *RC, *RS, *AA, *pairs, *parts;
+  double *gfreq, *amp, *phase, *IP, *SL, *lc, *ls, *aa, *rc, *rs, *logLb;
+};
+// max_region: the largest U = fgrid[(r+1) J] - fgrid[r J]
+void launch_het_tables(const PhdRec* d_rec, const NetGeom& g, const HetBuild& q, int max_region, cudaStream_t s);
 
 // ---- multi-event launches: parameter set b belongs to event event_of[b]; its signal bins are cut
 // into tiles of tile_bins bins; the (set, tile) work items are processed by a persistent kernel.
