@@ -63,6 +63,7 @@ struct DeviceState {
   double2* d_tabA = nullptr;
   double2* d_tabB = nullptr;
   float2* d_tabC = nullptr;
+  double2* d_tabD = nullptr;   // (1/i, i^{3/4})
   int tab_n = 0;
   int* d_bucket = nullptr;   // QNM interval index per 0.001 of final spin
 };
@@ -135,10 +136,12 @@ static int ensure_bin_tables(DeviceState& ds, int n) {
   int want = std::max(n, 1 << 20);
   double2 *a = nullptr, *b = nullptr;
   float2* c = nullptr;
+  double2* dd = nullptr;
   CU(cudaMalloc(&a, (size_t)want * sizeof(double2)));
   CU(cudaMalloc(&b, (size_t)want * sizeof(double2)));
   CU(cudaMalloc(&c, (size_t)want * sizeof(float2)));
-  launch_fill_bin_tables(a, b, c, want, 0);
+  CU(cudaMalloc(&dd, (size_t)want * sizeof(double2)));
+  launch_fill_bin_tables(a, b, c, dd, want, 0);
   tls_launches += 1;
   CU(cudaDeviceSynchronize());
   // The smaller tables stay allocated: batches copy the table pointers into their device event
@@ -146,6 +149,7 @@ static int ensure_bin_tables(DeviceState& ds, int n) {
   ds.d_tabA = a;
   ds.d_tabB = b;
   ds.d_tabC = c;
+  ds.d_tabD = dd;
   ds.tab_n = want;
   return QCBC_OK;
 }
@@ -327,6 +331,7 @@ static EventData event_data(const qcbc_event* ev) {
   d.tabA = ds.d_tabA;
   d.tabB = ds.d_tabB;
   d.tabC = ds.d_tabC;
+  d.tabD = ds.d_tabD;
   return d;
 }
 
@@ -419,7 +424,7 @@ static int event_upload(qcbc_event* ev, const double* const* Drows, const double
   std::vector<double> freq(nh);
   freq[0] = 1.0 / ev->g.Tobs;
   for (int i = 1; i < nh; i++) freq[i] = (double)i / ev->g.Tobs;
-  const size_t b64 = (size_t)nI * 3 * nh * 8, bm = qcbc::mixed_plane_floats(nI, nh) * sizeof(float),
+  const size_t b64 = qcbc::w64_doubles(nI, nh) * 8, bm = qcbc::mixed_plane_floats(nI, nh) * sizeof(float),
                bD = Dall.size() * 8, bS = Sall.size() * 8, bf = freq.size() * 8;
   if (!ev->d_w64) {
     CU(cudaMalloc(&ev->d_w64, b64));
@@ -484,17 +489,40 @@ extern "C" long long qcbc_event_device_bytes(const qcbc_event* ev) {
 }
 
 // ------------------------------------------------------------------ launch choice
-// Blocks per parameter set: enough blocks to fill 148 SMs several times over,
-// but at least ~512 bins per block.  The measured variant (tune_full) overrides.
+// Blocks per parameter set.  Mixed: enough blocks of 256 threads to fill 148 SMs several times over,
+// but at least ~512 bins per block.
+// FP64: blocks of 64 threads (eight per SM at 128 registers), because a block's start (record, tables)
+// and end are short serial stretches that other blocks have to fill: 2048 sets at 16 s take 191 us with
+// one 64-thread block per set, 196 with 128 threads, 223 with 256.  The tile count minimises a model of
+// the launch fitted to sweeps at 4, 16 and 128 s and 1 to 2048 sets (within 5 % of the best count there
+// but for one case at 9 %): a block costs its rows of 64 bins plus 28 rows of start and end; f = blocks
+// over resident blocks; below one wave an SM runs each block faster the fewer it holds; above, the part of
+// the last wave that is empty is lost.  Several tiles cost 12 % more below a wave (partial sums, no order
+// by length).
 static FullLaunch heuristic_launch(const qcbc_event* ev, int B, int prec) {
   FullLaunch L;
+  const int bins = std::max(1, ev->g.imax - ev->g.imin);
+  if (prec == QCBC_FP64) {
+    constexpr int kThreads = 64, kSlots = 148 * 8;
+    const int tmax = std::max(1, bins / kThreads);
+    double best = 0.0;
+    L.threads = kThreads;
+    L.tiles = 1;
+    for (int t = 1; t <= tmax; t += 1 + t / 8) {
+      const double f = (double)B * t / kSlots;
+      if (t > 1 && f > 8.0) break;
+      const double rows = ceil((double)bins / ((double)t * kThreads)) + 28.0;
+      const double c = f <= 1.0 ? rows * (0.35 + 0.65 * f) * (t > 1 ? 1.12 : 1.0)
+                                : rows * (f + 0.35 * (ceil(f) - f) / floor(f));
+      if (t == 1 || c < best) { best = c; L.tiles = t; }
+    }
+    return L;
+  }
   L.threads = 256;
-  int bins = std::max(1, ev->g.imax - ev->g.imin);
   int want_blocks = 148 * 8;
   int tiles = (want_blocks + B - 1) / B;
   int max_tiles = std::max(1, bins / 512);
   L.tiles = std::max(1, std::min(tiles, max_tiles));
-  (void)prec;
   return L;
 }
 
@@ -1276,7 +1304,7 @@ static int multi_graph(qcbc_batch* bt, int Bcap, int prec, MultiGraph** out) {
     launch_scan_expand(m->d_ntile, Bcap, m->d_off, m->d_items, m->items_cap, s);
     launch_lnl_multi(m->d_recs, bt->d_events, m->d_off, m->d_items, Bcap, m->tile_bins, m->items_cap, P, m->threads,
                      m->blocks, m->d_counter, m->d_part, s);
-    launch_finalize_multi(m->d_part, m->d_recs, m->d_status, m->d_off, bt->d_events, Bcap, m->items_cap, P, m->d_lnl,
+    launch_finalize_multi(m->d_part, m->d_recs, m->d_status, m->d_off, bt->d_events, Bcap, m->items_cap, m->d_lnl,
                           m->d_rho, s);
     if (with_copies) {
       cudaMemcpyAsync(m->h_lnl, m->d_lnl, sizeof(double) * Bcap, cudaMemcpyDeviceToHost, s);
@@ -2430,8 +2458,7 @@ extern "C" int qcbc_lnl_full_noalloc(qcbc_event* ev, const double* d_params, int
   EventData ed = event_data(ev);
   launch_setup(d_params, B, ev->g, ds.qnm, recs, status, s);
   launch_lnl_full(recs, B, ev->g, ed, precision == QCBC_MIXED ? kMixed : kFP64, L, part, s);
-  launch_finalize_full(part, recs, status, B, L.tiles, ev->g, ed, precision == QCBC_MIXED ? kMixed : kFP64, d_lnl,
-                       d_rho, s);
+  launch_finalize_full(part, recs, status, B, L.tiles, ev->g, ed, d_lnl, d_rho, s);
   tls_launches += 3;
   CU(cudaGetLastError());
   return QCBC_OK;

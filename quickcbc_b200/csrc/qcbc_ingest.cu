@@ -264,12 +264,11 @@ __global__ void k_event_weights(const double* __restrict__ D, int N, const doubl
   const double wr = 4.0 * sigma * Dr[i] / s;
   const double wi = 4.0 * sigma * Dr[N - i] / s;
   const double ws = 4.0 * sigma * sigma / s;
-  double* r = w64 + (size_t)id * 3 * nh;
-  r[i] = wr;
-  r[nh + i] = wi;
-  r[2 * nh + i] = ws;
-  // the mixed kernel's planes (EventData::wm) carry the amplitude's bin factor i^{-7/6}
+  // both forms carry the amplitude's bin factor i^{-7/6} (EventData::w64, wm)
   const double p = pow((double)i, -7.0 / 6.0);
+  double* grp = w64 + (size_t)(i >> 5) * (96 * nifo);          // 32 bins of 3 nifo doubles
+  reinterpret_cast<double2*>(grp)[32 * id + (i & 31)] = make_double2(wr * p, wi * p);
+  grp[64 * nifo + 32 * id + (i & 31)] = ws * (p * p);
   const float fr = (float)(wr * p), fi = (float)(wi * p), fs = (float)(ws * (p * p));
   const size_t n = (size_t)nh;
   if (nifo == 1) {

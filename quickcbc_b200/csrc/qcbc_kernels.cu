@@ -1000,30 +1000,6 @@ __device__ __forceinline__ void kahan_add(float& s, float& comp, float x) {
 //   <d|h> = K SD,  <h|h> = K^2 SH   (QuickCBC.c:4258-4266, Utilities.c:716-736).
 // Results land in acc[2*NIFO] of every thread (summed over the block by the caller).
 
-// FP64 form: IMRPhenomD evaluated bin by bin as the reference does.
-template <int NIFO>
-__device__ __forceinline__ void tile_fp64(const PhdRec& c, const NetGeom& g, const EventData& ev, int i0, int i1,
-                                          double* acc) {
-  const size_t nh = (size_t)ev.nh;
-  for (int i = i0 + threadIdx.x; i <= i1; i += blockDim.x) {
-    double f = bin_freq(g, i);
-    double Mf = c.Msec * f;
-    double amp, ph;
-    phd_eval64(c, Mf, amp, ph);
-#pragma unroll
-    for (int id = 0; id < NIFO; id++) {
-      // x = 2 pi f (ts - td) + lambda - phi, evaluated in the reference's order
-      double x = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(kTwoPi, f), c.ts - c.td[id]), c.lam[id]), -ph);
-      double sx, cx;
-      sincos(reduce_2pi(x), &sx, &cx);
-      const double* w = ev.w64 + (size_t)id * 3 * nh;
-      double wr = __ldg(w + i), wi = __ldg(w + nh + i), ws = __ldg(w + 2 * nh + i);
-      acc[2 * id] += amp * (wr * cx + wi * sx);
-      acc[2 * id + 1] += amp * amp * ws;
-    }
-  }
-}
-
 // Mixed form.  Per bin i (f = i df, Mf = Msec f), with the phase written as the ringdown's linear
 // part R0 + i Ri plus a rest (MixPoly):
 //  * the rest of the inspiral and intermediate pieces in FP64 from per-bin tables:
@@ -1332,6 +1308,420 @@ __device__ __forceinline__ void tile_mixed(const PhdRec& c, const NetGeom& g, co
   }
 }
 
+// ---- FP64 tile body.  The same decomposition as the mixed one (folded per-set polynomials over the
+// per-bin tables, linear phase and detector delays through rotation tables), every step in FP64:
+//  * phase of detector 0 in cycles = lin0 + i lin1 - rest(i), one sincos of it per bin; detectors 1, 2
+//    follow by the relative rotation e^{2 pi i (f (td0 - td) + (lam - lam0) / 2 pi)} = base(thread) R[row];
+//  * the ringdown's exponential is a geometric sequence in i: E(thread) E[row];
+//  * its arctangent is atan(z_c) of the warp's centre bin (table) plus atan(w), w = (z - z_c)/(1 + z z_c),
+//    |w| <= 0.265 on 32 bins, one polynomial; the reciprocal 1/(1 + z z_c) and the Lorentzian's
+//    1/(dfr^2 + fg^2) come from one reciprocal of their product;
+//  * the weighted data carry i^{-7/6}, so a bin needs no power, logarithm or division.
+// The FP64 pipe bounds it (58 % busy, about 68 FP64 of 130 instructions per signal bin at three detectors);
+// evaluating pow, log, atan, exp, ten divisions and three sincos per bin took four times as long: 2048 sets
+// at 16 s 741 -> 191 us per call, 201 sets at 128 s 889 -> 218 us.  Two rows at a time (QCBC_U64) read the
+// constants once for both: 126 M warp instructions per launch against 155 M one by one; three rows gain
+// another 1 %, four spill.  128 registers: 16 warps per SM with two rows each beat 20 at 96 (201 us) and 24
+// at 80 (209 us).
+// Sets outside the tables' range (a piece order IMRPhenomD does not have, |w| beyond the polynomial,
+// exponents near overflow) take the per-bin functions in the same loop (AP = PP = -1).
+
+// sin and cos of 2 pi t, |t| <= 1/8, and atan(w)/w, |w| <= 0.2645: polynomials in t^2 and w^2,
+// interpolated at Chebyshev nodes in 60-digit arithmetic and rounded; relative errors 3.9e-17, 2.1e-17
+// and 2.5e-17.
+__constant__ double c_sin2pi[7] = {6.283185307179586, -41.341702240399634, 81.60524927594804, -76.70585970427454,
+                                   42.058685020160894, -15.093804209987114, 3.7808689593022957};
+__constant__ double c_cos2pi[8] = {1.0, -19.739208802178716, 64.93939402266795, -85.45681720652271,
+                                   60.244641328867296, -26.426250908622137, 7.903091687751697, -1.6968494702918826};
+__constant__ double c_atan64[9] = {1.0, -0.33333333333330495, 0.19999999998915635, -0.14285714126071508,
+                                   0.11111099310073162, -0.09090417358899357, 0.07680201267088747,
+                                   -0.06490960023860128, 0.04468242583532965};
+constexpr double kAtanRange = 0.2645;
+
+// sin and cos of 2 pi cyc of U values.  Any: cyc may be beyond 2^45, infinite or NaN (the tile's bound on
+// its phase, Tile64, keeps the others below).
+template <int U, bool Any>
+__device__ __forceinline__ void sincos_cycles(const double (&cyc)[U], double (&sv)[U], double (&cv)[U]) {
+  constexpr double kMagic = 6755399441055744.0;         // 1.5 2^52: the add rounds to an integer
+  int k[U];                                             // quadrant
+  double t[U], z[U], s[U], c[U];
+#pragma unroll
+  for (int j = 0; j < U; j++) {
+    double x = cyc[j];
+    if (Any && (__double2hiint(x) & 0x7fffffff) > 0x42c00000) x -= rint(x);
+    const double q = fma(x, 4.0, kMagic);
+    k[j] = __double2loint(q);
+    t[j] = fma(q - kMagic, -0.25, x);
+    z[j] = t[j] * t[j];
+    s[j] = c_sin2pi[6];
+    c[j] = c_cos2pi[7];
+  }
+#pragma unroll
+  for (int m = 6; m >= 0; m--) {
+    const double b = c_cos2pi[m];
+#pragma unroll
+    for (int j = 0; j < U; j++) c[j] = fma(z[j], c[j], b);
+    if (m < 6) {
+      const double a = c_sin2pi[m];
+#pragma unroll
+      for (int j = 0; j < U; j++) s[j] = fma(z[j], s[j], a);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < U; j++) {
+    const double st = s[j] * t[j];
+    const double a = (k[j] & 1) ? c[j] : st, d = (k[j] & 1) ? st : c[j];
+    sv[j] = __hiloint2double(__double2hiint(a) ^ ((k[j] & 2) << 30), __double2loint(a));
+    cv[j] = __hiloint2double(__double2hiint(d) ^ (((k[j] + 1) & 2) << 30), __double2loint(d));
+  }
+}
+__device__ __forceinline__ void sincos_cycles(double cyc, double& sv, double& cv) {
+  const double x[1] = {cyc};
+  double s[1], c[1];
+  sincos_cycles<1, true>(x, s, c);
+  sv = s[0];
+  cv = c[0];
+}
+
+// 1/x for finite normal x: the hardware's approximation (about 2^-20) and one third-order step
+__device__ __forceinline__ double recip64(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+constexpr int kSeg64 = 64;                 // rows of blockDim.x bins per table segment
+struct alignas(16) Tab64 {
+  double2 rot[kSeg64][kMaxIfo - 1];        // relative rotations of detectors 1, 2 per row
+  double2 sub[kSeg64 * 8];                 // (z_c, Rat atan z_c) per row and warp
+  double er[kSeg64];                       // the exponential's row factor
+  double al[8];                            // inspiral amplitude
+};
+
+// The weighted FP64 data (EventData::w64): groups of 32 bins, in a group the pairs (wr', wi') of each
+// detector's 32 bins, then the ws' of each detector's.  A bin's pairs are 16-byte aligned, a warp's loads
+// are contiguous, and a thread's next row lies a constant number of bytes on, so a row costs two pointer
+// increments instead of an address per plane.
+__host__ __device__ constexpr int w64_group(int nifo) { return 32 * 3 * nifo; }    // doubles
+
+// a thread's sums: detector 0's real part, detectors 1, 2 before their rotation base, <h|h> terms
+template <int NIFO>
+struct Acc64 {
+  double r0, sx[NIFO], sy[NIFO], sh[NIFO];
+  __device__ __forceinline__ void zero() {
+    r0 = 0.0;
+#pragma unroll
+    for (int id = 0; id < NIFO; id++) { sx[id] = 0.0; sy[id] = 0.0; sh[id] = 0.0; }
+  }
+};
+
+// per-thread constants of a tile
+struct Tile64 {
+  double lin0, lin1;         // detector 0's linear phase, cycles
+  double D1, D0, Ru3, Rs, Rat;
+  double dn;                 // z - z_c of this lane
+  double fg2, E;             // Lorentzian width squared; fg g1 times the exponential at the first bin
+};
+
+// where a thread's next bin lies: its bin number and the addresses of its tables and data
+struct Cur64 {
+  double xi;
+  int b, k;                                  // bin, row of the table segment
+  const double2 *ab, *cd, *w;                // (i^{1/3}, i^{-1/3}), (log i | 1/i, i^{3/4}), data pairs
+  const double* ws;
+};
+
+__device__ __forceinline__ double amp64_ins(const Tab64& T, double xi, double t) {
+  const double2 a = sld2(T.al), b = sld2(T.al + 2), c = sld2(T.al + 4), d = sld2(T.al + 6);
+  const double inner = fma(xi, d.y, fma(t, fma(t, d.x, c.y), c.x));
+  const double mid = fma(xi, inner, fma(t, fma(t, b.y, b.x), a.y));
+  return fma(xi, mid, fma(t * t, a.x, 1.0));
+}
+__device__ __forceinline__ double amp64_int(const PhdRec& c, double xi) {
+  const double m = c.mdf, x = fma(xi, m, -c.hx1), y = fma(xi, m, -c.hx2), z = fma(xi, m, -c.hx3);
+  return fma(x, fma(x, fma(y, fma(z, c.hc[4], c.hc[3]), c.hc[2]), c.hc[1]), c.hc[0]);
+}
+
+// U consecutive rows of a thread, all in amplitude piece AP and phase piece PP (-1: decided per bin, with
+// the functions themselves in place of the ringdown's tables).  The U bins are evaluated side by side, so
+// that the polynomials' constants and the set's coefficients are read once for all of them.
+template <int NIFO, int AP, int PP, int U>
+__device__ __forceinline__ void step64(const PhdRec& c, const EventData& ev, const Tab64& T, const Tile64& q,
+                                       Acc64<NIFO>& A, const Cur64& p, int bs) {
+  constexpr bool kT = AP <= 0 || PP <= 0;              // i^{1/3} needed
+  constexpr int G = w64_group(NIFO);
+  const int nw = bs >> 5, warp = threadIdx.x >> 5;
+  double xi[U], t[U], u[U], L[U], s34[U], rest[U], amp[U];
+  double2 wri[U][NIFO];
+  double ws[U][NIFO];
+#pragma unroll
+  for (int j = 0; j < U; j++) {
+    xi[j] = j ? p.xi + (double)bs : p.xi;
+    t[j] = u[j] = L[j] = s34[j] = 0.0;
+    if (PP == 2) {                                     // u here is 1/i
+      const double2 v = __ldg(p.cd + j * bs);
+      u[j] = v.x;
+      s34[j] = v.y;
+      if (kT) t[j] = __ldg(&p.ab[j * bs].x);
+    } else {
+      const double2 v = __ldg(p.ab + j * bs);
+      t[j] = v.x;
+      u[j] = v.y;
+      if (PP < 0) {
+        const double2 l = __ldg(p.cd + j * bs);
+        L[j] = l.x;
+        s34[j] = l.y;
+      } else {
+        L[j] = __ldg(&p.cd[j * bs].x);
+      }
+    }
+#pragma unroll
+    for (int id = 0; id < NIFO; id++) {
+      wri[j][id] = __ldg(p.w + (size_t)(j * nw) * (G / 2) + id * 32);
+      ws[j][id] = __ldg(p.ws + (size_t)(j * nw) * G + id * 32);
+    }
+  }
+  if (PP == 2) {
+    double v[U], v2[U], pl[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+      const double2 zc = T.sub[(p.k + j) * nw + warp];
+      const double z = fma(xi[j], q.D1, -q.D0), den = fma(z, zc.x, 1.0);
+      double rd;
+      if (AP == 2) {
+        const double dfr = fma(xi[j], c.mdf, -c.fRD), lor = fma(dfr, dfr, q.fg2), rp = recip64(den * lor);
+        rd = rp * lor;
+        amp[j] = (q.E * T.er[p.k + j]) * (rp * den);
+      } else {
+        rd = recip64(den);
+      }
+      v[j] = q.dn * rd;
+      v2[j] = v[j] * v[j];
+      rest[j] = fma(q.Rs, s34[j], fma(u[j], q.Ru3, zc.y));
+      pl[j] = c_atan64[8];
+    }
+#pragma unroll
+    for (int k = 7; k >= 0; k--) {
+      const double a = c_atan64[k];
+#pragma unroll
+      for (int j = 0; j < U; j++) pl[j] = fma(v2[j], pl[j], a);
+    }
+#pragma unroll
+    for (int j = 0; j < U; j++) rest[j] = fma(q.Rat * v[j], pl[j], rest[j]);
+  } else if (PP == 1) {
+#pragma unroll
+    for (int j = 0; j < U; j++) rest[j] = mph_int(c.mix.pint, xi[j], u[j], L[j]);
+  } else if (PP == 0) {
+    const MixPhIns& m = c.mix.pins;
+    const double2 c0 = sld2(&m.A0), c1 = sld2(&m.Att), c2 = sld2(&m.AL), c3 = sld2(&m.Auu), c4 = sld2(&m.Au5),
+                  c5 = sld2(&m.Ait), c6 = sld2(&m.Aii);
+#pragma unroll
+    for (int j = 0; j < U; j++) {          // mph_ins with the coefficients read once
+      double ph = fma(t[j], fma(t[j], c1.x, c0.y), c0.x);
+      ph = fma(L[j], fma(t[j], c1.y, c2.x), ph);
+      double pu = fma(u[j] * u[j], c4.x, c3.y);
+      pu = fma(u[j], pu, c3.x);
+      pu = fma(u[j], pu, c2.y);
+      ph = fma(u[j], pu, ph);
+      rest[j] = fma(xi[j], fma(xi[j], c6.x, fma(t[j], fma(t[j], c5.y, c5.x), c4.y)), ph);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+      const int pp = ph_piece(c.mix, p.b + j * bs);
+      if (pp == 0) rest[j] = mph_ins(c.mix.pins, xi[j], t[j], u[j], L[j]);
+      else if (pp == 1) rest[j] = mph_int(c.mix.pint, xi[j], u[j], L[j]);
+      else rest[j] = fma(q.Ru3, u[j] * u[j] * u[j], fma(q.Rs, s34[j], q.Rat * atan(fma(xi[j], q.D1, -q.D0))));
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < U; j++) {
+    if (AP == 0) amp[j] = amp64_ins(T, xi[j], t[j]);
+    else if (AP == 1) amp[j] = amp64_int(c, xi[j]);
+    else if (AP < 0) {
+      const int ap = amp_piece(c.mix, p.b + j * bs);
+      if (ap == 0) amp[j] = amp64_ins(T, xi[j], t[j]);
+      else if (ap == 1) amp[j] = amp64_int(c, xi[j]);
+      else {
+        const double fg = c.fDM * c.g3, dfr = fma(xi[j], c.mdf, -c.fRD);
+        amp[j] = exp(-dfr * c.g2 / fg) * (fg * c.g1) / (dfr * dfr + fg * fg);
+      }
+    }
+  }
+  double sv[U], cv[U];
+#pragma unroll
+  for (int j = 0; j < U; j++) rest[j] = fma(xi[j], q.lin1, q.lin0) - rest[j];
+  sincos_cycles<U, (PP < 0)>(rest, sv, cv);
+#pragma unroll
+  for (int j = 0; j < U; j++) {
+    const double ex = amp[j] * cv[j], ey = amp[j] * sv[j], a2 = amp[j] * amp[j];
+    A.r0 = fma(wri[j][0].x, ex, fma(wri[j][0].y, ey, A.r0));
+    A.sh[0] = fma(a2, ws[j][0], A.sh[0]);
+#pragma unroll
+    for (int id = 1; id < NIFO; id++) {
+      const double2 R = T.rot[p.k + j][id - 1];
+      const double qx = fma(R.x, ex, -(R.y * ey)), qy = fma(R.x, ey, R.y * ex);
+      A.sx[id] = fma(wri[j][id].x, qx, fma(wri[j][id].y, qy, A.sx[id]));
+      A.sy[id] = fma(wri[j][id].x, qy, fma(-wri[j][id].y, qx, A.sy[id]));
+      A.sh[id] = fma(a2, ws[j][id], A.sh[id]);
+    }
+  }
+}
+
+#ifndef QCBC_U64
+#define QCBC_U64 2
+#endif
+// Rows [k, k_end) of the thread's bins (k relative to the table segment), in one pair of pieces.
+template <int NIFO, int AP, int PP>
+__device__ __forceinline__ void rows64(const PhdRec& c, const EventData& ev, const Tab64& T, const Tile64& q,
+                                       Acc64<NIFO>& A, int k, int k_end, int i, int i1, int bs) {
+  if (i > i1) return;
+  int n = min(k_end - k, (i1 - i) / bs + 1);
+  constexpr int G = w64_group(NIFO);
+  const int nw = bs >> 5;
+  const double* grp = ev.w64 + (size_t)(i >> 5) * G;
+  Cur64 p;
+  p.xi = (double)i;
+  p.b = i;
+  p.k = k;
+  p.ab = ev.tabA + i;
+  p.cd = (PP == 2 ? ev.tabD : ev.tabB) + i;
+  p.w = reinterpret_cast<const double2*>(grp) + (i & 31);
+  p.ws = grp + 64 * NIFO + (i & 31);
+  auto advance = [&](int m) {
+    p.xi += (double)(m * bs);
+    p.b += m * bs;
+    p.k += m;
+    p.ab += m * bs;
+    p.cd += m * bs;
+    p.w += (size_t)(m * nw) * (G / 2);
+    p.ws += (size_t)(m * nw) * G;
+  };
+  constexpr int U = PP < 0 ? 1 : QCBC_U64;
+#pragma unroll 1
+  for (; n >= U; n -= U) {
+    step64<NIFO, AP, PP, U>(c, ev, T, q, A, p, bs);
+    advance(U);
+  }
+  if (U > 1) {
+#pragma unroll 1
+    for (; n > 0; n--) {
+      step64<NIFO, AP, PP, 1>(c, ev, T, q, A, p, bs);
+      advance(1);
+    }
+  }
+}
+
+// One tile: bins [i0, i1] walked by the block's threads in rows of blockDim.x.  Contains
+// __syncthreads(): every thread of the block calls it, with the same i0 and i1.
+template <int NIFO>
+__device__ __forceinline__ void tile_fp64(const PhdRec& c, const NetGeom& g, const EventData& ev, int i0, int i1,
+                                          Tab64& T, double* acc) {
+  const int tid = threadIdx.x, bs = blockDim.x, nw = bs >> 5, lane = tid & 31;
+  const int nk = mixed_table_len(i0, i1, bs);
+  const MixPoly& P = c.mix;
+  constexpr double kInv2Pi = 0.15915494309189533577;
+  const double m = c.mdf, ie = c.inv_eta, rdm = 1.0 / c.fDM, fg = c.fDM * c.g3, gx = c.g2 / fg;
+  Tile64 q;
+  q.lin1 = g.df * (c.ts - c.td[0]) - P.pmrd.Ri;
+  q.lin0 = c.lam[0] * kInv2Pi - P.pmrd.R0;
+  q.D1 = m * rdm;
+  q.D0 = c.al5 * c.fRD * rdm;
+  q.Ru3 = kInv2Pi * (-c.al2 * (c.mdf_rthird * c.mdf_rthird * c.mdf_rthird) * ie);
+  q.Rs = kInv2Pi * ((4.0 / 3.0) * c.al3 * c.mdf_34 * ie);
+  q.Rat = kInv2Pi * (c.al4 * ie);
+  q.dn = q.D1 * ((double)lane - 15.5);
+  q.fg2 = fg * fg;
+  // the ringdown's tables hold for this set, and no phase in the tile exceeds 2^45 cycles: every term is
+  // monotonic in i, so the sum of their sizes at the tile's two ends bounds it
+  const bool fast = fabs(q.D1) * 16.0 <= kAtanRange && fabs(m * gx) * (double)i1 + fabs(c.fRD * gx) < 500.0;
+  // (a bound only, so in FP32; infinite or NaN counts as not small)
+  bool small;
+  {
+    const float x1 = (float)i1, u0 = __powf((float)max(i0, 1), -1.0f / 3.0f), t1 = __powf(x1 + 1.0f, 1.0f / 3.0f),
+                L1 = __logf(x1 + 1.0f), u3 = u0 * u0 * u0;
+    const MixPhIns& a = P.pins;
+    auto f = [](double v) { return fabsf((float)v); };
+    const float ins = f(a.A0) + t1 * (f(a.At) + t1 * f(a.Att)) + L1 * (f(a.AL) + t1 * f(a.AtL)) +
+                      u0 * (f(a.Au) + u0 * (f(a.Auu) + u0 * (f(a.Au3) + u0 * u0 * f(a.Au5)))) +
+                      x1 * (f(a.Ai) + t1 * (f(a.Ait) + t1 * f(a.Aitt)) + x1 * f(a.Aii));
+    const float mid = f(P.pint.B0) + x1 * f(P.pint.Bi) + u3 * u3 * u3 * f(P.pint.Bu9) + L1 * f(P.pint.BL);
+    const float mrd = u3 * f(q.Ru3) + x1 * f(q.Rs) + 1.6f * f(q.Rat);
+    small = f(q.lin0) + x1 * f(q.lin1) + ins + mid + mrd < 3.0e13f;
+  }
+  q.E = 0.0;
+  if (fast && i1 >= P.iF) q.E = fg * c.g1 * exp(-gx * (m * (double)(i0 + tid) - c.fRD));
+  if (tid < 8) {                           // ai[k] (Msec df)^{n/3}, n = 2 .. 9
+    double p = c.mdf_third * c.mdf_third;
+    for (int k = 0; k < tid; k++) p *= c.mdf_third;
+    T.al[tid] = c.ai[tid] * p;
+  }
+  Acc64<NIFO> A;
+  A.zero();
+  for (int k0 = 0; k0 < nk; k0 += kSeg64) {
+    const int kn = min(kSeg64, nk - k0), first = i0 + k0 * bs, last = min(first + kn * bs - 1, i1);
+    if (k0) __syncthreads();               // the previous segment's rows are done with the tables
+    if (NIFO > 1) {
+      for (int e = tid; e < kn * (NIFO - 1); e += bs) {
+        const int r = NIFO > 1 ? e / (NIFO - 1 > 0 ? NIFO - 1 : 1) : 0, id = e - r * (NIFO - 1) + 1;
+        const double cyc = (double)(k0 + r) * ((double)bs * g.df * (c.td[0] - c.td[id]));
+        double sv, cv;
+        sincos_cycles(cyc, sv, cv);
+        T.rot[r][id - 1] = make_double2(cv, sv);
+      }
+    }
+    if (fast && last >= P.iM) {
+      for (int e = tid; e < kn * nw; e += bs) {
+        const int r = e / nw, w = e - r * nw, row = first + r * bs;
+        if (row + bs > P.iM) {
+          const double z = fma((double)(row + w * 32) + 15.5, q.D1, -q.D0);
+          T.sub[e] = make_double2(z, q.Rat * atan(z));
+        }
+      }
+    }
+    if (fast && last >= P.iF)
+      for (int r = tid; r < kn; r += bs) T.er[r] = exp(-(m * gx) * ((double)bs * (double)(k0 + r)));
+    __syncthreads();
+    int k = 0;
+    while (k < kn) {                       // block-uniform
+      const int r0 = first + k * bs, r1 = min(r0 + bs - 1, i1);
+      const int a0 = amp_piece(P, r0), p0 = ph_piece(P, r0), code = a0 * 3 + p0;
+      const bool table = small && (code == 0 || code == 3 || code == 4 || (fast && (code == 5 || code == 8)));
+      int k_end = k + 1;
+      const int i = r0 + tid;
+      if (!table || a0 != amp_piece(P, r1) || p0 != ph_piece(P, r1)) {
+        rows64<NIFO, -1, -1>(c, ev, T, q, A, k, k_end, i, i1, bs);
+      } else {
+        int nxt = last + 1;                // the pieces can only change at a threshold
+        if (P.iA > r0 && P.iA < nxt) nxt = P.iA;
+        if (P.iF > r0 && P.iF < nxt) nxt = P.iF;
+        if (P.iP > r0 && P.iP < nxt) nxt = P.iP;
+        if (P.iM > r0 && P.iM < nxt) nxt = P.iM;
+        k_end = nxt > last ? kn : max(k + 1, (nxt - first - bs) / bs + 1);
+        switch (code) {
+          case 0: rows64<NIFO, 0, 0>(c, ev, T, q, A, k, k_end, i, i1, bs); break;
+          case 3: rows64<NIFO, 1, 0>(c, ev, T, q, A, k, k_end, i, i1, bs); break;
+          case 4: rows64<NIFO, 1, 1>(c, ev, T, q, A, k, k_end, i, i1, bs); break;
+          case 5: rows64<NIFO, 1, 2>(c, ev, T, q, A, k, k_end, i, i1, bs); break;
+          default: rows64<NIFO, 2, 2>(c, ev, T, q, A, k, k_end, i, i1, bs); break;
+        }
+      }
+      k = k_end;
+    }
+  }
+  acc[0] = A.r0;
+  acc[1] = A.sh[0];
+#pragma unroll
+  for (int id = 1; id < NIFO; id++) {
+    const double cyc = (double)(i0 + tid) * g.df * (c.td[0] - c.td[id]) + (c.lam[id] - c.lam[0]) * kInv2Pi;
+    double sv, cv;
+    sincos_cycles(cyc, sv, cv);
+    acc[2 * id] = cv * A.sx[id] - sv * A.sy[id];
+    acc[2 * id + 1] = A.sh[id];
+  }
+}
+
 // rotation-table entries per detector that a block of a launch needs: ceil(max bins per tile /
 // threads) + 1
 __host__ __device__ __forceinline__ int mixed_nk_cap(int band, int tiles, int threads) {
@@ -1384,14 +1774,14 @@ __device__ __forceinline__ void tile_range(const PhdRec& c, int tiles, int t, in
 
 // lnL (and rho, or the per-detector SNR^2 of the intrinsic model) of one set from its per-detector
 // sums sd[id] = S[2 id], sh[id] = S[2 id + 1]; rho_b may be null
-__device__ __noinline__ void finalize_set(const PhdRec& c, const double* S, const NetGeom& g, const EventData& ev, int mixed,
-                             int model, double* lnl_b, double* rho_b) {
+__device__ __noinline__ void finalize_set(const PhdRec& c, const double* S, const NetGeom& g, const EventData& ev, int model,
+                                          double* lnl_b, double* rho_b) {
   double L = 0.0;
   int loud = 0;
   for (int id = 0; id < g.nifo; id++) {
     const double sd = S[2 * id], sh = S[2 * id + 1];
     double K = c.Fs[id] * kH22fac * c.amp_scale / c.sqT * ev.inv_sigma[id];
-    if (mixed) K *= c.a0 * c.mdf_m76;       // the mixed kernel sums the amplitude without this factor
+    K *= c.a0 * c.mdf_m76;                  // the tiles sum the amplitude without this factor
     double HD = K * sd, HH = K * K * sh;
     double x = HD - 0.5 * HH;
     if (model == kModelIntrinsic) {
@@ -1422,7 +1812,7 @@ __device__ void reject_set(const NetGeom& g, double* lnl_b, double* rho_b) {
 struct FinalOut {
   double* lnl;
   double* rho;
-  int mixed, model;
+  int model;
   SetOrder order;      // order.cnt non-null: block k evaluates the k-th set longest first (one tile per set)
   int B;
   int* done;           // several tiles per set: per-set tile counts, zero before the launch
@@ -1471,7 +1861,7 @@ __device__ __forceinline__ void finish_tile(const PhdRec& rec, const double* acc
     double S[2 * kMaxIfo];
 #pragma unroll
     for (int k = 0; k < 2 * kMaxIfo; k++) S[k] = k < 2 * NIFO ? acc[k] : 0.0;
-    finalize_set(rec, S, g, ev, fo.mixed, fo.model, fo.lnl + b, rho_b);
+    finalize_set(rec, S, g, ev, fo.model, fo.lnl + b, rho_b);
     return;
   }
   double* out = partials + ((size_t)b * tiles + t) * (2 * kMaxIfo);
@@ -1495,13 +1885,17 @@ __device__ __forceinline__ void finish_tile(const PhdRec& rec, const double* acc
 #pragma unroll
     for (int k = 0; k < 2 * NIFO; k++) S[k] += __ldcg(p + k);
   }
-  finalize_set(rec, S, g, ev, fo.mixed, fo.model, fo.lnl + b, rho_b);
+  finalize_set(rec, S, g, ev, fo.model, fo.lnl + b, rho_b);
 }
 
+#ifndef QCBC_FP64_REGS
+#define QCBC_FP64_REGS 128     // see the FP64 tile body
+#endif
 template <int PREC, int NIFO>
-__global__ void __launch_bounds__(256) k_lnl_full(const PhdRec* __restrict__ recs, NetGeom g, EventData ev, int tiles,
+__global__ void __maxnreg__(QCBC_FP64_REGS) k_lnl_full(const PhdRec* __restrict__ recs, NetGeom g, EventData ev, int tiles,
                                                   double* __restrict__ partials, FinalOut fo) {
   __shared__ PhdRec rec;
+  __shared__ Tab64 tab;
   __shared__ double red[32 * 2 * kMaxIfo];
   pdl_wait();          // records (and class lists) of the setup
   const int bi = blockIdx.x / tiles, t = blockIdx.x - bi * tiles;
@@ -1514,7 +1908,7 @@ __global__ void __launch_bounds__(256) k_lnl_full(const PhdRec* __restrict__ rec
   double acc[2 * NIFO];
 #pragma unroll
   for (int k = 0; k < 2 * NIFO; k++) acc[k] = 0.0;
-  tile_fp64<NIFO>(rec, g, ev, i0, i1, acc);
+  tile_fp64<NIFO>(rec, g, ev, i0, i1, tab, acc);
   block_sum<2 * NIFO>(acc, red);
   if (threadIdx.x == 0) finish_tile<NIFO>(rec, acc, g, ev, fo, b, tiles, t, partials);
 }
@@ -1633,7 +2027,7 @@ static void launch_full_prec(const PhdRec* r, int B, const NetGeom& g, const Eve
 void launch_lnl_full(const PhdRec* d_recs, int B, const NetGeom& g, const EventData& ev, Precision prec,
                      const FullLaunch& L, double* d_partials, cudaStream_t s) {
   if (B <= 0) return;
-  const FinalOut none{nullptr, nullptr, 0, 0, SetOrder{nullptr, nullptr}, B, nullptr};
+  const FinalOut none{nullptr, nullptr, 0, SetOrder{nullptr, nullptr}, B, nullptr};
   if (prec == kFP64) launch_full_prec<kFP64>(d_recs, B, g, ev, L, d_partials, none, s);
   else launch_full_mixed(d_recs, B, g, ev, L, d_partials, none, s);
 }
@@ -1644,10 +2038,10 @@ bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, con
   if (B <= 0) return true;
   if (L.tiles != 1 && !d_done) {
     launch_lnl_full(d_recs, B, g, ev, prec, L, d_partials, s);
-    launch_finalize_full(d_partials, d_recs, d_status, B, L.tiles, g, ev, prec, d_lnl, d_rho, s, model);
+    launch_finalize_full(d_partials, d_recs, d_status, B, L.tiles, g, ev, d_lnl, d_rho, s, model);
     return false;
   }
-  const FinalOut fo{d_lnl, d_rho, prec == kMixed ? 1 : 0, model,
+  const FinalOut fo{d_lnl, d_rho, model,
                     (order && L.tiles == 1) ? *order : SetOrder{nullptr, nullptr}, B,
                     L.tiles == 1 ? nullptr : d_done};
   if (prec == kFP64) launch_full_prec<kFP64>(d_recs, B, g, ev, L, d_partials, fo, s);
@@ -1657,7 +2051,7 @@ bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, con
 
 __global__ void k_finalize_full(const double* __restrict__ partials, const PhdRec* __restrict__ recs,
                                 const int* __restrict__ status, int B, int tiles, NetGeom g, EventData ev,
-                                int mixed, int model, double* __restrict__ lnl, double* __restrict__ rho) {
+                                int model, double* __restrict__ lnl, double* __restrict__ rho) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   double* rho_b = rho ? rho + (size_t)b * g.nifo : nullptr;
@@ -1671,29 +2065,32 @@ __global__ void k_finalize_full(const double* __restrict__ partials, const PhdRe
     const double* p = partials + ((size_t)b * tiles + t) * (2 * kMaxIfo);
     for (int k = 0; k < 2 * g.nifo; k++) S[k] += p[k];
   }
-  finalize_set(recs[b], S, g, ev, mixed, model, lnl + b, rho_b);
+  finalize_set(recs[b], S, g, ev, model, lnl + b, rho_b);
 }
 
 void launch_finalize_full(const double* d_partials, const PhdRec* d_recs, const int* d_status, int B, int tiles,
-                          const NetGeom& g, const EventData& ev, Precision prec, double* d_lnl, double* d_rho,
+                          const NetGeom& g, const EventData& ev, double* d_lnl, double* d_rho,
                           cudaStream_t s, int model) {
   if (B <= 0) return;
   k_finalize_full<<<(B + 127) / 128, 128, 0, s>>>(d_partials, d_recs, d_status, B, tiles, g, ev,
-                                                  prec == kMixed ? 1 : 0, model, d_lnl, d_rho);
+                                                  model, d_lnl, d_rho);
 }
 
-__global__ void k_fill_bin_tables(double2* __restrict__ A, double2* __restrict__ Bt, float2* __restrict__ C, int n) {
+__global__ void k_fill_bin_tables(double2* __restrict__ A, double2* __restrict__ Bt, float2* __restrict__ C,
+                                  double2* __restrict__ D, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double x = (double)(i > 0 ? i : 1);
     double c3 = cbrt(x), s = pow(x, 0.75);
     A[i] = make_double2(c3, 1.0 / c3);
     Bt[i] = make_double2(log(x), s);
     C[i] = make_float2((float)(1.0 / x), (float)s);
+    D[i] = make_double2(1.0 / x, s);
   }
 }
 
-void launch_fill_bin_tables(double2* d_tabA, double2* d_tabB, float2* d_tabC, int n, cudaStream_t s) {
-  k_fill_bin_tables<<<(n + 255) / 256, 256, 0, s>>>(d_tabA, d_tabB, d_tabC, n);
+void launch_fill_bin_tables(double2* d_tabA, double2* d_tabB, float2* d_tabC, double2* d_tabD, int n,
+                            cudaStream_t s) {
+  k_fill_bin_tables<<<(n + 255) / 256, 256, 0, s>>>(d_tabA, d_tabB, d_tabC, d_tabD, n);
 }
 
 // ---------------------------------------------------------------- multi-event launches
@@ -1763,7 +2160,7 @@ void launch_scan_expand(const int* d_ntile, int B, int* d_off, int* d_items, int
 // registers, the mixed body reads its piece coefficients from shared memory and keeps each
 // thread's sums there (tile_mixed_smem).
 template <int PREC>
-__global__ void __launch_bounds__(256, PREC == kFP64 ? 4 : QCBC_MULTI_MINBLOCKS) k_lnl_multi(const PhdRec* __restrict__ recs,
+__global__ void __launch_bounds__(256, PREC == kFP64 ? 2 : QCBC_MULTI_MINBLOCKS) k_lnl_multi(const PhdRec* __restrict__ recs,
                                                       const EventDesc* __restrict__ events,
                                                       const int* __restrict__ off, const int* __restrict__ items,
                                                       int B, int tile_bins, int items_cap, int* __restrict__ counter,
@@ -1772,7 +2169,7 @@ __global__ void __launch_bounds__(256, PREC == kFP64 ? 4 : QCBC_MULTI_MINBLOCKS)
   __shared__ EventDesc evd;
   __shared__ int s_item, s_b;
   __shared__ double red[32 * 2 * kMaxIfo];
-  extern __shared__ __align__(16) float2 s_rot[];   // mixed: rotation table [nk][4], then the threads' state
+  extern __shared__ __align__(16) float2 s_rot[];   // FP64: Tab64; mixed: rotation table [nk][4], then the threads' state
   int total = off[B];
   if (total > items_cap) total = items_cap;
   for (;;) {
@@ -1796,9 +2193,10 @@ __global__ void __launch_bounds__(256, PREC == kFP64 ? 4 : QCBC_MULTI_MINBLOCKS)
     for (int k = 0; k < 2 * kMaxIfo; k++) acc[k] = 0.0;
     const int nifo = evd.g.nifo;
     if (PREC == kFP64) {
-      if (nifo == 1) tile_fp64<1>(rec, evd.g, evd.ev, i0, i1, acc);
-      else if (nifo == 2) tile_fp64<2>(rec, evd.g, evd.ev, i0, i1, acc);
-      else tile_fp64<3>(rec, evd.g, evd.ev, i0, i1, acc);
+      Tab64& tab = *reinterpret_cast<Tab64*>(s_rot);
+      if (nifo == 1) tile_fp64<1>(rec, evd.g, evd.ev, i0, i1, tab, acc);
+      else if (nifo == 2) tile_fp64<2>(rec, evd.g, evd.ev, i0, i1, tab, acc);
+      else tile_fp64<3>(rec, evd.g, evd.ev, i0, i1, tab, acc);
     } else {
       const int nk = (tile_bins + blockDim.x - 1) / blockDim.x + 1;
       if (nifo == 1) tile_mixed_smem<1>(rec, evd.g, evd.ev, i0, i1, s_rot, nk, kMaxIfo, acc);
@@ -1816,7 +2214,7 @@ __global__ void __launch_bounds__(256, PREC == kFP64 ? 4 : QCBC_MULTI_MINBLOCKS)
 }
 
 static size_t multi_smem(Precision prec, int threads, int tile_bins) {
-  if (prec == kFP64) return 0;
+  if (prec == kFP64) return sizeof(Tab64);
   int nk = (tile_bins + threads - 1) / threads + 1;
   return (size_t)nk * mix_rs(kMaxIfo) * sizeof(float2) + mixed_state_bytes(threads, kMaxIfo);
 }
@@ -1848,7 +2246,7 @@ void launch_lnl_multi(const PhdRec* d_recs, const EventDesc* d_events, const int
 
 __global__ void k_finalize_multi(const double* __restrict__ partials, const PhdRec* __restrict__ recs,
                                  const int* __restrict__ status, const int* __restrict__ off,
-                                 const EventDesc* __restrict__ events, int B, int items_cap, int mixed,
+                                 const EventDesc* __restrict__ events, int B, int items_cap,
                                  double* __restrict__ lnl, double* __restrict__ rho) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
@@ -1872,7 +2270,7 @@ __global__ void k_finalize_multi(const double* __restrict__ partials, const PhdR
       sh += partials[(size_t)it * (2 * kMaxIfo) + 2 * id + 1];
     }
     double K = c.Fs[id] * kH22fac * c.amp_scale / c.sqT * e.ev.inv_sigma[id];
-    if (mixed) K *= c.a0 * c.mdf_m76;
+    K *= c.a0 * c.mdf_m76;
     double HD = K * sd, HH = K * K * sh;
     if (rho) rho[(size_t)b * kMaxIfo + id] = HD / sqrt(HH);
     L += HD - 0.5 * HH;
@@ -1881,11 +2279,11 @@ __global__ void k_finalize_multi(const double* __restrict__ partials, const PhdR
 }
 
 void launch_finalize_multi(const double* d_partials, const PhdRec* d_recs, const int* d_status, const int* d_off,
-                           const EventDesc* d_events, int B, int items_cap, Precision prec, double* d_lnl,
-                           double* d_rho, cudaStream_t s) {
+                           const EventDesc* d_events, int B, int items_cap, double* d_lnl, double* d_rho,
+                           cudaStream_t s) {
   if (B <= 0) return;
   k_finalize_multi<<<(B + 127) / 128, 128, 0, s>>>(d_partials, d_recs, d_status, d_off, d_events, B, items_cap,
-                                                   prec == kMixed ? 1 : 0, d_lnl, d_rho);
+                                                   d_lnl, d_rho);
 }
 
 // ---------------------------------------------------------------- heterodyned lnL

@@ -21,7 +21,10 @@ struct NetGeom {
 // sigma[id] so that the FP32 copy stays in range:
 //   wr = 4 sigma Re(D)/S,  wi = 4 sigma Im(D)/S,  ws = 4 sigma^2 / S  per bin.
 struct EventData {
-  const double* w64;     // [nifo][3][nh]: wr, wi, ws rows (FP64 kernels)
+  // FP64 weighted data with the amplitude's bin factor folded in (as wm), in groups of 32 bins
+  // (w64_doubles in all): group j holds the pairs (wr', wi') of bins 32 j .. 32 j + 31 of each detector,
+  // then their ws' of each detector
+  const double* w64;
   // FP32 weighted data of the mixed kernel with the amplitude's bin factor folded in:
   // wr' = wr i^{-7/6}, wi' = wi i^{-7/6}, ws' = ws i^{-7/3}, 12 B per detector-bin in planes that
   // one thread reads with the fewest aligned loads (MixW):
@@ -32,13 +35,16 @@ struct EventData {
   int nh;                // row length (N/2)
   double inv_sigma[kMaxIfo];
   // per-bin constants shared by all events on a device (index = bin number i >= 1):
-  // tabA = (i^{1/3}, i^{-1/3}), tabB = (log i, i^{3/4}), tabC = (1/i, i^{3/4}) rounded to float
+  // tabA = (i^{1/3}, i^{-1/3}), tabB = (log i, i^{3/4}), tabC = tabD = (1/i, i^{3/4}), tabC rounded to float
   const double2* tabA;
   const double2* tabB;
   const float2* tabC;
+  const double2* tabD;
   int tab_n;
 };
-// Floats of the mixed kernel's planes for an event of nifo detectors: 3 per detector-bin over nh bins.
+// Doubles of the FP64 data (whole groups of 32 bins) and floats of the mixed kernel's planes for an event
+// of nifo detectors: 3 per detector-bin over nh bins.
+inline size_t w64_doubles(int nifo, size_t nh) { return (nh + 31) / 32 * 32 * 3 * (size_t)nifo; }
 inline size_t mixed_plane_floats(int nifo, size_t nh) { return (size_t)3 * nifo * nh; }
 
 // Heterodyne summary tables on the device (layouts as the reference's struct Het, flattened):
@@ -115,7 +121,7 @@ void launch_lnl_full(const PhdRec* d_recs, int B, const NetGeom& g, const EventD
 // d_rho: full model rho[id] = HD / sqrt(HH); intrinsic model the per-detector SNR^2 = 2 (HD - HH/2)
 // (and lnL = 0 unless at least two detectors exceed 25 when Nifo > 1, QuickCBC.c:4117-4128)
 void launch_finalize_full(const double* d_partials, const PhdRec* d_recs, const int* d_status, int B, int tiles,
-                          const NetGeom& g, const EventData& ev, Precision prec, double* d_lnl, double* d_rho,
+                          const NetGeom& g, const EventData& ev, double* d_lnl, double* d_rho,
                           cudaStream_t s, int model = kModelFull);
 // lnL of B sets with the finaliser folded into the lnL kernel: when each set is one tile (L.tiles ==
 // 1), longest first when order is given (filled by launch_setup_ordered); at several tiles per set
@@ -126,7 +132,8 @@ bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, con
                            Precision prec, const FullLaunch& L, double* d_partials, double* d_lnl, double* d_rho,
                            int model, const SetOrder* order, cudaStream_t s, int* d_done = nullptr);
 // fill the per-bin tables for bins [0, n)
-void launch_fill_bin_tables(double2* d_tabA, double2* d_tabB, float2* d_tabC, int n, cudaStream_t s);
+void launch_fill_bin_tables(double2* d_tabA, double2* d_tabB, float2* d_tabC, double2* d_tabD, int n,
+                            cudaStream_t s);
 void launch_lnl_het(const PhdRec* d_recs, const int* d_status, int B, const NetGeom& g, const HetData& h,
                     Precision prec, double* d_lnl, cudaStream_t s);
 // shared memory of one set's warp in the heterodyned kernels (its record and [3][nifo][M] doubles)
@@ -214,8 +221,8 @@ void launch_lnl_multi(const PhdRec* d_recs, const EventDesc* d_events, const int
                       int tile_bins, int items_cap, Precision prec, int threads, int blocks, int* d_counter,
                       double* d_partials, cudaStream_t s);
 void launch_finalize_multi(const double* d_partials, const PhdRec* d_recs, const int* d_status, const int* d_off,
-                           const EventDesc* d_events, int B, int items_cap, Precision prec, double* d_lnl,
-                           double* d_rho, cudaStream_t s);
+                           const EventDesc* d_events, int B, int items_cap, double* d_lnl, double* d_rho,
+                           cudaStream_t s);
 int multi_blocks_per_sm(Precision prec, int threads, int tile_bins);
 
 void upload_tables();    // constant-memory tables; call once per device
