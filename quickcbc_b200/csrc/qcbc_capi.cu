@@ -972,13 +972,15 @@ extern "C" int qcbc_het_fisher(qcbc_event* ev, const double* params, int B, doub
 }
 
 // ------------------------------------------------------------------ heterodyne grid search
-static int run_het_space(const NetGeom& g, const double* h_S, int sn_stride, const double* h_freq, int N, double Tobs,
-                         double fmin, double fmax, const double* params, const double* pmin, const double* pmax,
-                         HetSpaceOut& out) {
+static int run_het_space(const NetGeom& g, const double* S, int sn_stride, const double* freq, bool on_device, int N,
+                         double Tobs, double fmin, double fmax, const double* params, const double* pmin,
+                         const double* pmax, HetSpaceOut& out) {
   Workspace* w;
   int rc = workspace(w);
   if (rc) return rc;
-  HetSpaceIn in{g, g_dev[current_device()].qnm, h_S, sn_stride, h_freq, N, Tobs, fmin, fmax, w->stream};
+  const double* none = nullptr;
+  HetSpaceIn in{g, g_dev[current_device()].qnm, on_device ? S : none, on_device ? freq : none, on_device ? none : S,
+                on_device ? none : freq, sn_stride, N, Tobs, fmin, fmax, w->stream};
   std::string err;
   rc = het_space_run(in, params, pmin, pmax, out, err);
   tls_launches += out.launches;
@@ -991,13 +993,9 @@ extern "C" int qcbc_het_space(qcbc_event* ev, const double* params, const double
                               int* MN, int* MM) {
   if (!ev || !params || !pmin || !pmax) return fail(QCBC_EINVAL, "NULL argument");
   if (!ev->has_data) return fail(QCBC_EINVAL, "event has no data");
-  const int nI = ev->g.nifo, nh = ev->nh;
-  std::vector<double> S((size_t)nI * (nh + 1)), freq((size_t)nh);
-  CU(cudaMemcpy(S.data(), ev->d_S, S.size() * sizeof(double), cudaMemcpyDeviceToHost));
-  CU(cudaMemcpy(freq.data(), ev->d_freq, freq.size() * sizeof(double), cudaMemcpyDeviceToHost));
   HetSpaceOut out;
-  int rc = run_het_space(ev->g, S.data(), nh + 1, freq.data(), ev->g.N, ev->g.Tobs, ev->fmin, ev->fmax, params, pmin,
-                         pmax, out);
+  int rc = run_het_space(ev->g, ev->d_S, ev->nh + 1, ev->d_freq, true, ev->g.N, ev->g.Tobs, ev->fmin, ev->fmax, params,
+                         pmin, pmax, out);
   if (rc) return rc;
   ev->space_grid = out.fgrid;
   ev->space_MN = out.MN;
@@ -2332,7 +2330,7 @@ extern "C" void het_space(struct Net* net, struct Het* het, double* params, doub
   NetGeom g;
   fill_geom(g, nI, net->labels, net->Tobs, net->GMST, N, g_band_fmin, g_band_fmax);
   HetSpaceOut out;
-  if (run_het_space(g, S.data(), nh, freq->data, N, Tobs, g_band_fmin, g_band_fmax, params, min, max, out)) return;
+  if (run_het_space(g, S.data(), nh, freq->data, false, N, Tobs, g_band_fmin, g_band_fmax, params, min, max, out)) return;
   // the struct Het fields het_space sets, allocated as CreateRealVector / int_vector do
   // (IMRPhenomD_internals.c:148-156, Utilities.c:2941-2944) so freehet releases them
   het->MN = out.MN;

@@ -1,12 +1,12 @@
 // Heterodyne grid search: het_space (QuickCBC.c:4570-4910) with limits (4275-4385),
 // Fisher_All (2695-2817), FisherEvec (2449-2530), efix (4387-4567) and diff (4913-4964).
 //
-// The control logic (band limits from the SNR accumulation, the eigen-directions of the Fisher
-// matrix, the bracketing/secant search of efix, the adaptive grid walk and its flattening to
-// J = 2 regions) runs on the host in FP64, restated from the reference.  Every waveform it needs
-// is computed on the device: the reference set and its 22 central-difference neighbours over the
-// whole band for the Fisher matrix (one launch), each efix trial point, and the 12 sets of the
-// grid walk, whose phase/amplitude ratios are formed on the device as well.
+// The control logic (the eigen-directions of the Fisher matrix, the bracketing/secant search of efix, the
+// flattening of the grid to J = 2 regions) runs on the host in FP64, restated from the reference.  The
+// device computes the waveforms and everything that runs over bins: the band limits from the SNR
+// accumulation, the Fisher sums over the reference set's 22 central-difference neighbours, the distances
+// of each round of efix trial points (all directions search in step), the ratios of the 11 scaled steps to
+// the reference, and the adaptive grid walk.  Only those results cross to the host, through pinned memory.
 //
 // Differences from the reference, on purpose: no diagnostic files (fspace.dat, df.dat,
 // df_flat.dat, ratio.dat) and no printing; the grid is copied out before its scratch is released
@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <algorithm>
 #include <functional>
 #include <string>
 #include <vector>
@@ -177,13 +178,15 @@ void step_point(const double* params, double a, const double* e, const double* p
   } while (0)
 
 // Device scratch of the grid searches of one host thread, kept from call to call (grow-only, per
-// device).  The Fisher waves alone are (2 NP + 1) nifo N/2 doubles twice, about 290 MB at 128 s and
-// 4096 Hz, and allocating and releasing them on every call cost up to a second.  A search ends with
+// device).  The Fisher waves are (2 NP + 1) nifo doubles twice per in-band bin and their terms 66 nifo, about
+// 350 MB together at 128 s and 4096 Hz, and allocating and releasing them on every call cost up to a second.  A search ends with
 // its stream synchronised, so the next search of the thread may reuse the buffers.  They are
 // released with the process.
 struct ScratchCache {
   std::vector<void*> p[16];
   std::vector<size_t> cap[16];
+  void *h[16] = {}, *m[16] = {};     // pinned host block and its device address
+  size_t hcap[16] = {};
 };
 thread_local ScratchCache tls_scratch;
 
@@ -215,6 +218,23 @@ struct Scratch {
     *out = static_cast<T*>(p[next++]);
     return cudaSuccess;
   }
+  // the thread's pinned host block as a T, and the device's view of it
+  template <class T>
+  cudaError_t host(T** h, T** m) {
+    ScratchCache& c = tls_scratch;
+    if (c.hcap[device] < sizeof(T)) {
+      cudaFreeHost(c.h[device]);
+      c.h[device] = nullptr;
+      c.hcap[device] = 0;
+      cudaError_t e = cudaMallocHost(&c.h[device], sizeof(T));
+      if (e == cudaSuccess) e = cudaHostGetDevicePointer(&c.m[device], c.h[device], 0);
+      if (e != cudaSuccess) return e;
+      c.hcap[device] = sizeof(T);
+    }
+    *h = static_cast<T*>(c.h[device]);
+    *m = static_cast<T*>(c.m[device]);
+    return cudaSuccess;
+  }
 };
 
 }  // namespace
@@ -222,40 +242,55 @@ struct Scratch {
 void fisher_evec_11(const double (&F)[11][11], double* ej, double (&ev)[11][11]) { fisher_evec(F, ej, ev); }
 
 int efix_run(const double* params, const double* pmin, const double* pmax, double* eval, const double (&evec)[11][11],
-             double zs, const std::function<int(const double*, double&)>& dist) {
+             double zs, const std::function<int(const double*, int, double*)>& dist) {
   const double zmx = zs * 2.0, zmn = zs / 2.0;
-  double px[NP], e[NP];
-  int rc;
-  for (int i = 0; i < NP; ++i) {
-    double dzmin = 1.0e20, alpham = 1.0, alpha0 = 1.0, z0 = 0.0, z = 0.0;
-    for (int j = 0; j < NP; j++) e[j] = eval[i] * evec[i][j];
+  struct Search {
+    double e[NP], dzmin = 1.0e20, alpham = 1.0, alpha0 = 1.0, alpha = 0.0, z0 = 0.0;
     int k = 0;
-    do {
-      step_point(params, alpha0, e, pmin, pmax, px);
-      if ((rc = dist(px, z0))) return rc;
-      double dz = fabs(z0 - zs);
-      if (dz < dzmin) { dzmin = dz; alpham = alpha0; }
-      if (z0 < zmn) alpha0 *= 2.0;
-      if (z0 > zmx) alpha0 /= 1.9;
-      k++;
-    } while ((z0 > zmx || z0 < zmn) && k < 15 && fabs(alpha0 < 1.0e4));
-    double alpha = alpha0 * 1.1;
-    k = 0;
-    do {
-      step_point(params, alpha, e, pmin, pmax, px);
-      if ((rc = dist(px, z))) return rc;
-      double alphanew;
-      if (alpha > alpha0) alphanew = alpha0 + (zs - z0) / (z - z0) * (alpha - alpha0);
-      else alphanew = alpha + (zs - z) / (z0 - z) * (alpha0 - alpha);
-      double dz = fabs(z - zs);
-      if (dz < dzmin) { dzmin = dz; alpham = alpha; }
-      z0 = z;
-      alpha0 = alpha;
-      alpha = alphanew;
-      k++;
-    } while (fabs(z - zs) > 0.2 && k < 10 && fabs(alpha < 1.0e4));
-    if (dzmin / zs > 1.0) alpham = 0.0;               // kill any failed direction
-    eval[i] *= alpham;
+    bool secant = false, done = false;
+  } dir[NP];
+  for (int i = 0; i < NP; i++)
+    for (int j = 0; j < NP; j++) dir[i].e[j] = eval[i] * evec[i][j];
+  for (;;) {
+    double px[NP * NP], z[NP];
+    int who[NP], n = 0;
+    for (int i = 0; i < NP; i++) {
+      if (dir[i].done) continue;
+      step_point(params, dir[i].secant ? dir[i].alpha : dir[i].alpha0, dir[i].e, pmin, pmax, px + (size_t)n * NP);
+      who[n++] = i;
+    }
+    if (n == 0) break;
+    if (int rc = dist(px, n, z)) return rc;
+    for (int q = 0; q < n; q++) {
+      Search& d = dir[who[q]];
+      const double dz = fabs(z[q] - zs);
+      if (!d.secant) {                                // bracket: double or divide until within a factor of two
+        d.z0 = z[q];
+        if (dz < d.dzmin) { d.dzmin = dz; d.alpham = d.alpha0; }
+        if (d.z0 < zmn) d.alpha0 *= 2.0;
+        if (d.z0 > zmx) d.alpha0 /= 1.9;
+        d.k++;
+        if (!((d.z0 > zmx || d.z0 < zmn) && d.k < 15 && fabs(d.alpha0 < 1.0e4))) {
+          d.alpha = d.alpha0 * 1.1;
+          d.k = 0;
+          d.secant = true;
+        }
+      } else {
+        double next;
+        if (d.alpha > d.alpha0) next = d.alpha0 + (zs - d.z0) / (z[q] - d.z0) * (d.alpha - d.alpha0);
+        else next = d.alpha + (zs - z[q]) / (d.z0 - z[q]) * (d.alpha0 - d.alpha);
+        if (dz < d.dzmin) { d.dzmin = dz; d.alpham = d.alpha; }
+        d.z0 = z[q];
+        d.alpha0 = d.alpha;
+        d.alpha = next;
+        d.k++;
+        if (!(fabs(z[q] - zs) > 0.2 && d.k < 10 && fabs(d.alpha < 1.0e4))) d.done = true;
+      }
+    }
+  }
+  for (int i = 0; i < NP; i++) {
+    if (dir[i].dzmin / zs > 1.0) dir[i].alpham = 0.0;  // kill any failed direction
+    eval[i] *= dir[i].alpham;
   }
   return 0;
 }
@@ -268,29 +303,40 @@ int het_space_run(const HetSpaceIn& in, const double* params, const double* pmin
   const int ss = in.sn_stride;
   cudaStream_t s = in.stream;
   Scratch sc(s);
-  double *d_freq, *d_S, *d_par, *d_amp, *d_ph, *d_out;
+  constexpr int kSets = 2 * NP + 1, kChunks = 148, kHostGrid = 4096;
+  double *d_freq, *d_S, *d_amp, *d_ph, *d_dS, *d_bsum;
   PhdRec* d_rec;
   int* d_st;
-  const size_t wave_cap = (size_t)(2 * NP + 1) * nifo * N2;     // the Fisher waves are the largest
-  HS_CU(sc.alloc(&d_freq, (size_t)N2));
-  HS_CU(sc.alloc(&d_S, (size_t)nifo * ss));
-  HS_CU(sc.alloc(&d_par, (size_t)(2 * NP + 1) * NP));
-  HS_CU(sc.alloc(&d_rec, (size_t)(2 * NP + 1)));
-  HS_CU(sc.alloc(&d_st, (size_t)(2 * NP + 1)));
-  HS_CU(sc.alloc(&d_amp, wave_cap));
-  HS_CU(sc.alloc(&d_ph, wave_cap));
-  HS_CU(sc.alloc(&d_out, (size_t)NP * NP));
-  HS_CU(cudaMemcpyAsync(d_freq, in.h_freq, sizeof(double) * N2, cudaMemcpyHostToDevice, s));
-  HS_CU(cudaMemcpyAsync(d_S, in.h_S, sizeof(double) * nifo * ss, cudaMemcpyHostToDevice, s));
+  HsLimits* d_lim;
+  int imin = (int)(Tobs * in.fmin), imax = (int)(Tobs * in.fmax);   // band of the Fisher matrix
+  if (imax > N2) imax = N2;
+  const int nfish = imax > imin ? imax - imin : 0;
+  HS_CU(sc.alloc(&d_rec, (size_t)kSets));
+  HS_CU(sc.alloc(&d_st, (size_t)kSets));
+  HS_CU(sc.alloc(&d_amp, (size_t)nifo * N2));                       // the reference set's waves
+  HS_CU(sc.alloc(&d_ph, (size_t)nifo * N2));
+  HS_CU(sc.alloc(&d_dS, (size_t)N2));
+  HS_CU(sc.alloc(&d_bsum, (size_t)N2 / 1024 + 1));
+  HS_CU(sc.alloc(&d_lim, 1));
+  HS_CU(sc.alloc(&d_freq, in.d_freq ? 1 : (size_t)N2));
+  HS_CU(sc.alloc(&d_S, in.d_S ? 1 : (size_t)nifo * ss));
+  // pinned host memory the kernels read and write: parameters, limits, distances, the Fisher matrix, the grid
+  struct Pinned {
+    HsLimits lim;
+    double par[kSets * NP], part[NP * kChunks], fish[NP * NP];
+    int count, grid[kHostGrid];
+  }*h, *m;
+  HS_CU(sc.host(&h, &m));
+  if (!in.d_freq) HS_CU(cudaMemcpyAsync(d_freq, in.h_freq, sizeof(double) * N2, cudaMemcpyHostToDevice, s));
+  if (!in.d_S) HS_CU(cudaMemcpyAsync(d_S, in.h_S, sizeof(double) * nifo * ss, cudaMemcpyHostToDevice, s));
+  const double *freq = in.d_freq ? in.d_freq : d_freq, *S = in.d_S ? in.d_S : d_S;
   int launches = 0;
 
-  // waves of `nset` parameter sets (host rows of NP) over n bins into d_amp/d_ph
-  auto waves = [&](const double* h_par, int nset, int n, double* amp, double* ph) -> int {
-    HS_CU(cudaMemcpyAsync(d_par, h_par, sizeof(double) * NP * nset, cudaMemcpyHostToDevice, s));
-    launch_setup(d_par, nset, g, in.qnm, d_rec, d_st, s);
-    launch_waves(d_rec, nset, g, d_freq, n, amp, ph, s);
-    launches += 2;
-    return 0;
+  // records of `nset` parameter sets (host rows of NP); the stream has been waited for since the last
+  auto records = [&](const double* par, int nset) {
+    memcpy(h->par, par, sizeof(double) * NP * nset);
+    launch_setup(m->par, nset, g, in.qnm, d_rec, d_st, s);
+    launches += 1;
   };
 
   // ---- limits (QuickCBC.c:4275-4385)
@@ -299,78 +345,41 @@ int het_space_run(const HetSpaceIn& in, const double* params, const double* pmin
   int M = (int)(fstop * Tobs);
   if (M > N2) M = N2;
   if (M < 2) { err = "het_space: signal band below two bins"; return -2; }
-  int rc = waves(params, 1, M, d_amp, d_ph);        // the reference set, kept for diff
-  if (rc) return rc;
-  PhdRec rec0;
-  std::vector<double> Ar((size_t)nifo * M);
-  HS_CU(cudaMemcpyAsync(&rec0, d_rec, sizeof(PhdRec), cudaMemcpyDeviceToHost, s));
-  HS_CU(cudaMemcpyAsync(Ar.data(), d_amp, sizeof(double) * nifo * M, cudaMemcpyDeviceToHost, s));
+  records(params, 1);                                 // the reference set, its waves kept for diff and the ratios
+  launch_waves(d_rec, 1, g, freq, M, d_amp, d_ph, s);
+  launch_hs_limits(d_rec, d_amp, nifo, M, S, ss, in.fmin, Tobs, d_dS, d_bsum, d_lim, &m->lim, s);
+  launches += 3;
+  HS_CU(cudaGetLastError());
   HS_CU(cudaStreamSynchronize(s));
-  const double fs = rec0.fs;                          // fbegin(params), Utilities.c:587
-  const int jmin0 = (in.fmin > fs) ? (int)(Tobs * in.fmin) : (int)(Tobs * fs);
-  std::vector<double> SNRsq(M, 0.0), dSNRsq(M, 0.0), ratio((size_t)N2 + 1, 1.0);
-  {
-    double dx = 0.0;
-    for (int j = jmin0; j < M; j++) {
-      for (int id = 0; id < nifo; id++) {
-        const double a = Ar[(size_t)id * M + j];
-        const double x = 4.0 * (a * a) / in.h_S[(size_t)id * ss + j];
-        dSNRsq[j] += x;
-        dx += x;
-      }
-      SNRsq[j] = dx;
-    }
-  }
-  int stst0 = jmin0, stst1 = M - 1;
-  {
-    const double SNRsqT = SNRsq[M - 1];
-    bool f1 = false, f2 = false;
-    for (int j = jmin0; j < M; j++) {
-      if (!f1 && SNRsq[j] > 0.001) { f1 = true; stst0 = j; }
-      if (!f2 && SNRsqT - SNRsq[j] < 0.001) { f2 = true; stst1 = j; }
-    }
-    if (!f2) stst1 = M - 1;
-    if (stst0 < jmin0) stst0 = jmin0;
-    const double x = SNRsqT / (double)(stst1 - stst0);   // average contribution per significant bin
-    for (int j = 1; j < M; j++) {
-      const double d = dSNRsq[j] / x;
-      ratio[j] = 1.0;
-      if (d > 0.0) ratio[j] = 1.0 / d;
-    }
-  }
-  const int MN = stst0, MM = stst1, J = 2;
+  const int MN = h->lim.MN, MM = h->lim.MM, J = 2;
   const double tol = 0.003;
   if (MM <= MN) { err = "het_space: empty signal band"; return -2; }
+  int rc;
 
   // ---- Fisher_All (QuickCBC.c:2695-2817) and FisherEvec
   double F[NP][NP];
   for (int i = 0; i < NP; i++)
     for (int j = 0; j < NP; j++) F[i][j] = i == j ? 1.0e4 : 0.0;
   if (fabs(params[2]) < 0.9999 && fabs(params[3]) < 0.9999) {
-    std::vector<double> P((size_t)(2 * NP + 1) * NP);
-    for (int k = 0; k < 2 * NP + 1; k++) memcpy(&P[(size_t)k * NP], params, NP * sizeof(double));
+    std::vector<double> P((size_t)kSets * NP);
+    for (int k = 0; k < kSets; k++) memcpy(&P[(size_t)k * NP], params, NP * sizeof(double));
     for (int i = 0; i < NP; i++) {
       P[(size_t)(1 + 2 * i) * NP + i] += kEps;
       P[(size_t)(2 + 2 * i) * NP + i] -= kEps;
     }
-    // the reference set's waves over M bins stay in d_amp/d_ph[0..nifo*M); the Fisher waves go after
-    double* fa = d_amp + (size_t)nifo * M;
-    double* fp = d_ph + (size_t)nifo * M;
-    if ((size_t)nifo * M + (size_t)(2 * NP + 1) * nifo * N2 > wave_cap) {
-      double *a2, *p2;
-      HS_CU(sc.alloc(&a2, (size_t)(2 * NP + 1) * nifo * N2));
-      HS_CU(sc.alloc(&p2, (size_t)(2 * NP + 1) * nifo * N2));
-      fa = a2;
-      fp = p2;
-    }
-    if ((rc = waves(P.data(), 2 * NP + 1, N2, fa, fp))) return rc;
-    int imin = (int)(Tobs * in.fmin), imax = (int)(Tobs * in.fmax);
-    if (imax > N2) imax = N2;
-    launch_fisher_full(fa, fp, 1, g, N2, d_S, ss, imin, imax, kEps, d_out, s);
-    launches += 1;
-    double G[NP * NP];
-    HS_CU(cudaMemcpyAsync(G, d_out, sizeof(G), cudaMemcpyDeviceToHost, s));
+    double *fa, *fp, *d_fparts;
+    HS_CU(sc.alloc(&fa, (size_t)kSets * nifo * std::max(nfish, 1)));
+    HS_CU(sc.alloc(&fp, (size_t)kSets * nifo * std::max(nfish, 1)));
+    double* d_terms;
+    HS_CU(sc.alloc(&d_terms, (size_t)NP * (NP + 1) / 2 * nifo * std::max(nfish, 1)));
+    HS_CU(sc.alloc(&d_fparts, (size_t)NP * (NP + 1) / 2 * 8));
+    records(P.data(), kSets);
+    launch_waves(d_rec, kSets, g, freq + imin, nfish, fa, fp, s);
+    launch_fisher_full(fa, fp, g, nfish, S + imin, ss, kEps, d_terms, d_fparts, m->fish, s);
+    launches += 4;
+    HS_CU(cudaGetLastError());
     HS_CU(cudaStreamSynchronize(s));
+    const double* G = h->fish;
     for (int i = 0; i < NP; i++)
       for (int j = i; j < NP; j++) F[i][j] = F[j][i] = G[i * NP + j];
   }
@@ -378,85 +387,80 @@ int het_space_run(const HetSpaceIn& in, const double* params, const double* pmin
   fisher_evec(F, eval, evec);
 
   // ---- efix (QuickCBC.c:4387-4567), zs = 30, diff on the full grid
-  const int imin_d = (in.fmin > fs) ? (int)(Tobs * in.fmin) : (int)(Tobs * fs);
-  double* trial_a = d_amp + (size_t)nifo * M;        // one trial set after the reference waves
-  double* trial_p = d_ph + (size_t)nifo * M;
-  constexpr int kChunks = 148;
-  double* d_part;
-  HS_CU(sc.alloc(&d_part, (size_t)kChunks));
-  auto diff = [&](const double* px, double& z) -> int {
-    if ((rc = waves(px, 1, M, trial_a, trial_p))) return rc;
-    launch_diff_full(d_amp, d_ph, trial_a, trial_p, 1, g, M, imin_d, M, d_S, ss, kChunks, d_part, s);
+  auto dist = [&](const double* px, int n, double* z) -> int {
+    records(px, n);
+    launch_wave_diff(d_rec, n, g, freq, d_amp, d_ph, M, h->lim.jmin, M, S, ss, kChunks, m->part, s);
     launches += 1;
-    double part[kChunks];
-    HS_CU(cudaMemcpyAsync(part, d_part, sizeof(part), cudaMemcpyDeviceToHost, s));
+    HS_CU(cudaGetLastError());
     HS_CU(cudaStreamSynchronize(s));
-    z = 0.0;
-    for (int c = 0; c < kChunks; c++) z += part[c];
+    for (int q = 0; q < n; q++) {
+      z[q] = 0.0;
+      for (int c = 0; c < kChunks; c++) z[q] += h->part[q * kChunks + c];
+    }
     return 0;
   };
-  auto dist = [&](const double* px, double& z) -> int { return diff(px, z); };
   rc = efix_run(params, pmin, pmax, eval, evec, 30.0, dist);
   if (rc != 0) return rc;
 
-  // ---- grid walk (QuickCBC.c:4624-4765): the 12 sets' waves, their ratios and the walk on the device
-  std::vector<double> P((size_t)(NP + 1) * NP);
-  memcpy(P.data(), params, NP * sizeof(double));
+  // ---- grid walk (QuickCBC.c:4624-4765): the 11 steps' waves as ratios to the reference's, and the walk
+  std::vector<double> P((size_t)NP * NP);
   for (int i = 0; i < NP; ++i) {
     double e[NP];
     for (int j = 0; j < NP; j++) e[j] = eval[i] * evec[i][j];
-    step_point(params, 1.0, e, pmin, pmax, &P[(size_t)(1 + i) * NP]);
+    step_point(params, 1.0, e, pmin, pmax, &P[(size_t)i * NP]);
   }
-  if ((rc = waves(P.data(), NP + 1, MM, d_amp, d_ph))) return rc;
+  records(P.data(), NP);
   const int W = MM - MN, per = NP * nifo;
-  double *d_Cs, *d_Sn, *d_DH, *d_ratio;
-  int *d_grid, *d_count;
+  double *d_Cs, *d_Sn;
+  int *d_grid, *d_first;
   HS_CU(sc.alloc(&d_Cs, (size_t)per * W));
   HS_CU(sc.alloc(&d_Sn, (size_t)per * W));
-  HS_CU(sc.alloc(&d_DH, (size_t)per * W));
-  HS_CU(sc.alloc(&d_ratio, ratio.size()));
   HS_CU(sc.alloc(&d_grid, (size_t)W + 2));
-  HS_CU(sc.alloc(&d_count, 1));
-  HS_CU(cudaMemcpyAsync(d_ratio, ratio.data(), sizeof(double) * ratio.size(), cudaMemcpyHostToDevice, s));
-  launch_hs_ratios(d_amp, d_ph, NP + 1, nifo, MM, MN, MM, d_Cs, d_Sn, d_DH, s);
+  HS_CU(sc.alloc(&d_first, 3));
+  launch_hs_ratios(d_rec, NP, g, freq, d_amp, d_ph, M, MN, MM, d_Cs, d_Sn, s);
   const int djmax = (int)(100.0 * Tobs);                 // maximum spacing
-  launch_hs_walk(d_Cs, d_Sn, d_DH, d_ratio, per, MN, MM, djmax, tol, W + 2, d_grid, d_count, s);
+  HS_CU(launch_hs_walk(d_Cs, d_Sn, d_dS, d_lim, per, MN, MM, djmax, tol, W + 2, d_first, d_grid, m->grid,
+                       kHostGrid, &m->count, s));
   launches += 2;
-  int count = 0;
-  HS_CU(cudaMemcpyAsync(&count, d_count, sizeof(int), cudaMemcpyDeviceToHost, s));
   HS_CU(cudaStreamSynchronize(s));
+  const int count = h->count;
   if (count < 1) { err = "het_space: grid walk did not finish"; return -2; }
   std::vector<int> fgrid((size_t)count);
-  HS_CU(cudaMemcpy(fgrid.data(), d_grid, sizeof(int) * count, cudaMemcpyDeviceToHost));
+  if (count <= kHostGrid) memcpy(fgrid.data(), h->grid, sizeof(int) * count);
+  else HS_CU(cudaMemcpy(fgrid.data(), d_grid, sizeof(int) * count, cudaMemcpyDeviceToHost));
   const int Mr = (int)fgrid.size() - 1;
 
-  // ---- spacing per bin and the flattened grid with J = 2 points per region (QuickCBC.c:4767-4864)
-  std::vector<int> dfa((size_t)N2, 100);
-  for (int ii = 0; ii < Mr; ii++) {
-    const int d = fgrid[ii + 1] - fgrid[ii];
-    for (int i = fgrid[ii]; i < fgrid[ii + 1]; ++i) dfa[i] = d;
-  }
-  {
-    const int d = MM - fgrid[Mr];
-    for (int i = fgrid[Mr]; i < MM; ++i) dfa[i] = d;
-  }
+  // ---- spacing per bin and the flattened grid with J = 2 points per region (QuickCBC.c:4767-4864).  The
+  // spacing is constant between grid points (100 outside them), so its smallest value over a range of bins
+  // is found over the few stretches that overlap the range.
+  struct Stretch { int lo, hi, d; };                     // bins [lo, hi)
+  std::vector<Stretch> st;
+  st.push_back({0, fgrid[0], 100});
+  for (int i = 0; i < Mr; i++) st.push_back({fgrid[i], fgrid[i + 1], fgrid[i + 1] - fgrid[i]});
+  st.push_back({fgrid[Mr], MM, MM - fgrid[Mr]});
+  st.push_back({MM, N2, 100});
+  auto spacing_min = [&](int a, int b, int least) {      // smallest spacing of bins [a, b] within [0, N/2)
+    size_t lo = 0, hi = st.size();
+    while (lo < hi) {                                    // first stretch that ends beyond a
+      const size_t mid = (lo + hi) / 2;
+      if (st[mid].hi > a) hi = mid; else lo = mid + 1;
+    }
+    for (; lo < st.size() && st[lo].lo <= b; lo++)
+      if (st[lo].hi > st[lo].lo && st[lo].d < least) least = st[lo].d;
+    return least;
+  };
   std::vector<int> fg;
   fg.reserve(1024);
   int j = MN, k = 0, ii = 0;
   fg.push_back(j);
   do {
-    int jm = dfa[j];
+    int jm = spacing_min(j, j, 2147483647);
     bool flag;
     do {
-      flag = false;
       k = j + jm * J;
-      for (int i = j; i <= k; ++i) {
-        if (i < N2) {
-          if (dfa[i] < jm) { jm = dfa[i]; flag = true; }
-        } else {
-          flag = false;
-        }
-      }
+      const int least = spacing_min(j, k, jm);
+      flag = least < jm && k < N2;                       // a range that leaves the bins is not tried again
+      jm = least;
     } while (flag);
     j = k;
     for (int i = 0; i < J; ++i) {

@@ -16,6 +16,7 @@
 // :587-629, 716-736, 995-1109; IMRPhenomD.c:413-563.
 #include "qcbc_kernels.cuh"
 #include "qcbc_ptstep.h"
+#include <cooperative_groups.h>
 #include <cmath>
 #include <cstdio>
 
@@ -2600,178 +2601,366 @@ void launch_het_waves(const PhdRec* d_recs, int B, const NetGeom& g, const HetDa
   launch_waves(d_recs, B, g, h.freq, h.M, d_amp, d_phase, s);
 }
 
-// Fisher_All (QuickCBC.c:2695-2817): one block per (matrix f, pair i <= j) over the full band:
-// sum over detectors and bins k in [imin, imax) of 4 (dA_i dA_j + A^2 dphi_i dphi_j) / S, with
-// the central differences of the 23 wave sets of matrix f (as k_het_fisher) on n bins.
-__global__ void __launch_bounds__(256) k_fisher_full(const double* __restrict__ amp, const double* __restrict__ ph,
-                                                     NetGeom g, int n, const double* __restrict__ S, int sn_stride,
-                                                     int imin, int imax, double eps, double* __restrict__ fish) {
-  __shared__ double red[32];
-  __shared__ int s_ij[2];
-  const int f = blockIdx.y, nifo = g.nifo;
-  if (threadIdx.x == 0) {
-    int q = blockIdx.x, i = 0;
-    while (q >= kNP - i) { q -= kNP - i; i++; }
-    s_ij[0] = i;
-    s_ij[1] = i + q;
+// ---- the grid search's device pieces (het_space).  Each is spread over the whole chip; what bounds the
+// search is the number of dependent steps (about ten rounds of trial points, fifty grid points), not their
+// work: 33.4 ms -> 2.4 ms at 3 detectors, 128 s, 4096 Hz.
+
+// Fisher_All (QuickCBC.c:2695-2817) from the 23 wave sets (point, then +/- eps along each parameter) on n bins:
+// sum over detectors and bins of 4 (dA_i dA_j + A^2 dphi_i dphi_j) / S.  With one detector the matrix has a
+// null space, whose basis (and so the grid) can follow the last bits of these sums (one of ten one-detector
+// grids moved when they were reordered): a pair's 256 partial sums therefore run over the bins k, k + 256, ...
+// of detector after detector, each a serial chain, and are added in one fixed order, with fixed roundings in
+// each term.  The terms of all 66 pairs are computed first, a thread per bin reading the 45 wave arrays
+// once; the chains then only load and add, 32 loads ahead.  185 us at 3 x 128 k bins, where one block per
+// pair, reading nine wave arrays row by row, took 2.6 ms (a sum in any order, over the bins of the whole
+// chip, would take 45 us).
+constexpr int kNPairs = kNP * (kNP + 1) / 2;
+__global__ void __launch_bounds__(128) k_fisher_terms(const double* __restrict__ amp, const double* __restrict__ ph,
+                                                      int nifo, int n, const double* __restrict__ S, int sn_stride,
+                                                      double eps, double* __restrict__ terms) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nifo * n) return;
+  const int id = t / n;
+  const size_t row = (size_t)nifo * n;
+  double dA[kNP], dP[kNP];
+#pragma unroll
+  for (int i = 0; i < kNP; i++) {
+    dA[i] = (__ldg(amp + (1 + 2 * i) * row + t) - __ldg(amp + (2 + 2 * i) * row + t)) / (2.0 * eps);
+    dP[i] = (__ldg(ph + (1 + 2 * i) * row + t) - __ldg(ph + (2 + 2 * i) * row + t)) / (2.0 * eps);
   }
-  __syncthreads();
-  const int i = s_ij[0], j = s_ij[1];
-  const size_t set0 = (size_t)f * kFisherSets;
-  double acc[1] = {0.0};
-  for (int id = 0; id < nifo; id++) {
-    const double* A0 = amp + (set0 * nifo + id) * n;
-    const double* Api = amp + ((set0 + 1 + 2 * i) * nifo + id) * n;
-    const double* Ami = amp + ((set0 + 2 + 2 * i) * nifo + id) * n;
-    const double* Apj = amp + ((set0 + 1 + 2 * j) * nifo + id) * n;
-    const double* Amj = amp + ((set0 + 2 + 2 * j) * nifo + id) * n;
-    const double* Ppi = ph + ((set0 + 1 + 2 * i) * nifo + id) * n;
-    const double* Pmi = ph + ((set0 + 2 + 2 * i) * nifo + id) * n;
-    const double* Ppj = ph + ((set0 + 1 + 2 * j) * nifo + id) * n;
-    const double* Pmj = ph + ((set0 + 2 + 2 * j) * nifo + id) * n;
-    const double* Sd = S + (size_t)id * sn_stride;
-    for (int k = imin + threadIdx.x; k < imax; k += blockDim.x) {
-      const double dAi = (Api[k] - Ami[k]) / (2.0 * eps), dAj = (Apj[k] - Amj[k]) / (2.0 * eps);
-      const double dPi = (Ppi[k] - Pmi[k]) / (2.0 * eps), dPj = (Ppj[k] - Pmj[k]) / (2.0 * eps);
-      acc[0] += 4.0 * (dAi * dAj + A0[k] * A0[k] * dPi * dPj) / Sd[k];
+  const double A0 = __ldg(amp + t), A2 = A0 * A0, Sd = __ldg(S + (size_t)id * sn_stride + (t - id * n));
+  int q = 0;
+#pragma unroll
+  for (int i = 0; i < kNP; i++)
+#pragma unroll
+    for (int j = i; j < kNP; j++, q++)
+      terms[q * row + t] = 4.0 * __fma_rn(dA[i], dA[j], __dmul_rn(__dmul_rn(A2, dP[i]), dP[j])) / Sd;
+}
+
+// block: chains 32 y .. 32 y + 31 of pair x; the warp's butterfly sum into parts[x][y]
+__global__ void __launch_bounds__(32) k_fisher_chains(const double* __restrict__ terms, int nifo, int n,
+                                                      double* __restrict__ parts) {
+  const double* p = terms + (size_t)blockIdx.x * nifo * n;
+  double acc = 0.0;
+  constexpr int R = 32;
+  for (int id = 0; id < nifo; id++, p += n)
+    for (int k = blockIdx.y * 32 + threadIdx.x; k < n; k += 256 * R) {
+      double v[R];
+#pragma unroll
+      for (int r = 0; r < R; r++) v[r] = k + 256 * r < n ? __ldg(p + k + 256 * r) : 0.0;
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        if (k + 256 * r < n) acc += v[r];
     }
-  }
-  block_sum<1>(acc, red);
-  if (threadIdx.x == 0) fish[((size_t)f * kNP + i) * kNP + j] = acc[0];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (threadIdx.x == 0) parts[blockIdx.x * 8 + blockIdx.y] = acc;
 }
 
-void launch_fisher_full(const double* d_amp, const double* d_phase, int nmat, const NetGeom& g, int n,
-                        const double* d_S, int sn_stride, int imin, int imax, double eps, double* d_fish,
-                        cudaStream_t s) {
-  if (nmat <= 0) return;
-  dim3 grid(kNP * (kNP + 1) / 2, (unsigned)nmat);
-  k_fisher_full<<<grid, 256, 0, s>>>(d_amp, d_phase, g, n, d_S, sn_stride, imin, imax, eps, d_fish);
+// a pair's eight warp sums into the upper triangle of fish[11][11]: a warp per pair
+__global__ void __launch_bounds__(32) k_fisher_sum(const double* __restrict__ parts, double* __restrict__ fish) {
+  int q = blockIdx.x, i = 0;
+  double v = threadIdx.x < 8 ? parts[q * 8 + threadIdx.x] : 0.0;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  while (q >= kNP - i) { q -= kNP - i; i++; }
+  if (threadIdx.x == 0) fish[i * kNP + i + q] = v;
 }
 
-// diff (QuickCBC.c:4913-4964): partial sums over detectors and bins j in [imin, m) of
-// 4 |h_ref - h_b|^2 / S for the reference waves (one set) and B other wave sets on n bins; block
-// (c, b) covers chunk c of the bins of set b and writes out[b * gridDim.x + c].
-__global__ void __launch_bounds__(256) k_diff_full(const double* __restrict__ amp_ref, const double* __restrict__ ph_ref,
-                                                   const double* __restrict__ amp, const double* __restrict__ ph,
-                                                   NetGeom g, int n, int imin, int m, const double* __restrict__ S,
-                                                   int sn_stride, double* __restrict__ out) {
+void launch_fisher_full(const double* d_amp, const double* d_phase, const NetGeom& g, int n, const double* d_S,
+                        int sn_stride, double eps, double* d_terms, double* d_parts, double* d_fish, cudaStream_t s) {
+  if (n > 0)
+    k_fisher_terms<<<(g.nifo * n + 127) / 128, 128, 0, s>>>(d_amp, d_phase, g.nifo, n, d_S, sn_stride, eps, d_terms);
+  k_fisher_chains<<<dim3(kNPairs, 8), 32, 0, s>>>(d_terms, g.nifo, n, d_parts);
+  k_fisher_sum<<<kNPairs, 32, 0, s>>>(d_parts, d_fish);
+}
+
+// The tapered amplitude (without its detector factor) and the phase of record c at frequency f, as
+// k_waves computes them.
+__device__ __forceinline__ void wave_point(const PhdRec& c, double f, double& amp, double& ph, double& y) {
+  y = 1.0;
+  if (f < c.fs) y = exp(10.0 * (f - c.fs) / c.fs);
+  amp = 0.0;
+  ph = 0.0;
+  if (!(f > c.fCut)) { phd_eval64(c, c.Msec * f, amp, ph); amp *= c.amp_scale; }
+}
+
+// diff (QuickCBC.c:4913-4964): partial sums over detectors and bins j in [imin, m) of 4 |h_ref - h_b|^2 / S
+// between the reference waves (amp_ref, ph_ref [nifo][n]) and the waveform of record b, evaluated here
+// bin by bin (the trial waves are never written); block (c, b) covers chunk c of the bins and writes
+// out[b * gridDim.x + c].
+__global__ void __launch_bounds__(256) k_wave_diff(const PhdRec* __restrict__ recs, NetGeom g,
+                                                   const double* __restrict__ freq, const double* __restrict__ amp_ref,
+                                                   const double* __restrict__ ph_ref, int n, int imin, int m,
+                                                   const double* __restrict__ S, int sn_stride,
+                                                   double* __restrict__ out) {
+  __shared__ PhdRec c;
   __shared__ double red[32];
-  const int b = blockIdx.y, nifo = g.nifo;
+  load_record(c, recs + blockIdx.y);
+  __syncthreads();
   const int span = (m - imin + gridDim.x - 1) / gridDim.x;
   const int j0 = imin + blockIdx.x * span, j1 = min(m, j0 + span);
   double acc[1] = {0.0};
-  for (int id = 0; id < nifo; id++) {
-    const double* Ar = amp_ref + (size_t)id * n;
-    const double* Pr = ph_ref + (size_t)id * n;
-    const double* Ap = amp + ((size_t)b * nifo + id) * n;
-    const double* Pp = ph + ((size_t)b * nifo + id) * n;
-    const double* Sd = S + (size_t)id * sn_stride;
-    for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-      const double d = Pr[j] - Pp[j];
-      const double re = Ar[j] - Ap[j] * cos(d), im = Ap[j] * sin(d);
-      acc[0] += 4.0 * (re * re + im * im) / Sd[j];
+  for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
+    const double f = __ldg(freq + j);
+    double amp, ph, y;
+    wave_point(c, f, amp, ph, y);
+    for (int id = 0; id < g.nifo; id++) {
+      const double Ap = c.Fs[id] * kH22fac * amp / c.sqT * y;
+      const double Pp = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(kTwoPi, f), c.ts - c.td[id]), c.lam[id]), -ph);
+      const double Ar = __ldg(amp_ref + (size_t)id * n + j), d = __ldg(ph_ref + (size_t)id * n + j) - Pp;
+      double sd, cd;
+      sincos(d, &sd, &cd);
+      const double re = Ar - Ap * cd, im = Ap * sd;
+      acc[0] += 4.0 * (re * re + im * im) / __ldg(S + (size_t)id * sn_stride + j);
     }
   }
   block_sum<1>(acc, red);
-  if (threadIdx.x == 0) out[(size_t)b * gridDim.x + blockIdx.x] = acc[0];
+  if (threadIdx.x == 0) out[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = acc[0];
 }
 
-void launch_diff_full(const double* d_amp_ref, const double* d_ph_ref, const double* d_amp, const double* d_ph, int B,
-                      const NetGeom& g, int n, int imin, int m, const double* d_S, int sn_stride, int chunks,
+void launch_wave_diff(const PhdRec* d_recs, int B, const NetGeom& g, const double* d_freq, const double* d_amp_ref,
+                      const double* d_ph_ref, int n, int imin, int m, const double* d_S, int sn_stride, int chunks,
                       double* d_out, cudaStream_t s) {
   if (B <= 0 || chunks <= 0) return;
-  dim3 grid((unsigned)chunks, (unsigned)B);
-  k_diff_full<<<grid, 256, 0, s>>>(d_amp_ref, d_ph_ref, d_amp, d_ph, g, n, imin, m, d_S, sn_stride, d_out);
+  k_wave_diff<<<dim3((unsigned)chunks, (unsigned)B), 256, 0, s>>>(d_recs, g, d_freq, d_amp_ref, d_ph_ref, n, imin, m,
+                                                                  d_S, sn_stride, d_out);
 }
 
-// het_space's ratios to the reference waveform (QuickCBC.c:4688-4702) for the wave sets
-// 1..nset-1 against set 0, bins [j0, j1) of n: Cs = 1 - Ap/Ar cos(Pr - Pp), Sn = Ap/Ar sin(Pr - Pp),
-// DH = Cs^2 + Sn^2, each [j1-j0][nset-1][nifo] (bin-major, as the grid walk reads them).
-__global__ void k_hs_ratios(const double* __restrict__ amp, const double* __restrict__ ph, int nset, int nifo, int n,
-                            int j0, int j1, double* __restrict__ Cs, double* __restrict__ Sn,
-                            double* __restrict__ DH) {
-  const int per = (nset - 1) * nifo;
-  const long long total = (long long)per * (j1 - j0);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(t % per);
-    const int j = j0 + (int)(t / per);
-    const int id = r % nifo, i = r / nifo;
-    const double Ar = amp[(size_t)id * n + j], Pr = ph[(size_t)id * n + j];
-    const double Ap = amp[((size_t)(i + 1) * nifo + id) * n + j], Pp = ph[((size_t)(i + 1) * nifo + id) * n + j];
-    const double c = 1.0 - Ap / Ar * cos(Pr - Pp);
-    const double sv = Ap / Ar * sin(Pr - Pp);
-    Cs[t] = c;
-    Sn[t] = sv;
-    DH[t] = c * c + sv * sv;
+// het_space's ratios to the reference waveform (QuickCBC.c:4688-4702) of the records recs[0 .. nset),
+// bins [j0, j1): Cs = 1 - Ap/Ar cos(Pr - Pp), Sn = Ap/Ar sin(Pr - Pp) in rows [nset][nifo] of j1 - j0 bins.
+__global__ void __launch_bounds__(256) k_hs_ratios(const PhdRec* __restrict__ recs, NetGeom g,
+                                                   const double* __restrict__ freq, const double* __restrict__ amp_ref,
+                                                   const double* __restrict__ ph_ref, int n, int j0, int j1,
+                                                   double* __restrict__ Cs, double* __restrict__ Sn) {
+  __shared__ PhdRec c;
+  load_record(c, recs + blockIdx.y);
+  __syncthreads();
+  const int j = j0 + blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= j1) return;
+  const double f = __ldg(freq + j);
+  double amp, ph, y;
+  wave_point(c, f, amp, ph, y);
+  for (int id = 0; id < g.nifo; id++) {
+    const double Ap = c.Fs[id] * kH22fac * amp / c.sqT * y;
+    const double Pp = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(kTwoPi, f), c.ts - c.td[id]), c.lam[id]), -ph);
+    const double q = Ap / __ldg(amp_ref + (size_t)id * n + j), d = __ldg(ph_ref + (size_t)id * n + j) - Pp;
+    double sd, cd;
+    sincos(d, &sd, &cd);
+    const double cv = 1.0 - q * cd, sv = q * sd;
+    const size_t o = ((size_t)blockIdx.y * g.nifo + id) * (j1 - j0) + (j - j0);
+    Cs[o] = cv;
+    Sn[o] = sv;
   }
 }
 
-void launch_hs_ratios(const double* d_amp, const double* d_ph, int nset, int nifo, int n, int j0, int j1,
-                      double* d_Cs, double* d_Sn, double* d_DH, cudaStream_t s) {
-  long long total = (long long)(nset - 1) * nifo * (j1 - j0);
-  if (total <= 0) return;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 4736) blocks = 4736;
-  k_hs_ratios<<<(unsigned)blocks, 256, 0, s>>>(d_amp, d_ph, nset, nifo, n, j0, j1, d_Cs, d_Sn, d_DH);
+void launch_hs_ratios(const PhdRec* d_recs, int nset, const NetGeom& g, const double* d_freq, const double* d_amp_ref,
+                      const double* d_ph_ref, int n, int j0, int j1, double* d_Cs, double* d_Sn, cudaStream_t s) {
+  if (nset <= 0 || j1 <= j0) return;
+  k_hs_ratios<<<dim3((unsigned)((j1 - j0 + 255) / 256), (unsigned)nset), 256, 0, s>>>(
+      d_recs, g, d_freq, d_amp_ref, d_ph_ref, n, j0, j1, d_Cs, d_Sn);
 }
 
-// het_space's grid walk (QuickCBC.c:4720-4765) in one block: from the current grid point jmin,
-// the next one is the first bin j > jmin at which the linear interpolation between jmin and j of
-// any ratio (Cs, Sn, DH of any direction and detector) misses its value at the mid-point by more
-// than tl = max(tol ratio[j], tol), or at which j - jmin exceeds djmax.  The block tests 1024
-// consecutive bins at a time and keeps the first hit.  grid[0..*count) gets the points; the walk
-// stops at the cap (*count = -1 then).
-__global__ void __launch_bounds__(1024) k_hs_walk(const double* __restrict__ Cs, const double* __restrict__ Sn,
-                                                  const double* __restrict__ DH, const double* __restrict__ ratio,
-                                                  int per, int MN, int MM, int djmax, double tol, int cap,
-                                                  int* __restrict__ grid, int* __restrict__ count) {
-  __shared__ int s_first;
-  int jmin = MN, nout = 0;
-  if (threadIdx.x == 0) grid[nout] = jmin;
-  nout++;
-  for (;;) {
-    int found = MM;
-    for (int base = jmin + 1; base < MM && found == MM; base += blockDim.x) {
-      if (threadIdx.x == 0) s_first = MM;
-      __syncthreads();
-      const int j = base + threadIdx.x;
-      bool flag = false;
-      if (j < MM) {
-        double tl = tol * ratio[j];
-        if (tl < tol) tl = tol;
-        const int jmid = (j + jmin) / 2;
-        const double w0 = (double)(j - jmid), w1 = (double)(jmid - jmin), dw = (double)(j - jmin);
-        const size_t oa = (size_t)(jmin - MN) * per, ob = (size_t)(j - MN) * per, om = (size_t)(jmid - MN) * per;
-        for (int r = 0; r < per && !flag; r++) {
-          const double cmid = (Cs[oa + r] * w0 + Cs[ob + r] * w1) / dw;
-          const double smid = (Sn[oa + r] * w0 + Sn[ob + r] * w1) / dw;
-          const double dmid = (DH[oa + r] * w0 + DH[ob + r] * w1) / dw;
-          if (fabs(Cs[om + r] - cmid) > tl || fabs(Sn[om + r] - smid) > tl || fabs(DH[om + r] - dmid) > tl)
-            flag = true;
-        }
-        if (j - jmin > djmax) flag = true;
+// limits (QuickCBC.c:4275-4385): SNR^2 per bin, dS[j] = sum over detectors of 4 A^2 / S from jmin on
+// (jmin = Tobs max(fmin, fbegin)), zero before, and the sum of each block's 1024 bins.
+__device__ __forceinline__ int hs_jmin(const PhdRec& c, double fmin, double Tobs) {
+  return fmin > c.fs ? (int)(Tobs * fmin) : (int)(Tobs * c.fs);
+}
+__global__ void __launch_bounds__(1024) k_hs_power(const PhdRec* __restrict__ rec, const double* __restrict__ amp,
+                                                   int nifo, int M, const double* __restrict__ S, int sn_stride,
+                                                   double fmin, double Tobs, double* __restrict__ dS,
+                                                   double* __restrict__ bsum) {
+  __shared__ double red[32];
+  const int j = blockIdx.x * 1024 + threadIdx.x, jmin = hs_jmin(*rec, fmin, Tobs);
+  double v[1] = {0.0};
+  if (j < M) {
+    if (j >= jmin)
+      for (int id = 0; id < nifo; id++) {
+        const double a = __ldg(amp + (size_t)id * M + j);
+        v[0] += 4.0 * (a * a) / __ldg(S + (size_t)id * sn_stride + j);
       }
-      if (flag) atomicMin(&s_first, j);
+    dS[j] = v[0];
+  }
+  block_sum<1>(v, red);
+  if (threadIdx.x == 0) bsum[blockIdx.x] = v[0];
+}
+
+// The signal band from the accumulated SNR^2: MN = first bin where it exceeds 0.001, MM = first bin where
+// less than 0.001 of it is left, x = its average per bin between them.  One block: thread 0 runs through
+// the block sums and notes the two blocks, a scan of each finds the bin.
+__global__ void __launch_bounds__(1024) k_hs_limits(const PhdRec* __restrict__ rec, const double* __restrict__ dS,
+                                                    const double* __restrict__ bsum, int M, double fmin, double Tobs,
+                                                    HsLimits* __restrict__ out, HsLimits* __restrict__ out_host) {
+  __shared__ double s_sum[1024], s_w[32], s_before[2], s_total;
+  __shared__ int s_blk[2], s_bin[2];
+  const int nb = (M + 1023) / 1024, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int jmin = hs_jmin(*rec, fmin, Tobs);
+  if (tid == 0) {
+    s_blk[0] = s_blk[1] = -1;
+    s_bin[0] = s_bin[1] = 2147483647;
+    s_total = 0.0;
+  }
+  for (int pass = 0; pass < 2; pass++) {         // the total, then the blocks
+    double run = 0.0;
+    for (int b0 = 0; b0 < nb; b0 += 1024) {
       __syncthreads();
-      found = s_first;
+      if (b0 + tid < nb) s_sum[tid] = bsum[b0 + tid];
       __syncthreads();
+      if (tid == 0) {
+        const int m = min(1024, nb - b0);
+        for (int k = 0; k < m; k++) {
+          const double before = run;
+          run += s_sum[k];
+          if (pass == 1) {
+            if (s_blk[0] < 0 && run > 0.001) { s_blk[0] = b0 + k; s_before[0] = before; }
+            if (s_blk[1] < 0 && (b0 + k + 1) * 1024 > jmin && s_total - run < 0.001) {
+              s_blk[1] = b0 + k;
+              s_before[1] = before;
+            }
+          }
+        }
+        if (pass == 0) s_total = run;
+      }
     }
+  }
+  __syncthreads();
+  for (int e = 0; e < 2; e++) {
+    const int blk = s_blk[e];
+    if (blk >= 0) {                              // block-uniform
+      const int j = blk * 1024 + tid;
+      double v = j < M ? dS[j] : 0.0;
+      for (int o = 1; o < 32; o <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+      }
+      if (lane == 31) s_w[w] = v;
+      __syncthreads();
+      double p = s_before[e];
+      for (int k = 0; k < w; k++) p += s_w[k];
+      p += v;
+      const bool hit = j < M && j >= jmin && (e == 0 ? p > 0.001 : s_total - p < 0.001);
+      if (hit) atomicMin(&s_bin[e], j);
+      __syncthreads();
+      // the block's own sum crossed the line; its last bin stands in when the scan's rounding does not
+      if (tid == 0 && s_bin[e] == 2147483647) s_bin[e] = min(blk * 1024 + 1023, M - 1);
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    HsLimits r;
+    r.jmin = jmin;
+    r.MN = s_blk[0] >= 0 ? s_bin[0] : jmin;
+    r.MM = s_blk[1] >= 0 ? s_bin[1] : M - 1;
+    if (r.MN < jmin) r.MN = jmin;
+    r.x = s_total / (double)(r.MM - r.MN);
+    *out = r;
+    *out_host = r;
+  }
+}
+
+void launch_hs_limits(const PhdRec* d_rec, const double* d_amp, int nifo, int M, const double* d_S, int sn_stride,
+                      double fmin, double Tobs, double* d_dS, double* d_bsum, HsLimits* d_out, HsLimits* m_out,
+                      cudaStream_t s) {
+  k_hs_power<<<(M + 1023) / 1024, 1024, 0, s>>>(d_rec, d_amp, nifo, M, d_S, sn_stride, fmin, Tobs, d_dS, d_bsum);
+  k_hs_limits<<<1, 1024, 0, s>>>(d_rec, d_dS, d_bsum, M, fmin, Tobs, d_out, m_out);
+}
+
+// het_space's grid walk (QuickCBC.c:4720-4765): from the current grid point jmin, the next one is the
+// first bin j > jmin at which the linear interpolation between jmin and j of any ratio (Cs, Sn and
+// DH = Cs^2 + Sn^2 of any direction and detector) misses its value at the mid-point by more than tl = max(tol ratio[j], tol),
+// ratio[j] = x / dS[j], or at which j - jmin exceeds djmax.  One cooperative launch over the chip: the
+// warps take (32 bins, kWalkRows ratios) pieces of the window [jmin + 1, jmin + djmax + 1], which holds the
+// next point, keep the first hit in one of three turns of *first (reset a step before its use), and meet at
+// the grid barrier once per point.  A step is bound by the latency of its loads (the ratios exceed L2), so a
+// piece is small enough for one warp to have all its loads in flight: 41 points in 375 us, 995 us with
+// eleven ratios one after another, 19.9 ms with one block testing 1024 bins at a time.  grid[0..*count) gets
+// the points (and m_grid, mapped host memory, the first m_cap of them); the walk stops at the cap
+// (*count = -1 then).
+constexpr int kWalkRows = 4, kWalkThreads = 1024;
+__global__ void __launch_bounds__(kWalkThreads) k_hs_walk(const double* __restrict__ Cs, const double* __restrict__ Sn,
+                                                 const double* __restrict__ dS,
+                                                 const HsLimits* __restrict__ lim, int per, int MN, int MM, int djmax,
+                                                 double tol, int cap, int* first, int* __restrict__ grid,
+                                                 int* __restrict__ m_grid, int m_cap, int* __restrict__ count) {
+  cooperative_groups::grid_group all = cooperative_groups::this_grid();
+  const int lane = threadIdx.x & 31, gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarp = (gridDim.x * blockDim.x) >> 5;
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  const size_t W = (size_t)(MM - MN);
+  const int nsl = (per + kWalkRows - 1) / kWalkRows;
+  const double x = lim->x;
+  int jmin = MN, nout = 0, turn = 0;
+  if (lead) {
+    first[0] = first[1] = first[2] = MM;
+    grid[0] = jmin;
+    if (m_cap > 0) m_grid[0] = jmin;
+  }
+  nout++;
+  all.sync();
+  for (;;) {
+    const int end = djmax < MM - jmin - 1 ? jmin + djmax + 2 : MM;      // bins [jmin + 1, end)
+    const int tasks = ((end - jmin - 1 + 31) / 32) * nsl;
+    volatile int* hit = first + turn;
+    for (int t = gw; t < tasks; t += nwarp) {
+      const int j0 = jmin + 1 + (t / nsl) * 32, j = j0 + lane, r0 = (t % nsl) * kWalkRows;
+      int known = lane == 0 ? *hit : 0;
+      known = __shfl_sync(0xffffffffu, known, 0);
+      if (known <= j0) break;                      // a later piece of this warp starts later still
+      bool flag = false;
+      if (j < end) {
+        const int jmid = (j + jmin) / 2;
+        double ca[kWalkRows], cb[kWalkRows], cm[kWalkRows], sa[kWalkRows], sb[kWalkRows], sm[kWalkRows];
+#pragma unroll
+        for (int q = 0; q < kWalkRows; q++) {      // the last piece repeats its last ratio
+          const size_t row = (size_t)min(r0 + q, per - 1) * W - MN;
+          ca[q] = Cs[row + jmin]; cb[q] = Cs[row + j]; cm[q] = Cs[row + jmid];
+          sa[q] = Sn[row + jmin]; sb[q] = Sn[row + j]; sm[q] = Sn[row + jmid];
+        }
+        const double d = dS[j] / x;
+        double tl = tol * (d > 0.0 && j > 0 ? 1.0 / d : 1.0);
+        if (tl < tol) tl = tol;
+        const double w0 = (double)(j - jmid), w1 = (double)(jmid - jmin), dw = (double)(j - jmin);
+        flag = j - jmin > djmax;
+#pragma unroll
+        for (int q = 0; q < kWalkRows; q++) {
+          const double da = ca[q] * ca[q] + sa[q] * sa[q], db = cb[q] * cb[q] + sb[q] * sb[q],
+                       dm = cm[q] * cm[q] + sm[q] * sm[q];
+          const double cmid = (ca[q] * w0 + cb[q] * w1) / dw;
+          const double smid = (sa[q] * w0 + sb[q] * w1) / dw;
+          const double dmid = (da * w0 + db * w1) / dw;
+          flag = flag || fabs(cm[q] - cmid) > tl || fabs(sm[q] - smid) > tl || fabs(dm - dmid) > tl;
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, flag);
+      if (m && lane == 0) atomicMin(first + turn, j0 + __ffs(m) - 1);
+    }
+    all.sync();
+    const int found = *hit;
+    const int prev = turn == 0 ? 2 : turn - 1;     // read by every block before this barrier
+    if (lead) first[prev] = MM;
+    turn = turn == 2 ? 0 : turn + 1;
     if (found >= MM) break;
     jmin = found;
     if (nout >= cap) {
-      if (threadIdx.x == 0) *count = -1;
+      if (lead) *count = -1;
       return;
     }
-    if (threadIdx.x == 0) grid[nout] = jmin;
+    if (lead) {
+      grid[nout] = jmin;
+      if (nout < m_cap) m_grid[nout] = jmin;
+    }
     nout++;
   }
-  if (threadIdx.x == 0) *count = nout;
+  if (lead) *count = nout;
 }
 
-void launch_hs_walk(const double* d_Cs, const double* d_Sn, const double* d_DH, const double* d_ratio, int per, int MN,
-                    int MM, int djmax, double tol, int cap, int* d_grid, int* d_count, cudaStream_t s) {
-  k_hs_walk<<<1, 1024, 0, s>>>(d_Cs, d_Sn, d_DH, d_ratio, per, MN, MM, djmax, tol, cap, d_grid, d_count);
+cudaError_t launch_hs_walk(const double* d_Cs, const double* d_Sn, const double* d_dS,
+                           const HsLimits* d_lim, int per, int MN, int MM, int djmax, double tol, int cap, int* d_first,
+                           int* d_grid, int* m_grid, int m_cap, int* m_count, cudaStream_t s) {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  void* args[] = {&d_Cs, &d_Sn, &d_dS, &d_lim, &per, &MN, &MM, &djmax, &tol, &cap, &d_first, &d_grid, &m_grid,
+                  &m_cap, &m_count};
+  return cudaLaunchCooperativeKernel((const void*)k_hs_walk, dim3((unsigned)sms), dim3(kWalkThreads), args, 0, s);
 }
 
 // The slow-term quadrature of the heterodyne summary for one detector and the regions

@@ -149,24 +149,36 @@ void launch_het_waves(const PhdRec* d_recs, int B, const NetGeom& g, const HetDa
 // fullphaseamp on any frequency list freq[0..M) for B records: amp/phase [B][nifo][M]
 void launch_waves(const PhdRec* d_recs, int B, const NetGeom& g, const double* d_freq, int M, double* d_amp,
                   double* d_phase, cudaStream_t s);
-// Fisher_All (QuickCBC.c:2695-2817) from the 23 wave sets per matrix (layout of launch_het_fisher) on n
-// bins, PSD rows S [nifo][sn_stride], bins [imin, imax): upper triangle of d_fish[nmat][11][11]
-void launch_fisher_full(const double* d_amp, const double* d_phase, int nmat, const NetGeom& g, int n,
-                        const double* d_S, int sn_stride, int imin, int imax, double eps, double* d_fish,
-                        cudaStream_t s);
-// diff (QuickCBC.c:4913-4964) of B wave sets against one reference wave set, bins [imin, m) of n,
-// as `chunks` partial sums per set: d_out[B][chunks] (sum them in order)
-void launch_diff_full(const double* d_amp_ref, const double* d_ph_ref, const double* d_amp, const double* d_ph, int B,
-                      const NetGeom& g, int n, int imin, int m, const double* d_S, int sn_stride, int chunks,
+// Fisher_All (QuickCBC.c:2695-2817) from 23 wave sets (layout of launch_het_fisher) on n bins, PSD rows
+// S [nifo][sn_stride] from the first of them: upper triangle of d_fish[11][11].  Scratch: d_terms of
+// 66 nifo n doubles, d_parts of 66 x 8.
+void launch_fisher_full(const double* d_amp, const double* d_phase, const NetGeom& g, int n, const double* d_S,
+                        int sn_stride, double eps, double* d_terms, double* d_parts, double* d_fish, cudaStream_t s);
+// diff (QuickCBC.c:4913-4964) of the waveforms of B records against one reference wave set [nifo][n], bins
+// [imin, m), as `chunks` partial sums per record: d_out[B][chunks] (sum them in order)
+void launch_wave_diff(const PhdRec* d_recs, int B, const NetGeom& g, const double* d_freq, const double* d_amp_ref,
+                      const double* d_ph_ref, int n, int imin, int m, const double* d_S, int sn_stride, int chunks,
                       double* d_out, cudaStream_t s);
-// het_space ratios Cs, Sn, DH (QuickCBC.c:4688-4702) of wave sets 1..nset-1 to set 0, bins [j0, j1),
-// bin-major [j1-j0][nset-1][nifo]
-void launch_hs_ratios(const double* d_amp, const double* d_ph, int nset, int nifo, int n, int j0, int j1,
-                      double* d_Cs, double* d_Sn, double* d_DH, cudaStream_t s);
-// het_space grid walk (QuickCBC.c:4720-4765) over the ratios (per = (nset-1) nifo values per bin) and
-// the per-bin tolerance scale ratio[j]: d_grid[0..*d_count) (count -1 when it would exceed cap)
-void launch_hs_walk(const double* d_Cs, const double* d_Sn, const double* d_DH, const double* d_ratio, int per, int MN,
-                    int MM, int djmax, double tol, int cap, int* d_grid, int* d_count, cudaStream_t s);
+// limits (QuickCBC.c:4275-4385): the signal band [MN, MM] of the reference waves d_amp [nifo][M] from
+// jmin = Tobs max(fmin, fbegin) on, and x, the average SNR^2 per significant bin; d_dS [M] receives the
+// SNR^2 per bin, d_bsum is scratch for ceil(M / 1024) doubles.  m_out: mapped host memory.
+struct HsLimits {
+  int jmin, MN, MM, pad;
+  double x;
+};
+void launch_hs_limits(const PhdRec* d_rec, const double* d_amp, int nifo, int M, const double* d_S, int sn_stride,
+                      double fmin, double Tobs, double* d_dS, double* d_bsum, HsLimits* d_out, HsLimits* m_out,
+                      cudaStream_t s);
+// het_space ratios Cs, Sn (QuickCBC.c:4688-4702) of the waveforms of nset records to the reference
+// waves [nifo][n], bins [j0, j1): rows [nset][nifo] of j1 - j0
+void launch_hs_ratios(const PhdRec* d_recs, int nset, const NetGeom& g, const double* d_freq, const double* d_amp_ref,
+                      const double* d_ph_ref, int n, int j0, int j1, double* d_Cs, double* d_Sn, cudaStream_t s);
+// het_space grid walk (QuickCBC.c:4720-4765) over the ratios (per = nset nifo rows) with the tolerance
+// scaled by x / d_dS[j]: d_grid[0..*m_count) (count -1 when it would exceed cap), its first m_cap entries
+// also in m_grid; d_first: three ints of scratch; m_grid, m_count: mapped host memory.  A cooperative launch.
+cudaError_t launch_hs_walk(const double* d_Cs, const double* d_Sn, const double* d_dS,
+                           const HsLimits* d_lim, int per, int MN, int MM, int djmax, double tol, int cap, int* d_first,
+                           int* d_grid, int* m_grid, int m_cap, int* m_count, cudaStream_t s);
 // het_diff (QuickCBC.c:4966-5051) for npair pairs of wave sets (2p, 2p+1) -> d_out[npair]
 void launch_het_diff(const double* d_amp, const double* d_phase, int npair, const NetGeom& g, const HetData& h,
                      double* d_out, cudaStream_t s);

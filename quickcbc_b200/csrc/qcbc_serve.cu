@@ -329,8 +329,12 @@ static int fisher_jumps(Run* r) {
   int rc = qcbc_het_fisher(r->ev, r->start, 1, &F[0][0]);
   if (rc != QCBC_OK) return rc;
   qcbc::fisher_evec_11(F, r->ejump, r->evec);
-  auto dist = [&](const double* px, double& z) -> int {
-    if (qcbc_het_diff(r->ev, r->start, px, 1, &z) != QCBC_OK || !(z == z)) z = 1.0e20;
+  auto dist = [&](const double* px, int n, double* z) -> int {
+    double start[11 * 11];
+    for (int k = 0; k < 11; k++) memcpy(start + 11 * k, r->start, sizeof(double) * 11);
+    const bool ok = qcbc_het_diff(r->ev, start, px, n, z) == QCBC_OK;
+    for (int k = 0; k < n; k++)
+      if (!ok || !(z[k] == z[k])) z[k] = 1.0e20;
     return 0;
   };
   return qcbc::efix_run(r->start, r->pmin, r->pmax, r->ejump, r->evec, 1.0, dist);
