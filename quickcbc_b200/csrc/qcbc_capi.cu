@@ -66,6 +66,7 @@ struct DeviceState {
   double2* d_tabD = nullptr;   // (1/i, i^{3/4})
   int tab_n = 0;
   int* d_bucket = nullptr;   // QNM interval index per 0.001 of final spin
+  double* d_cubic = nullptr; // QnmTable::cubic
 };
 static std::mutex g_mu;
 constexpr int kMaxDevices = 16;        // devices the library keeps state for (device ids 0..15)
@@ -124,9 +125,33 @@ static int upload_qnm(DeviceState& ds) {
   CU(cudaMemcpy(ds.d_bucket, bucket.data(), nb * sizeof(int), cudaMemcpyHostToDevice));
   bool uniform_ok = x.front() >= -1.0 && x.back() <= 1.0;
   for (int i = 1; i < n && uniform_ok; i++) uniform_ok = (x[i] - x[i - 1]) >= 0.999e-3;
+  // the same spline as a cubic per interval, the two that a bucket can meet in one row
+  std::vector<double> cubic((size_t)nb * kQnmRow);
+  for (int k = 0; k < nb; k++)
+    for (int t = 0; t < 2; t++) {
+      const int j = std::min(bucket[k] + t, n - 2);
+      const double h = x[j + 1] - x[j];
+      double* c = &cubic[(size_t)k * kQnmRow + 9 * t];
+      // no next interval: a start beyond any spin keeps the first
+      c[0] = t == 1 && bucket[k] + 1 > n - 2 ? 4.0 : x[j];
+      for (int y = 0; y < 2; y++) {
+        const std::vector<double>& f = g_qnm_host[1 + y];
+        const std::vector<double>& m2 = y == 0 ? mr : md;
+        double* d = c + 1 + 4 * y;
+        d[0] = f[j];
+        d[1] = (f[j + 1] - f[j]) / h - h * (2.0 * m2[j] + m2[j + 1]) / 6.0;
+        d[2] = 0.5 * m2[j];
+        d[3] = (m2[j + 1] - m2[j]) / (6.0 * h);
+      }
+    }
+  if (ds.d_cubic) cudaFree(ds.d_cubic);
+  CU(cudaMalloc(&ds.d_cubic, cubic.size() * sizeof(double)));
+  CU(cudaMemcpy(ds.d_cubic, cubic.data(), cubic.size() * sizeof(double), cudaMemcpyHostToDevice));
+  const double* fits = fits_table();
+  if (!fits) return fail(QCBC_ECUDA, "fit table has no device address");
   ds.n = n;
   ds.qnm = QnmTable{ds.d_qnm, ds.d_qnm + n, ds.d_qnm + 2 * n, ds.d_qnm + 3 * n, ds.d_qnm + 4 * n,
-                    uniform_ok ? ds.d_bucket : nullptr, n, nb};
+                    uniform_ok ? ds.d_bucket : nullptr, n, nb, uniform_ok ? ds.d_cubic : nullptr, fits};
   return QCBC_OK;
 }
 
@@ -355,6 +380,7 @@ static HetData het_data(const qcbc_event* ev) {
   d.tabA = ds.d_tabA;
   d.tabB = ds.d_tabB;
   d.tabC = ds.d_tabC;
+  d.tab_n = ds.tab_n;
   return d;
 }
 
@@ -571,7 +597,7 @@ static int enqueue_full(Workspace* w, qcbc_event* ev, const double* d_params, in
     if ((rc = grow(w->d_olist, w->c_olist, (size_t)kOrderClasses * B))) return rc;
     CU(cudaMemsetAsync(w->d_ocnt, 0, sizeof(int) * kOrderClasses, s));
     const SetOrder o{w->d_ocnt, w->d_olist};
-    launch_setup_ordered(d_params, B, g, ds.qnm, w->d_recs, w->d_status, o, s, model);
+    launch_setup_lnl(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, model, o);
     if (k0) cudaEventRecord(k0, s);
     launch_lnl_full_final(w->d_recs, w->d_status, B, g, ed, kp, L, w->d_part, d_lnl, d_rho, model, &o, s);
     if (k1) cudaEventRecord(k1, s);
@@ -583,7 +609,7 @@ static int enqueue_full(Workspace* w, qcbc_event* ev, const double* d_params, in
     const size_t had = w->c_done;
     if ((rc = grow(w->d_done, w->c_done, (size_t)B))) return rc;
     if (w->c_done != had) CU(cudaMemsetAsync(w->d_done, 0, sizeof(int) * w->c_done, s));
-    launch_setup(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, model);
+    launch_setup_lnl(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, model);
     if (k0) cudaEventRecord(k0, s);
     launch_lnl_full_final(w->d_recs, w->d_status, B, g, ed, kp, L, w->d_part, d_lnl, d_rho, model, nullptr, s,
                           w->d_done);
@@ -784,7 +810,7 @@ static int het_setup_queue(qcbc_event* ev, Workspace* w, const double* pref, con
   q.SL = (double*)hd.SL; q.lc = (double*)hd.lc; q.ls = (double*)hd.ls;
   q.aa = (double*)hd.aa; q.rc = (double*)hd.rc; q.rs = (double*)hd.rs;
   q.logLb = w->m_lnl;
-  launch_setup(w->m_params, 1, ev->g, ds.qnm, w->d_recs, w->d_status, s);
+  launch_setup_lnl(w->m_params, 1, ev->g, ds.qnm, w->d_recs, w->d_status, s);
   launch_het_tables(w->d_recs, ev->g, q, max_region, s);
   tls_launches += 4;
   CU(cudaGetLastError());
@@ -823,20 +849,18 @@ static int enqueue_het(Workspace* w, qcbc_event* ev, const double* d_params, int
   if ((rc = grow(w->d_status, w->c_status, (size_t)B))) return rc;
   DeviceState& ds = g_dev[current_device()];
   const HetData hd = het_data(ev);
-  // the setup's threads pull the heterodyne tables (and, for the mixed form, the bin tables at the
-  // grid's bins) into L2 for the heterodyned launch
+  // the setup's threads pull the heterodyne tables and the bin tables at the grid's bins into L2 for
+  // the heterodyned launch
   SetupPrefetch pf;
   pf.buf = ev->het.buf;
   pf.bytes = het_doubles(ev->g.nifo, ev->het.M, ev->het.J) * sizeof(double);
-  if (prec == QCBC_MIXED) {
-    pf.bins = ev->het.d_fgrid;
-    pf.nbins = ev->het.M;
-    pf.tabA = hd.tabA;
-    pf.tabB = hd.tabB;
-    pf.tabC = hd.tabC;
-    pf.tab_n = g_dev[ev->device].tab_n;
-  }
-  launch_setup(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, kModelFull, pf);
+  pf.bins = ev->het.d_fgrid;
+  pf.nbins = ev->het.M;
+  pf.tabA = hd.tabA;
+  pf.tabB = hd.tabB;
+  pf.tabC = prec == QCBC_MIXED ? hd.tabC : nullptr;
+  pf.tab_n = hd.tab_n;
+  launch_setup_lnl(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, kModelFull, SetOrder{nullptr, nullptr}, pf);
   launch_lnl_het(w->d_recs, w->d_status, B, g, hd, prec == QCBC_MIXED ? kMixed : kFP64, d_lnl, s);
   tls_launches += 2;
   CU(cudaGetLastError());
@@ -2454,7 +2478,7 @@ extern "C" int qcbc_lnl_full_noalloc(qcbc_event* ev, const double* d_params, int
   cudaStream_t s = (cudaStream_t)stream;
   DeviceState& ds = g_dev[dev];
   EventData ed = event_data(ev);
-  launch_setup(d_params, B, ev->g, ds.qnm, recs, status, s);
+  launch_setup_lnl(d_params, B, ev->g, ds.qnm, recs, status, s);
   launch_lnl_full(recs, B, ev->g, ed, precision == QCBC_MIXED ? kMixed : kFP64, L, part, s);
   launch_finalize_full(part, recs, status, B, L.tiles, ev->g, ed, d_lnl, d_rho, s);
   tls_launches += 3;

@@ -115,7 +115,16 @@ enum FitId { F_RHO1, F_RHO2, F_RHO3, F_GAM1, F_GAM2, F_GAM3, F_V2, F_AL1, F_AL2,
 // x[n], fring[n], fring''[n], fdamp[n], fdamp''[n]
 // bucket[k] = index of the interval holding spin -1 + k/1000 (k = 0..2000), so one or two
 // comparisons find the interval instead of a binary search over the table.
-struct QnmTable { const double *x, *yr, *mr, *yd, *md; const int* bucket; int n, nbucket; };
+// cubic[k]: kQnmRow doubles for bucket k, the interval at its lower end and the next one, each as (x, fring as
+// a cubic in s - x, fdamp as a cubic): one load level finds and evaluates the spline.  Null, as bucket, when
+// the table's spacing is below 0.001.  fits: Table V's coefficients [F_COUNT][11] in global memory.
+constexpr int kQnmRow = 18;
+struct QnmTable {
+  const double *x, *yr, *mr, *yd, *md;
+  const int* bucket;
+  int n, nbucket;
+  const double *cubic, *fits;
+};
 
 struct Pow6 { double sixth, third, two_thirds, four_thirds, five_thirds, two, seven_thirds, eight_thirds; };
 

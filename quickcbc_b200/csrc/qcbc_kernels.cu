@@ -81,6 +81,10 @@ struct SetupConst {
   double vj[9];        // v^k at v = cbrt(pi * 0.018), k = 0..8
   double logvj;        // log v there
   double log_fj;       // log 0.018
+  // reciprocals and quotients of the above that the likelihood setup multiplies by
+  double r_pi_third, r_pi_two_thirds, r_pi_five_thirds, a0;    // a0 = sqrt(2/3) / pi^{1/6}
+  double r_fj_third;   // 0.018^{-1/3}
+  double dj_scale, dj_s2, dj_s3, dj_s4;                        // of the inspiral phase's slope at the join
 };
 __constant__ SetupConst c_setup;
 
@@ -107,8 +111,22 @@ void upload_tables() {
   for (int k = 1; k < 9; k++) h.vj[k] = v * h.vj[k - 1];
   h.logvj = std::log(v);
   h.log_fj = std::log(kPhiJoin);
+  h.r_pi_third = 1.0 / h.pi6.third;
+  h.r_pi_two_thirds = 1.0 / h.pi6.two_thirds;
+  h.r_pi_five_thirds = 1.0 / h.pi6.five_thirds;
+  h.a0 = std::sqrt(2.0 / 3.0) / h.pi6.sixth;
+  h.r_fj_third = 1.0 / h.fjp.third;
+  h.dj_scale = kPi / (3.0 * h.vj[8]);
+  h.dj_s2 = h.vj[1] / h.pi6.third;
+  h.dj_s3 = h.vj[2] / h.pi6.two_thirds;
+  h.dj_s4 = h.vj[3] / kPi;
   cudaMemcpyToSymbol(c_setup, &h, sizeof(h));
 }   // tables are statically initialised __constant__ data
+
+const double* fits_table() {
+  void* p = nullptr;
+  return cudaGetSymbolAddress(&p, c_fits) == cudaSuccess ? static_cast<const double*>(p) : nullptr;
+}
 
 // ---------------------------------------------------------------- setup
 // The 39 antenna monomials for one sky position / polarisation (straight-line code).
@@ -374,11 +392,11 @@ __device__ __forceinline__ double phd_fmax(const PhdRec& c) {
 
 // Intermediate amplitude: quartic with value and slope at f1, value at f2, value and slope at
 // f3 (eqs. 21-26 of arXiv:1508.07253), kept in Newton form on nodes f1,f1,f2,f3,f3.
-__device__ __forceinline__ void phd_amp_int(PhdRec& c, double v2) {
+// v3: amp_mrd at fmax.
+__device__ __forceinline__ void phd_amp_int_v3(PhdRec& c, double v2, double v3) {
   double f1 = kAmpJoin, f3 = c.fmax, f2 = f1 + (f3 - f1) / 2.0;
   const Pow6 p1 = c_setup.f1p;
   double v1 = amp_ins(c, f1, p1), d1 = damp_ins_p(c, f1, p1);
-  double v3 = amp_mrd<MO>(c, f3);
   double fg3 = c.fDM * c.g3, df3 = f3 - c.fRD;
   double d2 = v3 * (-c.g2 / fg3 - 2.0 * df3 / (df3 * df3 + fg3 * fg3));
   double q01 = d1, q12 = (v2 - v1) / (f2 - f1), q23 = (v3 - v2) / (f3 - f2), q34 = d2;
@@ -387,6 +405,8 @@ __device__ __forceinline__ void phd_amp_int(PhdRec& c, double v2) {
   c.hx1 = f1; c.hx2 = f2; c.hx3 = f3;
   c.hc[0] = v1; c.hc[1] = q01; c.hc[2] = q012; c.hc[3] = q0123; c.hc[4] = (q1234 - q0123) / (f3 - f1);
 }
+
+__device__ __forceinline__ void phd_amp_int(PhdRec& c, double v2) { phd_amp_int_v3(c, v2, amp_mrd<MO>(c, c.fmax)); }
 
 // C^1 join inspiral -> intermediate at Mf = 0.018 (IMRPhenomD_internals.c:1547-1566).
 __device__ __forceinline__ void phd_join_int(PhdRec& c, const double* pv, const double* pvl, const double* s) {
@@ -477,6 +497,7 @@ __device__ __forceinline__ FbeginHead fbegin_head(const double* p) {
   h.th = MO::pow(eta * p[5] / (5.0 * M), -1.0 / 8.0);
   return h;
 }
+template <class F = MO>
 __device__ __forceinline__ double fbegin_tail(const FbeginHead& h, double c1, double c2) {
   const double gE = 0.5772156649;
   double M = h.M, eta = h.eta, chi = h.chi, th = h.th;
@@ -488,7 +509,7 @@ __device__ __forceinline__ double fbegin_tail(const FbeginHead& h, double c1, do
   double PN25 = -(7729.0 / 21504.0 - 13.0 / 256.0 * eta) * kPi * t5;
   double PN3 = (-720817631400877.0 / 288412611379200.0 + 53.0 / 200.0 * kPi * kPi + 107.0 / 280.0 * gE +
                 (25302017977.0 / 4161798144.0 - 451.0 / 2048.0 * kPi * kPi) * eta - 30913.0 / 1835008.0 * eta * eta +
-                235925.0 / 1769472.0 * eta * eta * eta + 107.0 / 280.0 * MO::log(2.0 * th)) * t6;
+                235925.0 / 1769472.0 * eta * eta * eta + 107.0 / 280.0 * F::log(2.0 * th)) * t6;
   return t3 / (8.0 * M * kPi) * (1.0 + PN1 + PN15 + PN2 + PN25 + PN3);
 }
 
@@ -589,17 +610,6 @@ __device__ __forceinline__ int last_bin_below(const NetGeom& g, double fCut) {
   return hi;
 }
 
-// Scales of Mf = (Msec df) i for the per-bin tables of the mixed kernel.
-__device__ __forceinline__ void set_mdf(PhdRec& c, const NetGeom& g) {
-  c.mdf = c.Msec * g.df;
-  c.mdf_third = MO::cbrt(c.mdf);
-  c.mdf_rthird = 1.0 / c.mdf_third;
-  c.mdf_log = MO::log(c.mdf);
-  double sixth = sqrt(c.mdf_third), sq = sqrt(c.mdf);
-  c.mdf_m76 = 1.0 / (c.mdf * sixth);
-  c.mdf_34 = sqrt(c.mdf * sq);
-}
-
 // ---- coefficients of the mixed-precision kernel (MixPoly), from the finished FP64 record
 constexpr double kInv2PiD = 0.15915494309189533577;
 constexpr double kLnPi = 1.1447298858494002;
@@ -621,8 +631,8 @@ __device__ __forceinline__ void split_f2(double v, float (&p)[2]) {
 }
 
 // inspiral phase but its constant, and the intermediate / ringdown pieces but the parts that
-// need the ringdown join (needs pq, alpha/beta, the intermediate join, t0, the mdf scales)
-__device__ __forceinline__ void mix_phase_main(PhdRec& c) {
+// need the ringdown join (needs pq, alpha/beta, the intermediate join, t0, the mdf scales); rdm = 1 / fDM
+__device__ __forceinline__ void mix_phase_main(PhdRec& c, double rdm) {
   MixPoly& P = c.mix;
   const double* q = c.pq;
   const double K = kInv2PiD, T = c.mdf_third, U = c.mdf_rthird, m = c.mdf, ie = c.inv_eta;
@@ -646,7 +656,6 @@ __device__ __forceinline__ void mix_phase_main(PhdRec& c) {
   split_f2(K * (-c.al2 * U3 * ie), P.pmrd.Ru3);
   split_f2(K * ((4.0 / 3.0) * c.al3 * c.mdf_34 * ie), P.pmrd.Rs);
   split_f2(K * (c.al4 * ie), P.pmrd.Rat);
-  const double rdm = 1.0 / c.fDM;
   split_f2(m * rdm, P.pmrd.D1);
   split_f2(c.al5 * c.fRD * rdm, P.pmrd.D0);
 }
@@ -669,8 +678,8 @@ __device__ __forceinline__ void mix_phase_slopes(PhdRec& c) {
   c.mix.pint.Bi -= c.mix.pmrd.Ri;
 }
 
-// FP32 amplitude coefficients (needs ai, the intermediate Newton form, g1..g3, fDM)
-__device__ __forceinline__ void mix_amp(PhdRec& c) {
+// FP32 amplitude coefficients (needs ai, the intermediate Newton form, g1..g3, fDM); rfg = 1 / (fDM g3)
+__device__ __forceinline__ void mix_amp(PhdRec& c, double rfg) {
   MixPoly& P = c.mix;
   const double T = c.mdf_third, m = c.mdf, T2 = T * T, m2 = m * m;
   float* al = P.ains.al;
@@ -690,25 +699,22 @@ __device__ __forceinline__ void mix_amp(PhdRec& c) {
   const double fg = c.fDM * c.g3;
   split_f2(m, P.amrd.m);
   split_f2(c.fRD, P.amrd.fRD);
-  P.amrd.g2_over_fg = (float)(c.g2 / fg);
+  P.amrd.g2_over_fg = (float)(c.g2 * rfg);
   P.amrd.fg_g1 = (float)(fg * c.g1);
   P.amrd.fg2 = (float)(fg * fg);
 }
 
-// ---- cooperative setup: a block of 4 warps builds the records of 32 parameter sets, lane l
+// ---- setup of the waveform outputs: a block of 4 warps builds the records of 32 parameter sets, lane l
 // of every warp working on set l.  Each warp takes a different independent piece of the
 // record in each of four phases, so the dependency chain of one record is about a third of
 // the serial one and the lanes of a warp still run the same code:
 //   phase 1  w0 masses/scales        w1 fbegin head, ts      w2 projection, det 0-1   w3 projection, det 2
 //                                                            (or detector offsets)
-//   phase 2  w0 fRD, fDM             w1 fits, fbegin tail    w2 a0, ai[0..4], mdf, hi w3 TaylorF2, MfRef
-//   phase 3  w0 fmax, intermediate,  w1 join int, phi(fRef)  w2 MRD join pieces       w3 t0, bin iP
-//            bin iA
-//   phase 4  w0 MRD join, phi_pre,   w1 mixed-kernel phase,   w2 mixed-kernel          w3 first bin lo
-//            mixed-kernel constants      bin iM                  amplitude, bin iF
-// Each piece runs in the first phase whose inputs exist, spread so that the longest warp of each
-// phase is as short as the dependencies allow (measured per warp with clock64: the four phases'
-// longest pieces went from 7.1k + 11.5k + 7.1k + 7.5k to 6.2k + 8.0k + 7.6k + 4.3k cycles).
+//   phase 2  w0 fRD, fDM             w1 fits, fbegin tail    w2 a0, ai[0..4]          w3 TaylorF2, MfRef
+//   phase 3  w0 fmax, intermediate   w1 join int, phi(fRef)  w2 MRD join pieces       w3 t0
+//   phase 4  w0 MRD join, phi_pre
+// (The likelihood launches have their own setup below.  This one keeps its arithmetic: the grid search's
+// Fisher matrix differences these waveforms, and its null directions follow their last bits.)
 struct SetupScratch {
   double p[kMaxParams];
   PhdMass m;
@@ -716,7 +722,7 @@ struct SetupScratch {
   double v2, s[4], pv[8], pvl[8];
   MrdJoin mj;
   double phr_raw;
-  int phr_branch, st, hi, live;
+  int phr_branch, st, live;
 };
 
 constexpr int kSetupSets = 32;
@@ -748,12 +754,10 @@ __device__ __forceinline__ int length_class(int bins, int band) {
   return min(kOrderClasses - 1, __float2int_rz((float)bins * ((float)kOrderClasses / (float)max(band, 1))));
 }
 
-// ocnt / olist non-null: each set is filed under its length class (SetOrder)
 template <class Geom>
 __device__ __forceinline__ void setup_coop_block(const double* __restrict__ params, int B, const Geom& geo,
-                                                 const QnmTable& q, int tile_bins, PhdRec* __restrict__ recs,
-                                                 int* __restrict__ status, int* __restrict__ ntile, int model,
-                                                 int* __restrict__ ocnt = nullptr, int* __restrict__ olist = nullptr) {
+                                                 const QnmTable& q, PhdRec* __restrict__ recs,
+                                                 int* __restrict__ status, int model) {
   __shared__ __align__(16) PhdRec s_rec[kSetupSets];
   __shared__ SetupScratch s_x[kSetupSets];
   __shared__ NetGeom s_g[kSetupSets];
@@ -810,7 +814,6 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
   __syncthreads();
   // phase 2
   if (on) {
-    const NetGeom& g = s_g[lane];
     if (w == 0) {
       x.st = x.m.st | phd_ringdown(c, x.m, q);
     } else if (w == 1) {
@@ -818,8 +821,6 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
       c.fs = fbegin_tail(x.fb, x.p[2], x.p[3]);
     } else if (w == 2) {
       phd_amp_prefactors(c, x.m);
-      set_mdf(c, g);
-      x.hi = last_bin_below(g, c.fCut);
     } else {
       phd_taylorf2(c, x.m, x.pv, x.pvl);
       c.MfRef = c.Msec * kFref;
@@ -831,7 +832,6 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
     if (w == 0) {
       c.fmax = phd_fmax(c);
       phd_amp_int(c, x.v2);
-      c.mix.iA = first_bin_mf_at_least(s_g[lane], c.Msec, kAmpJoin);
     } else if (w == 1) {
       phd_pq_sigma(c, x.s);
       phd_join_int(c, x.pv, x.pvl, x.s);
@@ -840,65 +840,469 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
       x.mj = phd_mrd_pieces(c);
     } else {
       c.t0 = dphi_mrd<MO>(c, phd_fmax(c));
-      c.mix.iP = first_bin_mf_at_least(s_g[lane], c.Msec, kPhiJoin);
     }
   }
   __syncthreads();
   // phase 4
-  if (on && w != 0) {
-    if (w == 1) {
-      mix_phase_main(c);
-      c.mix.iM = first_bin_mf_at_least(s_g[lane], c.Msec, 0.5 * c.fRD);
-    } else if (w == 2) {
-      mix_amp(c);
-      c.mix.iF = first_bin_mf_at_least(s_g[lane], c.Msec, c.fmax);
-    } else {
-      c.i_lo = first_bin_above(s_g[lane], c.fs);
-    }
-  }
   if (w == 0 && lane < nb) {
     int st;
     if (on) {
       phd_join_mrd(c, x.mj);
       phd_phi_ref(c, model == kModelIntrinsic ? x.p[4] : 0.5 * x.p[4], x.phr_raw, x.phr_branch);
-      mix_phase_join(c);
       st = x.st;
       c.flags = (st == kStOK) ? kRecValid : 0;
-      c.i_hi = x.hi;
       c.event = s_ev[lane];
     } else {
       st = kStNoEvent;
       c.flags = 0;
       c.event = -1;
-      c.i_lo = 1;
-      c.i_hi = 0;
     }
     status[b] = st;
   }
-  __syncthreads();
-  if (ntile && w == 0 && lane < nb) {  // needs i_lo from warp 3
-    const int bins = (c.flags & kRecValid) ? c.i_hi - c.i_lo + 1 : 0;
-    ntile[b] = bins > 0 ? (bins + tile_bins - 1) / tile_bins : 0;
-  }
-  if (ocnt && w == 0) {                // all lanes of warp 0: one global atomic per class present
-    int cl = -1;
-    if (lane < nb) cl = length_class((c.flags & kRecValid) ? max(0, c.i_hi - c.i_lo + 1) : 0,
-                                     s_g[lane].imax - s_g[lane].imin);
-    const unsigned peers = __match_any_sync(0xffffffffu, cl);
-    const int leader = __ffs(peers) - 1;
-    int first = 0;
-    if (lane == leader && cl >= 0) first = atomicAdd(ocnt + cl, __popc(peers));
-    first = __shfl_sync(0xffffffffu, first, leader);
-    const int r = first + __popc(peers & ((1u << lane) - 1u));
-    if (cl >= 0 && r < B) olist[(size_t)cl * B + r] = b;   // r >= B only if the counts were not cleared
-  }
-  if (on && w == 1) mix_phase_slopes(c);   // needs Ri from warp 0
   __syncthreads();
   // the block's records are contiguous in shared and in global memory
   const int4* src = reinterpret_cast<const int4*>(s_rec);
   int4* dst = reinterpret_cast<int4*>(recs + b0);
   const int words = nb * (int)(sizeof(PhdRec) / 16);
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+}
+
+// ---- setup of the likelihood launches: 8 lanes per parameter set, four warps per four sets.
+// What bounds a setup is one set's chain of dependent FP64 work, not throughput.  So the lanes of a group
+// share every expensive function: one exp, log, cbrt, atan, sqrt or quotient per step serves up to eight
+// arguments side by side (the values meet by shuffle), the fits take a lane each, and everything else is
+// evaluated by all lanes of the group alike; quotients of ordinary numbers (but the masses') are a reciprocal
+// approximation with one third-order step, a quarter of the division's latency; and the warps take
+// independent pieces:
+//           until the first barrier                                  until the second
+//   warp 0  masses, final spin, QNM (one row per 0.001 of spin       joins, phase at fRef, folded phase
+//           holds both cubics it can need), alpha/beta/gamma fits,
+//           the pieces' functions at fRD/2, fmax, MfRef, Msec df
+//   warp 1  antenna response and delays (lane d: F+ of detector d,   -
+//           lane 3 + d: Fx), fbegin and the first bin
+//   warp 2  masses, rho/sigma/v2 fits, amplitude prefactors,         intermediate amplitude, folded
+//           TaylorF2                                                 amplitude
+//   warp 3  masses, fCut, amplitude scale, last bin                  first bins of the pieces
+// One set read from mapped host memory is ready 6.3 us after the kernel starts (2.2 us of it the read), where
+// four warps with a set per lane and out-of-line functions took about 20 us; a one-set heterodyned call went
+// from 38.0 to 25.4 us and the 4096-set launch sequence from 46.3 to 34.8 us with it and the kernels below.
+struct SetupVals {
+  double p[kMaxParams], v[F_COUNT], pv[8], pvl[8];
+  NetGeom g;
+  MrdJoin mj;
+  double phr, tref, rref, v3, rdm, rfg;
+  int br, ev, live, lo, hi, st;
+};
+constexpr int kLnlSets = 4, kLnlLanes = 8, kLnlThreads = 128;
+
+__device__ __forceinline__ double lane_of(double v, int src) { return __shfl_sync(0xffffffffu, v, src, kLnlLanes); }
+
+// 1/x for finite normal x: the hardware's approximation (about 2^-20) and one third-order step
+__device__ __forceinline__ double recip64(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// masses (Msun) and what follows from them, rounded as set_phys and phd_masses round them: the mixed kernel
+// rounds its coefficients and rotations to floats, so a last bit here can move a rotation by a float's.
+// exp of ln Mc, ln Mt and ln D side by side, then both masses in one division.  st: validity bits
+struct SetMass { double M, m1, m2, chi1, chi2, eta, Seta, chi, dist; int st; };
+__device__ __forceinline__ SetMass set_masses(const double* p, int l) {
+  SetMass m;
+  const double ex = exp(l == 0 ? p[0] : l == 1 ? p[1] : p[6]), mt = lane_of(ex, 1);
+  m.dist = lane_of(ex, 2);
+  const double eta0 = pow(lane_of(ex, 0) / mt, 5.0 / 3.0);
+  const double dm = eta0 > 0.25 ? 0.0 : sqrt(1.0 - 4.0 * eta0);
+  const double mq = (l == 0 ? mt * (1.0 + dm) / 2.0 : mt * (1.0 - dm) / 2.0) / kMsun;
+  const double a = lane_of(mq, 0), b = lane_of(mq, 1);
+  m.st = kStOK;
+  if (!(a > 0.0) || !(b > 0.0)) m.st |= kStBadMass;
+  if (!(m.dist > 0.0)) m.st |= kStBadDist;
+  if (!(p[2] <= 1.0 && p[2] >= -1.0 && p[3] <= 1.0 && p[3] >= -1.0)) m.st |= kStBadSpin;
+  const bool swap = !(a > b);
+  m.m1 = swap ? b : a; m.m2 = swap ? a : b;
+  m.chi1 = swap ? p[3] : p[2]; m.chi2 = swap ? p[2] : p[3];
+  m.M = m.m1 + m.m2;
+  m.eta = m.m1 * m.m2 / (m.M * m.M);
+  m.Seta = sqrt(1.0 - 4.0 * m.eta);
+  m.chi = (m.chi1 + m.chi2) / 2.0 * (1.0 - m.eta * 76.0 / 113.0) + m.Seta * ((m.chi1 - m.chi2) / 2.0);
+  return m;
+}
+
+// fit k of Table V at (eta, chi) from the block's copy of the coefficients
+__device__ __forceinline__ double fit_lane(const double* s_fits, int k, double eta, double chi) {
+  const double* t = s_fits + 11 * k;
+  const double xi = -1 + chi, xi2 = xi * xi, xi3 = xi2 * xi, e2 = eta * eta;
+  return t[0] + t[1] * eta + (t[2] + t[3] * eta + t[4] * e2) * xi + (t[5] + t[6] * eta + t[7] * e2) * xi2 +
+         (t[8] + t[9] * eta + t[10] * e2) * xi3;
+}
+
+// phi_ins at f with t = f^{1/3}, rt = 1/t and log v given
+__device__ __forceinline__ double phi_ins_roots(const PhdRec& c, double f, double t, double rt, double logv) {
+  const double* q = c.pq;
+  const double t2 = t * t, r2 = rt * rt, r3 = r2 * rt;
+  return q[0] + q[1] * t2 + (q[2] + q[3] * logv) * t + q[4] * logv + q[5] * rt + q[6] * r2 + q[7] * r3 +
+         q[8] * (r3 * r2) + f * (q[9] + q[10] * t + q[11] * t2 + q[12] * f) * c.inv_eta;
+}
+
+// warp 0 until the first barrier
+__device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const double* s_fits, const QnmTable& q, int l) {
+  const SetMass m = set_masses(x.p, l);
+  const double eta = m.eta, e2 = eta * eta, e3 = e2 * eta, e4 = e3 * eta;
+  // final spin and radiated energy (eqs. 3.6-3.8 of arXiv:1508.07250); the latter as a quotient er = N / D
+  const double a1 = 0.5 * (1.0 + m.Seta), a2 = 0.5 * (1.0 - m.Seta), a1s = a1 * a1, a2s = a2 * a2;
+  const double sp = a1s * m.chi1 + a2s * m.chi2, s2 = sp * sp, s3 = s2 * sp, s4 = s3 * sp, aq = a1s + a2s;
+  double fsp = 3.4641016151377544 * eta - 4.399247300629289 * e2 + 9.397292189321194 * e3 - 13.180949901606242 * e4 +
+               (1 - 0.0850917821418767 * eta - 5.837029316602263 * e2) * sp +
+               (0.1014665242971878 * eta - 2.0967746996832157 * e2) * s2 +
+               (-1.3546806617824356 * eta + 4.108962025369336 * e2) * s3 +
+               (-0.8676969352555539 * eta + 2.064046835273906 * e2) * s4;
+  int st = m.st;
+  if (!(fsp <= 1.0)) { st |= kStBadSpinFinal; fsp = 1.0; }
+  if (!(fsp >= -1.0)) fsp = -1.0;
+  x.st = st;
+  double yr, yd;                                   // fring, fdamp at the final spin
+  if (q.cubic) {
+    int k = (int)floor((fsp + 1.0) * 1000.0);
+    k = k < 0 ? 0 : (k >= q.nbucket ? q.nbucket - 1 : k);
+    const double2* t = reinterpret_cast<const double2*>(q.cubic + (size_t)k * kQnmRow);
+    double2 w[kQnmRow / 2];
+#pragma unroll
+    for (int i = 0; i < kQnmRow / 2; i++) w[i] = __ldg(t + i);
+    // (x, fring cubic, fdamp cubic) of the bucket's interval, then of the next
+    const bool nx = fsp >= w[4].y;
+    const double h = fsp - (nx ? w[4].y : w[0].x);
+    yr = (nx ? w[5].x : w[0].y) + h * ((nx ? w[5].y : w[1].x) + h * ((nx ? w[6].x : w[1].y) + h * (nx ? w[6].y : w[2].x)));
+    yd = (nx ? w[7].x : w[2].y) + h * ((nx ? w[7].y : w[3].x) + h * ((nx ? w[8].x : w[3].y) + h * (nx ? w[8].y : w[4].x)));
+  } else {
+    const int qi = qnm_interval(q, fsp);
+    yr = qnm_eval_at(q, q.yr, q.mr, qi, fsp);
+    yd = qnm_eval_at(q, q.yd, q.md, qi, fsp);
+  }
+  const double N = (0.055974469826360077 * eta + 0.5809510763115132 * e2 - 0.9606726679372312 * e3 + 3.352411249771192 * e4) *
+                   (aq + (-0.0030302335878845507 - 2.0066110851351073 * eta + 7.7050567802399215 * e2) * sp);
+  const double D = aq + (-0.6714403054720589 - 1.4756929437702908 * eta + 7.304676214885011 * e2) * sp;
+  // gamma_1..3, alpha_1..5 by lane, then beta_1..3
+  static_assert(F_GAM2 == F_GAM1 + 1 && F_GAM3 == F_GAM1 + 2 && F_AL5 == F_AL1 + 4 && F_BE3 == F_BE1 + 2, "lane order");
+  const double fa = fit_lane(s_fits, l < 3 ? F_GAM1 + l : F_AL1 + l - 3, eta, m.chi);
+  const double fb = fit_lane(s_fits, F_BE1 + (l < 3 ? l : 0), eta, m.chi);
+  const double g1 = lane_of(fa, 0), g2 = lane_of(fa, 1), g3 = lane_of(fa, 2);
+  const double al1 = lane_of(fa, 3), al2 = lane_of(fa, 4), al3 = lane_of(fa, 5), al4 = lane_of(fa, 6), al5 = lane_of(fa, 7);
+  const double b1 = lane_of(fb, 0), b2 = lane_of(fb, 1), b3 = lane_of(fb, 2);
+  const double rq = recip64(l == 0 ? eta : l == 1 ? g2 : D - N);
+  const double inv_eta = lane_of(rq, 0), re = D * lane_of(rq, 2), fRD = yr * re, fDM = yd * re, fg = fDM * g3;
+  const double root = g2 <= 1 ? sqrt(1 - g2 * g2) : 0.0;
+  const double fmax = fabs(fRD + fg * (root - 1.0) * lane_of(rq, 1));
+  const double Msec = m.M * kMtsun, mdf = Msec * x.g.df, MfRef = Msec * kFref, fm = 0.5 * fRD, dx = fmax - fRD;
+  // the functions at four frequencies side by side: lane 0 fRD/2, 1 fmax, 2 MfRef, 3 Msec df
+  const double f = l == 0 ? fm : l == 1 ? fmax : l == 2 ? MfRef : mdf, xr = f - al5 * fRD;
+  const double rr = recip64(l == 0 ? fDM : l == 1 ? fg : dx * dx + fg * fg);
+  const double rdm = lane_of(rr, 0), rfg = lane_of(rr, 1);
+  const double L = log(f), C = cbrt(f), sq = sqrt(f), f34 = sqrt(f * sq), at = atan(xr * rdm);
+  const double v3 = exp(-dx * g2 * rfg) * (fg * g1) * lane_of(rr, 2);
+  const double d3 = recip64(f), r2 = d3 * d3, rx = recip64(fDM * fDM + xr * xr);
+  const double pint = b1 * f - b3 * (1.0 / 3.0) * (r2 * d3) + b2 * L;
+  const double dpint = (b1 + b3 * (r2 * r2) + b2 * d3) * inv_eta;
+  const double pmrd = -(al2 * d3) + (4.0 / 3.0) * (al3 * f34) + al1 * f + al4 * at;
+  const double dpmrd = (al1 + al2 * r2 + al3 * (f34 * d3) + al4 * fDM * rx) * inv_eta;
+  c.eta = eta; c.inv_eta = inv_eta;
+  c.Msec = Msec; c.MfRef = MfRef; c.mdf = mdf;
+  c.fRD = fRD; c.fDM = fDM; c.fmax = fmax; c.fMRDJoin = fm;
+  c.g1 = g1; c.g2 = g2; c.g3 = g3;
+  c.b1 = b1; c.b2 = b2; c.b3 = b3;
+  c.al1 = al1; c.al2 = al2; c.al3 = al3; c.al4 = al4; c.al5 = al5;
+  c.pi_third = c_setup.pi6.third;
+  x.v3 = v3;
+  x.rdm = rdm;
+  x.rfg = rfg;
+  x.mj.phi_int = lane_of(pint, 0);
+  x.mj.dphi_int = lane_of(dpint, 0);
+  x.mj.phi_mrd = lane_of(pmrd, 0);
+  x.mj.dphi_mrd = lane_of(dpmrd, 0);
+  c.t0 = lane_of(dpmrd, 1);
+  // the phase at MfRef: the ringdown's or intermediate piece's value; the inspiral's needs TaylorF2, so its
+  // arguments (cube root and logarithm of MfRef) go on
+  x.br = MfRef < kPhiJoin ? 0 : (MfRef >= fm ? 1 : 2);
+  x.phr = lane_of(x.br == 0 ? L : x.br == 1 ? pmrd : pint, 2);
+  x.tref = lane_of(C, 2);
+  x.rref = lane_of(d3, 2);
+  // scales of Mf = (Msec df) i
+  const double T = lane_of(C, 3), r4 = recip64(l == 0 ? T : mdf * sqrt(T));
+  c.mdf_third = T;
+  c.mdf_log = lane_of(L, 3);
+  c.mdf_34 = lane_of(f34, 3);
+  c.mdf_rthird = lane_of(r4, 0);
+  c.mdf_m76 = lane_of(r4, 1);
+}
+
+// warp 0 until the second barrier: C^1 joins (IMRPhenomD_internals.c:1547-1584), phase at fRef, folded phase
+__device__ __forceinline__ void setup_joins(PhdRec& c, SetupVals& x, int model) {
+  const double* v = c_setup.vj;
+  const double *pv = x.pv, *pvl = x.pvl, ie = c.inv_eta, fj = kPhiJoin;
+  const double s1 = x.v[F_SI1], s2 = x.v[F_SI2], s3 = x.v[F_SI3], s4 = x.v[F_SI4];
+  const double D = (2.0 * pv[7] * v[7] + (pv[6] + pvl[6] * (1.0 + c_setup.logvj)) * v[6] + pvl[5] * v[5] - pv[4] * v[4] -
+                    2.0 * pv[3] * v[3] - 3.0 * pv[2] * v[2] - 4.0 * pv[1] * v[1] - 5.0 * pv[0]) * c_setup.dj_scale +
+                   (s1 + s2 * c_setup.dj_s2 + s3 * c_setup.dj_s3 + s4 * c_setup.dj_s4) * ie;
+  constexpr double rf = 1.0 / kPhiJoin;
+  c.C2Int = D - (c.b1 + c.b3 * (rf * rf * rf * rf) + c.b2 * rf) * ie;
+  const double pin = phi_ins_roots(c, fj, c_setup.fjp.third, c_setup.r_fj_third, c_setup.logvj);
+  c.C1Int = pin - ie * (c.b1 * fj - c.b3 * (rf * rf * rf / 3.0) + c.b2 * c_setup.log_fj) - c.C2Int * fj;
+  const double fm = c.fMRDJoin;
+  const double phiT = ie * x.mj.phi_int + c.C1Int + c.C2Int * fm;
+  c.C2MRD = c.C2Int + x.mj.dphi_int - x.mj.dphi_mrd;
+  c.C1MRD = phiT - ie * x.mj.phi_mrd - c.C2MRD * fm;
+  const double f = c.MfRef;
+  double phr;
+  if (x.br == 0) {
+    const double t = x.tref;
+    phr = phi_ins_roots(c, f, t, x.rref * t * t, (x.phr + kLnPi) * (1.0 / 3.0));
+  } else if (x.br == 1) {
+    phr = ie * x.phr + c.C1MRD + c.C2MRD * f;
+  } else {
+    phr = ie * x.phr + c.C1Int + c.C2Int * f;
+  }
+  c.phi_pre = 2. * (model == kModelIntrinsic ? x.p[4] : 0.5 * x.p[4]) + phr;
+  mix_phase_main(c, x.rdm);
+  mix_phase_join(c);
+  mix_phase_slopes(c);
+}
+
+// warp 1: projection (or the intrinsic model's offsets), fbegin and the first bin above it
+__device__ __forceinline__ void setup_project(PhdRec& c, SetupVals& x, int model, int l) {
+  const double* p = x.p;
+  const NetGeom& g = x.g;
+  c.ts = g.Tobs - p[5];
+  c.sqT = sqrt(g.Tobs);
+  const double ex = exp(l == 0 ? p[1] : (5.0 / 3.0) * (p[0] - p[1]));
+  if (model == kModelIntrinsic) {
+    set_offsets(c, p, g.nifo);
+  } else {
+    double sv, cv;
+    sincos(l == 0 ? g.GMST - p[7] : p[9], &sv, &cv);     // F_ant uses alpha - GMST
+    const double sa = lane_of(sv, 0), ca = lane_of(cv, 0), sps = lane_of(sv, 1), cps = lane_of(cv, 1);
+    const double Ap = (1.0 + p[10] * p[10]) / 2.0, Ac = -p[10], sd = p[8], cd = sqrt(1.0 - sd * sd);
+    double mp[21], mx[18];
+    antenna_basis(cps, sps, cd, sd, ca, -sa, mp, mx);
+    const bool plus = l < 3;
+    const int id = plus ? l : (l < 6 ? l - 3 : 0), lab = id < g.nifo ? g.labels[id] : 0;
+    double fv = 0.0;
+    const double* cP = c_antP[lab];
+    const double* cX = c_antX[lab];
+#pragma unroll
+    for (int k = 0; k < 18; k++) fv += (plus ? cP[k] : cX[k]) * (plus ? mp[k] : mx[k]);
+    if (plus)
+#pragma unroll
+      for (int k = 18; k < 21; k++) fv += cP[k] * mp[k];
+    const double fx = lane_of(fv, (l + 3) & (kLnlLanes - 1));
+    double lam = atan2(Ac * fx, Ap * fv);
+    if (lam < 0.0) lam += kTwoPi;
+    if (l < g.nifo) {
+      c.Fs[l] = sqrt(Ap * Ap * fv * fv + Ac * Ac * fx * fx);
+      c.lam[l] = lam;
+      const double r = c_detpos[lab][0] * cd * ca + c_detpos[lab][1] * cd * sa + c_detpos[lab][2] * sd;
+      c.td[l] = -r / kClight;
+    }
+  }
+  FbeginHead h;
+  double eta = lane_of(ex, 1);
+  if (eta > 0.25) eta = 0.25;
+  const double dm = sqrt(1.0 - 4.0 * eta);
+  h.M = lane_of(ex, 0) / kMsun * kTsunCBC;
+  h.eta = eta;
+  h.chi = 0.5 * ((1.0 + dm) * p[2] + (1.0 - dm) * p[3]);
+  h.th = 1.0 / sqrt(sqrt(sqrt(eta * p[5] / (5.0 * h.M))));
+  c.fs = fbegin_tail<MathInline>(h, p[2], p[3]);
+  x.lo = first_bin_above(g, c.fs);
+}
+
+// warp 2 until the first barrier: rho/sigma/v2 fits, a0 and the analytic amplitude prefactors (Appendix B of
+// arXiv:1508.07253), TaylorF2 with its aligned-spin terms but the 3PN spin-spin term PhenomD was not tuned
+// with, and the inspiral phase prefactors (phd_amp_prefactors, phd_taylorf2 without their divisions)
+__device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const double* s_fits, int l) {
+  const SetMass m = set_masses(x.p, l);
+  static_assert(F_RHO3 == F_RHO1 + 2 && F_SI4 == F_SI1 + 3, "lane order");
+  const double fv = fit_lane(s_fits, l < 3 ? F_RHO1 + l : l < 7 ? F_SI1 + l - 3 : F_V2, m.eta, m.chi);
+  const double s1 = lane_of(fv, 3), s2 = lane_of(fv, 4), s3 = lane_of(fv, 5), s4 = lane_of(fv, 6);
+  c.ai[5] = lane_of(fv, 0);
+  c.ai[6] = lane_of(fv, 1);
+  c.ai[7] = lane_of(fv, 2);
+  x.v[F_SI1] = s1; x.v[F_SI2] = s2; x.v[F_SI3] = s3; x.v[F_SI4] = s4;
+  x.v[F_V2] = lane_of(fv, 7);
+  const Pow6 pip = c_setup.pi6;
+  const double eta = m.eta, Seta = m.Seta, x1 = m.chi1, x2 = m.chi2, x1s = x1 * x1, x2s = x2 * x2, e2 = eta * eta,
+               e3 = eta * e2, Pi = kPi, Pi2 = pip.two;
+  c.a0 = c_setup.a0 * sqrt(eta);
+  c.ai[0] = (-969 + 1804 * eta) * (pip.two_thirds * (1.0 / 672.));
+  c.ai[1] = (x1 * (81 * (1 + Seta) - 44 * eta) + x2 * (81 - 81 * Seta - 44 * eta)) * (kPi / 48.);
+  c.ai[2] = (-27312085.0 - 10287648 * x2s - 10287648 * x1s * (1 + Seta) + 10287648 * x2s * Seta +
+             24 * (-1975055 + 857304 * x1s - 994896 * x1 * x2 + 857304 * x2s) * eta + 35371056 * e2) *
+            (pip.four_thirds * (1.0 / 8.128512e6));
+  c.ai[3] = (pip.five_thirds * (1.0 / 32256.)) *
+            (x2 * (-285197 * (-1 + Seta) + 4 * (-91902 + 1579 * Seta) * eta - 35632 * e2) +
+             x1 * (285197 * (1 + Seta) - 4 * (91902 + 1579 * Seta) * eta - 35632 * e2) + 42840 * (-1.0 + 4 * eta) * Pi);
+  c.ai[4] = -(Pi2 * (1.0 / 6.0085960704e10)) *
+            (-336 * (-3248849057.0 + 2943675504 * x1s - 3339284256 * x1 * x2 + 2943675504 * x2s) * e2 - 324322727232 * e3 -
+             7 * (-177520268561 + 107414046432 * x2s + 107414046432 * x1s * (1 + Seta) - 107414046432 * x2s * Seta +
+                  11087290368 * (x1 + x2 + x1 * Seta - x2 * Seta) * Pi) +
+             12 * eta * (-545384828789 - 176491177632 * x1 * x2 + 202603761360 * x2s +
+                         77616 * x1s * (2610335 + 995766 * Seta) - 77287373856 * x2s * Seta +
+                         5841690624 * (x1 + x2) * Pi + 21384760320 * Pi2));
+  const double m1M = 0.5 * (1.0 + Seta), m2M = 0.5 * (1.0 - Seta), q1 = m1M * m1M * x1s, q2 = m2M * m2M * x2s, xx = x1 * x2;
+  const double SL = m1M * m1M * x1 + m2M * m2M * x2, dS = Seta * (m2M * x2 - m1M * x1);
+  const double pf = (3.0 / 128.0) * recip64(eta);
+  const double sig = eta * (721.0 / 48.0 - 247.0 / 48.0) * xx + ((720.0 - 1.0) / 96.0 - (240.0 - 7.0) / 96.0) * (q1 + q2);
+  const double gam = (554345.0 / 1134.0 + 110.0 / 9.0 * eta) * SL + (13915.0 / 84.0 - 10.0 / 3.0 * eta) * dS;
+  double v[8], w5, w6;
+  v[0] = pf;
+  v[1] = 0.0;
+  v[2] = (5.0 / 9.0 * (743.0 / 84.0 + 11.0 * eta)) * pf;
+  v[3] = (-16.0 * Pi + 188.0 / 3.0 * SL + 25.0 * dS) * pf;
+  v[4] = (5.0 / 72.0 * (3058.673 / 7.056 + 5429.0 / 7.0 * eta + 617.0 * e2) - 10.0 * sig) * pf;
+  v[5] = (5.0 / 9.0 * (7729.0 / 84.0 - 13.0 * eta) * Pi - gam) * pf;
+  w5 = (5.0 / 3.0 * (7729.0 / 84.0 - 13.0 * eta) * Pi - 3.0 * gam) * pf;
+  v[6] = ((11583.231236531 / 4.694215680 - 640.0 / 3.0 * Pi * Pi - 6848.0 / 21.0 * kGammaE -
+           6848.0 / 21.0 * 1.3862943611198906) +
+          eta * (-15737.765635 / 3.048192 + 2255. / 12. * Pi * Pi) + e2 * (76055.0 / 1728.0) - e3 * (127825.0 / 1296.0) +
+          Pi / 3.0 * (3760.0 * SL + 1490.0 * dS)) * pf;
+  w6 = -6848.0 / 21.0 * pf;
+  v[7] = (Pi * (77096675.0 / 254016.0 + 378515.0 / 1512.0 * eta - 74045.0 / 756.0 * e2) +
+          (-8980424995.0 / 762048.0 + 6586595.0 / 756.0 * eta - 305.0 / 36.0 * e2) * SL -
+          (170978035.0 / 48384.0 - 2876425.0 / 672.0 * eta - 4735.0 / 144.0 * e2) * dS) * pf;
+#pragma unroll
+  for (int k = 0; k < 8; k++) x.pv[k] = v[k];
+  x.pvl[5] = w5;
+  x.pvl[6] = w6;
+  c.pq[0] = v[5] - kPi4;
+  c.pq[1] = v[7] * pip.two_thirds;
+  c.pq[2] = v[6] * pip.third;
+  c.pq[3] = w6 * pip.third;
+  c.pq[4] = w5;
+  c.pq[5] = v[4] * c_setup.r_pi_third;
+  c.pq[6] = v[3] * c_setup.r_pi_two_thirds;
+  c.pq[7] = v[2] * (1.0 / kPi);
+  c.pq[8] = v[0] * c_setup.r_pi_five_thirds;
+  c.pq[9] = s1;
+  c.pq[10] = s2 * (3.0 / 4.0);
+  c.pq[11] = s3 * (3.0 / 5.0);
+  c.pq[12] = s4 / 2.0;
+}
+
+// warp 2 until the second barrier: the intermediate amplitude's quartic through value and slope at f1 and f3
+// and the value at the middle (phd_amp_int), and the folded amplitude
+__device__ __forceinline__ void setup_amplitude(PhdRec& c, const SetupVals& x) {
+  const double f1 = kAmpJoin, f3 = c.fmax, h = f3 - f1, f2 = f1 + h / 2.0, rh = recip64(h), df3 = f3 - c.fRD,
+               fg = c.fDM * c.g3;
+  const Pow6 p1 = c_setup.f1p;
+  const double v1 = amp_ins(c, f1, p1), d1 = damp_ins_p(c, f1, p1), v2 = x.v[F_V2], v3 = x.v3;
+  const double d2 = v3 * (-c.g2 * x.rfg - 2.0 * df3 * recip64(df3 * df3 + fg * fg));
+  const double q12 = (v2 - v1) * (2.0 * rh), q23 = (v3 - v2) * (2.0 * rh);
+  const double q012 = (q12 - d1) * (2.0 * rh), q123 = (q23 - q12) * rh, q234 = (d2 - q23) * (2.0 * rh);
+  const double q0123 = (q123 - q012) * rh, q1234 = (q234 - q123) * rh;
+  c.hx1 = f1; c.hx2 = f2; c.hx3 = f3;
+  c.hc[0] = v1; c.hc[1] = d1; c.hc[2] = q012; c.hc[3] = q0123; c.hc[4] = (q1234 - q0123) * rh;
+  mix_amp(c, x.rfg);
+}
+
+// warp 3 until the first barrier: scales and the model's last bin
+__device__ __forceinline__ void setup_scales(PhdRec& c, SetupVals& x, int l) {
+  const SetMass m = set_masses(x.p, l);
+  const double Msec = m.M * kMtsun;
+  const double d = (l == 0 ? kFcut : m.M * kMrsun * m.M * kMtsun) / (l == 0 ? Msec : m.dist);
+  const double fCut = lane_of(d, 0);
+  c.fCut = fCut;
+  c.amp_scale = lane_of(d, 1);
+  x.hi = last_bin_below(x.g, fCut);
+}
+
+// A block's sets from their parameters and geometries in s_x to their records in s_rec: 8 lanes of each of
+// four warps per set.  Contains __syncthreads(): every thread of the block calls it.
+__device__ __forceinline__ void setup_roles(PhdRec& c, SetupVals& x, const double* s_fits, const QnmTable& q, int model) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & (kLnlLanes - 1);
+  if (w == 0) setup_ringdown(c, x, s_fits, q, l);
+  else if (w == 1) setup_project(c, x, model, l);
+  else if (w == 2) setup_inspiral(c, x, s_fits, l);
+  else if (w == 3) setup_scales(c, x, l);
+  __syncthreads();
+  if (w == 0) {
+    setup_joins(c, x, model);
+  } else if (w == 2) {
+    setup_amplitude(c, x);
+  } else if (w == 3) {
+    // first bins of the pieces, a lane each
+    const int bin = first_bin_mf_at_least(x.g, c.Msec, l == 0 ? kAmpJoin : l == 1 ? kPhiJoin : l == 2 ? c.fMRDJoin : c.fmax);
+    c.mix.iA = __shfl_sync(0xffffffffu, bin, 0, kLnlLanes);
+    c.mix.iP = __shfl_sync(0xffffffffu, bin, 1, kLnlLanes);
+    c.mix.iM = __shfl_sync(0xffffffffu, bin, 2, kLnlLanes);
+    c.mix.iF = __shfl_sync(0xffffffffu, bin, 3, kLnlLanes);
+  } else if (w == 1 && l == 0) {
+    if (x.live) {
+      c.flags = x.st == kStOK ? kRecValid : 0;
+      c.i_lo = x.lo;
+      c.i_hi = x.hi;
+      c.event = x.ev;
+    } else {
+      x.st = kStNoEvent;
+      c.flags = 0;
+      c.event = -1;
+      c.i_lo = 1;
+      c.i_hi = 0;
+    }
+  }
+  __syncthreads();
+}
+
+// ocnt / olist non-null: each set is filed under its length class (SetOrder); ntile non-null: its tile count
+template <class Geom>
+__device__ __forceinline__ void setup_lnl_block(const double* __restrict__ params, int B, const Geom& geo,
+                                                const QnmTable& q, int tile_bins, PhdRec* __restrict__ recs,
+                                                int* __restrict__ status, int* __restrict__ ntile, int model,
+                                                int* __restrict__ ocnt, int* __restrict__ olist) {
+  __shared__ __align__(16) PhdRec s_rec[kLnlSets];
+  __shared__ SetupVals s_x[kLnlSets];
+  __shared__ double s_fits[F_COUNT * 11];
+  const int b0 = blockIdx.x * kLnlSets, nb = min(kLnlSets, B - b0), tid = threadIdx.x;
+  {
+    // the block's parameters are contiguous: one load per thread, one round trip also from mapped host
+    // memory; a group past the last set repeats that set's (its record is not stored)
+    const int ps = geo.stride(model), set = tid / ps, k = tid - set * ps;
+    const double v = set < kLnlSets ? params[(size_t)(b0 + min(set, nb - 1)) * ps + k] : 0.0;
+    for (int i = tid; i < F_COUNT * 11; i += kLnlThreads) s_fits[i] = __ldg(q.fits + i);
+    if (tid < kLnlSets) {
+      NetGeom g;
+      int e = -1;
+      const bool live = geo.get(b0 + min(tid, nb - 1), g, e);
+      if (!live) {                       // a harmless stand-in: the record is marked invalid
+        memset(&g, 0, sizeof(g));
+        g.N = 8; g.imin = 1; g.imax = 2;
+        g.Tobs = 1.0; g.df = 1.0; g.div_exact = 1;
+      }
+      s_x[tid].g = g;
+      s_x[tid].ev = e;
+      s_x[tid].live = live;
+    }
+    if (set < kLnlSets) s_x[set].p[k] = v;
+  }
+  __syncthreads();
+  const int set = (tid & 31) / kLnlLanes;
+  SetupVals& x = s_x[set];
+  setup_roles(s_rec[set], x, s_fits, q, model);
+  if (tid < 32 && (tid & (kLnlLanes - 1)) == 0 && set < nb) {
+    const PhdRec& c = s_rec[set];
+    const int b = b0 + set, bins = (c.flags & kRecValid) ? max(0, c.i_hi - c.i_lo + 1) : 0;
+    status[b] = x.st;
+    if (ntile) ntile[b] = (bins + tile_bins - 1) / tile_bins;
+    if (ocnt) {
+      const int cl = length_class(bins, x.g.imax - x.g.imin), r = atomicAdd(ocnt + cl, 1);
+      if (r < B) olist[(size_t)cl * B + r] = b;      // r >= B only if the counts were not cleared
+    }
+  }
+  // the block's records are contiguous in shared and in global memory
+  const int4* src = reinterpret_cast<const int4*>(s_rec);
+  int4* dst = reinterpret_cast<int4*>(recs + b0);
+  const int words = nb * (int)(sizeof(PhdRec) / 16);
+  for (int i = tid; i < words; i += kLnlThreads) dst[i] = src[i];
 }
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may be scheduled while the
@@ -925,19 +1329,17 @@ static void launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, 
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// One line of the following launch's tables per thread (SetupPrefetch); every address lies inside
-// its array.
+// The following launch's tables (SetupPrefetch), a line or a bin's entries per thread and turn; every
+// address lies inside its array.
 __device__ __forceinline__ void setup_prefetch(const SetupPrefetch& pf) {
-  size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t lines = (pf.bytes + 127) / 128;
-  if (t < lines) {
-    prefetch_l2(static_cast<const char*>(pf.buf) + t * 128);
-    return;
-  }
-  t -= lines;
-  if (t < (size_t)pf.nbins) {
-    const int i = pf.bins[t];
-    if (i < 0 || i >= pf.tab_n) return;
+  const size_t lines = (pf.bytes + 127) / 128, step = (size_t)gridDim.x * blockDim.x;
+  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < lines + (size_t)pf.nbins; t += step) {
+    if (t < lines) {
+      prefetch_l2(static_cast<const char*>(pf.buf) + t * 128);
+      continue;
+    }
+    const int i = pf.bins[t - lines];
+    if (i < 0 || i >= pf.tab_n) continue;
     if (pf.tabA) prefetch_l2(pf.tabA + i);
     if (pf.tabB) prefetch_l2(pf.tabB + i);
     if (pf.tabC) prefetch_l2(pf.tabC + i);
@@ -946,26 +1348,31 @@ __device__ __forceinline__ void setup_prefetch(const SetupPrefetch& pf) {
 
 __global__ void __launch_bounds__(kSetupThreads) k_setup(const double* __restrict__ params, int B, NetGeom g,
                                                          QnmTable q, PhdRec* __restrict__ recs,
-                                                         int* __restrict__ status, int model, SetOrder o,
-                                                         SetupPrefetch pf) {
-  pdl_trigger();       // a dependent launch (the lnL kernel) may be scheduled; it waits for this grid
-  setup_prefetch(pf);
+                                                         int* __restrict__ status, int model) {
   GeomOne geo{g};
-  setup_coop_block(params, B, geo, q, 1, recs, status, nullptr, model, o.cnt, o.list);
+  setup_coop_block(params, B, geo, q, recs, status, model);
 }
 
 void launch_setup(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
-                  int* d_status, cudaStream_t s, int model, const SetupPrefetch& pf) {
+                  int* d_status, cudaStream_t s, int model) {
   if (B <= 0) return;
-  k_setup<<<(B + kSetupSets - 1) / kSetupSets, kSetupThreads, 0, s>>>(d_params, B, g, q, d_recs, d_status, model,
-                                                                      SetOrder{nullptr, nullptr}, pf);
+  k_setup<<<(B + kSetupSets - 1) / kSetupSets, kSetupThreads, 0, s>>>(d_params, B, g, q, d_recs, d_status, model);
 }
 
-void launch_setup_ordered(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
-                          int* d_status, const SetOrder& o, cudaStream_t s, int model) {
+__global__ void __launch_bounds__(kLnlThreads) k_setup_lnl(const double* __restrict__ params, int B, NetGeom g,
+                                                           QnmTable q, PhdRec* __restrict__ recs,
+                                                           int* __restrict__ status, int model, SetOrder o,
+                                                           SetupPrefetch pf) {
+  pdl_trigger();       // a dependent launch (the lnL kernel) may be scheduled; it waits for this grid
+  setup_prefetch(pf);
+  GeomOne geo{g};
+  setup_lnl_block(params, B, geo, q, 1, recs, status, nullptr, model, o.cnt, o.list);
+}
+
+void launch_setup_lnl(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
+                      int* d_status, cudaStream_t s, int model, const SetOrder& o, const SetupPrefetch& pf) {
   if (B <= 0) return;
-  k_setup<<<(B + kSetupSets - 1) / kSetupSets, kSetupThreads, 0, s>>>(d_params, B, g, q, d_recs, d_status, model, o,
-                                                                      SetupPrefetch{});
+  k_setup_lnl<<<(B + kLnlSets - 1) / kLnlSets, kLnlThreads, 0, s>>>(d_params, B, g, q, d_recs, d_status, model, o, pf);
 }
 
 // ---------------------------------------------------------------- reductions
@@ -1382,14 +1789,6 @@ __device__ __forceinline__ void sincos_cycles(double cyc, double& sv, double& cv
   sincos_cycles<1, true>(x, s, c);
   sv = s[0];
   cv = c[0];
-}
-
-// 1/x for finite normal x: the hardware's approximation (about 2^-20) and one third-order step
-__device__ __forceinline__ double recip64(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
 }
 
 constexpr int kSeg64 = 64;                 // rows of blockDim.x bins per table segment
@@ -2095,21 +2494,20 @@ void launch_fill_bin_tables(double2* d_tabA, double2* d_tabB, float2* d_tabC, do
 }
 
 // ---------------------------------------------------------------- multi-event launches
-__global__ void __launch_bounds__(kSetupThreads) k_setup_multi(const double* __restrict__ params,
+__global__ void __launch_bounds__(kLnlThreads) k_setup_multi(const double* __restrict__ params,
                                                                const int* __restrict__ event_of, int B,
                                                                const EventDesc* __restrict__ events, int n_events,
                                                                QnmTable q, int tile_bins, PhdRec* __restrict__ recs,
                                                                int* __restrict__ status, int* __restrict__ ntile) {
   GeomTable geo{event_of, events, n_events};
-  setup_coop_block(params, B, geo, q, tile_bins, recs, status, ntile, kModelFull);
+  setup_lnl_block(params, B, geo, q, tile_bins, recs, status, ntile, kModelFull, nullptr, nullptr);
 }
 
 void launch_setup_multi(const double* d_params, const int* d_event_of, int B, const EventDesc* d_events, int n_events,
                         const QnmTable& q, int tile_bins, PhdRec* d_recs, int* d_status, int* d_ntile, cudaStream_t s) {
   if (B <= 0) return;
-  k_setup_multi<<<(B + kSetupSets - 1) / kSetupSets, kSetupThreads, 0, s>>>(d_params, d_event_of, B, d_events,
-                                                                           n_events, q, tile_bins, d_recs, d_status,
-                                                                           d_ntile);
+  k_setup_multi<<<(B + kLnlSets - 1) / kLnlSets, kLnlThreads, 0, s>>>(d_params, d_event_of, B, d_events, n_events, q,
+                                                                     tile_bins, d_recs, d_status, d_ntile);
 }
 
 // One block: exclusive scan of ntile into off[0..B], then expansion into items (bounded by items_cap).
@@ -2301,142 +2699,264 @@ constexpr int kRecDoubles = (int)(sizeof(PhdRec) / 8);
 // doubles of shared memory one set's warp uses (a multiple of 2, so the next record stays 16-B aligned)
 __host__ __device__ inline int het_warp_doubles(int nifo, int M) { return kRecDoubles + (3 * nifo * M + 1) / 2 * 2; }
 
+// What a grid point needs besides the set: its bin's table entries and the reference waveform there.  Loaded
+// before the record is there where the kernel waits for it.
+struct HetPre {
+  double f;
+  int i;
+  bool bin;                  // FP64: f is bin i of the event and the tables hold it
+  double2 tA, tB;
+  float2 tC;
+  double aref[kMaxIfo], pcyc[kMaxIfo];      // reference amplitude (FP64: its reciprocal), phase in cycles
+};
+template <int PREC>
+__device__ __forceinline__ HetPre het_pre(const NetGeom& g, const HetData& h, int j) {
+  constexpr double kInv2Pi = 0.15915494309189533577;
+  HetPre e;
+  e.f = __ldg(h.freq + j);
+  e.i = (int)rint(e.f * g.Tobs);
+  e.bin = PREC != kFP64 || (e.i >= 1 && e.i < h.tab_n && bin_freq(g, e.i) == e.f);
+  e.tA = e.tB = make_double2(0.0, 0.0);
+  e.tC = make_float2(0.f, 0.f);
+  if (e.bin) {
+    e.tA = __ldg(h.tabA + e.i);
+    e.tB = __ldg(h.tabB + e.i);
+    if (PREC != kFP64) e.tC = __ldg(h.tabC + e.i);
+  }
+  for (int id = 0; id < kMaxIfo; id++) {
+    if (id >= g.nifo) break;
+    e.aref[id] = __ldg(h.amp + id * h.M + j);
+    if (PREC == kFP64) e.aref[id] = 1.0 / e.aref[id];
+    e.pcyc[id] = __ldg(h.phase + id * h.M + j) * kInv2Pi;
+  }
+  return e;
+}
+
 // The mixed-precision waveform at bin i of the event (a heterodyne grid point, f = i/Tobs) from
 // the folded polynomials of the mixed full-likelihood kernel (MixPoly) and the per-bin tables:
 // phc = phase / 2 pi = R0 + i Ri + the piece's rest (FP64 for the inspiral and intermediate
 // rests, FP32 for the ringdown's few cycles), amp = a0 Mf^{-7/6} A(Mf) in FP32 (the piece's
 // amplitude times a0 (Msec df)^{-7/6} i^{-7/6}).  No log, cube root or FP64 division per point.
 // The record must be in shared memory (its coefficients are read with shared loads).
-__device__ __forceinline__ void mixed_point(const PhdRec& c, const HetData& h, int i, float& amp, double& phc) {
+__device__ __forceinline__ void mixed_point(const PhdRec& c, const HetPre& e, float& amp, double& phc) {
   const MixPoly& P = c.mix;
-  const double2 tA = __ldg(h.tabA + i), tB = __ldg(h.tabB + i);
-  const float2 tC = __ldg(h.tabC + i);
+  const int i = e.i;
   const double xi = (double)i;
   const float xf = (float)i;
   const int pp = ph_piece(P, i), ap = amp_piece(P, i);
   double rest;
-  if (pp == 0) rest = mph_ins(P.pins, xi, tA.x, tA.y, tB.x);
-  else if (pp == 1) rest = mph_int(P.pint, xi, tA.y, tB.x);
-  else rest = (double)mph_mrd(P.pmrd, xf, tC);
+  if (pp == 0) rest = mph_ins(P.pins, xi, e.tA.x, e.tA.y, e.tB.x);
+  else if (pp == 1) rest = mph_int(P.pint, xi, e.tA.y, e.tB.x);
+  else rest = (double)mph_mrd(P.pmrd, xf, e.tC);
   const double2 r = sld2(&P.pmrd.R0);                          // (R0, Ri)
   phc = fma(xi, r.y, r.x) + rest;
-  const float a = ap == 0 ? mamp_ins(P.ains, xf, (float)tA.x) : (ap == 1 ? mamp_int(P.aint, xf) : mamp_mrd(P.amrd, xf));
-  const float u = (float)tA.y;                                // i^{-1/3}
+  const float a = ap == 0 ? mamp_ins(P.ains, xf, (float)e.tA.x) : (ap == 1 ? mamp_int(P.aint, xf) : mamp_mrd(P.amrd, xf));
+  const float u = (float)e.tA.y;                              // i^{-1/3}
   amp = a * (u * u * u) * sqrtf(u) * (float)(c.a0 * c.mdf_m76);
 }
 
-// Phase 1 of a set: the waveform at grid points j0, j0 + jstep, ... and the per-detector ratios
-// to the reference into the set's shared memory sm ([3][nifo][M]: hc, hs, cc).
+// The same in FP64 throughout: the folded polynomials for the inspiral and intermediate phase, the pieces
+// themselves for the rest, every power of Mf = m i from the tables' i^{1/3}, i^{-1/3}, log i, i^{3/4}.  amp
+// without amp_scale.  One atan or exp at most, where evaluating Mf^{1/6}, log Mf and the pieces' divisions
+// made a point 4.3 us of a one-set call.
+__device__ __forceinline__ void fp64_point(const PhdRec& c, const HetPre& e, double& amp, double& phc) {
+  constexpr double kInv2Pi = 0.15915494309189533577;
+  const MixPoly& P = c.mix;
+  const int pp = ph_piece(P, e.i), ap = amp_piece(P, e.i);
+  const double xi = (double)e.i, m = c.mdf, Mf = m * xi, u = e.tA.y, th = c.mdf_third * e.tA.x;
+  double rest;
+  if (pp == 0) {
+    rest = mph_ins(P.pins, xi, e.tA.x, u, e.tB.x);
+  } else if (pp == 1) {
+    rest = mph_int(P.pint, xi, u, e.tB.x);
+  } else {
+    const double r = c.mdf_rthird * u;
+    rest = kInv2Pi * c.inv_eta * (-c.al2 * (r * r * r) + (4.0 / 3.0) * (c.al3 * (c.mdf_34 * e.tB.y)) +
+                                  c.al4 * atan((Mf - c.al5 * c.fRD) / c.fDM));
+  }
+  const double2 r = sld2(&P.pmrd.R0);                          // (R0, Ri)
+  phc = fma(xi, r.y, r.x) + rest;
+  double a;
+  if (ap == 0) {
+    Pow6 p;
+    p.third = th;
+    p.two_thirds = th * th;
+    p.four_thirds = Mf * th;
+    p.five_thirds = p.four_thirds * th;
+    p.two = Mf * Mf;
+    p.seven_thirds = p.two * th;
+    p.eight_thirds = p.two * p.two_thirds;
+    a = amp_ins(c, Mf, p);
+  } else {
+    a = ap == 1 ? amp_int(c, Mf) : amp_mrd(c, Mf);
+  }
+  amp = a * (c.a0 * c.mdf_m76) * (u * u * u * sqrt(u));
+}
+
+// Phase 1 of a set at grid point j: the waveform and the per-detector ratios to the reference into the
+// set's shared memory sm ([3][nifo][M]: hc, hs, cc).
 template <int PREC>
-__device__ __forceinline__ void het_points(const PhdRec& c, const NetGeom& g, const HetData& h, double* sm, int j0,
-                                           int jstep) {
+__device__ __forceinline__ void het_point(const PhdRec& c, const NetGeom& g, const HetData& h, const HetPre& e,
+                                          double* sm, int j) {
   const int M = h.M, nifo = g.nifo;
   double* s_hc = sm;                 // [nifo][M]
   double* s_hs = sm + nifo * M;
   double* s_cc = sm + 2 * nifo * M;
   constexpr double kInv2Pi = 0.15915494309189533577;
-  for (int j = j0; j < M; j += jstep) {
-    double f = __ldg(h.freq + j);
-    double y = 1.0;
-    if (f < c.fs) y = exp(10.0 * (f - c.fs) / c.fs);          // taper below fbegin (QuickCBC.c:3859)
-    if (PREC == kFP64) {
-      double amp = 0.0, ph = 0.0;
-      if (!(f > c.fCut)) { phd_eval64(c, c.Msec * f, amp, ph); amp *= c.amp_scale; }
-      for (int id = 0; id < nifo; id++) {
-        double A = c.Fs[id] * kH22fac * amp / c.sqT * y;
-        double x = __dadd_rn(__dadd_rn(__dmul_rn(__dmul_rn(kTwoPi, f), c.ts - c.td[id]), c.lam[id]), -ph);
-        double aref = __ldg(h.amp + id * M + j), pref = __ldg(h.phase + id * M + j);
-        double sx, cx;
-        sincos(reduce_2pi(pref - x), &sx, &cx);
-        double cc = 2.0 * (aref - A * cx), ss = 2.0 * A * sx;
-        double hc = cc / aref, hs = ss / aref;
-        s_hc[id * M + j] = hc;
-        s_hs[id * M + j] = hs;
-        s_cc[id * M + j] = hc * hc + hs * hs;
-      }
-    } else {
-      float amp = 0.f;
-      double phc = 0.0;
-      if (!(f > c.fCut)) mixed_point(c, h, (int)rint(f * g.Tobs), amp, phc);
-      for (int id = 0; id < nifo; id++) {
-        double aref = __ldg(h.amp + id * M + j), pref = __ldg(h.phase + id * M + j);
-        float ratio = amp * (float)(c.Fs[id] * kH22fac * c.amp_scale / c.sqT * y / aref);
-        double cyc = pref * kInv2Pi - fma(f, c.ts - c.td[id], c.lam[id] * kInv2Pi - phc);
-        float r = (float)(cyc - rint(cyc));
-        float sx, cx;
-        sincospif(2.0f * r, &sx, &cx);
-        float hc = 2.0f * (1.0f - ratio * cx), hs = 2.0f * ratio * sx;
-        s_hc[id * M + j] = (double)hc;
-        s_hs[id * M + j] = (double)hs;
-        s_cc[id * M + j] = (double)hc * (double)hc + (double)hs * (double)hs;
+  const double f = e.f;
+  double y = 1.0;
+  if (f < c.fs) y = exp(10.0 * (f - c.fs) / c.fs);          // taper below fbegin (QuickCBC.c:3859)
+  if (PREC == kFP64) {
+    double amp = 0.0, phc = 0.0;
+    if (!(f > c.fCut)) {
+      if (e.bin) {
+        fp64_point(c, e, amp, phc);
+      } else {                                              // a grid off the event's bins
+        phd_eval64(c, c.Msec * f, amp, phc);
+        phc *= kInv2Pi;
       }
     }
-  }
-}
-
-// Phase 2 of a set, by one warp once phase 1 is in sm: the region contractions (lane r takes
-// regions r, r + 32, ...), a butterfly warp sum, and lane 0 writes lnL to *out.
-__device__ __forceinline__ void het_regions(const NetGeom& g, const HetData& h, const double* sm, double* out) {
-  const int lane = threadIdx.x & 31;
-  const int M = h.M, nifo = g.nifo;
-  const double* s_hc = sm;
-  const double* s_hs = sm + nifo * M;
-  const double* s_cc = sm + 2 * nifo * M;
-  const int J = h.J, J1 = J + 1, NR = h.NR;
-  double acc[4 * kMaxIfo];           // per detector: HH, HR, x, y
-#pragma unroll
-  for (int k = 0; k < 4 * kMaxIfo; k++) acc[k] = 0.0;
-  for (int r = lane; r < NR; r += 32) {
-    const double* ip = h.IP + (size_t)r * J1 * J1;
-#pragma unroll
-    for (int id = 0; id < kMaxIfo; id++) {     // unrolled: acc stays in registers
-      if (id >= nifo) break;
-      const double* sl = h.SL + ((size_t)r * nifo + id) * J1;
-      const double* lc = h.lc + ((size_t)r * nifo + id) * J1;
-      const double* ls = h.ls + ((size_t)r * nifo + id) * J1;
-      const double* vc = s_cc + id * M + r * J;
-      const double* vh = s_hc + id * M + r * J;
-      const double* vs = s_hs + id * M + r * J;
-      double HH = 0.0, HR = 0.0;
-      for (int a = 0; a < J1; a++) {
-        double u1 = 0.0, u2 = 0.0, u3 = 0.0;
-        for (int k = 0; k < J1; k++) {
-          double w = __ldg(ip + a * J1 + k);
-          u1 += w * vc[k];
-          u2 += w * vh[k];
-          u3 += w * vs[k];
-        }
-        HH += u1 * __ldg(sl + a);
-        HR += u2 * __ldg(lc + a) + u3 * __ldg(ls + a);
-      }
-      acc[4 * id] += HH;
-      acc[4 * id + 1] += HR;
-      if (r < NR - 2) {
-        acc[4 * id + 2] += __ldg(h.aa + id * NR + r + 1) * vc[J];
-        acc[4 * id + 3] += __ldg(h.rc + id * NR + r + 1) * vh[J] + __ldg(h.rs + id * NR + r + 1) * vs[J];
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 4 * kMaxIfo; k++)
-    for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  if (lane == 0) {
-    double L = h.logLb;
+    amp *= c.amp_scale * (kH22fac * y) / c.sqT;
     for (int id = 0; id < nifo; id++) {
-      double HH = acc[4 * id] - acc[4 * id + 2], HR = acc[4 * id + 1] - acc[4 * id + 3];
-      L -= (HR + 0.5 * HH);
+      const double ratio = c.Fs[id] * amp * e.aref[id];
+      const double cyc = e.pcyc[id] - fma(f, c.ts - c.td[id], c.lam[id] * kInv2Pi - phc);
+      double sx, cx;
+      sincos_cycles(cyc, sx, cx);
+      const double hc = 2.0 * (1.0 - ratio * cx), hs = 2.0 * ratio * sx;
+      s_hc[id * M + j] = hc;
+      s_hs[id * M + j] = hs;
+      s_cc[id * M + j] = hc * hc + hs * hs;
     }
-    *out = L;
+  } else {
+    float amp = 0.f;
+    double phc = 0.0;
+    if (!(f > c.fCut)) mixed_point(c, e, amp, phc);
+    for (int id = 0; id < nifo; id++) {
+      float ratio = amp * (float)(c.Fs[id] * kH22fac * c.amp_scale / c.sqT * y / e.aref[id]);
+      double cyc = e.pcyc[id] - fma(f, c.ts - c.td[id], c.lam[id] * kInv2Pi - phc);
+      float r = (float)(cyc - rint(cyc));
+      float sx, cx;
+      sincospif(2.0f * r, &sx, &cx);
+      float hc = 2.0f * (1.0f - ratio * cx), hs = 2.0f * ratio * sx;
+      s_hc[id * M + j] = (double)hc;
+      s_hs[id * M + j] = (double)hs;
+      s_cc[id * M + j] = (double)hc * (double)hc + (double)hs * (double)hs;
+    }
   }
 }
 
-// lnL of one set by one warp: phase 1 over the warp's lanes, then phase 2
+// Phase 2: one region of one detector, from the region's tables.  acc: HH, HR, and the edge values x, y.
+struct HetRegion {             // three points per region (J = 2)
+  double ip[9], sl[3], lc[3], ls[3], aa, rc, rs;
+  __device__ __forceinline__ void load(const HetData& h, int nifo, int id, int r) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) ip[k] = __ldg(h.IP + (size_t)r * 9 + k);
+    const size_t o = ((size_t)r * nifo + id) * 3;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      sl[a] = __ldg(h.SL + o + a);
+      lc[a] = __ldg(h.lc + o + a);
+      ls[a] = __ldg(h.ls + o + a);
+    }
+    aa = rc = rs = 0.0;
+    if (r < h.NR - 2) {
+      aa = __ldg(h.aa + id * h.NR + r + 1);
+      rc = __ldg(h.rc + id * h.NR + r + 1);
+      rs = __ldg(h.rs + id * h.NR + r + 1);
+    }
+  }
+  __device__ __forceinline__ void add(const double* vc, const double* vh, const double* vs, bool edge,
+                                      double (&acc)[4]) const {
+    double HH = 0.0, HR = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      double u1 = 0.0, u2 = 0.0, u3 = 0.0;
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const double w = ip[3 * a + k];
+        u1 = fma(w, vc[k], u1);
+        u2 = fma(w, vh[k], u2);
+        u3 = fma(w, vs[k], u3);
+      }
+      HH = fma(u1, sl[a], HH);
+      HR = fma(u2, lc[a], fma(u3, ls[a], HR));
+    }
+    acc[0] += HH;
+    acc[1] += HR;
+    if (edge) {
+      acc[2] = fma(aa, vc[2], acc[2]);
+      acc[3] = fma(rc, vh[2], fma(rs, vs[2], acc[3]));
+    }
+  }
+};
+
+// Detector id's sums over the regions r = lane, lane + 32, ... by one warp, summed over the warp (every lane
+// gets them).  pre: this lane's first region already loaded (J = 2), or null.
+__device__ __forceinline__ void het_detector(const NetGeom& g, const HetData& h, const double* sm, int id,
+                                             const HetRegion* pre, double (&acc)[4]) {
+  const int lane = threadIdx.x & 31, M = h.M, nifo = g.nifo, J = h.J, J1 = J + 1, NR = h.NR;
+  const double* s_hc = sm + id * M;
+  const double* s_hs = sm + (nifo + id) * M;
+  const double* s_cc = sm + (2 * nifo + id) * M;
+#pragma unroll
+  for (int k = 0; k < 4; k++) acc[k] = 0.0;
+  for (int r = lane; r < NR; r += 32) {
+    const double* vc = s_cc + r * J;
+    const double* vh = s_hc + r * J;
+    const double* vs = s_hs + r * J;
+    const bool edge = r < NR - 2;
+    if (J == 2) {
+      if (pre && r == lane) {
+        pre->add(vc, vh, vs, edge, acc);
+      } else {
+        HetRegion R;
+        R.load(h, nifo, id, r);
+        R.add(vc, vh, vs, edge, acc);
+      }
+      continue;
+    }
+    const double* ip = h.IP + (size_t)r * J1 * J1;
+    const size_t o = ((size_t)r * nifo + id) * J1;
+    double HH = 0.0, HR = 0.0;
+    for (int a = 0; a < J1; a++) {
+      double u1 = 0.0, u2 = 0.0, u3 = 0.0;
+      for (int k = 0; k < J1; k++) {
+        const double w = __ldg(ip + a * J1 + k);
+        u1 = fma(w, vc[k], u1);
+        u2 = fma(w, vh[k], u2);
+        u3 = fma(w, vs[k], u3);
+      }
+      HH = fma(u1, __ldg(h.SL + o + a), HH);
+      HR = fma(u2, __ldg(h.lc + o + a), fma(u3, __ldg(h.ls + o + a), HR));
+    }
+    acc[0] += HH;
+    acc[1] += HR;
+    if (edge) {
+      acc[2] = fma(__ldg(h.aa + id * NR + r + 1), vc[J], acc[2]);
+      acc[3] = fma(__ldg(h.rc + id * NR + r + 1), vh[J], fma(__ldg(h.rs + id * NR + r + 1), vs[J], acc[3]));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+}
+
+// a detector's part of lnL: HR + HH / 2 without the over-counted edges
+__device__ __forceinline__ double het_part(const double* a) { return (a[1] - a[3]) + 0.5 * (a[0] - a[2]); }
+
+// lnL of one set by one warp: phase 1 over the warp's lanes, then phase 2 detector by detector
 template <int PREC>
 __device__ __forceinline__ void het_warp(const PhdRec& c, const NetGeom& g, const HetData& h, double* sm,
                                          double* out) {
-  het_points<PREC>(c, g, h, sm, threadIdx.x & 31, 32);
+  for (int j = threadIdx.x & 31; j < h.M; j += 32) het_point<PREC>(c, g, h, het_pre<PREC>(g, h, j), sm, j);
   __syncwarp();
-  het_regions(g, h, sm, out);
+  double L = h.logLb;
+  for (int id = 0; id < g.nifo; id++) {
+    double acc[4];
+    het_detector(g, h, sm, id, nullptr, acc);
+    L -= het_part(acc);
+  }
+  if ((threadIdx.x & 31) == 0) *out = L;
 }
 
 // the warp's record into its shared memory
@@ -2494,14 +3014,22 @@ size_t het_smem_bytes(const NetGeom& g, const HetData& h) {
   return (size_t)het_warp_doubles(g.nifo, h.M) * sizeof(double);
 }
 
-// Heterodyned lnL of a few sets (the reference-signature calls, alone or merged): one block per
-// set, phase 1 over all the block's threads (one grid point each while M <= blockDim), then phase 2
-// by warp 0 exactly as k_lnl_het's warp does it, so both kernels give the same bits.  The block's
-// shared memory: the record, then [3][nifo][M] doubles.
+// Heterodyned lnL of a few sets (the reference-signature calls, alone or merged): one block per set, phase
+// 1 over all the block's threads (one grid point each while M <= blockDim), then phase 2 with a warp per
+// detector, by the code and in the order of k_lnl_het's warp, so both kernels give the same bits.  What does
+// not depend on the set (the grid points' and regions' tables) is loaded while the kernel waits for the
+// setup.  The block's shared memory: the record, then [3][nifo][M] doubles.
 template <int PREC>
 __global__ void __launch_bounds__(128) k_lnl_het_wide(const PhdRec* __restrict__ recs, const int* __restrict__ status,
                                                      NetGeom g, HetData h, int B, double* __restrict__ lnl) {
   extern __shared__ __align__(16) double sm[];
+  __shared__ double s_part[kMaxIfo];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool mine = (int)threadIdx.x < h.M, have = h.J == 2 && w < g.nifo;
+  HetPre pre;
+  HetRegion reg;
+  if (mine) pre = het_pre<PREC>(g, h, threadIdx.x);
+  if (have && lane < h.NR) reg.load(h, g.nifo, w, lane);
   pdl_wait();          // records of the setup
   const int b = blockIdx.x;
   if (b >= B) return;
@@ -2512,9 +3040,22 @@ __global__ void __launch_bounds__(128) k_lnl_het_wide(const PhdRec* __restrict__
   const double* src = reinterpret_cast<const double*>(recs + b);
   for (int k = threadIdx.x; k < kRecDoubles; k += blockDim.x) sm[k] = src[k];
   __syncthreads();
-  het_points<PREC>(*reinterpret_cast<const PhdRec*>(sm), g, h, sm + kRecDoubles, threadIdx.x, blockDim.x);
+  const PhdRec& c = *reinterpret_cast<const PhdRec*>(sm);
+  if (mine) het_point<PREC>(c, g, h, pre, sm + kRecDoubles, threadIdx.x);
+  for (int j = threadIdx.x + blockDim.x; j < h.M; j += blockDim.x)
+    het_point<PREC>(c, g, h, het_pre<PREC>(g, h, j), sm + kRecDoubles, j);
   __syncthreads();
-  if (threadIdx.x < 32) het_regions(g, h, sm + kRecDoubles, lnl + b);
+  for (int id = w; id < g.nifo; id += blockDim.x >> 5) {
+    double acc[4];
+    het_detector(g, h, sm + kRecDoubles, id, have && id == w ? &reg : nullptr, acc);
+    if (lane == 0) s_part[id] = het_part(acc);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double L = h.logLb;
+    for (int id = 0; id < g.nifo; id++) L -= s_part[id];
+    lnl[b] = L;
+  }
 }
 
 // batches up to this size take k_lnl_het_wide
@@ -2552,7 +3093,7 @@ void launch_lnl_het(const PhdRec* d_recs, const int* d_status, int B, const NetG
   // (early blocks holding SMs slowed it).
   if (B <= kHetWideMaxSets) {
     auto kw = prec == kFP64 ? k_lnl_het_wide<kFP64> : k_lnl_het_wide<kMixed>;
-    const int threads = std::min(128, std::max(32, (h.M + 31) / 32 * 32));
+    const int threads = std::min(128, std::max(32 * g.nifo, (h.M + 31) / 32 * 32));
     launch_pdl(kw, dim3((unsigned)B), dim3(threads), smem, s, d_recs, d_status, g, h, B, d_lnl);
     return;
   }

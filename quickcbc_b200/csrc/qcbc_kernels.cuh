@@ -53,11 +53,12 @@ struct HetData {
   int M, J, NR, MN, MM;
   double logLb;
   const double *freq, *amp, *phase, *IP, *SL, *lc, *ls, *aa, *rc, *rs;
-  // the device's per-bin tables (EventData::tabA/B/C): the mixed form evaluates the waveform at
-  // the grid's bins with the folded polynomials of the mixed full-likelihood kernel
+  // the device's per-bin tables (EventData::tabA/B/C): the waveform at the grid's bins comes from the
+  // folded polynomials of the full-likelihood kernels
   const double2* tabA;
   const double2* tabB;
   const float2* tabC;
+  int tab_n;
 };
 
 enum Precision { kFP64 = 0, kMixed = 1 };
@@ -102,8 +103,9 @@ struct SetupPrefetch {
   const float2* tabC = nullptr;
   int tab_n = 0;                     // entries of each table; bins outside [0, tab_n) are skipped
 };
+// records of the waveform outputs (fullphaseamp, fulltemplates and the grid search)
 void launch_setup(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
-                  int* d_status, cudaStream_t s, int model = kModelFull, const SetupPrefetch& pf = SetupPrefetch{});
+                  int* d_status, cudaStream_t s, int model = kModelFull);
 // Launch order of the sets: the setup files each set under its length class (its bin count in
 // kOrderClasses classes of the band): cnt[c] counts class c, list[c * B + r] is its r-th set (r in
 // no particular order).  Block k of the one-tile lnL launch then takes the k-th set with the
@@ -114,8 +116,11 @@ struct SetOrder {
   int* cnt;        // [kOrderClasses]
   int* list;       // [kOrderClasses][B]
 };
-void launch_setup_ordered(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
-                          int* d_status, const SetOrder& o, cudaStream_t s, int model = kModelFull);
+// records of a likelihood launch; o: files the sets by length when its lists are given
+void launch_setup_lnl(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
+                      int* d_status, cudaStream_t s, int model = kModelFull,
+                      const SetOrder& o = SetOrder{nullptr, nullptr}, const SetupPrefetch& pf = SetupPrefetch{});
+const double* fits_table();      // Table V's coefficients in global memory (QnmTable::fits) on the current device
 void launch_lnl_full(const PhdRec* d_recs, int B, const NetGeom& g, const EventData& ev, Precision prec,
                      const FullLaunch& L, double* d_partials, cudaStream_t s);
 // d_rho: full model rho[id] = HD / sqrt(HH); intrinsic model the per-detector SNR^2 = 2 (HD - HH/2)
