@@ -525,9 +525,22 @@ extern "C" long long qcbc_event_device_bytes(const qcbc_event* ev) {
 // over resident blocks; below one wave an SM runs each block faster the fewer it holds; above, the part of
 // the last wave that is empty is lost.  Several tiles cost 12 % more below a wave (partial sums, no order
 // by length).
+// Few sets take the kernel whose blocks make the records (full_small_fits), where a block's start is the setup:
+// fewer, longer blocks of 256 threads.  One block on two of three SMs is the best count while that leaves a
+// thread a few dozen bins (one set at 4 s: 28.2 us with 12 to 37 tiles, 32 with 8 or 74, 40 with 592; 16 sets at
+// 16 s: 20.6 us with 6 tiles, 22.6 with 18), two per SM beyond (32 sets at 128 s: 65 us with 9 tiles, 74 with 4);
+// above 37 tiles the count of the tiles costs more than the shorter tile gives (one set at 128 s: 32.1 us with
+// 74, 32.4 with 37, 37 with 148).  Against the two launches: 1 to 148 sets at 4 s 1.5 to 5 us less, 1 to 48
+// sets at 128 s 1 to 8 us less; 64 sets and more at 16 s or 128 s are up to 2 us slower, so the line is there.
 static FullLaunch heuristic_launch(const qcbc_event* ev, int B, int prec) {
   FullLaunch L;
   const int bins = std::max(1, ev->g.imax - ev->g.imin);
+  const long long work = (long long)B * bins;
+  if (prec == QCBC_FP64 && (B <= 48 || (B <= 148 && work <= 600000))) {
+    L.threads = 256;
+    L.tiles = std::max(1, std::min({(work <= 300000 ? 96 : 148 * 2) / B, 37, (bins + 255) / 256}));
+    return L;
+  }
   if (prec == QCBC_FP64) {
     constexpr int kThreads = 64, kSlots = 148 * 8;
     const int tmax = std::max(1, bins / kThreads);
@@ -578,17 +591,42 @@ extern "C" int qcbc_get_full_launch(qcbc_event* ev, int B, int precision, int* t
 }
 
 // ------------------------------------------------------------------ full likelihood
+// Do the results of a call lie in its parameters' memory?  Then the setup has to have read them all before the
+// first result is written: its own launch.
+static bool in_place(const double* d_params, size_t n_params, const double* out, size_t n_out) {
+  return out && out < d_params + n_params && d_params < out + n_out;
+}
+
 static int enqueue_full(Workspace* w, qcbc_event* ev, const double* d_params, int B, double* d_lnl, double* d_rho,
                         int prec, cudaStream_t s, const NetGeom& g, cudaEvent_t k0 = nullptr,
-                        cudaEvent_t k1 = nullptr, int model = kModelFull, const FullLaunch* shape = nullptr) {
+                        cudaEvent_t k1 = nullptr, int model = kModelFull, const FullLaunch* shape = nullptr,
+                        const double* h_params = nullptr) {
   FullLaunch L = shape ? *shape : choose_launch(ev, B, prec);
   int rc;
+  const Precision kp = prec == QCBC_MIXED ? kMixed : kFP64;
+  const size_t np = (size_t)B * param_stride(model, g.nifo);
+  if (full_small_fits(B, kp, L) && !in_place(d_params, np, d_lnl, (size_t)B) &&
+      !in_place(d_params, np, d_rho, (size_t)B * g.nifo)) {
+    // each tile's block makes its set's record itself: one launch
+    if ((rc = grow(w->d_part, w->c_part, (size_t)B * L.tiles * 2 * kMaxIfo))) return rc;
+    if (L.tiles > 1) {
+      const size_t had = w->c_done;
+      if ((rc = grow(w->d_done, w->c_done, (size_t)B))) return rc;
+      if (w->c_done != had) CU(cudaMemsetAsync(w->d_done, 0, sizeof(int) * w->c_done, s));
+    }
+    if (k0) cudaEventRecord(k0, s);
+    launch_lnl_full_small(d_params, h_params, B, g, g_dev[current_device()].qnm, event_data(ev), kp, L, w->d_part, d_lnl,
+                          d_rho, model, w->d_done, s);
+    if (k1) cudaEventRecord(k1, s);
+    tls_launches += 1;
+    CU(cudaGetLastError());
+    return QCBC_OK;
+  }
   if ((rc = grow(w->d_recs, w->c_recs, (size_t)B))) return rc;
   if ((rc = grow(w->d_status, w->c_status, (size_t)B))) return rc;
   if ((rc = grow(w->d_part, w->c_part, (size_t)B * L.tiles * 2 * kMaxIfo))) return rc;
   DeviceState& ds = g_dev[current_device()];
   EventData ed = event_data(ev);
-  const Precision kp = prec == QCBC_MIXED ? kMixed : kFP64;
   if (L.tiles == 1) {
     // one tile per set: the sets run in order of length and the lnL kernel finalises each itself
     // The counts start at zero on this call's stream, whatever ran before: repeated calls, calls
@@ -647,7 +685,7 @@ static int run_full(qcbc_event* ev, const double* params, int B, double* lnl, do
   if ((rc = mapped_ptr(w->h_lnl, w->ch_lnl, w->m_lnl, w->m_lnl_of))) return rc;
   if (rho && (rc = mapped_ptr(w->h_rho, w->ch_rho, w->m_rho, w->m_rho_of))) return rc;
   if ((rc = enqueue_full(w, ev, w->m_params, B, w->m_lnl, rho ? w->m_rho : nullptr, prec, s, g, nullptr, nullptr,
-                         model, shape)))
+                         model, shape, w->h_params)))
     return rc;
   CU(cudaStreamSynchronize(s));
   memcpy(lnl, w->h_lnl, sizeof(double) * B);
@@ -843,12 +881,19 @@ extern "C" int qcbc_het_setup(qcbc_event* ev, const double* pref, const int* fgr
 }
 
 static int enqueue_het(Workspace* w, qcbc_event* ev, const double* d_params, int B, double* d_lnl, int prec,
-                       cudaStream_t s, const NetGeom& g) {
+                       cudaStream_t s, const NetGeom& g, const double* h_params = nullptr) {
   int rc;
-  if ((rc = grow(w->d_recs, w->c_recs, (size_t)B))) return rc;
-  if ((rc = grow(w->d_status, w->c_status, (size_t)B))) return rc;
   DeviceState& ds = g_dev[current_device()];
   const HetData hd = het_data(ev);
+  const Precision kp = prec == QCBC_MIXED ? kMixed : kFP64;
+  if (B <= kHetSmallSets && !in_place(d_params, (size_t)B * 11, d_lnl, (size_t)B)) {
+    launch_lnl_het_small(d_params, h_params, B, g, ds.qnm, hd, kp, d_lnl, s);
+    tls_launches += 1;
+    CU(cudaGetLastError());
+    return QCBC_OK;
+  }
+  if ((rc = grow(w->d_recs, w->c_recs, (size_t)B))) return rc;
+  if ((rc = grow(w->d_status, w->c_status, (size_t)B))) return rc;
   // the setup's threads pull the heterodyne tables and the bin tables at the grid's bins into L2 for
   // the heterodyned launch
   SetupPrefetch pf;
@@ -861,7 +906,7 @@ static int enqueue_het(Workspace* w, qcbc_event* ev, const double* d_params, int
   pf.tabC = prec == QCBC_MIXED ? hd.tabC : nullptr;
   pf.tab_n = hd.tab_n;
   launch_setup_lnl(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, kModelFull, SetOrder{nullptr, nullptr}, pf);
-  launch_lnl_het(w->d_recs, w->d_status, B, g, hd, prec == QCBC_MIXED ? kMixed : kFP64, d_lnl, s);
+  launch_lnl_het(w->d_recs, w->d_status, B, g, hd, kp, d_lnl, s);
   tls_launches += 2;
   CU(cudaGetLastError());
   return QCBC_OK;
@@ -883,7 +928,7 @@ extern "C" int qcbc_lnl_het(qcbc_event* ev, const double* params, int B, double*
   // writes lnL into, the pinned staging buffers through their mapped addresses (no copy calls)
   if ((rc = mapped_ptr(w->h_params, w->ch_params, w->m_params, w->m_params_of))) return rc;
   if ((rc = mapped_ptr(w->h_lnl, w->ch_lnl, w->m_lnl, w->m_lnl_of))) return rc;
-  if ((rc = enqueue_het(w, ev, w->m_params, B, w->m_lnl, precision, s, ev->g))) return rc;
+  if ((rc = enqueue_het(w, ev, w->m_params, B, w->m_lnl, precision, s, ev->g, w->h_params))) return rc;
   CU(cudaStreamSynchronize(s));
   memcpy(lnl, w->h_lnl, sizeof(double) * B);
   // a set fails the setup exactly when its lnL is the rejected-sample value

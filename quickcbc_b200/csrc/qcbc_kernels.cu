@@ -19,6 +19,7 @@
 #include <cooperative_groups.h>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 
 namespace qcbc {
 
@@ -894,6 +895,10 @@ struct SetupVals {
   int br, ev, live, lo, hi, st;
 };
 constexpr int kLnlSets = 4, kLnlLanes = 8, kLnlThreads = 128;
+// the block's sets (a kernel that makes one set's record uses the first): at a fixed place, so that the
+// out-of-line setup addresses it directly
+__shared__ __align__(16) PhdRec s_set_rec[kLnlSets];
+__shared__ SetupVals s_set[kLnlSets];
 
 __device__ __forceinline__ double lane_of(double v, int src) { return __shfl_sync(0xffffffffu, v, src, kLnlLanes); }
 
@@ -931,13 +936,19 @@ __device__ __forceinline__ SetMass set_masses(const double* p, int l) {
   return m;
 }
 
-// fit k of Table V at (eta, chi) from the block's copy of the coefficients
-__device__ __forceinline__ double fit_lane(const double* s_fits, int k, double eta, double chi) {
-  const double* t = s_fits + 11 * k;
-  const double xi = -1 + chi, xi2 = xi * xi, xi3 = xi2 * xi, e2 = eta * eta;
-  return t[0] + t[1] * eta + (t[2] + t[3] * eta + t[4] * e2) * xi + (t[5] + t[6] * eta + t[7] * e2) * xi2 +
-         (t[8] + t[9] * eta + t[10] * e2) * xi3;
-}
+// a lane's fit of Table V: its coefficients, loaded ahead of their use
+struct FitLane {
+  double t[11];
+  __device__ __forceinline__ void load(const double* fits, int k) {
+#pragma unroll
+    for (int j = 0; j < 11; j++) t[j] = __ldg(fits + 11 * k + j);
+  }
+  __device__ __forceinline__ double at(double eta, double chi) const {
+    const double xi = -1 + chi, xi2 = xi * xi, xi3 = xi2 * xi, e2 = eta * eta;
+    return t[0] + t[1] * eta + (t[2] + t[3] * eta + t[4] * e2) * xi + (t[5] + t[6] * eta + t[7] * e2) * xi2 +
+           (t[8] + t[9] * eta + t[10] * e2) * xi3;
+  }
+};
 
 // phi_ins at f with t = f^{1/3}, rt = 1/t and log v given
 __device__ __forceinline__ double phi_ins_roots(const PhdRec& c, double f, double t, double rt, double logv) {
@@ -948,7 +959,12 @@ __device__ __forceinline__ double phi_ins_roots(const PhdRec& c, double f, doubl
 }
 
 // warp 0 until the first barrier
-__device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const double* s_fits, const QnmTable& q, int l) {
+__device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const QnmTable& q, int l) {
+  // gamma_1..3, alpha_1..5 by lane, then beta_1..3
+  static_assert(F_GAM2 == F_GAM1 + 1 && F_GAM3 == F_GAM1 + 2 && F_AL5 == F_AL1 + 4 && F_BE3 == F_BE1 + 2, "lane order");
+  FitLane ta, tb;
+  ta.load(q.fits, l < 3 ? F_GAM1 + l : F_AL1 + l - 3);
+  tb.load(q.fits, F_BE1 + (l < 3 ? l : 0));
   const SetMass m = set_masses(x.p, l);
   const double eta = m.eta, e2 = eta * eta, e3 = e2 * eta, e4 = e3 * eta;
   // final spin and radiated energy (eqs. 3.6-3.8 of arXiv:1508.07250); the latter as a quotient er = N / D
@@ -984,10 +1000,7 @@ __device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const do
   const double N = (0.055974469826360077 * eta + 0.5809510763115132 * e2 - 0.9606726679372312 * e3 + 3.352411249771192 * e4) *
                    (aq + (-0.0030302335878845507 - 2.0066110851351073 * eta + 7.7050567802399215 * e2) * sp);
   const double D = aq + (-0.6714403054720589 - 1.4756929437702908 * eta + 7.304676214885011 * e2) * sp;
-  // gamma_1..3, alpha_1..5 by lane, then beta_1..3
-  static_assert(F_GAM2 == F_GAM1 + 1 && F_GAM3 == F_GAM1 + 2 && F_AL5 == F_AL1 + 4 && F_BE3 == F_BE1 + 2, "lane order");
-  const double fa = fit_lane(s_fits, l < 3 ? F_GAM1 + l : F_AL1 + l - 3, eta, m.chi);
-  const double fb = fit_lane(s_fits, F_BE1 + (l < 3 ? l : 0), eta, m.chi);
+  const double fa = ta.at(eta, m.chi), fb = tb.at(eta, m.chi);
   const double g1 = lane_of(fa, 0), g2 = lane_of(fa, 1), g3 = lane_of(fa, 2);
   const double al1 = lane_of(fa, 3), al2 = lane_of(fa, 4), al3 = lane_of(fa, 5), al4 = lane_of(fa, 6), al5 = lane_of(fa, 7);
   const double b1 = lane_of(fb, 0), b2 = lane_of(fb, 1), b3 = lane_of(fb, 2);
@@ -1120,10 +1133,12 @@ __device__ __forceinline__ void setup_project(PhdRec& c, SetupVals& x, int model
 // warp 2 until the first barrier: rho/sigma/v2 fits, a0 and the analytic amplitude prefactors (Appendix B of
 // arXiv:1508.07253), TaylorF2 with its aligned-spin terms but the 3PN spin-spin term PhenomD was not tuned
 // with, and the inspiral phase prefactors (phd_amp_prefactors, phd_taylorf2 without their divisions)
-__device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const double* s_fits, int l) {
-  const SetMass m = set_masses(x.p, l);
+__device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const QnmTable& q, int l) {
   static_assert(F_RHO3 == F_RHO1 + 2 && F_SI4 == F_SI1 + 3, "lane order");
-  const double fv = fit_lane(s_fits, l < 3 ? F_RHO1 + l : l < 7 ? F_SI1 + l - 3 : F_V2, m.eta, m.chi);
+  FitLane tf;
+  tf.load(q.fits, l < 3 ? F_RHO1 + l : l < 7 ? F_SI1 + l - 3 : F_V2);
+  const SetMass m = set_masses(x.p, l);
+  const double fv = tf.at(m.eta, m.chi);
   const double s1 = lane_of(fv, 3), s2 = lane_of(fv, 4), s3 = lane_of(fv, 5), s4 = lane_of(fv, 6);
   c.ai[5] = lane_of(fv, 0);
   c.ai[6] = lane_of(fv, 1);
@@ -1217,12 +1232,16 @@ __device__ __forceinline__ void setup_scales(PhdRec& c, SetupVals& x, int l) {
 }
 
 // A block's sets from their parameters and geometries in s_x to their records in s_rec: 8 lanes of each of
-// four warps per set.  Contains __syncthreads(): every thread of the block calls it.
-__device__ __forceinline__ void setup_roles(PhdRec& c, SetupVals& x, const double* s_fits, const QnmTable& q, int model) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & (kLnlLanes - 1);
-  if (w == 0) setup_ringdown(c, x, s_fits, q, l);
+// four warps per set.  Contains __syncthreads(): every thread of the block calls it.  Out of line, so that
+// every kernel runs the same instructions and a set's record has the same bits wherever it is made.
+// one: the block has one set, and all groups work on it alike.
+__device__ __noinline__ void setup_roles(const QnmTable q, int model, bool one) {
+  const int w = threadIdx.x >> 5, l = threadIdx.x & (kLnlLanes - 1), set = one ? 0 : (threadIdx.x & 31) / kLnlLanes;
+  PhdRec& c = s_set_rec[set];
+  SetupVals& x = s_set[set];
+  if (w == 0) setup_ringdown(c, x, q, l);
   else if (w == 1) setup_project(c, x, model, l);
-  else if (w == 2) setup_inspiral(c, x, s_fits, l);
+  else if (w == 2) setup_inspiral(c, x, q, l);
   else if (w == 3) setup_scales(c, x, l);
   __syncthreads();
   if (w == 0) {
@@ -1259,16 +1278,13 @@ __device__ __forceinline__ void setup_lnl_block(const double* __restrict__ param
                                                 const QnmTable& q, int tile_bins, PhdRec* __restrict__ recs,
                                                 int* __restrict__ status, int* __restrict__ ntile, int model,
                                                 int* __restrict__ ocnt, int* __restrict__ olist) {
-  __shared__ __align__(16) PhdRec s_rec[kLnlSets];
-  __shared__ SetupVals s_x[kLnlSets];
-  __shared__ double s_fits[F_COUNT * 11];
+  SetupVals* s_x = s_set;
   const int b0 = blockIdx.x * kLnlSets, nb = min(kLnlSets, B - b0), tid = threadIdx.x;
   {
     // the block's parameters are contiguous: one load per thread, one round trip also from mapped host
     // memory; a group past the last set repeats that set's (its record is not stored)
     const int ps = geo.stride(model), set = tid / ps, k = tid - set * ps;
     const double v = set < kLnlSets ? params[(size_t)(b0 + min(set, nb - 1)) * ps + k] : 0.0;
-    for (int i = tid; i < F_COUNT * 11; i += kLnlThreads) s_fits[i] = __ldg(q.fits + i);
     if (tid < kLnlSets) {
       NetGeom g;
       int e = -1;
@@ -1285,11 +1301,11 @@ __device__ __forceinline__ void setup_lnl_block(const double* __restrict__ param
     if (set < kLnlSets) s_x[set].p[k] = v;
   }
   __syncthreads();
+  setup_roles(q, model, false);
   const int set = (tid & 31) / kLnlLanes;
-  SetupVals& x = s_x[set];
-  setup_roles(s_rec[set], x, s_fits, q, model);
   if (tid < 32 && (tid & (kLnlLanes - 1)) == 0 && set < nb) {
-    const PhdRec& c = s_rec[set];
+    const SetupVals& x = s_x[set];
+    const PhdRec& c = s_set_rec[set];
     const int b = b0 + set, bins = (c.flags & kRecValid) ? max(0, c.i_hi - c.i_lo + 1) : 0;
     status[b] = x.st;
     if (ntile) ntile[b] = (bins + tile_bins - 1) / tile_bins;
@@ -1299,10 +1315,43 @@ __device__ __forceinline__ void setup_lnl_block(const double* __restrict__ param
     }
   }
   // the block's records are contiguous in shared and in global memory
-  const int4* src = reinterpret_cast<const int4*>(s_rec);
+  const int4* src = reinterpret_cast<const int4*>(s_set_rec);
   int4* dst = reinterpret_cast<int4*>(recs + b0);
   const int words = nb * (int)(sizeof(PhdRec) / 16);
   for (int i = tid; i < words; i += kLnlThreads) dst[i] = src[i];
+}
+
+// ---- small batches: the likelihood kernel makes the record itself.
+// A one-set call was two launches: the setup, its record through memory, and a wait of about two microseconds
+// for the first kernel's end before the second could start.  Below, every block of the likelihood kernel runs
+// the setup of its set (the set's four warps; the tiles of a set repeat it, side by side) and goes on with
+// the record in shared memory, and the parameters of up to kPackSets sets come as kernel arguments instead
+// of being read over the host link.  What bounds a call is the serial chain of one set's setup (5.5 us of the
+// kernel's 9.5) and the launch and the wait for it (12 us).  Calls from the host, two launches and now: one set at
+// 4 s 31.2 and 28.3 us, 16 sets 38.5 and 32.3; one heterodyned set 26.4 and 23.8.
+constexpr int kPackSets = 16;
+struct SrcPack {
+  double v[kPackSets * kMaxParams];
+  __device__ __forceinline__ double get(int i) const { return v[i]; }
+};
+struct SrcMem {
+  const double* p;
+  __device__ __forceinline__ double get(int i) const { return p[i]; }
+};
+
+// The record of set b into s_set_rec[0].  Blocks of at least kLnlThreads threads; contains __syncthreads().
+template <class Src>
+__device__ __forceinline__ void setup_one(const Src& src, int b, const NetGeom& g, const QnmTable& q, int model) {
+  const int tid = threadIdx.x, ps = param_stride(model, g.nifo);
+  SetupVals& x = s_set[0];
+  if (tid < ps) x.p[tid] = src.get(b * ps + tid);
+  if (tid == 0) {
+    x.g = g;
+    x.ev = 0;
+    x.live = 1;
+  }
+  __syncthreads();
+  setup_roles(q, model, true);
 }
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may be scheduled while the
@@ -2246,52 +2295,76 @@ __device__ int ordered_set(const FinalOut& fo, int k) {
   return s_set;
 }
 
-// thread 0's block sums of tile t of set b: the set's lnL (its only tile, or its last to finish), or
-// the tile's partials (FinalOut)
+// The sums over a set's tiles by one warp, S[k] in every lane: lane (u, k) adds quantity k of tiles u, u + 4, ...
+// and the four are joined in a fixed order.  One thread that adds them tile by tile takes 80 ns a tile, a fifth
+// of one set's whole launch at 74 tiles.
+template <int NV>
+__device__ __forceinline__ void tile_sums(const double* p, int tiles, double (&S)[2 * kMaxIfo]) {
+  const int lane = threadIdx.x & 31, k = lane & 7;
+  double x = 0.0;
+  if (k < NV) {
+    const double* q = p + (size_t)(lane >> 3) * (2 * kMaxIfo) + k;
+#pragma unroll 8
+    for (int u = lane >> 3; u < tiles; u += 4, q += 8 * kMaxIfo) x += __ldcg(q);
+  }
+  x += __shfl_xor_sync(0xffffffffu, x, 8);
+  x += __shfl_xor_sync(0xffffffffu, x, 16);
+#pragma unroll
+  for (int j = 0; j < 2 * kMaxIfo; j++) S[j] = j < NV ? __shfl_sync(0xffffffffu, x, j) : 0.0;
+}
+
+// By warp 0, whose lane 0 holds the block sums of tile t of set b: the set's lnL (its only tile, or its last to
+// finish), or the tile's partials (FinalOut)
 template <int NIFO>
 __device__ __forceinline__ void finish_tile(const PhdRec& rec, const double* acc, const NetGeom& g,
                                             const EventData& ev, const FinalOut& fo, int b, int tiles, int t,
                                             double* partials) {
+  const int lane = threadIdx.x & 31;
   double* rho_b = fo.rho ? fo.rho + (size_t)b * g.nifo : nullptr;
+  double S[2 * kMaxIfo];
   if (fo.lnl && tiles == 1) {
-    if (!(rec.flags & kRecValid)) {
-      reject_set(g, fo.lnl + b, rho_b);
-      return;
-    }
-    double S[2 * kMaxIfo];
 #pragma unroll
     for (int k = 0; k < 2 * kMaxIfo; k++) S[k] = k < 2 * NIFO ? acc[k] : 0.0;
-    finalize_set(rec, S, g, ev, fo.model, fo.lnl + b, rho_b);
-    return;
-  }
-  double* out = partials + ((size_t)b * tiles + t) * (2 * kMaxIfo);
+  } else {
+    int last = 0;
+    if (lane == 0) {
+      double* out = partials + ((size_t)b * tiles + t) * (2 * kMaxIfo);
 #pragma unroll
-  for (int k = 0; k < 2 * NIFO; k++) out[k] = acc[k];
-  if (!fo.lnl || !fo.done) return;
-  __threadfence();                               // the partials before the count
-  if (atomicAdd(fo.done + b, 1) != tiles - 1) return;
-  __threadfence();                               // every tile's partials after the count
-  fo.done[b] = 0;
-  if (!(rec.flags & kRecValid)) {
-    reject_set(g, fo.lnl + b, rho_b);
-    return;
+      for (int k = 0; k < 2 * NIFO; k++) out[k] = acc[k];
+      if (fo.lnl && fo.done) {
+        __threadfence();                         // the partials before the count
+        last = atomicAdd(fo.done + b, 1) == tiles - 1;
+      }
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();                             // every tile's partials after the count
+    // the same sum in the same order as k_finalize_full
+    tile_sums<2 * NIFO>(partials + (size_t)b * tiles * (2 * kMaxIfo), tiles, S);
+    if (lane == 0) fo.done[b] = 0;
   }
-  // the same sum in the same order as k_finalize_full
-  double S[2 * kMaxIfo];
-#pragma unroll
-  for (int k = 0; k < 2 * kMaxIfo; k++) S[k] = 0.0;
-  for (int u = 0; u < tiles; u++) {
-    const double* p = partials + ((size_t)b * tiles + u) * (2 * kMaxIfo);
-#pragma unroll
-    for (int k = 0; k < 2 * NIFO; k++) S[k] += __ldcg(p + k);
-  }
-  finalize_set(rec, S, g, ev, fo.model, fo.lnl + b, rho_b);
+  if (lane != 0) return;
+  if (!(rec.flags & kRecValid)) reject_set(g, fo.lnl + b, rho_b);
+  else finalize_set(rec, S, g, ev, fo.model, fo.lnl + b, rho_b);
 }
 
 #ifndef QCBC_FP64_REGS
 #define QCBC_FP64_REGS 128     // see the FP64 tile body
 #endif
-template <int PREC, int NIFO>
+template <int NIFO>
+__device__ __forceinline__ void full_tile_fp64(const PhdRec& rec, const NetGeom& g, const EventData& ev, Tab64& tab,
+                                               double* red, const FinalOut& fo, int b, int tiles, int t,
+                                               double* partials) {
+  int i0, i1;
+  tile_range(rec, tiles, t, i0, i1);
+  double acc[2 * NIFO];
+#pragma unroll
+  for (int k = 0; k < 2 * NIFO; k++) acc[k] = 0.0;
+  tile_fp64<NIFO>(rec, g, ev, i0, i1, tab, acc);
+  block_sum<2 * NIFO>(acc, red);
+  if (threadIdx.x < 32) finish_tile<NIFO>(rec, acc, g, ev, fo, b, tiles, t, partials);
+}
+
+template <int NIFO>
 __global__ void __maxnreg__(QCBC_FP64_REGS) k_lnl_full(const PhdRec* __restrict__ recs, NetGeom g, EventData ev, int tiles,
                                                   double* __restrict__ partials, FinalOut fo) {
   __shared__ PhdRec rec;
@@ -2303,14 +2376,18 @@ __global__ void __maxnreg__(QCBC_FP64_REGS) k_lnl_full(const PhdRec* __restrict_
   if (b < 0) return;   // whole block
   load_record(rec, recs + b);
   __syncthreads();
-  int i0, i1;
-  tile_range(rec, tiles, t, i0, i1);
-  double acc[2 * NIFO];
-#pragma unroll
-  for (int k = 0; k < 2 * NIFO; k++) acc[k] = 0.0;
-  tile_fp64<NIFO>(rec, g, ev, i0, i1, tab, acc);
-  block_sum<2 * NIFO>(acc, red);
-  if (threadIdx.x == 0) finish_tile<NIFO>(rec, acc, g, ev, fo, b, tiles, t, partials);
+  full_tile_fp64<NIFO>(rec, g, ev, tab, red, fo, b, tiles, t, partials);
+}
+
+template <int NIFO, class Src>
+__global__ void __maxnreg__(QCBC_FP64_REGS) k_lnl_full_small(const __grid_constant__ Src src, QnmTable q, NetGeom g,
+                                                             EventData ev, int tiles, double* __restrict__ partials,
+                                                             FinalOut fo) {
+  __shared__ Tab64 tab;
+  __shared__ double red[32 * 2 * kMaxIfo];
+  const int b = blockIdx.x / tiles, t = blockIdx.x - b * tiles;
+  setup_one(src, b, g, q, fo.model);
+  full_tile_fp64<NIFO>(s_set_rec[0], g, ev, tab, red, fo, b, tiles, t, partials);
 }
 
 #ifndef QCBC_MIXED_MINBLOCKS
@@ -2371,6 +2448,18 @@ __device__ __forceinline__ void mixed_prefetch(const NetGeom& g, const EventData
 
 // Mixed-precision full lnL over one tile of bins of one parameter set.
 template <int NIFO>
+__device__ __forceinline__ void full_tile_mixed(const PhdRec& rec, const NetGeom& g, const EventData& ev, float2* s_rot,
+                                                double* red, const FinalOut& fo, int b, int tiles, int t,
+                                                double* partials) {
+  int i0, i1;
+  tile_range(rec, tiles, t, i0, i1);
+  double acc[2 * NIFO];
+  tile_mixed_smem<NIFO>(rec, g, ev, i0, i1, s_rot, mixed_nk_cap(g.imax - g.imin, tiles, blockDim.x), NIFO, acc);
+  group_sum<2 * NIFO>(acc, red, blockDim.x);
+  if (threadIdx.x < 32) finish_tile<NIFO>(rec, acc, g, ev, fo, b, tiles, t, partials);
+}
+
+template <int NIFO>
 __global__ void __launch_bounds__(256, QCBC_MIXED_MINBLOCKS) k_lnl_full_mixed(const PhdRec* __restrict__ recs, NetGeom g,
                                                                                EventData ev, int tiles,
                                                                                double* __restrict__ partials,
@@ -2385,12 +2474,19 @@ __global__ void __launch_bounds__(256, QCBC_MIXED_MINBLOCKS) k_lnl_full_mixed(co
   if (b < 0) return;   // whole block
   load_record(rec, recs + b);
   __syncthreads();
-  int i0, i1;
-  tile_range(rec, tiles, t, i0, i1);
-  double acc[2 * NIFO];
-  tile_mixed_smem<NIFO>(rec, g, ev, i0, i1, s_rot, mixed_nk_cap(g.imax - g.imin, tiles, blockDim.x), NIFO, acc);
-  group_sum<2 * NIFO>(acc, red, blockDim.x);
-  if (threadIdx.x == 0) finish_tile<NIFO>(rec, acc, g, ev, fo, b, tiles, t, partials);
+  full_tile_mixed<NIFO>(rec, g, ev, s_rot, red, fo, b, tiles, t, partials);
+}
+
+template <int NIFO, class Src>
+__global__ void __launch_bounds__(256, 2) k_lnl_full_mixed_small(const __grid_constant__ Src src, QnmTable q, NetGeom g,
+                                                                 EventData ev, int tiles, double* __restrict__ partials,
+                                                                 FinalOut fo) {
+  __shared__ double red[32 * 2 * kMaxIfo];
+  extern __shared__ __align__(16) float2 s_rot[];
+  mixed_prefetch<NIFO>(g, ev);
+  const int b = blockIdx.x / tiles, t = blockIdx.x - b * tiles;
+  setup_one(src, b, g, q, fo.model);
+  full_tile_mixed<NIFO>(s_set_rec[0], g, ev, s_rot, red, fo, b, tiles, t, partials);
 }
 
 // rotation-table length per block for a launch: ceil(max bins per tile / threads)
@@ -2415,20 +2511,57 @@ static void launch_full_mixed(const PhdRec* r, int B, const NetGeom& g, const Ev
   }
 }
 
-template <int PREC>
-static void launch_full_prec(const PhdRec* r, int B, const NetGeom& g, const EventData& ev, const FullLaunch& L,
+static void launch_full_fp64(const PhdRec* r, int B, const NetGeom& g, const EventData& ev, const FullLaunch& L,
                              double* part, const FinalOut& fo, cudaStream_t s) {
   dim3 grid((unsigned)(B * L.tiles)), block(L.threads);
-  auto k = g.nifo == 1 ? k_lnl_full<PREC, 1> : (g.nifo == 2 ? k_lnl_full<PREC, 2> : k_lnl_full<PREC, 3>);
+  auto k = g.nifo == 1 ? k_lnl_full<1> : (g.nifo == 2 ? k_lnl_full<2> : k_lnl_full<3>);
   if (fo.order.cnt || fo.done) launch_pdl(k, grid, block, 0, s, r, g, ev, L.tiles, part, fo);
   else k<<<grid, block, 0, s>>>(r, g, ev, L.tiles, part, fo);
+}
+
+// Fits a launch of B sets the kernel that makes its records itself?  Its blocks have to be resident at once
+// (512 threads per SM at 128 registers, two mixed blocks), or the repeated setups add up: 32 sets of 18 tiles at
+// 4 s, more than that, take 48 us against 36 with 4 tiles.
+bool full_small_fits(int B, Precision prec, const FullLaunch& L) {
+  if (L.threads < kLnlThreads) return false;
+  const long long per_sm = prec == kFP64 ? 512 / L.threads : 2;
+  return (long long)B * L.tiles <= 148 * per_sm;
+}
+
+template <class Src>
+static void launch_small_src(const Src& src, int B, const NetGeom& g, const QnmTable& q, const EventData& ev,
+                             Precision prec, const FullLaunch& L, double* part, const FinalOut& fo, cudaStream_t s) {
+  dim3 grid((unsigned)(B * L.tiles)), block(L.threads);
+  if (prec == kFP64) {
+    auto k = g.nifo == 1 ? k_lnl_full_small<1, Src> : (g.nifo == 2 ? k_lnl_full_small<2, Src> : k_lnl_full_small<3, Src>);
+    k<<<grid, block, 0, s>>>(src, q, g, ev, L.tiles, part, fo);
+  } else {
+    auto k = g.nifo == 1 ? k_lnl_full_mixed_small<1, Src>
+                         : (g.nifo == 2 ? k_lnl_full_mixed_small<2, Src> : k_lnl_full_mixed_small<3, Src>);
+    const size_t smem = (size_t)mixed_nk(g, L) * mix_rs(g.nifo) * sizeof(float2) + mixed_state_bytes(L.threads, g.nifo);
+    k<<<grid, block, smem, s>>>(src, q, g, ev, L.tiles, part, fo);
+  }
+}
+
+void launch_lnl_full_small(const double* d_params, const double* h_params, int B, const NetGeom& g, const QnmTable& q,
+                           const EventData& ev, Precision prec, const FullLaunch& L, double* d_partials, double* d_lnl,
+                           double* d_rho, int model, int* d_done, cudaStream_t s) {
+  if (B <= 0) return;
+  const FinalOut fo{d_lnl, d_rho, model, SetOrder{nullptr, nullptr}, B, L.tiles == 1 ? nullptr : d_done};
+  if (h_params && B <= kPackSets) {
+    SrcPack p;
+    memcpy(p.v, h_params, sizeof(double) * B * param_stride(model, g.nifo));
+    launch_small_src(p, B, g, q, ev, prec, L, d_partials, fo, s);
+  } else {
+    launch_small_src(SrcMem{d_params}, B, g, q, ev, prec, L, d_partials, fo, s);
+  }
 }
 
 void launch_lnl_full(const PhdRec* d_recs, int B, const NetGeom& g, const EventData& ev, Precision prec,
                      const FullLaunch& L, double* d_partials, cudaStream_t s) {
   if (B <= 0) return;
   const FinalOut none{nullptr, nullptr, 0, SetOrder{nullptr, nullptr}, B, nullptr};
-  if (prec == kFP64) launch_full_prec<kFP64>(d_recs, B, g, ev, L, d_partials, none, s);
+  if (prec == kFP64) launch_full_fp64(d_recs, B, g, ev, L, d_partials, none, s);
   else launch_full_mixed(d_recs, B, g, ev, L, d_partials, none, s);
 }
 
@@ -2444,35 +2577,33 @@ bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, con
   const FinalOut fo{d_lnl, d_rho, model,
                     (order && L.tiles == 1) ? *order : SetOrder{nullptr, nullptr}, B,
                     L.tiles == 1 ? nullptr : d_done};
-  if (prec == kFP64) launch_full_prec<kFP64>(d_recs, B, g, ev, L, d_partials, fo, s);
+  if (prec == kFP64) launch_full_fp64(d_recs, B, g, ev, L, d_partials, fo, s);
   else launch_full_mixed(d_recs, B, g, ev, L, d_partials, fo, s);
   return true;
 }
 
+// one warp per set
 __global__ void k_finalize_full(const double* __restrict__ partials, const PhdRec* __restrict__ recs,
                                 const int* __restrict__ status, int B, int tiles, NetGeom g, EventData ev,
                                 int model, double* __restrict__ lnl, double* __restrict__ rho) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (b >= B) return;
   double* rho_b = rho ? rho + (size_t)b * g.nifo : nullptr;
-  if (status[b] != kStOK) {
-    reject_set(g, lnl + b, rho_b);
-    return;
-  }
   double S[2 * kMaxIfo];
-  for (int k = 0; k < 2 * kMaxIfo; k++) S[k] = 0.0;
-  for (int t = 0; t < tiles; t++) {
-    const double* p = partials + ((size_t)b * tiles + t) * (2 * kMaxIfo);
-    for (int k = 0; k < 2 * g.nifo; k++) S[k] += p[k];
-  }
-  finalize_set(recs[b], S, g, ev, model, lnl + b, rho_b);
+  const double* p = partials + (size_t)b * tiles * (2 * kMaxIfo);
+  if (g.nifo == 1) tile_sums<2>(p, tiles, S);
+  else if (g.nifo == 2) tile_sums<4>(p, tiles, S);
+  else tile_sums<6>(p, tiles, S);
+  if (lane != 0) return;
+  if (status[b] != kStOK) reject_set(g, lnl + b, rho_b);
+  else finalize_set(recs[b], S, g, ev, model, lnl + b, rho_b);
 }
 
 void launch_finalize_full(const double* d_partials, const PhdRec* d_recs, const int* d_status, int B, int tiles,
                           const NetGeom& g, const EventData& ev, double* d_lnl, double* d_rho,
                           cudaStream_t s, int model) {
   if (B <= 0) return;
-  k_finalize_full<<<(B + 127) / 128, 128, 0, s>>>(d_partials, d_recs, d_status, B, tiles, g, ev,
+  k_finalize_full<<<(B + 3) / 4, 128, 0, s>>>(d_partials, d_recs, d_status, B, tiles, g, ev,
                                                   model, d_lnl, d_rho);
 }
 
@@ -2971,7 +3102,6 @@ __global__ void __launch_bounds__(128, QCBC_HET_MINBLOCKS) k_lnl_het(const PhdRe
                                                  NetGeom g, HetData h, int B, int warp_doubles,
                                                  double* __restrict__ lnl) {
   extern __shared__ __align__(16) double sm[];
-  pdl_wait();          // records of the setup (immediate when launched the ordinary way)
   const int w = threadIdx.x >> 5;
   const int b = blockIdx.x * (blockDim.x >> 5) + w;
   if (b >= B) return;                // the whole warp leaves; no block barrier follows
@@ -3014,40 +3144,35 @@ size_t het_smem_bytes(const NetGeom& g, const HetData& h) {
   return (size_t)het_warp_doubles(g.nifo, h.M) * sizeof(double);
 }
 
-// Heterodyned lnL of a few sets (the reference-signature calls, alone or merged): one block per set, phase
-// 1 over all the block's threads (one grid point each while M <= blockDim), then phase 2 with a warp per
-// detector, by the code and in the order of k_lnl_het's warp, so both kernels give the same bits.  What does
-// not depend on the set (the grid points' and regions' tables) is loaded while the kernel waits for the
-// setup.  The block's shared memory: the record, then [3][nifo][M] doubles.
-template <int PREC>
-__global__ void __launch_bounds__(128) k_lnl_het_wide(const PhdRec* __restrict__ recs, const int* __restrict__ status,
-                                                     NetGeom g, HetData h, int B, double* __restrict__ lnl) {
+// Heterodyned lnL of a few sets (the reference-signature calls, alone or merged): one block per set, which
+// makes the set's record, evaluates phase 1 over all its threads (one grid point each while M <= blockDim) and
+// phase 2 with a warp per detector, by the code and in the order of k_lnl_het's warp, so both kernels give the
+// same bits.  What does not depend on the set (the grid points' and regions' tables) is loaded first, under
+// the parameters' way in.  Dynamic shared memory: [3][nifo][M] doubles.
+template <int PREC, class Src>
+__global__ void __launch_bounds__(128) k_lnl_het_small(const __grid_constant__ Src src, QnmTable q, NetGeom g, HetData h,
+                                                       double* __restrict__ lnl) {
   extern __shared__ __align__(16) double sm[];
   __shared__ double s_part[kMaxIfo];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.x;
   const bool mine = (int)threadIdx.x < h.M, have = h.J == 2 && w < g.nifo;
   HetPre pre;
   HetRegion reg;
   if (mine) pre = het_pre<PREC>(g, h, threadIdx.x);
   if (have && lane < h.NR) reg.load(h, g.nifo, w, lane);
-  pdl_wait();          // records of the setup
-  const int b = blockIdx.x;
-  if (b >= B) return;
-  if (status[b] != kStOK) {
+  setup_one(src, b, g, q, kModelFull);
+  const PhdRec& c = s_set_rec[0];
+  if (s_set[0].st != kStOK) {    // the whole block
     if (threadIdx.x == 0) lnl[b] = -1.0e20;
     return;
   }
-  const double* src = reinterpret_cast<const double*>(recs + b);
-  for (int k = threadIdx.x; k < kRecDoubles; k += blockDim.x) sm[k] = src[k];
-  __syncthreads();
-  const PhdRec& c = *reinterpret_cast<const PhdRec*>(sm);
-  if (mine) het_point<PREC>(c, g, h, pre, sm + kRecDoubles, threadIdx.x);
+  if (mine) het_point<PREC>(c, g, h, pre, sm, threadIdx.x);
   for (int j = threadIdx.x + blockDim.x; j < h.M; j += blockDim.x)
-    het_point<PREC>(c, g, h, het_pre<PREC>(g, h, j), sm + kRecDoubles, j);
+    het_point<PREC>(c, g, h, het_pre<PREC>(g, h, j), sm, j);
   __syncthreads();
   for (int id = w; id < g.nifo; id += blockDim.x >> 5) {
     double acc[4];
-    het_detector(g, h, sm + kRecDoubles, id, have && id == w ? &reg : nullptr, acc);
+    het_detector(g, h, sm, id, have && id == w ? &reg : nullptr, acc);
     if (lane == 0) s_part[id] = het_part(acc);
   }
   __syncthreads();
@@ -3058,8 +3183,6 @@ __global__ void __launch_bounds__(128) k_lnl_het_wide(const PhdRec* __restrict__
   }
 }
 
-// batches up to this size take k_lnl_het_wide
-constexpr int kHetWideMaxSets = 128;
 
 // sets per block: four warps while their shared memory stays within 96 KB
 static int het_sets_per_block(size_t warp_bytes) {
@@ -3087,18 +3210,23 @@ void launch_lnl_het(const PhdRec* d_recs, const int* d_status, int B, const NetG
   const int spb = het_sets_per_block(smem);
   const int wd = het_warp_doubles(g.nifo, h.M);
   const unsigned grid = (unsigned)((B + spb - 1) / spb);
-  // A small batch (the reference-signature calls, merged or not) takes a block per set and is
-  // launched with programmatic dependent launch after the setup, so its blocks wait on the SMs
-  // instead of behind a launch gap; a large one takes a warp per set, launched the ordinary way
-  // (early blocks holding SMs slowed it).
-  if (B <= kHetWideMaxSets) {
-    auto kw = prec == kFP64 ? k_lnl_het_wide<kFP64> : k_lnl_het_wide<kMixed>;
-    const int threads = std::min(128, std::max(32 * g.nifo, (h.M + 31) / 32 * 32));
-    launch_pdl(kw, dim3((unsigned)B), dim3(threads), smem, s, d_recs, d_status, g, h, B, d_lnl);
-    return;
-  }
   auto k = prec == kFP64 ? k_lnl_het<kFP64> : k_lnl_het<kMixed>;
   k<<<grid, 32 * spb, spb * smem, s>>>(d_recs, d_status, g, h, B, wd, d_lnl);
+}
+
+void launch_lnl_het_small(const double* d_params, const double* h_params, int B, const NetGeom& g, const QnmTable& q,
+                          const HetData& h, Precision prec, double* d_lnl, cudaStream_t s) {
+  if (B <= 0) return;
+  const size_t smem = het_smem_bytes(g, h) - kRecDoubles * sizeof(double);
+  if (h_params && B <= kPackSets) {
+    SrcPack p;
+    memcpy(p.v, h_params, sizeof(double) * 11 * B);
+    auto k = prec == kFP64 ? k_lnl_het_small<kFP64, SrcPack> : k_lnl_het_small<kMixed, SrcPack>;
+    k<<<(unsigned)B, kLnlThreads, smem, s>>>(p, q, g, h, d_lnl);
+  } else {
+    auto k = prec == kFP64 ? k_lnl_het_small<kFP64, SrcMem> : k_lnl_het_small<kMixed, SrcMem>;
+    k<<<(unsigned)B, kLnlThreads, smem, s>>>(SrcMem{d_params}, q, g, h, d_lnl);
+  }
 }
 
 // ---------------------------------------------------------------- heterodyne-grid waveforms, het_diff, Fisher_Het
@@ -4228,8 +4356,16 @@ void allow_dynamic_smem() {
   allow((const void*)k_lnl_het_multi<kMixed>);
   allow((const void*)k_lnl_het<kFP64>);
   allow((const void*)k_lnl_het<kMixed>);
-  allow((const void*)k_lnl_het_wide<kFP64>);
-  allow((const void*)k_lnl_het_wide<kMixed>);
+  allow((const void*)k_lnl_het_small<kFP64, SrcPack>);
+  allow((const void*)k_lnl_het_small<kMixed, SrcPack>);
+  allow((const void*)k_lnl_het_small<kFP64, SrcMem>);
+  allow((const void*)k_lnl_het_small<kMixed, SrcMem>);
+  allow((const void*)k_lnl_full_mixed_small<1, SrcPack>);
+  allow((const void*)k_lnl_full_mixed_small<2, SrcPack>);
+  allow((const void*)k_lnl_full_mixed_small<3, SrcPack>);
+  allow((const void*)k_lnl_full_mixed_small<1, SrcMem>);
+  allow((const void*)k_lnl_full_mixed_small<2, SrcMem>);
+  allow((const void*)k_lnl_full_mixed_small<3, SrcMem>);
 }
 
 }  // namespace qcbc

@@ -136,11 +136,23 @@ void launch_finalize_full(const double* d_partials, const PhdRec* d_recs, const 
 bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, const NetGeom& g, const EventData& ev,
                            Precision prec, const FullLaunch& L, double* d_partials, double* d_lnl, double* d_rho,
                            int model, const SetOrder* order, cudaStream_t s, int* d_done = nullptr);
+// The same for a batch small enough (full_small_fits) that each tile's block makes its set's record itself:
+// one launch, no records.  h_params, when given, are the same parameters on the host: those of up to 16
+// sets travel as kernel arguments.  d_partials and d_done as above (unused at one tile per set).
+bool full_small_fits(int B, Precision prec, const FullLaunch& L);
+void launch_lnl_full_small(const double* d_params, const double* h_params, int B, const NetGeom& g, const QnmTable& q,
+                           const EventData& ev, Precision prec, const FullLaunch& L, double* d_partials, double* d_lnl,
+                           double* d_rho, int model, int* d_done, cudaStream_t s);
 // fill the per-bin tables for bins [0, n)
 void launch_fill_bin_tables(double2* d_tabA, double2* d_tabB, float2* d_tabC, double2* d_tabD, int n,
                             cudaStream_t s);
 void launch_lnl_het(const PhdRec* d_recs, const int* d_status, int B, const NetGeom& g, const HetData& h,
                     Precision prec, double* d_lnl, cudaStream_t s);
+// the same with the setup in the kernel, a block per set (batches of at most kHetSmallSets sets); h_params as for
+// launch_lnl_full_small
+constexpr int kHetSmallSets = 128;
+void launch_lnl_het_small(const double* d_params, const double* h_params, int B, const NetGeom& g, const QnmTable& q,
+                          const HetData& h, Precision prec, double* d_lnl, cudaStream_t s);
 // shared memory of one set's warp in the heterodyned kernels (its record and [3][nifo][M] doubles)
 size_t het_smem_bytes(const NetGeom& g, const HetData& h);
 // heterodyned lnL of sets of many events (records from launch_setup_multi); d_het [n_events] (M = 0:
