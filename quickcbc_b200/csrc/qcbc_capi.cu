@@ -1153,27 +1153,26 @@ extern "C" int qcbc_time_lnl_het(qcbc_event* ev, const double* d_params, int B, 
 }
 
 // ================================================================== multi-event batches
-struct MultiGraph {
-  int Bcap = 0, items_cap = 0, tile_bins = 0, threads = 0, blocks = 0;
-  int prec = 0;
-  double* d_params = nullptr; int* d_eof = nullptr; PhdRec* d_recs = nullptr; int* d_status = nullptr;
-  int* d_ntile = nullptr; int* d_off = nullptr; int* d_items = nullptr; int* d_counter = nullptr;
-  double* d_part = nullptr; double* d_lnl = nullptr; double* d_rho = nullptr;
+struct MultiBuf {
+  int Bcap = 0, tile_bins = 0;
+  MultiWork w = {};
+  double* d_params = nullptr; int* d_eof = nullptr; double* d_lnl = nullptr; double* d_rho = nullptr;   // timed runs
+  // pinned staging of the host form, and its device addresses: the setup reads the parameters from, and the
+  // likelihood writes its results into, host memory
   double* h_params = nullptr; int* h_eof = nullptr; double* h_lnl = nullptr; double* h_rho = nullptr;
-  int* h_status = nullptr;
-  cudaGraphExec_t exec_full = nullptr, exec_dev = nullptr;
+  double* m_params = nullptr; int* m_eof = nullptr; double* m_lnl = nullptr; double* m_rho = nullptr;
 };
 
 // Scratch of the heterodyned multi-event path (grown on demand).
 struct HetMultiScratch {
   int cap = 0;
   double* d_params = nullptr; int* d_eof = nullptr; PhdRec* d_recs = nullptr; int* d_status = nullptr;
-  int* d_ntile = nullptr; double* d_lnl = nullptr;
+  double* d_lnl = nullptr;
   double* h_params = nullptr; int* h_eof = nullptr; double* h_lnl = nullptr; int* h_status = nullptr;
 };
 
 static void free_het_scratch(HetMultiScratch& h) {
-  cudaFree(h.d_params); cudaFree(h.d_eof); cudaFree(h.d_recs); cudaFree(h.d_status); cudaFree(h.d_ntile);
+  cudaFree(h.d_params); cudaFree(h.d_eof); cudaFree(h.d_recs); cudaFree(h.d_status);
   cudaFree(h.d_lnl);
   cudaFreeHost(h.h_params); cudaFreeHost(h.h_eof); cudaFreeHost(h.h_lnl); cudaFreeHost(h.h_status);
   h = HetMultiScratch();
@@ -1187,25 +1186,24 @@ struct qcbc_batch {
   std::vector<size_t> het_smem;        // per slot: shared memory of its heterodyned lnL
   HetMultiScratch hs;
   int nh_max = 0;
-  int tile_bins = 2048, threads = 256;
+  // the tiling of a mixed and of an FP64 launch until it is set: bins per tile, threads per block (multi_launch)
+  int tile_bins = 2048, threads = 256, tile64 = 4096, threads64 = 128;
   cudaStream_t stream = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   unsigned char* d_flush = nullptr;
   std::mutex mu;
-  std::map<long long, MultiGraph*> graphs;
+  std::map<long long, MultiBuf*> bufs;       // by (Bcap, tile_bins)
+  std::map<long long, int> blocks;           // resident blocks by (precision, threads, tile_bins)
 };
 
 extern "C" int qcbc_batch_destroy(qcbc_batch* bt);
 
-static void free_graph(MultiGraph* m) {
+static void free_multi(MultiBuf* m) {
   if (!m) return;
-  if (m->exec_full) cudaGraphExecDestroy(m->exec_full);
-  if (m->exec_dev) cudaGraphExecDestroy(m->exec_dev);
-  cudaFree(m->d_params); cudaFree(m->d_eof); cudaFree(m->d_recs); cudaFree(m->d_status); cudaFree(m->d_ntile);
-  cudaFree(m->d_off); cudaFree(m->d_items); cudaFree(m->d_counter); cudaFree(m->d_part); cudaFree(m->d_lnl);
-  cudaFree(m->d_rho);
+  cudaFree(m->w.recs); cudaFree(m->w.status); cudaFree(m->w.sets); cudaFree(m->w.done); cudaFree(m->w.ctl);
+  cudaFree(m->w.items); cudaFree(m->w.part);
+  cudaFree(m->d_params); cudaFree(m->d_eof); cudaFree(m->d_lnl); cudaFree(m->d_rho);
   cudaFreeHost(m->h_params); cudaFreeHost(m->h_eof); cudaFreeHost(m->h_lnl); cudaFreeHost(m->h_rho);
-  cudaFreeHost(m->h_status);
   delete m;
 }
 
@@ -1290,8 +1288,8 @@ extern "C" int qcbc_batch_destroy(qcbc_batch* bt) {
   {
     std::lock_guard<std::mutex> lk(bt->mu);
     cudaStreamSynchronize(bt->stream);
-    for (auto& kv : bt->graphs) free_graph(kv.second);
-    bt->graphs.clear();
+    for (auto& kv : bt->bufs) free_multi(kv.second);
+    bt->bufs.clear();
   }
   cudaFree(bt->d_events);
   cudaFree(bt->d_het);
@@ -1309,8 +1307,8 @@ extern "C" int qcbc_batch_set_tiling(qcbc_batch* bt, int tile_bins, int threads)
   if (tile_bins < 0 || (threads != 0 && threads != 64 && threads != 128 && threads != 256))
     return fail(QCBC_EINVAL, "tile_bins >= 0, threads in {64, 128, 256}");
   std::lock_guard<std::mutex> lk(bt->mu);
-  if (tile_bins > 0) bt->tile_bins = tile_bins;
-  if (threads > 0) bt->threads = threads;
+  if (tile_bins > 0) bt->tile_bins = bt->tile64 = tile_bins;
+  if (threads > 0) bt->threads = bt->threads64 = threads;
   return QCBC_OK;
 }
 
@@ -1321,73 +1319,58 @@ extern "C" int qcbc_batch_get_tiling(qcbc_batch* bt, int* tile_bins, int* thread
   return QCBC_OK;
 }
 
-// Buffers + captured graphs for (Bcap, precision, tiling); caller holds bt->mu.
-static int multi_graph(qcbc_batch* bt, int Bcap, int prec, MultiGraph** out) {
-  long long key = ((long long)Bcap << 24) ^ ((long long)bt->tile_bins << 4) ^ ((long long)bt->threads << 1) ^ prec;
-  auto it = bt->graphs.find(key);
-  if (it != bt->graphs.end()) { *out = it->second; return QCBC_OK; }
-  MultiGraph* m = new MultiGraph();
+// Buffers for up to Bcap sets at the batch's tiling; caller holds bt->mu.
+static int multi_buf(qcbc_batch* bt, int Bcap, int prec, MultiBuf** out) {
+  const int tile_bins = prec == QCBC_MIXED ? bt->tile_bins : bt->tile64;
+  const long long key = ((long long)Bcap << 24) ^ tile_bins;
+  auto it = bt->bufs.find(key);
+  if (it != bt->bufs.end()) { *out = it->second; return QCBC_OK; }
+  const long long tiles_per_set = (bt->nh_max + tile_bins - 1) / tile_bins;
+  const long long cap = (long long)Bcap * tiles_per_set;
+  if (cap > (1LL << 30)) return fail(QCBC_EINVAL, "work list too large");
+  MultiBuf* m = new MultiBuf();
   m->Bcap = Bcap;
-  m->prec = prec;
-  m->tile_bins = bt->tile_bins;
-  m->threads = bt->threads;
-  long long tiles_per_set = (bt->nh_max + m->tile_bins - 1) / m->tile_bins;
-  long long cap = (long long)Bcap * tiles_per_set;
-  if (cap > (1LL << 30)) { delete m; return fail(QCBC_EINVAL, "work list too large"); }
-  m->items_cap = (int)cap;
-  cudaDeviceProp prop;
-  CU(cudaGetDeviceProperties(&prop, bt->device));
-  Precision P = prec == QCBC_MIXED ? kMixed : kFP64;
-  m->blocks = prop.multiProcessorCount * multi_blocks_per_sm(P, m->threads, m->tile_bins);
-  bool ok = cudaMalloc(&m->d_params, sizeof(double) * 11 * Bcap) == cudaSuccess &&
-            cudaMalloc(&m->d_eof, sizeof(int) * Bcap) == cudaSuccess &&
-            cudaMalloc(&m->d_recs, sizeof(PhdRec) * Bcap) == cudaSuccess &&
-            cudaMalloc(&m->d_status, sizeof(int) * Bcap) == cudaSuccess &&
-            cudaMalloc(&m->d_ntile, sizeof(int) * Bcap) == cudaSuccess &&
-            cudaMalloc(&m->d_off, sizeof(int) * (Bcap + 1)) == cudaSuccess &&
-            cudaMalloc(&m->d_items, sizeof(int) * cap) == cudaSuccess &&
-            cudaMalloc(&m->d_counter, sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&m->d_part, sizeof(double) * 2 * kMaxIfo * cap) == cudaSuccess &&
-            cudaMalloc(&m->d_lnl, sizeof(double) * Bcap) == cudaSuccess &&
-            cudaMalloc(&m->d_rho, sizeof(double) * kMaxIfo * Bcap) == cudaSuccess &&
-            cudaMallocHost(&m->h_params, sizeof(double) * 11 * Bcap) == cudaSuccess &&
-            cudaMallocHost(&m->h_eof, sizeof(int) * Bcap) == cudaSuccess &&
-            cudaMallocHost(&m->h_lnl, sizeof(double) * Bcap) == cudaSuccess &&
-            cudaMallocHost(&m->h_rho, sizeof(double) * kMaxIfo * Bcap) == cudaSuccess &&
-            cudaMallocHost(&m->h_status, sizeof(int) * Bcap) == cudaSuccess;
-  if (!ok) { free_graph(m); return fail(QCBC_ENOMEM, "multi-event buffers for B=%d", Bcap); }
-  DeviceState& ds = g_dev[bt->device];
-  cudaStream_t s = bt->stream;
-  for (int with_copies = 1; with_copies >= 0; with_copies--) {
-    cudaGraph_t graph = nullptr;
-    CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    if (with_copies) {
-      cudaMemcpyAsync(m->d_params, m->h_params, sizeof(double) * 11 * Bcap, cudaMemcpyHostToDevice, s);
-      cudaMemcpyAsync(m->d_eof, m->h_eof, sizeof(int) * Bcap, cudaMemcpyHostToDevice, s);
-    }
-    cudaMemsetAsync(m->d_counter, 0, sizeof(int), s);
-    launch_setup_multi(m->d_params, m->d_eof, Bcap, bt->d_events, (int)bt->events.size(), ds.qnm, m->tile_bins,
-                       m->d_recs, m->d_status, m->d_ntile, s);
-    launch_scan_expand(m->d_ntile, Bcap, m->d_off, m->d_items, m->items_cap, s);
-    launch_lnl_multi(m->d_recs, bt->d_events, m->d_off, m->d_items, Bcap, m->tile_bins, m->items_cap, P, m->threads,
-                     m->blocks, m->d_counter, m->d_part, s);
-    launch_finalize_multi(m->d_part, m->d_recs, m->d_status, m->d_off, bt->d_events, Bcap, m->items_cap, m->d_lnl,
-                          m->d_rho, s);
-    if (with_copies) {
-      cudaMemcpyAsync(m->h_lnl, m->d_lnl, sizeof(double) * Bcap, cudaMemcpyDeviceToHost, s);
-      cudaMemcpyAsync(m->h_rho, m->d_rho, sizeof(double) * kMaxIfo * Bcap, cudaMemcpyDeviceToHost, s);
-      cudaMemcpyAsync(m->h_status, m->d_status, sizeof(int) * Bcap, cudaMemcpyDeviceToHost, s);
-    }
-    cudaError_t e = cudaStreamEndCapture(s, &graph);
-    if (e != cudaSuccess) { free_graph(m); return fail(QCBC_ECUDA, "graph capture: %s", cudaGetErrorString(e)); }
-    cudaGraphExec_t exec = nullptr;
-    e = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) { free_graph(m); return fail(QCBC_ECUDA, "graph instantiate: %s", cudaGetErrorString(e)); }
-    if (with_copies) m->exec_full = exec; else m->exec_dev = exec;
-  }
-  bt->graphs[key] = m;
+  m->tile_bins = tile_bins;
+  m->w.items_cap = (int)cap;
+  auto dev = [](auto*& p, size_t n) { return cudaMalloc(&p, n * sizeof(*p)) == cudaSuccess; };
+  auto pin = [](auto*& p, auto*& d, size_t n) {
+    return cudaHostAlloc(&p, n * sizeof(*p), cudaHostAllocMapped) == cudaSuccess &&
+           cudaHostGetDevicePointer((void**)&d, p, 0) == cudaSuccess;
+  };
+  const size_t n = (size_t)Bcap;
+  const bool ok = dev(m->w.recs, n) && dev(m->w.status, n) && dev(m->w.sets, n) && dev(m->w.done, n) &&
+                  dev(m->w.ctl, kMultiKinds + 2) && dev(m->w.items, (size_t)cap) && dev(m->w.part, 2 * kMaxIfo * (size_t)cap) &&
+                  dev(m->d_params, 11 * n) && dev(m->d_eof, n) && dev(m->d_lnl, n) && dev(m->d_rho, kMaxIfo * n) &&
+                  pin(m->h_params, m->m_params, 11 * n) && pin(m->h_eof, m->m_eof, n) && pin(m->h_lnl, m->m_lnl, n) &&
+                  pin(m->h_rho, m->m_rho, kMaxIfo * n);
+  if (!ok) { free_multi(m); return fail(QCBC_ENOMEM, "multi-event buffers for B=%d", Bcap); }
+  memset(m->h_params, 0, sizeof(double) * 11 * n);
+  for (size_t b = 0; b < n; b++) m->h_eof[b] = -1;         // no event, no work
+  bt->bufs[key] = m;
   *out = m;
+  return QCBC_OK;
+}
+
+// Caller holds bt->mu.  A set's tiles depend on its own bins alone, so its lnL does not depend on the other sets.
+// FP64 tiles start as 4096 bins in blocks of 128 threads: a tile's start (record, tables) costs as much as 20 to
+// 30 of its rows, so short tiles and wide blocks lose (24 events of 64 sets: 365 us with 2048 bins and 256
+// threads, 225 with 4096 and 128), but a few sets need several tiles each to fill the chip (3 events of 16 sets: 52
+// us, with 8192 bins 58).  The mixed tiles stay at 2048 bins and 256 threads: its rotations are relative to the
+// tile's start, so other tiles would change the results in FP32's last bits.
+static int multi_launch(qcbc_batch* bt, MultiBuf* m, const double* d_params, const int* d_eof, int B, int prec,
+                        double* d_lnl, double* d_rho, cudaStream_t s) {
+  const Precision P = prec == QCBC_MIXED ? kMixed : kFP64;
+  const int threads = P == kFP64 ? bt->threads64 : bt->threads;
+  int& blocks = bt->blocks[((long long)m->tile_bins << 16) ^ (threads << 1) ^ prec];
+  if (!blocks) {
+    int sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, bt->device));
+    blocks = sms * multi_blocks_per_sm(P, threads, m->tile_bins);
+  }
+  launch_lnl_multi(d_params, d_eof, B, bt->d_events, (int)bt->events.size(), g_dev[bt->device].qnm, P, m->tile_bins,
+                   threads, blocks, m->w, d_lnl, d_rho, s);
+  tls_launches += 3;
+  CU(cudaGetLastError());
   return QCBC_OK;
 }
 
@@ -1395,19 +1378,19 @@ static int bucket_of(int B) { return std::max(256, (B + 255) / 256 * 256); }
 
 static int run_multi(qcbc_batch* bt, const int* event_of, const double* params, int B, double* lnl, double* rho,
                      int precision) {
-  MultiGraph* m = nullptr;
-  int rc = multi_graph(bt, bucket_of(B), precision, &m);
+  MultiBuf* m = nullptr;
+  int rc = multi_buf(bt, bucket_of(B), precision, &m);
   if (rc) return rc;
   memcpy(m->h_params, params, sizeof(double) * 11 * (size_t)B);
   memcpy(m->h_eof, event_of, sizeof(int) * (size_t)B);
-  for (int b = B; b < m->Bcap; b++) m->h_eof[b] = -1;      // padding sets: no event, no work
-  CU(cudaGraphLaunch(m->exec_full, bt->stream));
-  tls_launches += 4;
+  if ((rc = multi_launch(bt, m, m->m_params, m->m_eof, B, precision, m->m_lnl, rho ? m->m_rho : nullptr, bt->stream)))
+    return rc;
   CU(cudaStreamSynchronize(bt->stream));
   memcpy(lnl, m->h_lnl, sizeof(double) * (size_t)B);
   if (rho) memcpy(rho, m->h_rho, sizeof(double) * kMaxIfo * (size_t)B);
+  // a set fails the setup exactly when its lnL is the rejected-sample value
   int bad = 0;
-  for (int b = 0; b < B; b++) bad += m->h_status[b] != 0;
+  for (int b = 0; b < B; b++) bad += lnl[b] == -1.0e20;
   if (bad) return fail(QCBC_EDOM, "%d of %d parameter sets invalid (bad input or event index; lnL=-1e20)", bad, B);
   return QCBC_OK;
 }
@@ -1432,17 +1415,10 @@ extern "C" int qcbc_lnl_multi_dev(qcbc_batch* bt, const int* d_event_of, const d
   if (precision != QCBC_FP64 && precision != QCBC_MIXED) return fail(QCBC_EINVAL, "precision %d", precision);
   if (B <= 0) return B == 0 ? QCBC_OK : fail(QCBC_EINVAL, "B < 0");
   std::lock_guard<std::mutex> lk(bt->mu);
-  MultiGraph* m = nullptr;
-  int rc = multi_graph(bt, bucket_of(B), precision, &m);
+  MultiBuf* m = nullptr;
+  int rc = multi_buf(bt, bucket_of(B), precision, &m);
   if (rc) return rc;
-  cudaStream_t s = stream ? (cudaStream_t)stream : bt->stream;
-  CU(cudaMemcpyAsync(m->d_params, d_params, sizeof(double) * 11 * (size_t)B, cudaMemcpyDeviceToDevice, s));
-  CU(cudaMemcpyAsync(m->d_eof, d_event_of, sizeof(int) * (size_t)B, cudaMemcpyDeviceToDevice, s));
-  if (m->Bcap > B) CU(cudaMemsetAsync(m->d_eof + B, 0xFF, sizeof(int) * (size_t)(m->Bcap - B), s));   // -1: no work
-  CU(cudaGraphLaunch(m->exec_dev, s));
-  CU(cudaMemcpyAsync(d_lnl, m->d_lnl, sizeof(double) * (size_t)B, cudaMemcpyDeviceToDevice, s));
-  tls_launches += 4;
-  return QCBC_OK;
+  return multi_launch(bt, m, d_params, d_event_of, B, precision, d_lnl, nullptr, stream ? (cudaStream_t)stream : bt->stream);
 }
 
 extern "C" int qcbc_lnl_multi_het_dev(qcbc_batch* bt, const int* d_event_of, const double* d_params, int B,
@@ -1461,7 +1437,6 @@ extern "C" int qcbc_lnl_multi_het_dev(qcbc_batch* bt, const int* d_event_of, con
     CU(cudaMalloc(&h.d_eof, n * sizeof(int)));
     CU(cudaMalloc(&h.d_recs, n * sizeof(PhdRec)));
     CU(cudaMalloc(&h.d_status, n * sizeof(int)));
-    CU(cudaMalloc(&h.d_ntile, n * sizeof(int)));
     CU(cudaMalloc(&h.d_lnl, n * sizeof(double)));
     CU(cudaMallocHost(&h.h_params, n * 11 * sizeof(double)));
     CU(cudaMallocHost(&h.h_eof, n * sizeof(int)));
@@ -1472,8 +1447,8 @@ extern "C" int qcbc_lnl_multi_het_dev(qcbc_batch* bt, const int* d_event_of, con
   size_t smem = 0;
   for (size_t k = 0; k < bt->het_smem.size(); k++) smem = std::max(smem, bt->het_smem[k]);
   DeviceState& ds = g_dev[current_device()];
-  launch_setup_multi(d_params, d_event_of, B, bt->d_events, (int)bt->events.size(), ds.qnm, bt->tile_bins, h.d_recs,
-                     h.d_status, h.d_ntile, s);
+  launch_setup_multi(d_params, d_event_of, B, bt->d_events, (int)bt->events.size(), ds.qnm, h.d_recs,
+                     h.d_status, s);
   launch_lnl_het_multi(h.d_recs, h.d_status, B, bt->d_events, bt->d_het, smem,
                        precision == QCBC_MIXED ? kMixed : kFP64, d_lnl, s);
   tls_launches += 2;
@@ -1495,7 +1470,6 @@ extern "C" int qcbc_lnl_multi_het(qcbc_batch* bt, const int* event_of, const dou
     CU(cudaMalloc(&h.d_eof, n * sizeof(int)));
     CU(cudaMalloc(&h.d_recs, n * sizeof(PhdRec)));
     CU(cudaMalloc(&h.d_status, n * sizeof(int)));
-    CU(cudaMalloc(&h.d_ntile, n * sizeof(int)));
     CU(cudaMalloc(&h.d_lnl, n * sizeof(double)));
     CU(cudaMallocHost(&h.h_params, n * 11 * sizeof(double)));
     CU(cudaMallocHost(&h.h_eof, n * sizeof(int)));
@@ -1511,8 +1485,8 @@ extern "C" int qcbc_lnl_multi_het(qcbc_batch* bt, const int* event_of, const dou
   CU(cudaMemcpyAsync(h.d_params, h.h_params, sizeof(double) * 11 * (size_t)B, cudaMemcpyHostToDevice, s));
   CU(cudaMemcpyAsync(h.d_eof, h.h_eof, sizeof(int) * (size_t)B, cudaMemcpyHostToDevice, s));
   DeviceState& ds = g_dev[current_device()];
-  launch_setup_multi(h.d_params, h.d_eof, B, bt->d_events, (int)bt->events.size(), ds.qnm, bt->tile_bins, h.d_recs,
-                     h.d_status, h.d_ntile, s);
+  launch_setup_multi(h.d_params, h.d_eof, B, bt->d_events, (int)bt->events.size(), ds.qnm, h.d_recs,
+                     h.d_status, s);
   launch_lnl_het_multi(h.d_recs, h.d_status, B, bt->d_events, bt->d_het, smem,
                        precision == QCBC_MIXED ? kMixed : kFP64, h.d_lnl, s);
   tls_launches += 2;
@@ -1531,16 +1505,18 @@ extern "C" int qcbc_lnl_multi_het(qcbc_batch* bt, const int* event_of, const dou
 extern "C" int qcbc_time_lnl_multi(qcbc_batch* bt, int B, int precision, int iters, int flush, float* ms) {
   if (!bt || !ms || iters <= 0 || B <= 0) return fail(QCBC_EINVAL, "bad argument");
   std::lock_guard<std::mutex> lk(bt->mu);
-  MultiGraph* m = nullptr;
-  int rc = multi_graph(bt, bucket_of(B), precision, &m);
+  MultiBuf* m = nullptr;
+  int rc = multi_buf(bt, bucket_of(B), precision, &m);
   if (rc) return rc;
+  // the sets of the last call from the host at this size, from device memory
+  CU(cudaMemcpyAsync(m->d_params, m->h_params, sizeof(double) * 11 * (size_t)B, cudaMemcpyHostToDevice, bt->stream));
+  CU(cudaMemcpyAsync(m->d_eof, m->h_eof, sizeof(int) * (size_t)B, cudaMemcpyHostToDevice, bt->stream));
   size_t fb = (size_t)512 << 20;
   if (flush && !bt->d_flush) CU(cudaMalloc(&bt->d_flush, fb));
   for (int it = 0; it < iters; it++) {
     if (flush) CU(cudaMemsetAsync(bt->d_flush, 0x5a, fb, bt->stream));
     CU(cudaEventRecord(bt->e0, bt->stream));
-    CU(cudaGraphLaunch(m->exec_dev, bt->stream));
-    tls_launches += 4;
+    if ((rc = multi_launch(bt, m, m->d_params, m->d_eof, B, precision, m->d_lnl, m->d_rho, bt->stream))) return rc;
     CU(cudaEventRecord(bt->e1, bt->stream));
     CU(cudaEventSynchronize(bt->e1));
     CU(cudaEventElapsedTime(&ms[it], bt->e0, bt->e1));
@@ -1550,7 +1526,8 @@ extern "C" int qcbc_time_lnl_multi(qcbc_batch* bt, int B, int precision, int ite
 
 extern "C" int qcbc_batch_autotune(qcbc_batch* bt, const int* event_of, const double* params, int B, int precision) {
   if (!bt || !event_of || !params || B <= 0) return fail(QCBC_EINVAL, "bad argument");
-  static const int cand[][2] = {{1024, 128}, {2048, 256}, {4096, 256}, {8192, 256}, {2048, 128}, {1024, 256}};
+  static const int cand[][2] = {{1024, 128}, {2048, 256}, {4096, 256}, {8192, 256}, {2048, 128}, {1024, 256},
+                                {4096, 128}, {8192, 128}};
   std::vector<double> lnl(B);
   float best = 1e30f;
   int bt_tiles = bt->tile_bins, bt_threads = bt->threads;
@@ -1559,6 +1536,7 @@ extern "C" int qcbc_batch_autotune(qcbc_batch* bt, const int* event_of, const do
       std::lock_guard<std::mutex> lk(bt->mu);
       bt->tile_bins = c[0];
       bt->threads = c[1];
+      if (precision == QCBC_FP64) { bt->tile64 = c[0]; bt->threads64 = c[1]; }
       int rc = run_multi(bt, event_of, params, B, lnl.data(), nullptr, precision);
       if (rc && rc != QCBC_EDOM) return rc;
     }
@@ -1571,6 +1549,7 @@ extern "C" int qcbc_batch_autotune(qcbc_batch* bt, const int* event_of, const do
   std::lock_guard<std::mutex> lk(bt->mu);
   bt->tile_bins = bt_tiles;
   bt->threads = bt_threads;
+  if (precision == QCBC_FP64) { bt->tile64 = bt_tiles; bt->threads64 = bt_threads; }
   return QCBC_OK;
 }
 

@@ -242,16 +242,32 @@ void launch_het_tables(const PhdRec* d_rec, const NetGeom& g, const HetBuild& q,
 // into tiles of tile_bins bins; the (set, tile) work items are processed by a persistent kernel.
 // A set's tiling depends only on its own bins, so its lnL is the same in any mix of events.
 void launch_setup_multi(const double* d_params, const int* d_event_of, int B, const EventDesc* d_events, int n_events,
-                        const QnmTable& q, int tile_bins, PhdRec* d_recs, int* d_status, int* d_ntile, cudaStream_t s);
-// d_off[0] = 0, d_off[b+1] = d_off[b] + ntile[b]; then d_items[d_off[b] + t] = b
-void launch_scan_expand(const int* d_ntile, int B, int* d_off, int* d_items, int items_cap, cudaStream_t s);
-// persistent kernel: `blocks` blocks pull work items from *d_counter (zeroed by the caller)
-void launch_lnl_multi(const PhdRec* d_recs, const EventDesc* d_events, const int* d_off, const int* d_items, int B,
-                      int tile_bins, int items_cap, Precision prec, int threads, int blocks, int* d_counter,
-                      double* d_partials, cudaStream_t s);
-void launch_finalize_multi(const double* d_partials, const PhdRec* d_recs, const int* d_status, const int* d_off,
-                           const EventDesc* d_events, int B, int items_cap, double* d_lnl, double* d_rho,
-                           cudaStream_t s);
+                        const QnmTable& q, PhdRec* d_recs, int* d_status, cudaStream_t s);
+// The work list.  A tile's kind is the number of detectors and the waveform pieces at its first bin: 3 x 5.
+constexpr int kMultiKinds = 15;
+// a set's tiles, its first kind, the slot of its first tile's partials, and for each of its five kinds the tiles
+// [t[k], t[k + 1]) and their place within the kind
+struct MultiSet {
+  int tiles, kind, first, t[6], at[5];
+};
+// tile t of set b, whose `tiles` tiles have their partials from slot `first` on
+struct MultiItem {
+  int b, t, tiles, first;
+};
+// device buffers of a launch of B sets: items_cap >= the sum over the sets of their tiles
+struct MultiWork {
+  PhdRec* recs;
+  MultiSet* sets;
+  int *status, *done;                  // [B] each
+  int* ctl;                            // tiles of each kind, all tiles, the item counter
+  MultiItem* items;                    // [items_cap]
+  double* part;                        // [items_cap][2 kMaxIfo]
+  int items_cap;
+};
+// lnL [B] and (d_rho may be null) rho [B][kMaxIfo]: setup, work list, and a persistent kernel of `blocks` blocks
+void launch_lnl_multi(const double* d_params, const int* d_event_of, int B, const EventDesc* d_events, int n_events,
+                      const QnmTable& q, Precision prec, int tile_bins, int threads, int blocks, const MultiWork& w,
+                      double* d_lnl, double* d_rho, cudaStream_t s);
 int multi_blocks_per_sm(Precision prec, int threads, int tile_bins);
 
 void upload_tables();    // constant-memory tables; call once per device
