@@ -2340,38 +2340,50 @@ __device__ __forceinline__ void tile_sums(const double* p, int tiles, double (&S
   for (int j = 0; j < 2 * kMaxIfo; j++) S[j] = j < NV ? __shfl_sync(0xffffffffu, x, j) : 0.0;
 }
 
+// By the warp that counted a set's last tile.  Out of line: it would cost the tile loops registers.
+template <int NIFO>
+__device__ __noinline__ void finish_set(const PhdRec& rec, const NetGeom& g, const EventData& ev, int model, int* done,
+                                        const double* p, int tiles, double* lnl_b, double* rho_b) {
+  double S[2 * kMaxIfo];
+  __threadfence();                               // every tile's partials after the count
+  tile_sums<2 * NIFO>(p, tiles, S);              // the same sum in the same order as k_finalize_full
+  if ((threadIdx.x & 31) != 0) return;
+  *done = 0;
+  if (!(rec.flags & kRecValid)) reject_set(g, lnl_b, rho_b);
+  else finalize_set(rec, S, g, ev, model, lnl_b, rho_b);
+}
+
 // By warp 0, whose lane 0 holds the block sums of tile t of set b: the set's lnL (its only tile, or its last to
 // finish), or the tile's partials (FinalOut)
 template <int NIFO>
 __device__ __forceinline__ void finish_tile(const PhdRec& rec, const double* acc, const NetGeom& g,
                                             const EventData& ev, const FinalOut& fo, int b, int tiles, int t,
                                             double* partials) {
-  const int lane = threadIdx.x & 31;
   double* rho_b = fo.rho ? fo.rho + (size_t)b * g.nifo : nullptr;
-  double S[2 * kMaxIfo];
   if (fo.lnl && tiles == 1) {
+    if (threadIdx.x != 0) return;
+    if (!(rec.flags & kRecValid)) {
+      reject_set(g, fo.lnl + b, rho_b);
+      return;
+    }
+    double S[2 * kMaxIfo];
 #pragma unroll
     for (int k = 0; k < 2 * kMaxIfo; k++) S[k] = k < 2 * NIFO ? acc[k] : 0.0;
-  } else {
-    int last = 0;
-    if (lane == 0) {
-      double* out = partials + ((size_t)b * tiles + t) * (2 * kMaxIfo);
-#pragma unroll
-      for (int k = 0; k < 2 * NIFO; k++) out[k] = acc[k];
-      if (fo.lnl && fo.done) {
-        __threadfence();                         // the partials before the count
-        last = atomicAdd(fo.done + b, 1) == tiles - 1;
-      }
-    }
-    if (!__shfl_sync(0xffffffffu, last, 0)) return;
-    __threadfence();                             // every tile's partials after the count
-    // the same sum in the same order as k_finalize_full
-    tile_sums<2 * NIFO>(partials + (size_t)b * tiles * (2 * kMaxIfo), tiles, S);
-    if (lane == 0) fo.done[b] = 0;
+    finalize_set(rec, S, g, ev, fo.model, fo.lnl + b, rho_b);
+    return;
   }
-  if (lane != 0) return;
-  if (!(rec.flags & kRecValid)) reject_set(g, fo.lnl + b, rho_b);
-  else finalize_set(rec, S, g, ev, fo.model, fo.lnl + b, rho_b);
+  int last = 0;
+  if (threadIdx.x == 0) {
+    double* out = partials + ((size_t)b * tiles + t) * (2 * kMaxIfo);
+#pragma unroll
+    for (int k = 0; k < 2 * NIFO; k++) out[k] = acc[k];
+    if (fo.lnl && fo.done) {
+      __threadfence();                           // the partials before the count
+      last = atomicAdd(fo.done + b, 1) == tiles - 1;
+    }
+  }
+  if (__shfl_sync(0xffffffffu, last, 0))
+    finish_set<NIFO>(rec, g, ev, fo.model, fo.done + b, partials + (size_t)b * tiles * (2 * kMaxIfo), tiles, fo.lnl + b, rho_b);
 }
 
 #ifndef QCBC_FP64_REGS
@@ -2398,7 +2410,9 @@ __global__ void __maxnreg__(QCBC_FP64_REGS) k_lnl_full(const PhdRec* __restrict_
   __shared__ Tab64 tab;
   __shared__ double red[32 * 2 * kMaxIfo];
   pdl_wait();          // records (and class lists) of the setup
-  const int bi = blockIdx.x / tiles, t = blockIdx.x - bi * tiles;
+  // the same tile of every set before the next tile: blocks that run side by side are then in the same waveform
+  // pieces and read the same bins (600 sets at 16 s: FP64 90.3 -> 86.2 us a call, mixed 74.2 -> 69.3)
+  const int t = blockIdx.x / fo.B, bi = blockIdx.x - t * fo.B;
   const int b = fo.order.cnt ? ordered_set(fo, bi) : bi;
   if (b < 0) return;   // whole block
   load_record(rec, recs + b);
@@ -2412,7 +2426,7 @@ __global__ void __maxnreg__(QCBC_FP64_REGS) k_lnl_full_small(const __grid_consta
                                                              FinalOut fo) {
   __shared__ Tab64 tab;
   __shared__ double red[32 * 2 * kMaxIfo];
-  const int b = blockIdx.x / tiles, t = blockIdx.x - b * tiles;
+  const int t = blockIdx.x / fo.B, b = blockIdx.x - t * fo.B;
   setup_one(src, b, g, q, fo.model);
   full_tile_fp64<NIFO>(s_set_rec[0], g, ev, tab, red, fo, b, tiles, t, partials);
 }
@@ -2496,7 +2510,7 @@ __global__ void __launch_bounds__(256, QCBC_MIXED_MINBLOCKS) k_lnl_full_mixed(co
   extern __shared__ __align__(16) float2 s_rot[];   // [nk][mix_rs(NIFO)], then the threads' state
   mixed_prefetch<NIFO>(g, ev);
   pdl_wait();          // records (and class lists) of the setup
-  const int bi = blockIdx.x / tiles, t = blockIdx.x - bi * tiles;
+  const int t = blockIdx.x / fo.B, bi = blockIdx.x - t * fo.B;
   const int b = fo.order.cnt ? ordered_set(fo, bi) : bi;
   if (b < 0) return;   // whole block
   load_record(rec, recs + b);
@@ -2511,7 +2525,7 @@ __global__ void __launch_bounds__(256, 2) k_lnl_full_mixed_small(const __grid_co
   __shared__ double red[32 * 2 * kMaxIfo];
   extern __shared__ __align__(16) float2 s_rot[];
   mixed_prefetch<NIFO>(g, ev);
-  const int b = blockIdx.x / tiles, t = blockIdx.x - b * tiles;
+  const int t = blockIdx.x / fo.B, b = blockIdx.x - t * fo.B;
   setup_one(src, b, g, q, fo.model);
   full_tile_mixed<NIFO>(s_set_rec[0], g, ev, s_rot, red, fo, b, tiles, t, partials);
 }
