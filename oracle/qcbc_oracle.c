@@ -77,7 +77,8 @@ int ora_set_qnm(const double *a, const double *fr, const double *fd, int n) {
   return 0;
 }
 
-static void qnm_default(void) {
+/* at load: the first evaluations may come from several threads at once */
+__attribute__((constructor)) static void qnm_default(void) {
   if (qnm_n == 0) ora_set_qnm(ORA_QNM_A, ORA_QNM_FRING, ORA_QNM_FDAMP, ORA_QNM_N);
 }
 
