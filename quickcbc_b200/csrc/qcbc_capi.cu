@@ -605,7 +605,7 @@ static int enqueue_full(Workspace* w, qcbc_event* ev, const double* d_params, in
   int rc;
   const Precision kp = prec == QCBC_MIXED ? kMixed : kFP64;
   const size_t np = (size_t)B * param_stride(model, g.nifo);
-  if (full_small_fits(B, kp, L) && !in_place(d_params, np, d_lnl, (size_t)B) &&
+  if (full_small_fits(B, kp, L, g) && !in_place(d_params, np, d_lnl, (size_t)B) &&
       !in_place(d_params, np, d_rho, (size_t)B * g.nifo)) {
     // each tile's block makes its set's record itself: one launch
     if ((rc = grow(w->d_part, w->c_part, (size_t)B * L.tiles * 2 * kMaxIfo))) return rc;
@@ -1408,7 +1408,7 @@ extern "C" int qcbc_lnl_multi(qcbc_batch* bt, const int* event_of, const double*
 
 // Device-buffer forms for callers that keep parameter sets and results on the device (the
 // service's device-resident sampler): no host copies, no synchronisation; work is ordered on
-// `stream`.  Calls on one batch must not overlap (they share the batch's graph buffers).
+// `stream`.  Calls on one batch must not overlap (they share the batch's buffers).
 extern "C" int qcbc_lnl_multi_dev(qcbc_batch* bt, const int* d_event_of, const double* d_params, int B, double* d_lnl,
                                   int precision, void* stream) {
   if (!bt || !d_event_of || !d_params || !d_lnl) return fail(QCBC_EINVAL, "NULL argument");
@@ -2516,7 +2516,7 @@ extern "C" int qcbc_lnl_full_noalloc(qcbc_event* ev, const double* d_params, int
 // tables built by qcbc_het_setup rebuilt about the same reference point and grid
 // (QuickCBC.c:1994-2010).  Tables given by qcbc_het_set are dropped.  Everything is queued on the
 // thread's stream and waited for once: at 128 s, 4096 Hz, three detectors a redraw with its tables
-// takes about 0.14 ms (11.8 ms with two host round trips and the host-side table gathers).
+// takes 0.12 ms (11.8 ms with two host round trips and the host-side table gathers).
 static int event_psd_changed(qcbc_event* ev, Workspace* w) {
   const int nI = ev->g.nifo, nh = ev->nh;
   const int lo = std::max(ev->g.imin, 1), hi = std::min(ev->g.imax, nh);

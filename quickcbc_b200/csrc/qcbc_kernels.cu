@@ -1,13 +1,15 @@
 // CUDA kernels of the QuickCBC likelihood hot path (sm_100a).
 //
-//   k_setup          one block of 4 warps per 32 parameter sets: IMRPhenomD
-//                    coefficients, start/cut-off bins and detector response,
-//                    all FP64, the warps working on independent pieces.
-//   k_lnl_full<P>    fused waveform -> projection -> PSD-weighted inner
-//                    products over one tile of bins of one parameter set; no
-//                    h(f) is written to memory.  P = FP64 or mixed.
+//   k_setup_lnl      records for the likelihoods, 8 lanes per parameter set:
+//                    IMRPhenomD coefficients, start/cut-off bins and detector
+//                    response, all FP64.  k_setup: the waveform kernels' form.
+//   k_lnl_full,      fused waveform -> projection -> PSD-weighted inner
+//   k_lnl_full_mixed products over one tile of bins of one parameter set; no
+//                    h(f) is written to memory.  FP64 or mixed.
+//   k_lnl_*_small    the same for few sets, making the records themselves.
 //   k_finalize_full  fixed-order sum of the tile partials -> lnL, rho.
-//   k_lnl_het<P>     heterodyned likelihood, one block per parameter set.
+//   k_lnl_het<P>     heterodyned likelihood, one warp per parameter set.
+//   k_lnl_multi<P>   many events: a persistent kernel over a work list.
 //   waveform kernels for the reference-signature entry points and the FP64
 //   heterodyne setup sums.
 //
@@ -2563,8 +2565,10 @@ static void launch_full_fp64(const PhdRec* r, int B, const NetGeom& g, const Eve
 // Fits a launch of B sets the kernel that makes its records itself?  Its blocks have to be resident at once
 // (512 threads per SM at 128 registers, two mixed blocks), or the repeated setups add up: 32 sets of 18 tiles at
 // 4 s, more than that, take 48 us against 36 with 4 tiles.
-bool full_small_fits(int B, Precision prec, const FullLaunch& L) {
+bool full_small_fits(int B, Precision prec, const FullLaunch& L, const NetGeom& g) {
   if (L.threads < kLnlThreads) return false;
+  // a long rotation table leaves no room for the setup's shared memory
+  if (prec == kMixed && (size_t)mixed_nk(g, L) * mix_rs(g.nifo) * sizeof(float2) > (size_t)96 << 10) return false;
   const long long per_sm = prec == kFP64 ? 512 / L.threads : 2;
   return (long long)B * L.tiles <= 148 * per_sm;
 }
@@ -3887,7 +3891,7 @@ void launch_fullphaseamp(const double* d_params, const NetGeom& g, const QnmTabl
 // band's raw data and PSD (9.4 MB at 3 x 131 k bins) are read once and the per-bin terms stay in L2.
 // The earlier form wrote the template, amplitude and phase of all N/2 bins to memory in two waveform
 // passes and copied five [nifo][N/2] arrays (31 MB at 128 s, 4096 Hz) to the host to pick out the
-// grid's entries: 11.9 ms per call there against 116 us.
+// grid's entries: 11.3 ms per call there against 109 us.
 
 // Discrete Legendre (Gram) polynomials P_0 .. P_J at point n of U + 1 (recurrence of QuickCBC.c:5055-5094).
 __device__ __forceinline__ void gram_values(int J, int U, int n, double (&P)[4]) {

@@ -139,7 +139,7 @@ bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, con
 // The same for a batch small enough (full_small_fits) that each tile's block makes its set's record itself:
 // one launch, no records.  h_params, when given, are the same parameters on the host: those of up to 16
 // sets travel as kernel arguments.  d_partials and d_done as above (unused at one tile per set).
-bool full_small_fits(int B, Precision prec, const FullLaunch& L);
+bool full_small_fits(int B, Precision prec, const FullLaunch& L, const NetGeom& g);
 void launch_lnl_full_small(const double* d_params, const double* h_params, int B, const NetGeom& g, const QnmTable& q,
                            const EventData& ev, Precision prec, const FullLaunch& L, double* d_partials, double* d_lnl,
                            double* d_rho, int model, int* d_done, cudaStream_t s);

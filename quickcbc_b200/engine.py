@@ -192,7 +192,7 @@ class Batch:
 
     Parameter set b belongs to events[event_of[b]]; networks, durations, sample
     rates and bands may differ between events.  One persistent kernel serves all
-    sets, launched as one captured CUDA graph per call.
+    sets.
     """
 
     def __init__(self, events):
