@@ -622,7 +622,7 @@ def interleaved_stream(q, b, evs, eo, P, Lm):
 
 
 def bench_cfg4_uneven(q):
-    """Config 4: 256 uneven events x (32 chains x 8 proposals) in one graph-captured
+    """Config 4: 256 uneven events x (32 chains x 8 proposals) in one
     persistent launch, autotuned tiling, mixed and FP64."""
     from quickcbc_b200 import synth
 

@@ -94,9 +94,8 @@ int qcbc_lnl_intrinsic(qcbc_event* ev, const double* params, int B, double* lnl,
 /* A batch groups open events (same device) so that parameter sets of different
  * analyses -- differing networks, durations, sample rates and bands -- are
  * evaluated together.  Each set's signal band is cut into tiles of tile_bins
- * bins; a persistent kernel takes (set, tile) work items from a device queue;
- * the sequence (copies, setup, work list, kernel, finalise) is one captured CUDA
- * graph per (batch-size bucket, precision), launched once per call.  A set's
+ * bins; a persistent kernel takes (set, tile) work items from a device queue,
+ * and a set's last tile writes its result: three launches per call.  A set's
  * lnL depends only on its own inputs and the tiling, not on the other sets in
  * the call.  Calls on one batch are serialised internally. */
 typedef struct qcbc_batch qcbc_batch;
@@ -137,7 +136,7 @@ int qcbc_lnl_multi_het_dev(qcbc_batch* batch, const int* d_event_of, const doubl
  * 4 x 4 Jacobian (skydensity_all).  x, y: [11] host arrays (y's angles not wrapped). */
 int qcbc_sky_ring_map(const double* x, double* y, double GMST, int label1, int label2, double rot,
                       double* log_jacobian);
-/* Device time of `iters` graph launches on inputs already uploaded by a previous
+/* Device time of `iters` calls on inputs uploaded from a previous
  * qcbc_lnl_multi call with the same B (no host copies inside the timed span). */
 int qcbc_time_lnl_multi(qcbc_batch* batch, int B, int precision, int iters, int flush_l2, float* ms);
 
