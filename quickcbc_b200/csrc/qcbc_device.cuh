@@ -244,6 +244,55 @@ __device__ __forceinline__ void phd_eval64(const PhdRec& c, double Mf, double& a
   phase = ph - (c.t0 * (Mf - c.MfRef) + c.phi_pre);
 }
 
+// ------------------------------------------------------------- folded coefficients (MixPoly)
+constexpr double kInv2PiD = 0.15915494309189533577;
+constexpr double kLnPi = 1.1447298858494002;
+
+// v as a pair of floats hi + lo (hi = v rounded, lo = the remainder rounded)
+__device__ __forceinline__ void split_f2(double v, float (&p)[2]) {
+  const float hi = (float)v;
+  p[0] = hi;
+  p[1] = (float)(v - (double)hi);
+}
+
+// Phase coefficients of the finished FP64 record (needs pq, alpha/beta, the joins, t0, phi_pre and the mdf
+// scales); rdm = 1 / fDM.  Every lane of a set's group runs this on the one record in shared memory, so nothing
+// here reads what it has written: whatever order the lanes store in, they store the same values.
+__device__ __forceinline__ void mix_phase(PhdRec& c, double rdm) {
+  MixPoly& P = c.mix;
+  const double* q = c.pq;
+  const double K = kInv2PiD, T = c.mdf_third, U = c.mdf_rthird, m = c.mdf, ie = c.inv_eta;
+  const double third = 1.0 / 3.0, lam3 = (c.mdf_log + kLnPi) * third;
+  const double T2 = T * T, U2 = U * U, U3 = U2 * U, U5 = U3 * U2, U9 = U3 * U3 * U3;
+  // the ringdown's linear part, which the other pieces are relative to
+  const double shift = c.t0 * c.MfRef - c.phi_pre;
+  const double R0 = K * (c.C1MRD + shift), Ri = K * (c.al1 * m * ie + c.C2MRD * m - c.t0 * m);
+  P.pins.A0 = K * (q[0] + q[4] * lam3 + shift) - R0;
+  P.pins.At = K * (q[2] * T + q[3] * T * lam3);
+  P.pins.Att = K * (q[1] * T2);
+  P.pins.AtL = K * (q[3] * T * third);
+  P.pins.AL = K * (q[4] * third);
+  P.pins.Au = K * (q[5] * U);
+  P.pins.Auu = K * (q[6] * U2);
+  P.pins.Au3 = K * (q[7] * U3);
+  P.pins.Au5 = K * (q[8] * U5);
+  P.pins.Ai = K * (ie * q[9] * m - c.t0 * m) - Ri;
+  P.pins.Ait = K * (ie * q[10] * T * m);
+  P.pins.Aitt = K * (ie * q[11] * T2 * m);
+  P.pins.Aii = K * (ie * q[12] * m * m);
+  P.pint.B0 = K * (c.b2 * ie * c.mdf_log + c.C1Int + shift) - R0;
+  P.pint.Bi = K * (c.b1 * m * ie + c.C2Int * m - c.t0 * m) - Ri;
+  P.pint.Bu9 = K * (-(c.b3 * third) * U9 * ie);
+  P.pint.BL = K * (c.b2 * ie);
+  P.pmrd.R0 = R0;
+  P.pmrd.Ri = Ri;
+  split_f2(K * (-c.al2 * U3 * ie), P.pmrd.Ru3);
+  split_f2(K * ((4.0 / 3.0) * c.al3 * c.mdf_34 * ie), P.pmrd.Rs);
+  split_f2(K * (c.al4 * ie), P.pmrd.Rat);
+  split_f2(m * rdm, P.pmrd.D1);
+  split_f2(c.al5 * c.fRD * rdm, P.pmrd.D0);
+}
+
 // Reduce x to [-pi, pi] in FP64 with a two-constant 2 pi (|x| < 1e9 keeps it exact to ~1e-15).
 __device__ __forceinline__ double reduce_2pi(double x) {
   constexpr double kInv2Pi = 0.15915494309189533577;

@@ -613,10 +613,6 @@ __device__ __forceinline__ int last_bin_below(const NetGeom& g, double fCut) {
   return hi;
 }
 
-// ---- coefficients of the mixed-precision kernel (MixPoly), from the finished FP64 record
-constexpr double kInv2PiD = 0.15915494309189533577;
-constexpr double kLnPi = 1.1447298858494002;
-
 // smallest bin i >= 0 with Msec f_i >= X (the comparison the FP64 evaluation makes)
 __device__ __forceinline__ int first_bin_mf_at_least(const NetGeom& g, double Msec, double X) {
   double x = X / Msec * g.Tobs;
@@ -625,60 +621,6 @@ __device__ __forceinline__ int first_bin_mf_at_least(const NetGeom& g, double Ms
   for (int k = 0; k < 3 && i > 0 && Msec * bin_freq(g, i - 1) >= X; k++) i--;
   for (int k = 0; k < 3 && !(Msec * bin_freq(g, i) >= X); k++) i++;
   return i;
-}
-
-// v as a pair of floats hi + lo (hi = v rounded, lo = the remainder rounded)
-__device__ __forceinline__ void split_f2(double v, float (&p)[2]) {
-  p[0] = (float)v;
-  p[1] = (float)(v - (double)p[0]);
-}
-
-// inspiral phase but its constant, and the intermediate / ringdown pieces but the parts that
-// need the ringdown join (needs pq, alpha/beta, the intermediate join, t0, the mdf scales); rdm = 1 / fDM
-__device__ __forceinline__ void mix_phase_main(PhdRec& c, double rdm) {
-  MixPoly& P = c.mix;
-  const double* q = c.pq;
-  const double K = kInv2PiD, T = c.mdf_third, U = c.mdf_rthird, m = c.mdf, ie = c.inv_eta;
-  const double third = 1.0 / 3.0, lam3 = (c.mdf_log + kLnPi) * third;
-  const double T2 = T * T, U2 = U * U, U3 = U2 * U, U5 = U3 * U2, U9 = U3 * U3 * U3;
-  P.pins.At = K * (q[2] * T + q[3] * T * lam3);
-  P.pins.Att = K * (q[1] * T2);
-  P.pins.AtL = K * (q[3] * T * third);
-  P.pins.AL = K * (q[4] * third);
-  P.pins.Au = K * (q[5] * U);
-  P.pins.Auu = K * (q[6] * U2);
-  P.pins.Au3 = K * (q[7] * U3);
-  P.pins.Au5 = K * (q[8] * U5);
-  P.pins.Ai = K * (ie * q[9] * m - c.t0 * m);
-  P.pins.Ait = K * (ie * q[10] * T * m);
-  P.pins.Aitt = K * (ie * q[11] * T2 * m);
-  P.pins.Aii = K * (ie * q[12] * m * m);
-  P.pint.Bi = K * (c.b1 * m * ie + c.C2Int * m - c.t0 * m);
-  P.pint.Bu9 = K * (-(c.b3 * third) * U9 * ie);
-  P.pint.BL = K * (c.b2 * ie);
-  split_f2(K * (-c.al2 * U3 * ie), P.pmrd.Ru3);
-  split_f2(K * ((4.0 / 3.0) * c.al3 * c.mdf_34 * ie), P.pmrd.Rs);
-  split_f2(K * (c.al4 * ie), P.pmrd.Rat);
-  split_f2(m * rdm, P.pmrd.D1);
-  split_f2(c.al5 * c.fRD * rdm, P.pmrd.D0);
-}
-
-// the rest of the phase pieces: constants (phi_pre) and the ringdown slope (C2MRD)
-__device__ __forceinline__ void mix_phase_join(PhdRec& c) {
-  MixPoly& P = c.mix;
-  const double K = kInv2PiD, m = c.mdf, ie = c.inv_eta;
-  const double shift = c.t0 * c.MfRef - c.phi_pre;
-  P.pmrd.R0 = K * (c.C1MRD + shift);
-  P.pmrd.Ri = K * (c.al1 * m * ie + c.C2MRD * m - c.t0 * m);
-  P.pins.A0 = K * (c.pq[0] + c.pq[4] * ((c.mdf_log + kLnPi) * (1.0 / 3.0)) + shift) - P.pmrd.R0;
-  P.pint.B0 = K * (c.b2 * ie * c.mdf_log + c.C1Int + shift) - P.pmrd.R0;
-}
-
-// the inspiral and intermediate slopes relative to the ringdown's (after mix_phase_main and
-// mix_phase_join)
-__device__ __forceinline__ void mix_phase_slopes(PhdRec& c) {
-  c.mix.pins.Ai -= c.mix.pmrd.Ri;
-  c.mix.pint.Bi -= c.mix.pmrd.Ri;
 }
 
 // FP32 amplitude coefficients (needs ai, the intermediate Newton form, g1..g3, fDM); rfg = 1 / (fDM g3)
@@ -1079,9 +1021,7 @@ __device__ __forceinline__ void setup_joins(PhdRec& c, SetupVals& x, int model) 
     phr = ie * x.phr + c.C1Int + c.C2Int * f;
   }
   c.phi_pre = 2. * (model == kModelIntrinsic ? x.p[4] : 0.5 * x.p[4]) + phr;
-  mix_phase_main(c, x.rdm);
-  mix_phase_join(c);
-  mix_phase_slopes(c);
+  mix_phase(c, x.rdm);
 }
 
 // warp 1: projection (or the intrinsic model's offsets), fbegin and the first bin above it
