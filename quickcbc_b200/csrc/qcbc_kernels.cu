@@ -17,6 +17,7 @@
 // lnL), 5112-5299 (heterodyne), 5303-5444 (heterodyned lnL); Utilities.c
 // :587-629, 716-736, 995-1109; IMRPhenomD.c:413-563.
 #include "qcbc_kernels.cuh"
+#include "qcbc_math.cuh"
 #include "qcbc_ptstep.h"
 #include <cooperative_groups.h>
 #include <cmath>
@@ -816,9 +817,7 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
 // What bounds a setup is one set's chain of dependent FP64 work, not throughput.  So the lanes of a group
 // share every expensive function: one exp, log, cbrt, atan, sqrt or quotient per step serves up to eight
 // arguments side by side (the values meet by shuffle), the fits take a lane each, and everything else is
-// evaluated by all lanes of the group alike; quotients of ordinary numbers (but the masses') are a reciprocal
-// approximation with one third-order step, a quarter of the division's latency; and the warps take
-// independent pieces:
+// evaluated by all lanes of the group alike; and the warps take independent pieces:
 //           until the first barrier                                  until the second
 //   warp 0  masses, final spin, QNM (one row per 0.001 of spin       joins, phase at fRef, folded phase
 //           holds both cubics it can need), alpha/beta/gamma fits,
@@ -845,14 +844,6 @@ __shared__ __align__(16) PhdRec s_set_rec[kLnlSets];
 __shared__ SetupVals s_set[kLnlSets];
 
 __device__ __forceinline__ double lane_of(double v, int src) { return __shfl_sync(0xffffffffu, v, src, kLnlLanes); }
-
-// 1/x for finite normal x: the hardware's approximation (about 2^-20) and one third-order step
-__device__ __forceinline__ double recip64(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
 
 // masses (Msun) and what follows from them, rounded as set_phys and phd_masses round them: the mixed kernel
 // rounds its coefficients and rotations to floats, so a last bit here can move a rotation by a float's.
@@ -948,18 +939,18 @@ __device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const Qn
   const double g1 = lane_of(fa, 0), g2 = lane_of(fa, 1), g3 = lane_of(fa, 2);
   const double al1 = lane_of(fa, 3), al2 = lane_of(fa, 4), al3 = lane_of(fa, 5), al4 = lane_of(fa, 6), al5 = lane_of(fa, 7);
   const double b1 = lane_of(fb, 0), b2 = lane_of(fb, 1), b3 = lane_of(fb, 2);
-  const double rq = recip64(l == 0 ? eta : l == 1 ? g2 : D - N);
+  const double rq = 1.0 / (l == 0 ? eta : l == 1 ? g2 : D - N);
   const double inv_eta = lane_of(rq, 0), re = D * lane_of(rq, 2), fRD = yr * re, fDM = yd * re, fg = fDM * g3;
   const double root = g2 <= 1 ? sqrt(1 - g2 * g2) : 0.0;
   const double fmax = fabs(fRD + fg * (root - 1.0) * lane_of(rq, 1));
   const double Msec = m.M * kMtsun, mdf = Msec * x.g.df, MfRef = Msec * kFref, fm = 0.5 * fRD, dx = fmax - fRD;
   // the functions at four frequencies side by side: lane 0 fRD/2, 1 fmax, 2 MfRef, 3 Msec df
   const double f = l == 0 ? fm : l == 1 ? fmax : l == 2 ? MfRef : mdf, xr = f - al5 * fRD;
-  const double rr = recip64(l == 0 ? fDM : l == 1 ? fg : dx * dx + fg * fg);
+  const double rr = 1.0 / (l == 0 ? fDM : l == 1 ? fg : dx * dx + fg * fg);
   const double rdm = lane_of(rr, 0), rfg = lane_of(rr, 1);
   const double L = log(f), C = cbrt(f), sq = sqrt(f), f34 = sqrt(f * sq), at = atan(xr * rdm);
   const double v3 = exp(-dx * g2 * rfg) * (fg * g1) * lane_of(rr, 2);
-  const double d3 = recip64(f), r2 = d3 * d3, rx = recip64(fDM * fDM + xr * xr);
+  const double d3 = 1.0 / f, r2 = d3 * d3, rx = 1.0 / (fDM * fDM + xr * xr);
   const double pint = b1 * f - b3 * (1.0 / 3.0) * (r2 * d3) + b2 * L;
   const double dpint = (b1 + b3 * (r2 * r2) + b2 * d3) * inv_eta;
   const double pmrd = -(al2 * d3) + (4.0 / 3.0) * (al3 * f34) + al1 * f + al4 * at;
@@ -986,7 +977,7 @@ __device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const Qn
   x.tref = lane_of(C, 2);
   x.rref = lane_of(d3, 2);
   // scales of Mf = (Msec df) i
-  const double T = lane_of(C, 3), r4 = recip64(l == 0 ? T : mdf * sqrt(T));
+  const double T = lane_of(C, 3), r4 = 1.0 / (l == 0 ? T : mdf * sqrt(T));
   c.mdf_third = T;
   c.mdf_log = lane_of(L, 3);
   c.mdf_34 = lane_of(f34, 3);
@@ -1108,7 +1099,7 @@ __device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const Qn
                          5841690624 * (x1 + x2) * Pi + 21384760320 * Pi2));
   const double m1M = 0.5 * (1.0 + Seta), m2M = 0.5 * (1.0 - Seta), q1 = m1M * m1M * x1s, q2 = m2M * m2M * x2s, xx = x1 * x2;
   const double SL = m1M * m1M * x1 + m2M * m2M * x2, dS = Seta * (m2M * x2 - m1M * x1);
-  const double pf = (3.0 / 128.0) * recip64(eta);
+  const double pf = (3.0 / 128.0) * (1.0 / eta);
   const double sig = eta * (721.0 / 48.0 - 247.0 / 48.0) * xx + ((720.0 - 1.0) / 96.0 - (240.0 - 7.0) / 96.0) * (q1 + q2);
   const double gam = (554345.0 / 1134.0 + 110.0 / 9.0 * eta) * SL + (13915.0 / 84.0 - 10.0 / 3.0 * eta) * dS;
   double v[8], w5, w6;
@@ -1149,11 +1140,11 @@ __device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const Qn
 // warp 2 until the second barrier: the intermediate amplitude's quartic through value and slope at f1 and f3
 // and the value at the middle (phd_amp_int), and the folded amplitude
 __device__ __forceinline__ void setup_amplitude(PhdRec& c, const SetupVals& x) {
-  const double f1 = kAmpJoin, f3 = c.fmax, h = f3 - f1, f2 = f1 + h / 2.0, rh = recip64(h), df3 = f3 - c.fRD,
+  const double f1 = kAmpJoin, f3 = c.fmax, h = f3 - f1, f2 = f1 + h / 2.0, rh = 1.0 / h, df3 = f3 - c.fRD,
                fg = c.fDM * c.g3;
   const Pow6 p1 = c_setup.f1p;
   const double v1 = amp_ins(c, f1, p1), d1 = damp_ins_p(c, f1, p1), v2 = x.v[F_V2], v3 = x.v3;
-  const double d2 = v3 * (-c.g2 * x.rfg - 2.0 * df3 * recip64(df3 * df3 + fg * fg));
+  const double d2 = v3 * (-c.g2 * x.rfg - 2.0 * df3 * (1.0 / (df3 * df3 + fg * fg)));
   const double q12 = (v2 - v1) * (2.0 * rh), q23 = (v3 - v2) * (2.0 * rh);
   const double q012 = (q12 - d1) * (2.0 * rh), q123 = (q23 - q12) * rh, q234 = (d2 - q23) * (2.0 * rh);
   const double q0123 = (q123 - q012) * rh, q1234 = (q234 - q123) * rh;
@@ -1752,61 +1743,12 @@ __device__ __forceinline__ void tile_mixed(const PhdRec& c, const NetGeom& g, co
 // Sets outside the tables' range (a piece order IMRPhenomD does not have, |w| beyond the polynomial,
 // exponents near overflow) take the per-bin functions in the same loop (AP = PP = -1).
 
-// sin and cos of 2 pi t, |t| <= 1/8, and atan(w)/w, |w| <= 0.2645: polynomials in t^2 and w^2,
-// interpolated at Chebyshev nodes in 60-digit arithmetic and rounded; relative errors 3.9e-17, 2.1e-17
-// and 2.5e-17.
-__constant__ double c_sin2pi[7] = {6.283185307179586, -41.341702240399634, 81.60524927594804, -76.70585970427454,
-                                   42.058685020160894, -15.093804209987114, 3.7808689593022957};
-__constant__ double c_cos2pi[8] = {1.0, -19.739208802178716, 64.93939402266795, -85.45681720652271,
-                                   60.244641328867296, -26.426250908622137, 7.903091687751697, -1.6968494702918826};
-__constant__ double c_atan64[9] = {1.0, -0.33333333333330495, 0.19999999998915635, -0.14285714126071508,
-                                   0.11111099310073162, -0.09090417358899357, 0.07680201267088747,
-                                   -0.06490960023860128, 0.04468242583532965};
-constexpr double kAtanRange = 0.2645;
-
-// sin and cos of 2 pi cyc of U values.  Any: cyc may be beyond 2^45, infinite or NaN (the tile's bound on
-// its phase, Tile64, keeps the others below).
-template <int U, bool Any>
-__device__ __forceinline__ void sincos_cycles(const double (&cyc)[U], double (&sv)[U], double (&cv)[U]) {
-  constexpr double kMagic = 6755399441055744.0;         // 1.5 2^52: the add rounds to an integer
-  int k[U];                                             // quadrant
-  double t[U], z[U], s[U], c[U];
-#pragma unroll
-  for (int j = 0; j < U; j++) {
-    double x = cyc[j];
-    if (Any && (__double2hiint(x) & 0x7fffffff) > 0x42c00000) x -= rint(x);
-    const double q = fma(x, 4.0, kMagic);
-    k[j] = __double2loint(q);
-    t[j] = fma(q - kMagic, -0.25, x);
-    z[j] = t[j] * t[j];
-    s[j] = c_sin2pi[6];
-    c[j] = c_cos2pi[7];
-  }
-#pragma unroll
-  for (int m = 6; m >= 0; m--) {
-    const double b = c_cos2pi[m];
-#pragma unroll
-    for (int j = 0; j < U; j++) c[j] = fma(z[j], c[j], b);
-    if (m < 6) {
-      const double a = c_sin2pi[m];
-#pragma unroll
-      for (int j = 0; j < U; j++) s[j] = fma(z[j], s[j], a);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < U; j++) {
-    const double st = s[j] * t[j];
-    const double a = (k[j] & 1) ? c[j] : st, d = (k[j] & 1) ? st : c[j];
-    sv[j] = __hiloint2double(__double2hiint(a) ^ ((k[j] & 2) << 30), __double2loint(a));
-    cv[j] = __hiloint2double(__double2hiint(d) ^ (((k[j] + 1) & 2) << 30), __double2loint(d));
-  }
-}
-__device__ __forceinline__ void sincos_cycles(double cyc, double& sv, double& cv) {
-  const double x[1] = {cyc};
-  double s[1], c[1];
-  sincos_cycles<1, true>(x, s, c);
-  sv = s[0];
-  cv = c[0];
+// 1/x in the tile's ringdown, where x is an ordinary positive number: its tables are used only for |D1| 16 <=
+// kAtanRange, so fDM is at least 60 Msec df, the Lorentzian at least (fDM g3)^2 and 1 + z z_c at least 0.9
+__device__ __forceinline__ double recip_tile(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return recip_newton(x, r);
 }
 
 constexpr int kSeg64 = 64;                 // rows of blockDim.x bins per table segment
@@ -1908,23 +1850,17 @@ __device__ __forceinline__ void step64(const PhdRec& c, const EventData& ev, con
       const double z = fma(xi[j], q.D1, -q.D0), den = fma(z, zc.x, 1.0);
       double rd;
       if (AP == 2) {
-        const double dfr = fma(xi[j], c.mdf, -c.fRD), lor = fma(dfr, dfr, q.fg2), rp = recip64(den * lor);
+        const double dfr = fma(xi[j], c.mdf, -c.fRD), lor = fma(dfr, dfr, q.fg2), rp = recip_tile(den * lor);
         rd = rp * lor;
         amp[j] = (q.E * T.er[p.k + j]) * (rp * den);
       } else {
-        rd = recip64(den);
+        rd = recip_tile(den);
       }
       v[j] = q.dn * rd;
       v2[j] = v[j] * v[j];
       rest[j] = fma(q.Rs, s34[j], fma(u[j], q.Ru3, zc.y));
-      pl[j] = c_atan64[8];
     }
-#pragma unroll
-    for (int k = 7; k >= 0; k--) {
-      const double a = c_atan64[k];
-#pragma unroll
-      for (int j = 0; j < U; j++) pl[j] = fma(v2[j], pl[j], a);
-    }
+    atan_ratio<U>(v2, pl);
 #pragma unroll
     for (int j = 0; j < U; j++) rest[j] = fma(q.Rat * v[j], pl[j], rest[j]);
   } else if (PP == 1) {
