@@ -17,6 +17,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 namespace qcbc {
 
@@ -246,7 +247,55 @@ __device__ __forceinline__ void phd_eval64(const PhdRec& c, double Mf, double& a
 
 // ------------------------------------------------------------- folded coefficients (MixPoly)
 constexpr double kInv2PiD = 0.15915494309189533577;
+constexpr double kInv2PiLo = -9.8393383376096589e-18;        // 1/(2 pi) - kInv2PiD
 constexpr double kLnPi = 1.1447298858494002;
+
+// fl(a b) and what the rounding left (Dekker's product by one fused multiply-add)
+__device__ __forceinline__ double two_prod(double a, double b, double& err) {
+  const double p = a * b;
+  err = fma(a, b, -p);
+  return p;
+}
+
+// What separates r = fl(1/t), t = fl(f^{1/3}), from f^{-1/3} = r (1 + eps): one Newton step of t^3 = f and one of
+// r t = 1, both residuals exact to first order.  rf = 1/f.
+__device__ __forceinline__ double rthird_eps(double f, double rf, double t, double r) {
+  double e2, e3;
+  const double t2 = two_prod(t, t, e2), t3 = two_prod(t2, t, e3);
+  return fma(-t, r, 1.0) - ((f - t3) - fma(e2, t, e3)) * (rf * (1.0 / 3.0));
+}
+
+// The linear phase n (df t - slope) in cycles at whole n, less its whole cycles, to 1e-16 of a cycle: n df t
+// reaches 1e6 cycles, where a rounded product or slope is off by 1e-10 rad, the slope's rounding alike in every bin.
+struct LinPhase {
+  double hi, lo;             // the slope as hi + lo, hi of 32 bits: n hi is exact for n < 2^21
+  __device__ __forceinline__ LinPhase(double df, double t, double slope) {
+    double e;
+    const double p = two_prod(df, t, e);
+    unsigned long long b;
+    const double s = p - slope;
+    memcpy(&b, &s, sizeof(b));
+    b &= ~((1ull << 21) - 1);
+    memcpy(&hi, &b, sizeof(b));
+    lo = ((p - hi) - slope) + e;
+  }
+  __device__ __forceinline__ double cycles(double n) const {
+    double e;
+    const double p = two_prod(n, hi, e), r = (p - rint(p)) + fma(n, lo, e);
+    return r - rint(r);
+  }
+};
+
+// (q + ql) (r (1 + eps))^5 / 2 pi as hi + lo.  The Newtonian phase is up to 1e5 rad where the likelihood
+// feels 1e-13 rad that all bins share, so the rounding of its coefficient must not be five times r's.
+__device__ __forceinline__ double fold_r5(double q, double ql, double r, double eps, double& lo) {
+  double e2, e4, e5, ep, ea;
+  const double r2 = two_prod(r, r, e2), r4 = two_prod(r2, r2, e4), r5 = two_prod(r4, r, e5);
+  e5 = fma(5.0 * eps, r5, fma(fma(2.0 * r2, e2, e4), r, e5));
+  const double p = two_prod(q, r5, ep), a = two_prod(kInv2PiD, p, ea);
+  lo = ea + fma(kInv2PiD, fma(q, e5, fma(ql, r5, ep)), kInv2PiLo * p);
+  return a;
+}
 
 // v as a pair of floats hi + lo (hi = v rounded, lo = the remainder rounded)
 __device__ __forceinline__ void split_f2(double v, float (&p)[2]) {
@@ -255,32 +304,34 @@ __device__ __forceinline__ void split_f2(double v, float (&p)[2]) {
   p[1] = (float)(v - (double)hi);
 }
 
-// Phase coefficients of the finished FP64 record (needs pq, alpha/beta, the joins, t0, phi_pre and the mdf
-// scales); rdm = 1 / fDM.  Every lane of a set's group runs this on the one record in shared memory, so nothing
+// Phase coefficients of the finished FP64 record (needs pq, alpha/beta, the joins, t0 and the mdf scales);
+// rdm = 1 / fDM, eps: of mdf^{-1/3} (rthird_eps), q8lo: of pq[8], shift: t0 MfRef - phi_pre in cycles, any whole
+// number of them left out.  Every lane of a set's group runs this on the one record in shared memory, so nothing
 // here reads what it has written: whatever order the lanes store in, they store the same values.
-__device__ __forceinline__ void mix_phase(PhdRec& c, double rdm) {
+__device__ __forceinline__ void mix_phase(PhdRec& c, double rdm, double eps, double q8lo, double shift) {
   MixPoly& P = c.mix;
   const double* q = c.pq;
   const double K = kInv2PiD, T = c.mdf_third, U = c.mdf_rthird, m = c.mdf, ie = c.inv_eta;
   const double third = 1.0 / 3.0, lam3 = (c.mdf_log + kLnPi) * third;
-  const double T2 = T * T, U2 = U * U, U3 = U2 * U, U5 = U3 * U2, U9 = U3 * U3 * U3;
+  const double T2 = T * T, U1 = fma(U, eps, U), U2 = U1 * U1, U3 = U2 * U1, U9 = U3 * U3 * U3;
   // the ringdown's linear part, which the other pieces are relative to
-  const double shift = c.t0 * c.MfRef - c.phi_pre;
-  const double R0 = K * (c.C1MRD + shift), Ri = K * (c.al1 * m * ie + c.C2MRD * m - c.t0 * m);
-  P.pins.A0 = K * (q[0] + q[4] * lam3 + shift) - R0;
+  const double R0 = K * c.C1MRD + shift, Ri = K * (c.al1 * m * ie + c.C2MRD * m - c.t0 * m);
+  P.pins.A0 = (K * (q[0] + q[4] * lam3) + shift) - R0;
   P.pins.At = K * (q[2] * T + q[3] * T * lam3);
   P.pins.Att = K * (q[1] * T2);
   P.pins.AtL = K * (q[3] * T * third);
   P.pins.AL = K * (q[4] * third);
-  P.pins.Au = K * (q[5] * U);
+  P.pins.Au = K * (q[5] * U1);
   P.pins.Auu = K * (q[6] * U2);
   P.pins.Au3 = K * (q[7] * U3);
-  P.pins.Au5 = K * (q[8] * U5);
+  double lo;
+  const double hi = fold_r5(q[8], q8lo, U, eps, lo);
+  P.pins.Au5 = hi + lo;
   P.pins.Ai = K * (ie * q[9] * m - c.t0 * m) - Ri;
   P.pins.Ait = K * (ie * q[10] * T * m);
   P.pins.Aitt = K * (ie * q[11] * T2 * m);
   P.pins.Aii = K * (ie * q[12] * m * m);
-  P.pint.B0 = K * (c.b2 * ie * c.mdf_log + c.C1Int + shift) - R0;
+  P.pint.B0 = (K * (c.b2 * ie * c.mdf_log + c.C1Int) + shift) - R0;
   P.pint.Bi = K * (c.b1 * m * ie + c.C2Int * m - c.t0 * m) - Ri;
   P.pint.Bu9 = K * (-(c.b3 * third) * U9 * ie);
   P.pint.BL = K * (c.b2 * ie);

@@ -86,7 +86,8 @@ struct SetupConst {
   double logvj;        // log v there
   double log_fj;       // log 0.018
   // reciprocals and quotients of the above that the likelihood setup multiplies by
-  double r_pi_third, r_pi_two_thirds, r_pi_five_thirds, a0;    // a0 = sqrt(2/3) / pi^{1/6}
+  double r_pi_third, r_pi_two_thirds, a0;                      // a0 = sqrt(2/3) / pi^{1/6}
+  double r_pi_five_thirds, r_pi_five_thirds_lo;                // pi^{-5/3} as hi + lo
   double r_fj_third;   // 0.018^{-1/3}
   double dj_scale, dj_s2, dj_s3, dj_s4;                        // of the inspiral phase's slope at the join
 };
@@ -115,9 +116,11 @@ void upload_tables() {
   for (int k = 1; k < 9; k++) h.vj[k] = v * h.vj[k - 1];
   h.logvj = std::log(v);
   h.log_fj = std::log(kPhiJoin);
-  h.r_pi_third = 1.0 / h.pi6.third;
-  h.r_pi_two_thirds = 1.0 / h.pi6.two_thirds;
-  h.r_pi_five_thirds = 1.0 / h.pi6.five_thirds;
+  const long double pi = 3.141592653589793238462643383279502884L, p53 = powl(pi, -5.0L / 3.0L);
+  h.r_pi_third = (double)powl(pi, -1.0L / 3.0L);
+  h.r_pi_two_thirds = (double)powl(pi, -2.0L / 3.0L);
+  h.r_pi_five_thirds = (double)p53;
+  h.r_pi_five_thirds_lo = (double)(p53 - (long double)h.r_pi_five_thirds);
   h.a0 = std::sqrt(2.0 / 3.0) / h.pi6.sixth;
   h.r_fj_third = 1.0 / h.fjp.third;
   h.dj_scale = kPi / (3.0 * h.vj[8]);
@@ -834,7 +837,7 @@ struct SetupVals {
   double p[kMaxParams], v[F_COUNT], pv[8], pvl[8];
   NetGeom g;
   MrdJoin mj;
-  double phr, tref, rref, v3, rdm, rfg;
+  double phr, tref, rref, eref, em, q8lo, v3, rdm, rfg;
   int br, ev, live, lo, hi, st;
 };
 constexpr int kLnlSets = 4, kLnlLanes = 8, kLnlThreads = 128;
@@ -885,12 +888,12 @@ struct FitLane {
   }
 };
 
-// phi_ins at f with t = f^{1/3}, rt = 1/t and log v given
+// phi_ins at f without its Newtonian term, with t = f^{1/3}, rt = 1/t and log v given
 __device__ __forceinline__ double phi_ins_roots(const PhdRec& c, double f, double t, double rt, double logv) {
   const double* q = c.pq;
   const double t2 = t * t, r2 = rt * rt, r3 = r2 * rt;
   return q[0] + q[1] * t2 + (q[2] + q[3] * logv) * t + q[4] * logv + q[5] * rt + q[6] * r2 + q[7] * r3 +
-         q[8] * (r3 * r2) + f * (q[9] + q[10] * t + q[11] * t2 + q[12] * f) * c.inv_eta;
+         f * (q[9] + q[10] * t + q[11] * t2 + q[12] * f) * c.inv_eta;
 }
 
 // warp 0 until the first barrier
@@ -950,7 +953,7 @@ __device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const Qn
   const double rdm = lane_of(rr, 0), rfg = lane_of(rr, 1);
   const double L = log(f), C = cbrt(f), sq = sqrt(f), f34 = sqrt(f * sq), at = atan(xr * rdm);
   const double v3 = exp(-dx * g2 * rfg) * (fg * g1) * lane_of(rr, 2);
-  const double d3 = 1.0 / f, r2 = d3 * d3, rx = 1.0 / (fDM * fDM + xr * xr);
+  const double d3 = 1.0 / f, Ci = 1.0 / C, ci = rthird_eps(f, d3, C, Ci), r2 = d3 * d3, rx = 1.0 / (fDM * fDM + xr * xr);
   const double pint = b1 * f - b3 * (1.0 / 3.0) * (r2 * d3) + b2 * L;
   const double dpint = (b1 + b3 * (r2 * r2) + b2 * d3) * inv_eta;
   const double pmrd = -(al2 * d3) + (4.0 / 3.0) * (al3 * f34) + al1 * f + al4 * at;
@@ -975,14 +978,16 @@ __device__ __forceinline__ void setup_ringdown(PhdRec& c, SetupVals& x, const Qn
   x.br = MfRef < kPhiJoin ? 0 : (MfRef >= fm ? 1 : 2);
   x.phr = lane_of(x.br == 0 ? L : x.br == 1 ? pmrd : pint, 2);
   x.tref = lane_of(C, 2);
-  x.rref = lane_of(d3, 2);
+  x.rref = lane_of(Ci, 2);
+  x.eref = lane_of(ci, 2);
+  x.em = lane_of(ci, 3);
   // scales of Mf = (Msec df) i
-  const double T = lane_of(C, 3), r4 = 1.0 / (l == 0 ? T : mdf * sqrt(T));
+  const double T = lane_of(C, 3);
   c.mdf_third = T;
   c.mdf_log = lane_of(L, 3);
   c.mdf_34 = lane_of(f34, 3);
-  c.mdf_rthird = lane_of(r4, 0);
-  c.mdf_m76 = lane_of(r4, 1);
+  c.mdf_rthird = lane_of(Ci, 3);
+  c.mdf_m76 = 1.0 / (mdf * sqrt(T));
 }
 
 // warp 0 until the second barrier: C^1 joins (IMRPhenomD_internals.c:1547-1584), phase at fRef, folded phase
@@ -995,24 +1000,30 @@ __device__ __forceinline__ void setup_joins(PhdRec& c, SetupVals& x, int model) 
                    (s1 + s2 * c_setup.dj_s2 + s3 * c_setup.dj_s3 + s4 * c_setup.dj_s4) * ie;
   constexpr double rf = 1.0 / kPhiJoin;
   c.C2Int = D - (c.b1 + c.b3 * (rf * rf * rf * rf) + c.b2 * rf) * ie;
-  const double pin = phi_ins_roots(c, fj, c_setup.fjp.third, c_setup.r_fj_third, c_setup.logvj);
+  const double rj = c_setup.r_fj_third, rj2 = rj * rj;
+  const double pin = phi_ins_roots(c, fj, c_setup.fjp.third, rj, c_setup.logvj) + c.pq[8] * (rj2 * rj2 * rj);
   c.C1Int = pin - ie * (c.b1 * fj - c.b3 * (rf * rf * rf / 3.0) + c.b2 * c_setup.log_fj) - c.C2Int * fj;
   const double fm = c.fMRDJoin;
   const double phiT = ie * x.mj.phi_int + c.C1Int + c.C2Int * fm;
   c.C2MRD = c.C2Int + x.mj.dphi_int - x.mj.dphi_mrd;
   c.C1MRD = phiT - ie * x.mj.phi_mrd - c.C2MRD * fm;
   const double f = c.MfRef;
-  double phr;
+  const double phi0 = model == kModelIntrinsic ? x.p[4] : 0.5 * x.p[4];
+  double phr, shift;                   // shift: t0 MfRef - phi_pre in cycles
   if (x.br == 0) {
-    const double t = x.tref;
-    phr = phi_ins_roots(c, f, t, x.rref * t * t, (x.phr + kLnPi) * (1.0 / 3.0));
+    double lo;
+    const double hi = fold_r5(c.pq[8], x.q8lo, x.rref, x.eref, lo);
+    const double rest = phi_ins_roots(c, f, x.tref, fma(x.rref, x.eref, x.rref), (x.phr + kLnPi) * (1.0 / 3.0));
+    phr = fma(hi, kTwoPi, rest);
+    shift = kInv2PiD * (c.t0 * f - 2. * phi0 - rest) - lo - (hi - rint(hi));
   } else if (x.br == 1) {
     phr = ie * x.phr + c.C1MRD + c.C2MRD * f;
   } else {
     phr = ie * x.phr + c.C1Int + c.C2Int * f;
   }
-  c.phi_pre = 2. * (model == kModelIntrinsic ? x.p[4] : 0.5 * x.p[4]) + phr;
-  mix_phase(c, x.rdm);
+  c.phi_pre = 2. * phi0 + phr;
+  if (x.br != 0) shift = kInv2PiD * (c.t0 * f - c.phi_pre);
+  mix_phase(c, x.rdm, x.em, x.q8lo, shift);
 }
 
 // warp 1: projection (or the intrinsic model's offsets), fbegin and the first bin above it
@@ -1099,7 +1110,7 @@ __device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const Qn
                          5841690624 * (x1 + x2) * Pi + 21384760320 * Pi2));
   const double m1M = 0.5 * (1.0 + Seta), m2M = 0.5 * (1.0 - Seta), q1 = m1M * m1M * x1s, q2 = m2M * m2M * x2s, xx = x1 * x2;
   const double SL = m1M * m1M * x1 + m2M * m2M * x2, dS = Seta * (m2M * x2 - m1M * x1);
-  const double pf = (3.0 / 128.0) * (1.0 / eta);
+  const double e128 = 128.0 * eta, pf = 3.0 / e128, pflo = fma(-e128, pf, 3.0) * pf * (1.0 / 3.0);
   const double sig = eta * (721.0 / 48.0 - 247.0 / 48.0) * xx + ((720.0 - 1.0) / 96.0 - (240.0 - 7.0) / 96.0) * (q1 + q2);
   const double gam = (554345.0 / 1134.0 + 110.0 / 9.0 * eta) * SL + (13915.0 / 84.0 - 10.0 / 3.0 * eta) * dS;
   double v[8], w5, w6;
@@ -1130,7 +1141,9 @@ __device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const Qn
   c.pq[5] = v[4] * c_setup.r_pi_third;
   c.pq[6] = v[3] * c_setup.r_pi_two_thirds;
   c.pq[7] = v[2] * (1.0 / kPi);
-  c.pq[8] = v[0] * c_setup.r_pi_five_thirds;
+  double q8e;
+  c.pq[8] = two_prod(pf, c_setup.r_pi_five_thirds, q8e);
+  x.q8lo = q8e + fma(pf, c_setup.r_pi_five_thirds_lo, pflo * c_setup.r_pi_five_thirds);
   c.pq[9] = s1;
   c.pq[10] = s2 * (3.0 / 4.0);
   c.pq[11] = s3 * (3.0 / 5.0);
@@ -1727,7 +1740,8 @@ __device__ __forceinline__ void tile_mixed(const PhdRec& c, const NetGeom& g, co
 
 // ---- FP64 tile body.  The same decomposition as the mixed one (folded per-set polynomials over the
 // per-bin tables, linear phase and detector delays through rotation tables), every step in FP64:
-//  * phase of detector 0 in cycles = lin0 + i lin1 - rest(i), one sincos of it per bin; detectors 1, 2
+//  * phase of detector 0 in cycles = lin0 + i lin1 - rest(i), one sincos of it per bin, with i lin1 (up to 1e6
+//    cycles) reduced exactly, per thread and per row (LinPhase); detectors 1, 2
 //    follow by the relative rotation e^{2 pi i (f (td0 - td) + (lam - lam0) / 2 pi)} = base(thread) R[row];
 //  * the ringdown's exponential is a geometric sequence in i: E(thread) E[row];
 //  * its arctangent is atan(z_c) of the warp's centre bin (table) plus atan(w), w = (z - z_c)/(1 + z z_c),
@@ -1756,6 +1770,7 @@ struct alignas(16) Tab64 {
   double2 rot[kSeg64][kMaxIfo - 1];        // relative rotations of detectors 1, 2 per row
   double2 sub[kSeg64 * 8];                 // (z_c, Rat atan z_c) per row and warp
   double er[kSeg64];                       // the exponential's row factor
+  double lin[kSeg64];                      // detector 0's linear phase per row, fraction of a cycle
   double al[8];                            // inspiral amplitude
 };
 
@@ -1778,7 +1793,7 @@ struct Acc64 {
 
 // per-thread constants of a tile
 struct Tile64 {
-  double lin0, lin1;         // detector 0's linear phase, cycles
+  double lin;                // detector 0's linear phase at the thread's first bin, cycles
   double D1, D0, Ru3, Rs, Rat;
   double dn;                 // z - z_c of this lane
   double fg2, E;             // Lorentzian width squared; fg g1 times the exponential at the first bin
@@ -1905,7 +1920,7 @@ __device__ __forceinline__ void step64(const PhdRec& c, const EventData& ev, con
   }
   double sv[U], cv[U];
 #pragma unroll
-  for (int j = 0; j < U; j++) rest[j] = fma(xi[j], q.lin1, q.lin0) - rest[j];
+  for (int j = 0; j < U; j++) rest[j] = (q.lin + T.lin[p.k + j]) - rest[j];
   sincos_cycles<U, (PP < 0)>(rest, sv, cv);
 #pragma unroll
   for (int j = 0; j < U; j++) {
@@ -1978,8 +1993,9 @@ __device__ __forceinline__ void tile_fp64(const PhdRec& c, const NetGeom& g, con
   constexpr double kInv2Pi = 0.15915494309189533577;
   const double m = c.mdf, ie = c.inv_eta, rdm = 1.0 / c.fDM, fg = c.fDM * c.g3, gx = c.g2 / fg;
   Tile64 q;
-  q.lin1 = g.df * (c.ts - c.td[0]) - P.pmrd.Ri;
-  q.lin0 = c.lam[0] * kInv2Pi - P.pmrd.R0;
+  const LinPhase lin(g.df, c.ts - c.td[0], P.pmrd.Ri);
+  const double lin0 = c.lam[0] * kInv2Pi - P.pmrd.R0;
+  q.lin = lin0 + lin.cycles((double)(i0 + tid));
   q.D1 = m * rdm;
   q.D0 = c.al5 * c.fRD * rdm;
   q.Ru3 = kInv2Pi * (-c.al2 * (c.mdf_rthird * c.mdf_rthird * c.mdf_rthird) * ie);
@@ -2002,7 +2018,7 @@ __device__ __forceinline__ void tile_fp64(const PhdRec& c, const NetGeom& g, con
                       x1 * (f(a.Ai) + t1 * (f(a.Ait) + t1 * f(a.Aitt)) + x1 * f(a.Aii));
     const float mid = f(P.pint.B0) + x1 * f(P.pint.Bi) + u3 * u3 * u3 * f(P.pint.Bu9) + L1 * f(P.pint.BL);
     const float mrd = u3 * f(q.Ru3) + x1 * f(q.Rs) + 1.6f * f(q.Rat);
-    small = f(q.lin0) + x1 * f(q.lin1) + ins + mid + mrd < 3.0e13f;
+    small = f(lin0) + x1 * f(lin.hi) + ins + mid + mrd < 3.0e13f;
   }
   q.E = 0.0;
   if (fast && i1 >= P.iF) q.E = fg * c.g1 * exp(-gx * (m * (double)(i0 + tid) - c.fRD));
@@ -2034,6 +2050,7 @@ __device__ __forceinline__ void tile_fp64(const PhdRec& c, const NetGeom& g, con
         }
       }
     }
+    for (int r = tid; r < kn; r += bs) T.lin[r] = lin.cycles((double)((k0 + r) * bs));
     if (fast && last >= P.iF)
       for (int r = tid; r < kn; r += bs) T.er[r] = exp(-(m * gx) * ((double)bs * (double)(k0 + r)));
     __syncthreads();
@@ -2747,7 +2764,8 @@ struct HetPre {
   bool bin;                  // FP64: f is bin i of the event and the tables hold it
   double2 tA, tB;
   float2 tC;
-  double aref[kMaxIfo], pcyc[kMaxIfo];      // reference amplitude (FP64: its reciprocal), phase in cycles
+  // reference amplitude (FP64: its reciprocal) and phase in cycles (FP64: their fraction)
+  double aref[kMaxIfo], pcyc[kMaxIfo];
 };
 template <int PREC>
 __device__ __forceinline__ HetPre het_pre(const NetGeom& g, const HetData& h, int j) {
@@ -2767,7 +2785,11 @@ __device__ __forceinline__ HetPre het_pre(const NetGeom& g, const HetData& h, in
     if (id >= g.nifo) break;
     e.aref[id] = __ldg(h.amp + id * h.M + j);
     if (PREC == kFP64) e.aref[id] = 1.0 / e.aref[id];
-    e.pcyc[id] = __ldg(h.phase + id * h.M + j) * kInv2Pi;
+    const double ph = __ldg(h.phase + id * h.M + j);
+    e.pcyc[id] = ph * kInv2Pi;
+    // the quotient by the 2 pi that the tables' phases were made with; its whole cycles go before its rounding
+    // (up to 1e-11 rad) can be felt
+    if (PREC == kFP64) e.pcyc[id] = (e.pcyc[id] - rint(e.pcyc[id])) + fma(-e.pcyc[id], kTwoPi, ph) * kInv2Pi;
   }
   return e;
 }
@@ -2859,7 +2881,9 @@ __device__ __forceinline__ void het_point(const PhdRec& c, const NetGeom& g, con
     amp *= c.amp_scale * (kH22fac * y) / c.sqT;
     for (int id = 0; id < nifo; id++) {
       const double ratio = c.Fs[id] * amp * e.aref[id];
-      const double cyc = e.pcyc[id] - fma(f, c.ts - c.td[id], c.lam[id] * kInv2Pi - phc);
+      double te;
+      const double t = two_prod(f, c.ts - c.td[id], te);
+      const double cyc = (e.pcyc[id] - ((t - rint(t)) + te)) - (c.lam[id] * kInv2Pi - phc);
       double sx, cx;
       sincos_cycles(cyc, sx, cx);
       const double hc = 2.0 * (1.0 - ratio * cx), hs = 2.0 * ratio * sx;

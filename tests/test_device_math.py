@@ -6,6 +6,7 @@ in the last place; the sine and cosine polynomials are within 2^-54 of their fun
 roundings act on at most one, so 1.5 2^-52 absolute near one quadrant's ends plus the argument's reduction, which is
 exact; the arctangent's last multiply-add and product round once each, two units."""
 import ctypes as C
+from fractions import Fraction
 
 import numpy as np
 
@@ -85,3 +86,50 @@ def test_arctangent(tmp_path):
     y = np.empty(len(w))
     L.at(_p(w), _p(y), len(w))
     assert _ulps(y, np.arctan(w.astype(LD))) <= 2.0
+
+
+PHASE = r"""
+#include "qcbc_device.cuh"
+extern "C" void lin(double df, double t, double slope, const double* n, double* y, int k) {
+  const qcbc::LinPhase p(df, t, slope);
+  for (int j = 0; j < k; j++) y[j] = p.cycles(n[j]);
+}
+extern "C" void fold(const double* q, const double* ql, const double* f, const double* t, double* y, int n) {
+  for (int k = 0; k < n; k++) {
+    const double r = 1.0 / t[k];
+    double lo;
+    const double hi = qcbc::fold_r5(q[k], ql[k], r, qcbc::rthird_eps(f[k], 1.0 / f[k], t[k], r), lo);
+    y[2 * k] = hi;
+    y[2 * k + 1] = lo;
+  }
+}
+"""
+
+
+def test_linear_phase_is_reduced_exactly(tmp_path):
+    """Against exact fractions: the slope's last part, n lo and the sum are rounded, 2^-52 of a cycle together."""
+    L = compile_host(str(tmp_path), PHASE)
+    n = np.concatenate([[0, 1, (1 << 20) - 1], np.random.default_rng(4).integers(0, 1 << 20, 500)]).astype(float)
+    for df, t, slope in ((1 / 128.0, 126.3, 1.7e-5), (1 / 7.3, 5.1, 2e-3), (0.25, 2.0, -0.4), (1 / 64.0, 61.99, 0.0)):
+        y = np.empty(len(n))
+        L.lin(C.c_double(df), C.c_double(t), C.c_double(slope), _p(n), _p(y), len(n))
+        step = Fraction(df) * Fraction(t) - Fraction(slope)
+        for k, got in zip(n, y):
+            d = Fraction(got) - int(k) * step
+            assert abs(d - round(d)) <= Fraction(1, 2 ** 52)
+
+
+def test_newtonian_coefficient(tmp_path):
+    """q f^{-5/3} / 2 pi from a cube root that is a unit in the last place off: to 2^-63 as hi + lo."""
+    L = compile_host(str(tmp_path), PHASE)
+    rng = np.random.default_rng(5)
+    n = 20000
+    f, q = 10.0 ** rng.uniform(-8, -1, n), rng.uniform(0.01, 5.0, n)
+    ql = q * rng.uniform(-1, 1, n) * 2.0 ** -53
+    t = np.cbrt(f) * (1 + rng.integers(-1, 2, n) * 2.0 ** -52)
+    y = np.empty(2 * n)
+    L.fold(_p(q), _p(ql), _p(f), _p(t), _p(y), n)
+    got = y[0::2].astype(LD) + y[1::2].astype(LD)
+    want = (q.astype(LD) + ql) * f.astype(LD) ** (LD(-5) / LD(3)) / LD("6.283185307179586476925286766559005768")
+    assert np.max(np.abs(got / want - 1)) <= 2.0 ** -60       # long double's own power has a few bits of its 64
+    assert np.max(np.abs(y[0::2] / want.astype(float) - 1)) > 2.0 ** -52        # the one-term product is not enough

@@ -17,7 +17,7 @@ extern "C" int rec_bytes() { return (int)sizeof(PhdRec); }
 extern "C" int differing(const void* start, double rdm, int runs) {
   PhdRec one, two;
   memcpy(&one, start, sizeof(one));
-  qcbc::mix_phase(one, rdm);
+  qcbc::mix_phase(one, rdm, 1e-16, 1e-17, 0.3);
   std::atomic<int> turn{0}, ready{0}, done{0};
   int bad = 0;
   auto lane = [&](bool lead) {
@@ -31,7 +31,7 @@ extern "C" int differing(const void* start, double rdm, int runs) {
       while (turn < k) std::this_thread::yield();
       ready++;
       while (ready < 2) std::this_thread::yield();
-      qcbc::mix_phase(two, rdm);
+      qcbc::mix_phase(two, rdm, 1e-16, 1e-17, 0.3);
       done++;
       if (lead) {
         while (done < 2) std::this_thread::yield();
