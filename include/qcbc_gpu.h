@@ -106,10 +106,13 @@ qcbc_batch* qcbc_batch_create(qcbc_event* const* events, int n_events);
 qcbc_batch* qcbc_batch_create_slots(int capacity, int max_bins);
 int qcbc_batch_set_slot(qcbc_batch* batch, int slot, qcbc_event* ev);
 int qcbc_batch_destroy(qcbc_batch* batch);
-/* tile_bins > 0 and threads in {64,128,256}; 0 keeps the current/automatic value */
+/* tile_bins > 0 and threads in {64,128,256}, for both precisions; 0 keeps the current value (at first 2048 x 256
+ * for QCBC_MIXED, 4096 x 128 for QCBC_FP64) */
 int qcbc_batch_set_tiling(qcbc_batch* batch, int tile_bins, int threads);
+/* The tiling of the launches of one precision, and that of the precision tuned last (QCBC_MIXED before any). */
+int qcbc_batch_get_tiling_of(qcbc_batch* batch, int precision, int* tile_bins, int* threads);
 int qcbc_batch_get_tiling(qcbc_batch* batch, int* tile_bins, int* threads);
-/* Times each candidate tiling on the given call and keeps the fastest. */
+/* Times each candidate tiling on the given call and keeps the fastest for that precision. */
 int qcbc_batch_autotune(qcbc_batch* batch, const int* event_of, const double* params, int B, int precision);
 /* event_of[B] indexes the batch's events; rho is [B][3] (unused detectors 0) or NULL. */
 int qcbc_lnl_multi(qcbc_batch* batch, const int* event_of, const double* params, int B, double* lnl, double* rho,

@@ -90,6 +90,7 @@ def lib():
         L.qcbc_batch_set_slot.argtypes = [vp, i, vp]
         L.qcbc_batch_set_tiling.argtypes = [vp, i, i]
         L.qcbc_batch_get_tiling.argtypes = [vp, pi, pi]
+        L.qcbc_batch_get_tiling_of.argtypes = [vp, i, pi, pi]
         L.qcbc_batch_autotune.argtypes = [vp, pi, _PD, i, i]
         L.qcbc_lnl_multi.argtypes = [vp, pi, _PD, i, _PD, _PD, i]
         L.qcbc_time_lnl_multi.argtypes = [vp, i, i, i, i, C.POINTER(C.c_float)]

@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <thread>
@@ -1178,6 +1179,9 @@ static void free_het_scratch(HetMultiScratch& h) {
   h = HetMultiScratch();
 }
 
+struct BatchTiling { int tile_bins, threads; };      // bins per tile, threads per block
+static_assert(QCBC_FP64 == 0 && QCBC_MIXED == 1, "tilings are indexed by precision");
+
 struct qcbc_batch {
   int device = 0;
   std::vector<qcbc_event*> events;
@@ -1186,14 +1190,16 @@ struct qcbc_batch {
   std::vector<size_t> het_smem;        // per slot: shared memory of its heterodyned lnL
   HetMultiScratch hs;
   int nh_max = 0;
-  // the tiling of a mixed and of an FP64 launch until it is set: bins per tile, threads per block (multi_launch)
-  int tile_bins = 2048, threads = 256, tile64 = 4096, threads64 = 128;
+  // the tiling of an FP64 and of a mixed launch (indexed by precision) until it is set or tuned (multi_launch), and
+  // the precision whose tiling was tuned last
+  BatchTiling tiling[2] = {{4096, 128}, {2048, 256}};
+  int shown = QCBC_MIXED;
   cudaStream_t stream = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   unsigned char* d_flush = nullptr;
   std::mutex mu;
-  std::map<long long, MultiBuf*> bufs;       // by (Bcap, tile_bins)
-  std::map<long long, int> blocks;           // resident blocks by (precision, threads, tile_bins)
+  std::map<std::array<int, 3>, MultiBuf*> bufs;       // by (Bcap, tile_bins, precision)
+  std::map<std::array<int, 3>, int> blocks;           // resident blocks by (precision, threads, tile_bins)
 };
 
 extern "C" int qcbc_batch_destroy(qcbc_batch* bt);
@@ -1307,22 +1313,31 @@ extern "C" int qcbc_batch_set_tiling(qcbc_batch* bt, int tile_bins, int threads)
   if (tile_bins < 0 || (threads != 0 && threads != 64 && threads != 128 && threads != 256))
     return fail(QCBC_EINVAL, "tile_bins >= 0, threads in {64, 128, 256}");
   std::lock_guard<std::mutex> lk(bt->mu);
-  if (tile_bins > 0) bt->tile_bins = bt->tile64 = tile_bins;
-  if (threads > 0) bt->threads = bt->threads64 = threads;
+  for (BatchTiling& t : bt->tiling) {
+    if (tile_bins > 0) t.tile_bins = tile_bins;
+    if (threads > 0) t.threads = threads;
+  }
+  return QCBC_OK;
+}
+
+extern "C" int qcbc_batch_get_tiling_of(qcbc_batch* bt, int precision, int* tile_bins, int* threads) {
+  if (!bt || !tile_bins || !threads) return fail(QCBC_EINVAL, "NULL argument");
+  if (precision != QCBC_FP64 && precision != QCBC_MIXED) return fail(QCBC_EINVAL, "precision %d", precision);
+  std::lock_guard<std::mutex> lk(bt->mu);
+  *tile_bins = bt->tiling[precision].tile_bins;
+  *threads = bt->tiling[precision].threads;
   return QCBC_OK;
 }
 
 extern "C" int qcbc_batch_get_tiling(qcbc_batch* bt, int* tile_bins, int* threads) {
-  if (!bt || !tile_bins || !threads) return fail(QCBC_EINVAL, "NULL argument");
-  *tile_bins = bt->tile_bins;
-  *threads = bt->threads;
-  return QCBC_OK;
+  if (!bt) return fail(QCBC_EINVAL, "NULL argument");
+  return qcbc_batch_get_tiling_of(bt, bt->shown, tile_bins, threads);
 }
 
 // Buffers for up to Bcap sets at the batch's tiling; caller holds bt->mu.
 static int multi_buf(qcbc_batch* bt, int Bcap, int prec, MultiBuf** out) {
-  const int tile_bins = prec == QCBC_MIXED ? bt->tile_bins : bt->tile64;
-  const long long key = ((long long)Bcap << 24) ^ tile_bins;
+  const int tile_bins = bt->tiling[prec].tile_bins;
+  const std::array<int, 3> key{Bcap, tile_bins, prec};     // a precision's own: its calls may run beside the other's
   auto it = bt->bufs.find(key);
   if (it != bt->bufs.end()) { *out = it->second; return QCBC_OK; }
   const long long tiles_per_set = (bt->nh_max + tile_bins - 1) / tile_bins;
@@ -1360,8 +1375,8 @@ static int multi_buf(qcbc_batch* bt, int Bcap, int prec, MultiBuf** out) {
 static int multi_launch(qcbc_batch* bt, MultiBuf* m, const double* d_params, const int* d_eof, int B, int prec,
                         double* d_lnl, double* d_rho, cudaStream_t s) {
   const Precision P = prec == QCBC_MIXED ? kMixed : kFP64;
-  const int threads = P == kFP64 ? bt->threads64 : bt->threads;
-  int& blocks = bt->blocks[((long long)m->tile_bins << 16) ^ (threads << 1) ^ prec];
+  const int threads = bt->tiling[prec].threads;
+  int& blocks = bt->blocks[{prec, threads, m->tile_bins}];
   if (!blocks) {
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, bt->device));
@@ -1528,29 +1543,32 @@ extern "C" int qcbc_batch_autotune(qcbc_batch* bt, const int* event_of, const do
   if (!bt || !event_of || !params || B <= 0) return fail(QCBC_EINVAL, "bad argument");
   static const int cand[][2] = {{1024, 128}, {2048, 256}, {4096, 256}, {8192, 256}, {2048, 128}, {1024, 256},
                                 {4096, 128}, {8192, 128}};
+  if (precision != QCBC_FP64 && precision != QCBC_MIXED) return fail(QCBC_EINVAL, "precision %d", precision);
   std::vector<double> lnl(B);
   float best = 1e30f;
-  int bt_tiles = bt->tile_bins, bt_threads = bt->threads;
+  BatchTiling found;
+  {
+    std::lock_guard<std::mutex> lk(bt->mu);
+    found = bt->tiling[precision];
+  }
+  int rc = QCBC_OK;
   for (auto& c : cand) {
     {
       std::lock_guard<std::mutex> lk(bt->mu);
-      bt->tile_bins = c[0];
-      bt->threads = c[1];
-      if (precision == QCBC_FP64) { bt->tile64 = c[0]; bt->threads64 = c[1]; }
-      int rc = run_multi(bt, event_of, params, B, lnl.data(), nullptr, precision);
-      if (rc && rc != QCBC_EDOM) return rc;
+      bt->tiling[precision] = {c[0], c[1]};
+      rc = run_multi(bt, event_of, params, B, lnl.data(), nullptr, precision);
+      if (rc == QCBC_EDOM) rc = QCBC_OK;
     }
     float ms[5];
-    int rc = qcbc_time_lnl_multi(bt, B, precision, 5, 0, ms);
-    if (rc) return rc;
+    if (rc || (rc = qcbc_time_lnl_multi(bt, B, precision, 5, 0, ms))) break;
     std::sort(ms, ms + 5);
-    if (ms[2] < best) { best = ms[2]; bt_tiles = c[0]; bt_threads = c[1]; }
+    if (ms[2] < best) { best = ms[2]; found = {c[0], c[1]}; }
   }
+  // the other precision's tiling stays; a candidate that fails leaves the best so far, or what was there before
   std::lock_guard<std::mutex> lk(bt->mu);
-  bt->tile_bins = bt_tiles;
-  bt->threads = bt_threads;
-  if (precision == QCBC_FP64) { bt->tile64 = bt_tiles; bt->threads64 = bt_threads; }
-  return QCBC_OK;
+  bt->tiling[precision] = found;
+  if (!rc) bt->shown = precision;
+  return rc;
 }
 
 // ================================================================== reference-signature drop-ins

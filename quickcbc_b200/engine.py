@@ -222,9 +222,13 @@ class Batch:
     def set_tiling(self, tile_bins=0, threads=0):
         check(lib().qcbc_batch_set_tiling(self._h, int(tile_bins), int(threads)))
 
-    def tiling(self):
+    def tiling(self, precision=None):
+        """(bins per tile, threads) of the launches of a precision; None: of the precision tuned last."""
         t, th = C.c_int(), C.c_int()
-        check(lib().qcbc_batch_get_tiling(self._h, C.byref(t), C.byref(th)))
+        if precision is None:
+            check(lib().qcbc_batch_get_tiling(self._h, C.byref(t), C.byref(th)))
+        else:
+            check(lib().qcbc_batch_get_tiling_of(self._h, precision_code(precision), C.byref(t), C.byref(th)))
         return t.value, th.value
 
     def autotune(self, event_of, params, precision=MIXED):

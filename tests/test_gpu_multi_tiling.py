@@ -57,3 +57,29 @@ def test_failed_tuning_changes_nothing(batch):
         assert L.qcbc_batch_get_tiling_of(h, prec, C.byref(t), C.byref(th)) == 0
         assert (t.value, th.value) == want
     L.qcbc_batch_destroy(h)
+
+
+def test_precisions_side_by_side_on_two_streams(batch):
+    """Device-form calls of the two precisions at one tiling, queued on two streams: neither waits for the other,
+    so they share no scratch."""
+    b, eo, P = batch
+    b.set_tiling(2048, 128)
+    n = 60
+    eo, P = np.tile(eo, n), np.tile(P, (n, 1))
+    want = {p: b.lnl(eo, P, p) for p in (q.FP64, q.MIXED)}
+    L, vp = _lib.lib(), C.c_void_p
+    dP, dE = q.DeviceBuffer(P.nbytes), q.DeviceBuffer(eo.nbytes)
+    dP.upload(P)
+    dE.upload(eo)
+    import torch
+    streams = {p: torch.cuda.Stream() for p in want}
+    outs = {p: [q.DeviceBuffer(8 * len(eo)) for _ in range(6)] for p in want}
+    for k in range(6):
+        for p in want:
+            assert L.qcbc_lnl_multi_dev(vp(b._h), vp(dE.ptr), vp(dP.ptr), len(eo), vp(outs[p][k].ptr), p,
+                                        vp(streams[p].cuda_stream)) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    for p in want:
+        for k in range(6):
+            assert np.array_equal(outs[p][k].download((len(eo),)), want[p]), (p, k)
+    b.set_tiling(2048, 256)
