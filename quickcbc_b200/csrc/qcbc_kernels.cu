@@ -2761,7 +2761,7 @@ __host__ __device__ inline int het_warp_doubles(int nifo, int M) { return kRecDo
 struct HetPre {
   double f;
   int i;
-  bool bin;                  // FP64: f is bin i of the event and the tables hold it
+  bool bin;                  // the tables hold bin i, and (FP64) it is f's
   double2 tA, tB;
   float2 tC;
   // reference amplitude (FP64: its reciprocal) and phase in cycles (FP64: their fraction)
@@ -2773,7 +2773,8 @@ __device__ __forceinline__ HetPre het_pre(const NetGeom& g, const HetData& h, in
   HetPre e;
   e.f = __ldg(h.freq + j);
   e.i = (int)rint(e.f * g.Tobs);
-  e.bin = PREC != kFP64 || (e.i >= 1 && e.i < h.tab_n && bin_freq(g, e.i) == e.f);
+  // tables given by a caller may name any frequency, also one beyond the model's cut-off that no set evaluates
+  e.bin = e.i >= 0 && e.i < h.tab_n && (PREC != kFP64 || (e.i >= 1 && bin_freq(g, e.i) == e.f));
   e.tA = e.tB = make_double2(0.0, 0.0);
   e.tC = make_float2(0.f, 0.f);
   if (e.bin) {
