@@ -24,8 +24,8 @@ CSRC = os.path.join(HERE, "csrc")
 GEN = os.path.join(CSRC, "_gen")
 LIB = os.path.join(HERE, "libqcbc_gpu.so")
 SOURCES = ["qcbc_kernels.cu", "qcbc_capi.cu", "qcbc_serve.cu", "qcbc_hetspace.cu", "qcbc_ptstep.cu", "qcbc_ingest.cu"]
-HEADERS = ["qcbc_device.cuh", "qcbc_math.cuh", "qcbc_kernels.cuh", "qcbc_hetspace.h", "qcbc_ptstep.h",
-           "qcbc_ingest_dev.h"]
+HEADERS = ["qcbc_device.cuh", "qcbc_math.cuh", "qcbc_kernels.cuh", "qcbc_hetspace.h", "qcbc_coop.h",
+           "qcbc_ptstep.h", "qcbc_ingest_dev.h"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall", "--expt-relaxed-constexpr"]
 

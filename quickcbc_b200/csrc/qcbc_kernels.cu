@@ -18,6 +18,7 @@
 // :587-629, 716-736, 995-1109; IMRPhenomD.c:413-563.
 #include "qcbc_kernels.cuh"
 #include "qcbc_math.cuh"
+#include "qcbc_coop.h"
 #include "qcbc_ptstep.h"
 #include <cooperative_groups.h>
 #include <cmath>
@@ -3563,7 +3564,10 @@ cudaError_t launch_hs_walk(const double* d_Cs, const double* d_Sn, const double*
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   void* args[] = {&d_Cs, &d_Sn, &d_dS, &d_lim, &per, &MN, &MM, &djmax, &tol, &cap, &d_first, &d_grid, &m_grid,
                   &m_cap, &m_count};
-  return cudaLaunchCooperativeKernel((const void*)k_hs_walk, dim3((unsigned)sms), dim3(kWalkThreads), args, 0, s);
+  // the walk's blocks share out whatever there is: any number of them finds the same points
+  return launch_coop(sms, [&](int blocks) {
+    return cudaLaunchCooperativeKernel((const void*)k_hs_walk, dim3((unsigned)blocks), dim3(kWalkThreads), args, 0, s);
+  });
 }
 
 // The slow-term quadrature of the heterodyne summary for one detector and the regions
