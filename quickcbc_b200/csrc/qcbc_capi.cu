@@ -341,7 +341,6 @@ struct qcbc_event {
   double inv_sigma[kMaxIfo] = {1, 1, 1};
   HetDev het;
   int fixed_tiles = 0, fixed_threads = 0;
-  std::map<long long, FullLaunch> tuned;
   long long bytes = 0;
   bool has_data = false;
 };
@@ -568,9 +567,6 @@ static FullLaunch heuristic_launch(const qcbc_event* ev, int B, int prec) {
 
 static FullLaunch choose_launch(qcbc_event* ev, int B, int prec) {
   if (ev->fixed_tiles > 0) return FullLaunch{ev->fixed_tiles, ev->fixed_threads > 0 ? ev->fixed_threads : 256};
-  long long key = ((long long)B << 2) | prec;
-  auto it = ev->tuned.find(key);
-  if (it != ev->tuned.end()) return it->second;
   return heuristic_launch(ev, B, prec);
 }
 
@@ -638,7 +634,7 @@ static int enqueue_full(Workspace* w, qcbc_event* ev, const double* d_params, in
     const SetOrder o{w->d_ocnt, w->d_olist};
     launch_setup_lnl(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, model, o);
     if (k0) cudaEventRecord(k0, s);
-    launch_lnl_full_final(w->d_recs, w->d_status, B, g, ed, kp, L, w->d_part, d_lnl, d_rho, model, &o, s);
+    launch_lnl_full_final(w->d_recs, B, g, ed, kp, L, w->d_part, d_lnl, d_rho, model, &o, s);
     if (k1) cudaEventRecord(k1, s);
     const cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) return fail(QCBC_ECUDA, "lnL launch: %s", cudaGetErrorString(le));
@@ -650,7 +646,7 @@ static int enqueue_full(Workspace* w, qcbc_event* ev, const double* d_params, in
     if (w->c_done != had) CU(cudaMemsetAsync(w->d_done, 0, sizeof(int) * w->c_done, s));
     launch_setup_lnl(d_params, B, g, ds.qnm, w->d_recs, w->d_status, s, model);
     if (k0) cudaEventRecord(k0, s);
-    launch_lnl_full_final(w->d_recs, w->d_status, B, g, ed, kp, L, w->d_part, d_lnl, d_rho, model, nullptr, s,
+    launch_lnl_full_final(w->d_recs, B, g, ed, kp, L, w->d_part, d_lnl, d_rho, model, nullptr, s,
                           w->d_done);
     if (k1) cudaEventRecord(k1, s);
     tls_launches += 2;

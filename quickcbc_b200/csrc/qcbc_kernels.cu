@@ -672,7 +672,7 @@ struct SetupScratch {
   double v2, s[4], pv[8], pvl[8];
   MrdJoin mj;
   double phr_raw;
-  int phr_branch, st, live;
+  int phr_branch, st;
 };
 
 constexpr int kSetupSets = 32;
@@ -704,31 +704,21 @@ __device__ __forceinline__ int length_class(int bins, int band) {
   return min(kOrderClasses - 1, __float2int_rz((float)bins * ((float)kOrderClasses / (float)max(band, 1))));
 }
 
-template <class Geom>
-__device__ __forceinline__ void setup_coop_block(const double* __restrict__ params, int B, const Geom& geo,
+__device__ __forceinline__ void setup_coop_block(const double* __restrict__ params, int B, const NetGeom& g,
                                                  const QnmTable& q, PhdRec* __restrict__ recs,
                                                  int* __restrict__ status, int model) {
   __shared__ __align__(16) PhdRec s_rec[kSetupSets];
   __shared__ SetupScratch s_x[kSetupSets];
-  __shared__ NetGeom s_g[kSetupSets];
-  __shared__ int s_ev[kSetupSets];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int b0 = blockIdx.x * kSetupSets, nb = min(kSetupSets, B - b0);
   const int b = b0 + lane;
   PhdRec& c = s_rec[lane];
   SetupScratch& x = s_x[lane];
-  if (w == 0 && lane < nb) {
-    NetGeom g;
-    int e;
-    x.live = geo.get(b, g, e);
-    s_g[lane] = g;
-    s_ev[lane] = e;
-  }
   {
     // The block's parameters are contiguous: every thread loads its share with independent loads
     // (one round trip, also when they are read from mapped host memory), then stores them.
     constexpr int kPer = (kSetupSets * kMaxParams + kSetupThreads - 1) / kSetupThreads;
-    const int ps = geo.stride(model), n = nb * ps;
+    const int ps = param_stride(model, g.nifo), n = nb * ps;
     const double* src = params + (size_t)b0 * ps;
     double v[kPer];
 #pragma unroll
@@ -743,7 +733,7 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
     }
   }
   __syncthreads();
-  const bool on = lane < nb && x.live;
+  const bool on = lane < nb;
   // phase 1
   if (on) {
     const double* p = x.p;
@@ -752,13 +742,13 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
       x.m = phd_masses(c, ph.m1, ph.m2, p[2], p[3], ph.dist);
     } else if (w == 1) {
       x.fb = fbegin_head(p);
-      c.ts = s_g[lane].Tobs - p[5];
-      c.sqT = sqrt(s_g[lane].Tobs);
+      c.ts = g.Tobs - p[5];
+      c.sqT = sqrt(g.Tobs);
     } else if (w == 2) {
-      if (model == kModelIntrinsic) set_offsets(c, p, s_g[lane].nifo);
-      else set_projection(c, p, s_g[lane], 0, 2);
+      if (model == kModelIntrinsic) set_offsets(c, p, g.nifo);
+      else set_projection(c, p, g, 0, 2);
     } else if (model != kModelIntrinsic) {
-      set_projection(c, p, s_g[lane], 2, kMaxIfo);     // the third detector, if any
+      set_projection(c, p, g, 2, kMaxIfo);     // the third detector, if any
     }
   }
   __syncthreads();
@@ -794,20 +784,12 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
   }
   __syncthreads();
   // phase 4
-  if (w == 0 && lane < nb) {
-    int st;
-    if (on) {
-      phd_join_mrd(c, x.mj);
-      phd_phi_ref(c, model == kModelIntrinsic ? x.p[4] : 0.5 * x.p[4], x.phr_raw, x.phr_branch);
-      st = x.st;
-      c.flags = (st == kStOK) ? kRecValid : 0;
-      c.event = s_ev[lane];
-    } else {
-      st = kStNoEvent;
-      c.flags = 0;
-      c.event = -1;
-    }
-    status[b] = st;
+  if (w == 0 && on) {
+    phd_join_mrd(c, x.mj);
+    phd_phi_ref(c, model == kModelIntrinsic ? x.p[4] : 0.5 * x.p[4], x.phr_raw, x.phr_branch);
+    c.flags = (x.st == kStOK) ? kRecValid : 0;
+    c.event = 0;
+    status[b] = x.st;
   }
   __syncthreads();
   // the block's records are contiguous in shared and in global memory
@@ -1372,8 +1354,7 @@ __device__ __forceinline__ void setup_prefetch(const SetupPrefetch& pf) {
 __global__ void __launch_bounds__(kSetupThreads) k_setup(const double* __restrict__ params, int B, NetGeom g,
                                                          QnmTable q, PhdRec* __restrict__ recs,
                                                          int* __restrict__ status, int model) {
-  GeomOne geo{g};
-  setup_coop_block(params, B, geo, q, recs, status, model);
+  setup_coop_block(params, B, g, q, recs, status, model);
 }
 
 void launch_setup(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
@@ -1823,7 +1804,7 @@ __device__ __forceinline__ double amp64_int(const PhdRec& c, double xi) {
 // the functions themselves in place of the ringdown's tables).  The U bins are evaluated side by side, so
 // that the polynomials' constants and the set's coefficients are read once for all of them.
 template <int NIFO, int AP, int PP, int U>
-__device__ __forceinline__ void step64(const PhdRec& c, const EventData& ev, const Tab64& T, const Tile64& q,
+__device__ __forceinline__ void step64(const PhdRec& c, const Tab64& T, const Tile64& q,
                                        Acc64<NIFO>& A, const Cur64& p, int bs) {
   constexpr bool kT = AP <= 0 || PP <= 0;              // i^{1/3} needed
   constexpr int G = w64_group(NIFO);
@@ -1971,13 +1952,13 @@ __device__ __forceinline__ void rows64(const PhdRec& c, const EventData& ev, con
   constexpr int U = PP < 0 ? 1 : QCBC_U64;
 #pragma unroll 1
   for (; n >= U; n -= U) {
-    step64<NIFO, AP, PP, U>(c, ev, T, q, A, p, bs);
+    step64<NIFO, AP, PP, U>(c, T, q, A, p, bs);
     advance(U);
   }
   if (U > 1) {
 #pragma unroll 1
     for (; n > 0; n--) {
-      step64<NIFO, AP, PP, 1>(c, ev, T, q, A, p, bs);
+      step64<NIFO, AP, PP, 1>(c, T, q, A, p, bs);
       advance(1);
     }
   }
@@ -2511,21 +2492,15 @@ void launch_lnl_full(const PhdRec* d_recs, int B, const NetGeom& g, const EventD
   else launch_full_mixed(d_recs, B, g, ev, L, d_partials, none, s);
 }
 
-bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, const NetGeom& g, const EventData& ev,
+void launch_lnl_full_final(const PhdRec* d_recs, int B, const NetGeom& g, const EventData& ev,
                            Precision prec, const FullLaunch& L, double* d_partials, double* d_lnl, double* d_rho,
                            int model, const SetOrder* order, cudaStream_t s, int* d_done) {
-  if (B <= 0) return true;
-  if (L.tiles != 1 && !d_done) {
-    launch_lnl_full(d_recs, B, g, ev, prec, L, d_partials, s);
-    launch_finalize_full(d_partials, d_recs, d_status, B, L.tiles, g, ev, d_lnl, d_rho, s, model);
-    return false;
-  }
+  if (B <= 0) return;
   const FinalOut fo{d_lnl, d_rho, model,
                     (order && L.tiles == 1) ? *order : SetOrder{nullptr, nullptr}, B,
                     L.tiles == 1 ? nullptr : d_done};
   if (prec == kFP64) launch_full_fp64(d_recs, B, g, ev, L, d_partials, fo, s);
   else launch_full_mixed(d_recs, B, g, ev, L, d_partials, fo, s);
-  return true;
 }
 
 // one warp per set

@@ -128,13 +128,11 @@ void launch_lnl_full(const PhdRec* d_recs, int B, const NetGeom& g, const EventD
 void launch_finalize_full(const double* d_partials, const PhdRec* d_recs, const int* d_status, int B, int tiles,
                           const NetGeom& g, const EventData& ev, double* d_lnl, double* d_rho,
                           cudaStream_t s, int model = kModelFull);
-// lnL of B sets with the finaliser folded into the lnL kernel: when each set is one tile (L.tiles ==
-// 1), longest first when order is given (filled by launch_setup_ordered); at several tiles per set
-// when d_done (B ints, zero before the launch and left zero after it) is given, the set's last
-// tile to finish finalises it.  Otherwise the lnL kernel and launch_finalize_full.  Returns true
-// when one launch did both.
-bool launch_lnl_full_final(const PhdRec* d_recs, const int* d_status, int B, const NetGeom& g, const EventData& ev,
-                           Precision prec, const FullLaunch& L, double* d_partials, double* d_lnl, double* d_rho,
+// lnL of B sets finalised by the lnL kernel itself.  One tile per set: longest first when order is given (its lists
+// filled by launch_setup_lnl).  Several: the set's last tile to finish finalises it, counted in d_done (B ints,
+// zero before the launch and left zero after it).
+void launch_lnl_full_final(const PhdRec* d_recs, int B, const NetGeom& g, const EventData& ev, Precision prec,
+                           const FullLaunch& L, double* d_partials, double* d_lnl, double* d_rho,
                            int model, const SetOrder* order, cudaStream_t s, int* d_done = nullptr);
 // The same for a batch small enough (full_small_fits) that each tile's block makes its set's record itself:
 // one launch, no records.  h_params, when given, are the same parameters on the host: those of up to 16
