@@ -602,20 +602,21 @@ def interleaved_stream(q, b, evs, eo, P, Lm):
     """The config-4 sets in round-robin event order (set k of every event, then set k + 1, ...):
     the blocks in flight read the data of all 256 events at once, about 16 B per detector-bin
     of each set (the FP32 weighted data), more than L2 holds; the work list by kind of tile brings them back
-    to an L2-sized part at a time.  Achieved bandwidth counts each set's in-band bins once."""
+    to an L2-sized part at a time, so the useful bytes (each set's in-band bins once) come from L2 and the
+    launch is bound by instruction issue."""
     order = np.lexsort((eo, np.arange(len(eo)) - np.searchsorted(eo, eo)))
     eo_i, P_i = eo[order], P[order]
     L_i = b.lnl(eo_i, P_i, q.MIXED)
     ms = b.time(len(P_i), q.MIXED, iters=5, flush_l2=True)
-    nbytes = 0
+    nbytes = flops = 0
     for e, ev in enumerate(evs):
         bins = min(int(ev.Tobs * 1024.0), ev.N // 2) - int(ev.Tobs * ev.fmin)
-        # useful bytes: FP32 (wr, wi, ws) per detector-bin and one FP32 bin factor per bin
-        nbytes += int(np.sum(eo == e)) * bins * 12 * len(ev.labels)
+        sets = int(np.sum(eo == e))
+        nbytes += sets * bins * 12 * len(ev.labels)       # FP32 (wr, wi, ws) per detector-bin
+        flops += sets * bins * (WF_FLOPS_PER_BIN + PROJ_FLOPS_PER_DET_BIN * len(ev.labels))
     t = float(np.median(ms)) * 1e-3
-    peak, kind = load_peaks()
-    return {"value": len(P_i) / t, "unit": "lnL evals/s", "ms": t * 1e3, "stream_bytes": nbytes,
-            "achieved_GBs": nbytes / t / 1e9, "frac_hbm": nbytes / t / 1e9 / peak, "peak_kind": kind,
+    return {"value": len(P_i) / t, "unit": "lnL evals/s", "ms": t * 1e3, "tiling": list(b.tiling(q.MIXED)),
+            "flops": flops, "stream_bytes": nbytes, "l2_served_GBs": nbytes / t / 1e9,
             "bytes_note": "12 B per detector-bin of every set (each set reads its event's band; the bin factor "
                           "i^-7/6 is folded into the weighted data)",
             "same_lnl_as_grouped_order": bool(np.array_equal(L_i, Lm[order]))}
@@ -632,11 +633,11 @@ def bench_cfg4_uneven(q):
     hs = [q.Event.from_synthetic(x) for x in evs]
     b = q.Batch(hs)
     eo, P = synth.uneven_params(evs)
-    tiling = b.autotune(eo, P, q.MIXED)
+    b.autotune(eo, P, q.MIXED)
     Lm = b.lnl(eo, P, q.MIXED)
     L64 = b.lnl(eo, P, q.FP64)
     out = {"workload": "config 4: 256 events (Tobs 4-64 s, fs 2048/4096 Hz, 1-3 det), 65536 sets per launch",
-           "tiling": list(tiling), "device_bytes": int(sum(h.device_bytes() for h in hs)),
+           "tiling": {"mixed": list(b.tiling(q.MIXED)), "fp64": list(b.tiling(q.FP64))}, "device_bytes": int(sum(h.device_bytes() for h in hs)),
            "max_abs_dlnL_mixed_vs_fp64": float(np.max(np.abs(Lm - L64)))}
     for prec, name, it in ((q.MIXED, "mixed", 8), (q.FP64, "fp64", 3)):
         ms = b.time(len(P), prec, iters=it, flush_l2=True)
@@ -645,7 +646,7 @@ def bench_cfg4_uneven(q):
     for _ in range(3):
         b.lnl(eo, P, q.MIXED)
     out["e2e_mixed"] = {"value": 3 * len(P) / (time.perf_counter() - t0), "unit": "lnL evals/s",
-                        "h2d_bytes_per_step": int(P.nbytes + eo.nbytes), "d2h_bytes_per_step": int(len(P) * 44)}
+                        "h2d_bytes_per_step": int(P.nbytes + eo.nbytes), "d2h_bytes_per_step": int(len(P) * 8)}
     out["mixed_interleaved"] = interleaved_stream(q, b, evs, eo, P, Lm)
     b.close()
     for h in hs:
@@ -985,17 +986,18 @@ def main():
         out["config3"] = bench_cfg3_het(q)
         out["config4_uneven"] = bench_cfg4_uneven(q)
         # the config-4 launch with the sets interleaved across all 256 events; its work list goes by kind of
-        # tile, and one kind's data fit in L2, so DRAM carries the events' data about once (traffic)
+        # tile, and one kind's data fit in L2, so DRAM carries the events' data about once (traffic, when the
+        # capture has this tiling's blocks)
         st = out["config4_uneven"]["mixed_interleaved"]
-        tr, ti = capture_traffic("k_lnl_multi_cfg4_kinds", "k_lnl_multi", None, None, st["ms"])
+        tr, ti = capture_traffic("k_lnl_multi_cfg4_kinds", "k_lnl_multi", None, f"({st['tiling'][1]},1,1)", st["ms"])
         out["roofline_stream"] = {
-            "bound": "issue", "achieved": st["achieved_GBs"], "peak": hbm_peak, "unit": "GB/s",
-            "frac": st["frac_hbm"], "traffic": tr, "peak_kind": peak_kind, "kernel": "k_lnl_multi (mixed)",
-            "kernel_ms": st["ms"], "bytes_per_launch": st["stream_bytes"], **ti,
-            "note": "config 4, 65536 sets interleaved across 256 events (1-3 detectors): useful bytes = "
-                    "12 B (FP32 wr, wi, ws) per detector-bin of every set's band; the waveform's bin factor "
-                    "is folded into those values, so no per-bin table is streamed; served from L2 (the tiles "
-                    "run by kind, and a kind's data fit there), peak is HBM's for comparison"}
+            "bound": "issue", "achieved": st["flops"] / (st["ms"] * 1e-3) / 1e12, "peak": fp32_peak, "unit": "TFLOP/s",
+            "frac": st["flops"] / (st["ms"] * 1e-3) / 1e12 / fp32_peak, "traffic": tr, "kernel": "k_lnl_multi (mixed)",
+            "kernel_ms": st["ms"], "flops_per_launch": st["flops"], "tiling": st["tiling"],
+            "useful_bytes_per_launch": st["stream_bytes"], "l2_served_GBs": st["l2_served_GBs"], **ti,
+            "note": "config 4, 65536 sets interleaved across 256 events (1-3 detectors): achieved counts FP32 flops "
+                    "per set-bin as in roofline; useful bytes = 12 B (FP32 wr, wi, ws) per detector-bin of every "
+                    "set's band, served from L2 (the tiles run by kind, and a kind's data fit there)"}
         out["input_stage"] = bench_input_stage(q)
         # config 5 as specified (32 runs of 16 x 8 chains x 20000 steps, Poisson 2/s): mixed against
         # plain FP64, heterodyned and full likelihood, chains stepped on the device
