@@ -518,8 +518,8 @@ extern "C" long long qcbc_event_device_bytes(const qcbc_event* ev) {
 // Blocks per parameter set.  Mixed: enough blocks of 256 threads to fill 148 SMs several times over,
 // but at least ~512 bins per block.
 // FP64: blocks of 64 threads (eight per SM at 128 registers), because a block's start (record, tables)
-// and end are short serial stretches that other blocks have to fill: 2048 sets at 16 s take 191 us with
-// one 64-thread block per set, 196 with 128 threads, 223 with 256.  The tile count minimises a model of
+// and end are short serial stretches that other blocks have to fill: 2048 sets at 16 s take 188.5 us with
+// one 64-thread block per set, 190 with 128 threads, 214 with 256.  The tile count minimises a model of
 // the launch fitted to sweeps at 4, 16 and 128 s and 1 to 2048 sets (within 5 % of the best count there
 // but for one case at 9 %): a block costs its rows of 64 bins plus 28 rows of start and end; f = blocks
 // over resident blocks; below one wave an SM runs each block faster the fewer it holds; above, the part of
@@ -527,10 +527,10 @@ extern "C" long long qcbc_event_device_bytes(const qcbc_event* ev) {
 // by length).
 // Few sets take the kernel whose blocks make the records (full_small_fits), where a block's start is the setup:
 // fewer, longer blocks of 256 threads.  One block on two of three SMs is the best count while that leaves a
-// thread a few dozen bins (one set at 4 s: 28.2 us with 12 to 37 tiles, 32 with 8 or 74, 40 with 592; 16 sets at
-// 16 s: 20.6 us with 6 tiles, 22.6 with 18), two per SM beyond (32 sets at 128 s: 65 us with 9 tiles, 74 with 4);
-// above 37 tiles the count of the tiles costs more than the shorter tile gives (one set at 128 s: 32.1 us with
-// 74, 32.4 with 37, 37 with 148).  Against the two launches: 1 to 148 sets at 4 s 1.5 to 5 us less, 1 to 48
+// thread a few dozen bins (one set at 4 s: 28.6 to 29.3 us with 12 to 37 tiles, 32 with 8, 29.6 with 74, 44 with
+// 592; 16 sets at 16 s from device memory: 21.7 us with 6 tiles, 24.7 with 3, 22.6 with 18), two per SM beyond (32
+// sets at 128 s: 67 us with 9 tiles, 78 with 4).  37 tiles at most: twice as many give one set at 128 s 3 % (35.2 and
+// 34.3 us) and cost the shorter bands as much; 148 lose (38.1).  Against the two launches: 1 to 148 sets at 4 s 1.5 to 5 us less, 1 to 48
 // sets at 128 s 1 to 8 us less; 64 sets and more at 16 s or 128 s are up to 2 us slower, so the line is there.
 static FullLaunch heuristic_launch(const qcbc_event* ev, int B, int prec) {
   FullLaunch L;

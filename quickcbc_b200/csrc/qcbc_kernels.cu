@@ -815,7 +815,8 @@ __device__ __forceinline__ void setup_coop_block(const double* __restrict__ para
 //   warp 3  masses, fCut, amplitude scale, last bin                  first bins of the pieces
 // One set read from mapped host memory is ready 6.3 us after the kernel starts (2.2 us of it the read), where
 // four warps with a set per lane and out-of-line functions took about 20 us; a one-set heterodyned call went
-// from 38.0 to 25.4 us and the 4096-set launch sequence from 46.3 to 34.8 us with it and the kernels below.
+// from 38.0 to 25.4 us and the 4096-set launch sequence from 46.3 to 34.8 us with it and the kernels below (36.0 since
+// it divides and carries what its phases round).
 struct SetupVals {
   double p[kMaxParams], v[F_COUNT], pv[8], pvl[8];
   NetGeom g;
@@ -1732,7 +1733,7 @@ __device__ __forceinline__ void tile_mixed(const PhdRec& c, const NetGeom& g, co
 //  * the weighted data carry i^{-7/6}, so a bin needs no power, logarithm or division.
 // The FP64 pipe bounds it (58 % busy, about 68 FP64 of 130 instructions per signal bin at three detectors);
 // evaluating pow, log, atan, exp, ten divisions and three sincos per bin took four times as long: 2048 sets
-// at 16 s 741 -> 191 us per call, 201 sets at 128 s 889 -> 218 us.  Two rows at a time (QCBC_U64) read the
+// at 16 s 740 -> 187 us per call, 201 sets at 128 s 888 -> 212 us.  Two rows at a time (QCBC_U64) read the
 // constants once for both: 126 M warp instructions per launch against 155 M one by one; three rows gain
 // another 1 %, four spill.  128 registers: 16 warps per SM with two rows each beat 20 at 96 (201 us) and 24
 // at 80 (209 us).
@@ -2571,8 +2572,8 @@ void launch_setup_multi(const double* d_params, const int* d_event_of, int B, co
 // in which the setup's blocks counted them.  Blocks that work at the same time are then in the same loop.  In the
 // order of the sets, with whole sets side by side, up to fifteen loops replaced one another in the instruction
 // caches and 60 % of the warps' cycles were waits for instructions (now 8 %): 64 events of 64 sets in FP64 took
-// 1025 us from call to result, now 603; 24 events of 64 sets 362 and 225; the mixed launches 694 and 683, 262
-// and 245.  Also clears the sets' tile counts, writes the rejected sets' results and sets the item counter to the
+// 1025 us from call to result, then 603; 24 events of 64 sets 362 and 225 (one draw of events; others hold up to 40 %
+// more bins); the mixed launches 694 and 683, 262 and 245.  Also clears the sets' tile counts, writes the rejected sets' results and sets the item counter to the
 // grid's size (a block's first item is its index).
 __global__ void __launch_bounds__(128) k_multi_items(MultiWork w, int B, int grid, double* __restrict__ lnl,
                                                      double* __restrict__ rho) {
@@ -3182,7 +3183,7 @@ void launch_het_waves(const PhdRec* d_recs, int B, const NetGeom& g, const HetDa
 
 // ---- the grid search's device pieces (het_space).  Each is spread over the whole chip; what bounds the
 // search is the number of dependent steps (about ten rounds of trial points, fifty grid points), not their
-// work: 33.4 ms -> 2.4 ms at 3 detectors, 128 s, 4096 Hz.
+// work: 34.0 ms -> 2.05 ms at 3 detectors, 128 s, 4096 Hz.
 
 // Fisher_All (QuickCBC.c:2695-2817) from the 23 wave sets (point, then +/- eps along each parameter) on n bins:
 // sum over detectors and bins of 4 (dA_i dA_j + A^2 dphi_i dphi_j) / S.  With one detector the matrix has a
@@ -3774,7 +3775,7 @@ void launch_fullphaseamp(const double* d_params, const NetGeom& g, const QnmTabl
 
 // ---------------------------------------------------------------- heterodyne setup (FP64)
 // The tables of heterodyne() (QuickCBC.c:5112-5299) in three launches after the reference point's
-// record, with nothing but logLb coming back to the host.  What bounds them is launch latency: the
+// record (the waveform outputs' setup), with nothing but logLb coming back to the host.  What bounds them is launch latency: the
 // band's raw data and PSD (9.4 MB at 3 x 131 k bins) are read once and the per-bin terms stay in L2.
 // The earlier form wrote the template, amplitude and phase of all N/2 bins to memory in two waveform
 // passes and copied five [nifo][N/2] arrays (31 MB at 128 s, 4096 Hz) to the host to pick out the

@@ -103,7 +103,7 @@ struct SetupPrefetch {
   const float2* tabC = nullptr;
   int tab_n = 0;                     // entries of each table; bins outside [0, tab_n) are skipped
 };
-// records of the waveform outputs (fullphaseamp, fulltemplates and the grid search)
+// records of the waveform outputs (fullphaseamp, fulltemplates, the grid search) and of the heterodyne tables
 void launch_setup(const double* d_params, int B, const NetGeom& g, const QnmTable& q, PhdRec* d_recs,
                   int* d_status, cudaStream_t s, int model = kModelFull);
 // Launch order of the sets: the setup files each set under its length class (its bin count in
