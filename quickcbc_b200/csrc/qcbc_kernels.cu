@@ -1092,8 +1092,11 @@ __device__ __forceinline__ void setup_inspiral(PhdRec& c, SetupVals& x, const Qn
              12 * eta * (-545384828789 - 176491177632 * x1 * x2 + 202603761360 * x2s +
                          77616 * x1s * (2610335 + 995766 * Seta) - 77287373856 * x2s * Seta +
                          5841690624 * (x1 + x2) * Pi + 21384760320 * Pi2));
-  const double m1M = 0.5 * (1.0 + Seta), m2M = 0.5 * (1.0 - Seta), q1 = m1M * m1M * x1s, q2 = m2M * m2M * x2s, xx = x1 * x2;
-  const double SL = m1M * m1M * x1 + m2M * m2M * x2, dS = Seta * (m2M * x2 - m1M * x1);
+  // the mass fractions and their difference from the masses: near equal masses sqrt(1 - 4 eta) has lost them (its
+  // error is eta's over its value)
+  const double mf = (l == 0 ? m.m1 : l == 1 ? m.m2 : m.m1 - m.m2) / m.M;
+  const double m1M = lane_of(mf, 0), m2M = lane_of(mf, 1), q1 = m1M * m1M * x1s, q2 = m2M * m2M * x2s, xx = x1 * x2;
+  const double SL = m1M * m1M * x1 + m2M * m2M * x2, dS = lane_of(mf, 2) * (m2M * x2 - m1M * x1);
   const double e128 = 128.0 * eta, pf = 3.0 / e128, pflo = fma(-e128, pf, 3.0) * pf * (1.0 / 3.0);
   const double sig = eta * (721.0 / 48.0 - 247.0 / 48.0) * xx + ((720.0 - 1.0) / 96.0 - (240.0 - 7.0) / 96.0) * (q1 + q2);
   const double gam = (554345.0 / 1134.0 + 110.0 / 9.0 * eta) * SL + (13915.0 / 84.0 - 10.0 / 3.0 * eta) * dS;
