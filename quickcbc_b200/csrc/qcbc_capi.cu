@@ -2532,7 +2532,7 @@ extern "C" int qcbc_lnl_full_noalloc(qcbc_event* ev, const double* d_params, int
 // tables built by qcbc_het_setup rebuilt about the same reference point and grid
 // (QuickCBC.c:1994-2010).  Tables given by qcbc_het_set are dropped.  Everything is queued on the
 // thread's stream and waited for once: at 128 s, 4096 Hz, three detectors a redraw with its tables
-// takes 0.12 ms (11.8 ms with two host round trips and the host-side table gathers).
+// takes 0.13 ms (11.8 ms with two host round trips and the host-side table gathers).
 static int event_psd_changed(qcbc_event* ev, Workspace* w) {
   const int nI = ev->g.nifo, nh = ev->nh;
   const int lo = std::max(ev->g.imin, 1), hi = std::min(ev->g.imax, nh);
