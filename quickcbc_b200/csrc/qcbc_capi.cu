@@ -1329,7 +1329,12 @@ extern "C" int qcbc_batch_get_tiling_of(qcbc_batch* bt, int precision, int* tile
 
 extern "C" int qcbc_batch_get_tiling(qcbc_batch* bt, int* tile_bins, int* threads) {
   if (!bt) return fail(QCBC_EINVAL, "NULL argument");
-  return qcbc_batch_get_tiling_of(bt, bt->shown, tile_bins, threads);
+  int shown;
+  {
+    std::lock_guard<std::mutex> lk(bt->mu);
+    shown = bt->shown;
+  }
+  return qcbc_batch_get_tiling_of(bt, shown, tile_bins, threads);
 }
 
 // Buffers for up to Bcap sets at the batch's tiling; caller holds bt->mu.
